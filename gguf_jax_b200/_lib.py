@@ -36,6 +36,7 @@ SIGNATURES = {
     "ggq_fused_batch_limit": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64]),
     "ggq_gemv_max_batch": (ctypes.c_int32, []),
     "ggq_workspace_bytes": (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32]),
+    "ggq_scratch_bytes": (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32]),
     "ggq_gemv": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                   ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32,
                                   ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]),

@@ -54,15 +54,33 @@ extern "C" int32_t ggq_fused_batch_limit(int32_t qtype, int64_t N, int64_t K) {
 
 static int sm_count_of(int dev) { return device_sm_count(dev); }
 
+// The formats whose batches up to 16 run without any scratch when none is given (streaming and MMA kernels); the tiled
+// kernel, two to five times as fast on them, is what ggq_scratch_bytes makes room for.
+static bool tile_scratch_is_optional(int qtype) {
+  return !is_k_quant(qtype) && qtype != QT_Q2_K && qtype != QT_IQ4_XS && qtype != QT_IQ2_XXS && qtype != QT_IQ2_XS && qtype != QT_IQ2_S &&
+         qtype != QT_IQ3_XXS && qtype != QT_IQ3_S && qtype != QT_IQ1_S && qtype != QT_IQ1_M;
+}
+
+static size_t tile_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
+  const int tmax = gemv_tile_max_batch(qtype);
+  return tmax && M <= kGemvMaxBatch && K % 256 == 0 ? gemv_tile_workspace_bytes(qtype, N, K, M < tmax ? M : tmax) : 0;
+}
+
+extern "C" size_t ggq_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
+  const TypeInfo* ti = type_info(qtype);
+  if (!ti || N <= 0 || K <= 0 || M <= 0) return 0;
+  const size_t need = ggq_workspace_bytes(qtype, N, K, M), tile = tile_scratch_bytes(qtype, N, K, M);
+  return need > tile ? need : tile;
+}
+
 extern "C" size_t ggq_workspace_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
   const TypeInfo* ti = type_info(qtype);
   if (!ti || N <= 0 || K <= 0) return 0;
   size_t need = 0;
   if (qtype == QT_Q4_K || qtype == QT_Q5_K || qtype == QT_Q6_K) need = gemv_q4k_workspace_bytes(N, kMaxSmCount);
-  if (M <= kGemvMaxBatch) {
-    const int tmax = gemv_tile_max_batch(qtype);
-    const size_t tile = tmax ? gemv_tile_workspace_bytes(qtype, N, K, M < tmax ? M : tmax) : 0;
-    if (tile > need && K % 256 == 0) need = tile;
+  if (!tile_scratch_is_optional(qtype)) {
+    const size_t tile = tile_scratch_bytes(qtype, N, K, M);
+    if (tile > need) need = tile;
   }
   if ((qtype == QT_Q4_K || qtype == QT_Q5_K || qtype == QT_Q6_K) && M >= 2 && K % 256 == 0) {
     const size_t wd = gemv_wide_workspace_bytes(qtype, N, K, M, kMaxSmCount);

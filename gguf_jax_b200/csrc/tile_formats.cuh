@@ -34,6 +34,9 @@
 //                       groups are loaded one at a time inside a real loop (keeps the loop body small)
 //   Run, load_run(ld, t)             what is read once per run and row
 //   Group, load_group(ld, run, t, grp)   the raw fields and the scale of group grp of the run
+//   kKv                 16-entry code book held in registers (Tables::kv): absent / 0 none, 1 IQ4 values + 128,
+//                       2 MXFP4 values + 12
+//   kScaleExp           the group scales carry 2^kScaleExp (taken back out of the row sums; 0 where the trait is absent)
 //   octet(group, q, tab, p)   the four A-operand registers of octet q of the group: p[0], p[1] = first
 //                       MMA (k-slot pairs 2t.. and 2t+8..), p[2], p[3] = second MMA
 //   fold(group, acc, xsum, out) -> float   out + the group's contribution given acc = sum(code * x)
@@ -180,7 +183,7 @@ struct BlockLd {
 // Per-CTA lookup tables in shared memory.
 struct Tables {
   uint32_t grid;           // shared-window address of the format's grid: 8 (IQ1, IQ2) or 4 (IQ3) code bytes per entry
-  uint32_t kv[4];          // IQ4_XS: the sixteen codes kvalues + 128, four per register
+  uint32_t kv[4];          // sixteen unsigned codes, four per register (formats with kKv)
 };
 #else
 struct BlockLd {
@@ -197,6 +200,34 @@ struct Tables {
 };
 #endif
 struct NoRun {};
+// Optional members of a format.
+template <class F, class = void> struct KvOf { static constexpr int value = 0; };
+template <class F> struct KvOf<F, decltype((void)F::kKv)> { static constexpr int value = F::kKv; };
+template <class F, class = void> struct ScaleExpOf { static constexpr int value = 0; };
+template <class F> struct ScaleExpOf<F, decltype((void)F::kScaleExp)> { static constexpr int value = F::kScaleExp; };
+
+// Sixteen-entry lookup of the four nibbles held in the low 16 bits of `sel`: result bytes in nibble
+// order (byte0.lo, byte0.hi, byte1.lo, byte1.hi).
+TF_HD uint32_t lookup4(const Tables& tb, uint32_t sel) {
+  const uint32_t s7 = sel & 0x7777u;
+  const uint32_t lo = prmt(tb.kv[0], tb.kv[1], s7), hi = prmt(tb.kv[2], tb.kv[3], s7);
+  return prmt(lo, hi, ((sel >> 1) & 0x4444u) | 0x3210u);
+}
+// An octet from one word of eight table nibbles (pair order 1: low nibbles a.., high nibbles b..).
+TF_HD void lookup_octet(const Tables& tb, uint32_t w, uint32_t (&p)[4]) {
+  const uint32_t c0 = lookup4(tb, w), c1 = lookup4(tb, w >> 16);
+  p[0] = pair02(c0); p[1] = pair13(c0); p[2] = pair02(c1); p[3] = pair13(c1);
+}
+// An octet from one word of eight plain nibbles (pair order 0: the four low nibbles, then the four high ones).
+TF_HD void nibble_octet(uint32_t w, uint32_t (&p)[4]) {
+  p[0] = w & 0x000F000Fu; p[1] = (w >> 8) & 0x000F000Fu; p[2] = (w >> 4) & 0x000F000Fu; p[3] = (w >> 12) & 0x000F000Fu;
+}
+// The same with a fifth bit per weight: bits 0-3 of `h` belong to the low nibbles, bits 16-19 to the high ones.
+TF_HD void nibble5_octet(uint32_t w, uint32_t h, uint32_t (&p)[4]) {
+  const uint32_t lo = (w & 0x0F0F0F0Fu) | (((h & 15u) * 0x02040810u) & 0x10101010u);
+  const uint32_t hi = ((w >> 4) & 0x0F0F0F0Fu) | ((((h >> 16) & 15u) * 0x02040810u) & 0x10101010u);
+  p[0] = pair02(lo); p[1] = pair13(lo); p[2] = pair02(hi); p[3] = pair13(hi);
+}
 
 // =============================================================================================
 // Q4_K  (144 B: d, dmin, 12 packed 6-bit scales/mins, 128 nibble bytes)
@@ -391,7 +422,7 @@ struct Q6K {
 // low nibbles (weights 4q..4q+3) and four high nibbles (16+4q..): MMA 1 takes the first two bytes
 // of the word, MMA 2 the last two (pair order 1).
 struct IQ4XS {
-  static constexpr int kQt = 23, kTs = 136, kAlign = 8, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 1;
+  static constexpr int kQt = 23, kTs = 136, kAlign = 8, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 1, kKv = 1;
   static constexpr bool kSums = true, kUnrollGroups = false;
   static constexpr int kTableBytes = 0;
   typedef NoRun Run;
@@ -412,18 +443,7 @@ struct IQ4XS {
     g.dl = mulf(f16_bits_to_float(h[0] & 0xFFFF), (float)ls);
     return g;
   }
-  // Sixteen-entry lookup of the four nibbles held in the low 16 bits of `sel`: result bytes in
-  // nibble order (byte0.lo, byte0.hi, byte1.lo, byte1.hi).
-  TF_HD static uint32_t lookup4(const Tables& tb, uint32_t sel) {
-    const uint32_t s7 = sel & 0x7777u;
-    const uint32_t lo = prmt(tb.kv[0], tb.kv[1], s7), hi = prmt(tb.kv[2], tb.kv[3], s7);
-    return prmt(lo, hi, ((sel >> 1) & 0x4444u) | 0x3210u);
-  }
-  TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
-    const uint32_t w = g.q[q];
-    const uint32_t c0 = lookup4(tb, w), c1 = lookup4(tb, w >> 16);
-    p[0] = pair02(c0); p[1] = pair13(c0); p[2] = pair02(c1); p[3] = pair13(c1);
-  }
+  TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) { lookup_octet(tb, g.q[q], p); }
   TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
     return fmaf_(g.dl, fmaf_(-128.0f, xsum, acc), out);
   }
@@ -657,6 +677,307 @@ struct IQ1M {
   }
   TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
     return fmaf_(g.dl8, fmaf_(-9.0f, xsum, acc), out);
+  }
+};
+
+// =============================================================================================
+// Q3_K  (110 B: 32 bytes of third bits, 64 quant bytes, 12 bytes of 6-bit scales, d)
+// weight e = 128 h + 32 s + p: code = (qs[32 h + p] >> 2 s) & 3 | third bit << 2 (bit 4 h + s of hmask[p]), value
+// d * (scale - 32) * (code - 4), scale index 8 h + 2 s + (p >> 4).
+// run t = (h, u) = (t >> 1, t & 1): p in [16 u, 16 u + 16); group = shift s, as in Q2_K.
+struct Q3K {
+  static constexpr int kQt = 11, kTs = 110, kAlign = 2, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t q[4], hm[4]; float dl[4]; int h4; };
+  struct Group { const Run* r; int s; float dl; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { Q2K::src_quads(t, oo, a, b); }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    const int h = t >> 1, u = t & 1;
+    ld.words<4, 2>(32 + 32 * h + 16 * u, r.q);
+    ld.words<4, 2>(16 * u, r.hm);
+    r.h4 = 4 * h;
+    uint32_t sc[3];
+    ld.words<3, 2>(96, sc);
+    const float d = f16_bits_to_float(ld.u16(108));
+    for (int s = 0; s < 4; s++) {
+      // low four bits: nibble h of byte j = 2 s + u; high two bits: field 2 h + (s >> 1) of byte 8 + (j & 3)
+      const uint32_t lo = (sc[s >> 1] >> (16 * (s & 1) + 8 * u + 4 * h)) & 15;
+      const uint32_t hi = (sc[2] >> (16 * (s & 1) + 8 * u + 4 * h + 2 * (s >> 1))) & 3;
+      r.dl[s] = mulf(d, (float)((int)(lo | (hi << 4)) - 32));
+    }
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) { return Group{&r, grp, r.dl[grp]}; }
+  TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) {
+    for (int i = 0; i < 2; i++) {
+      const uint32_t c = ((g.r->q[2 * q + i] >> (2 * g.s)) & 0x03030303u) |
+                         (((g.r->hm[2 * q + i] >> (g.r->h4 + g.s)) & 0x01010101u) << 2);
+      p[2 * i] = pair02(c); p[2 * i + 1] = pair13(c);
+    }
+  }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
+    return fmaf_(g.dl, fmaf_(-4.0f, xsum, acc), out);
+  }
+};
+
+// =============================================================================================
+// TQ2_0  (66 B: 64 bytes of 2-bit fields laid out as in Q2_K, d): value d * (code - 1), one scale per superblock
+struct TQ20 {
+  static constexpr int kQt = 35, kTs = 66, kAlign = 2, kOct = 8, kGroupOct = 8, kSumOct = 8, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t q[4]; float d; };
+  typedef const Run& Group;
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { Q2K::src_quads(t, oo, a, b); }
+  TF_HD static int x_exp(int, int oo) { return -2 * (oo >> 1); }
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    ld.words<4, 2>(16 * t, r.q);
+    r.d = f16_bits_to_float(ld.u16(64));
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int) { return r; }
+  TF_HD static void octet(Group g, int q, const Tables&, uint32_t (&p)[4]) {
+    const uint32_t m = 0x00030003u << (2 * (q >> 1)), w0 = g.q[2 * (q & 1)], w1 = g.q[2 * (q & 1) + 1];
+    p[0] = w0 & m; p[1] = (w0 >> 8) & m; p[2] = w1 & m; p[3] = (w1 >> 8) & m;
+  }
+  TF_HD static float fold(Group g, float acc, float xsum, float out) { return fmaf_(g.d, fmaf_(-1.0f, xsum, acc), out); }
+};
+
+// TQ1_0  (54 B: 48 + 4 bytes of base-3 digits, d): digit n of a byte v is (((v * 3^n) & 255) * 3) >> 8, value d * (digit - 1).
+// Octet g = 8 t + q (elements 8 g ..): g < 20 bytes 8 (g & 3).., digit g >> 2; g < 30 bytes 32 + 8 (g & 1).., digit
+// (g - 20) >> 1; the last two octets hold bytes 48..51 twice each, digits 2 (g - 30) and 2 (g - 30) + 1.
+struct TQ10 {
+  static constexpr int kQt = 34, kTs = 54, kAlign = 2, kOct = 8, kGroupOct = 8, kSumOct = 8, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { float d; int t; };
+  struct Group { BlockLd ld; float d; int t; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) { return Run{f16_bits_to_float(ld.u16(52)), t}; }
+  TF_HD static Group load_group(const BlockLd& ld, const Run& r, int, int) { return Group{ld, r.d, r.t}; }
+  TF_HD static uint32_t digits(uint32_t bytes02, uint32_t pow3) {
+    return ((((bytes02 & 0x00FF00FFu) * pow3) & 0x00FF00FFu) * 3u >> 8) & 0x00030003u;
+  }
+  TF_HD static uint32_t pow3(int n) { return n < 4 ? (0x1B090301u >> (8 * n)) & 0xFFu : 81u; }
+  TF_HD static void octet(const Group& gr, int q, const Tables&, uint32_t (&p)[4]) {
+    const int g = 8 * gr.t + q;
+    const int off = g < 20 ? 8 * (g & 3) : g < 30 ? 32 + 8 * (g & 1) : 48;
+    const int n = g < 20 ? g >> 2 : g < 30 ? (g - 20) >> 1 : 2 * (g - 30);
+    const int last = g >= 30 ? 1 : 0;
+    uint32_t w0[1], w1[1];
+    gr.ld.template words<1, 2>(off, w0);
+    gr.ld.template words<1, 2>(last ? off : off + 4, w1);
+    const uint32_t pa = pow3(n), pb = pow3(n + last);
+    p[0] = digits(w0[0], pa); p[1] = digits(w0[0] >> 8, pa); p[2] = digits(w1[0], pb); p[3] = digits(w1[0] >> 8, pb);
+  }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) { return fmaf_(g.d, fmaf_(-1.0f, xsum, acc), out); }
+};
+
+// =============================================================================================
+// Formats that ran on kernels decoding byte by byte to float32 before (streaming at batch 1, three bf16 terms per weight above).
+// Measured on B200, 14336 x 4096, us at batch 1 / 4 / 8 / 16, before -> here: Q8_0 26 / 55 / 57 / 55 -> 20 / 23 / 34 / 66,
+// Q4_0 31 / 86 / 87 / 92 -> 16 / 20 / 30 / 60, Q5_1 38 / 131 / 133 / 137 -> 18 / 22 / 38 / 75, MXFP4 36 / 90 / 92 / 98 ->
+// 24 / 26 / 36 / 69, Q3_K 43 / 102 / 102 / 97 -> 21 / 25 / 41 / 81, TQ1_0 68 / 91 / 92 / 98 -> 24 / 30 / 40 / 79.
+//
+// The 32-element formats: eight blocks make a superblock (kTs = 8 x block bytes), run t = blocks 2 t and 2 t + 1
+// = groups 0 and 1.  The run is read as aligned words; the block that starts two bytes into a word is shifted.
+
+// Q8_0 (34 B: d, 32 int8): codes q + 128
+struct Q80 {
+  static constexpr int kQt = 8, kTs = 272, kAlign = 16, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t q[16]; float d[2]; };
+  struct Group { const uint32_t* q; float d; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    uint32_t w[17];
+    ld.words<17, 4>(68 * t, w);
+    r.d[0] = f16_bits_to_float(w[0] & 0xFFFF);
+    r.d[1] = f16_bits_to_float(w[8] >> 16);
+    for (int i = 0; i < 8; i++) {
+      r.q[i] = funnel16(w[i], w[i + 1]) ^ 0x80808080u;
+      r.q[8 + i] = w[9 + i] ^ 0x80808080u;
+    }
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) { return Group{r.q + 8 * grp, r.d[grp]}; }
+  TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) { plain_octet(g.q[2 * q], g.q[2 * q + 1], p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
+    return fmaf_(g.d, fmaf_(-128.0f, xsum, acc), out);
+  }
+};
+
+// Nibble blocks: element e < 16 is the low nibble of byte e, element 16 + e its high nibble; octet q of a block is its
+// word q (weights 4 q.. and 16 + 4 q..).
+TF_HD void nibble_src(int t, int oo, int& a, int& b) { a = 64 * t + 32 * (oo >> 2) + 4 * (oo & 3); b = a + 16; }
+
+// Q4_0 (18 B: d, 16 nibble bytes): d * (code - 8)
+struct Q40 {
+  static constexpr int kQt = 2, kTs = 144, kAlign = 16, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t q[8]; float d[2]; };
+  struct Group { const uint32_t* q; float d; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    uint32_t w[9];
+    ld.words<9, 4>(36 * t, w);
+    r.d[0] = f16_bits_to_float(w[0] & 0xFFFF);
+    r.d[1] = f16_bits_to_float(w[4] >> 16);
+    for (int i = 0; i < 4; i++) { r.q[i] = funnel16(w[i], w[i + 1]); r.q[4 + i] = w[5 + i]; }
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) { return Group{r.q + 4 * grp, r.d[grp]}; }
+  TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) { nibble_octet(g.q[q], p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
+    return fmaf_(g.d, fmaf_(-8.0f, xsum, acc), out);
+  }
+};
+
+// IQ4_NL (18 B, laid out as Q4_0): nibbles select one of sixteen values, codes value + 128
+struct IQ4NL : Q40 {
+  static constexpr int kQt = 20, kPairOrder = 1, kKv = 1;
+  TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) { lookup_octet(tb, g.q[q], p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
+    return fmaf_(g.d, fmaf_(-128.0f, xsum, acc), out);
+  }
+};
+
+// Q4_1 (20 B: d, m, 16 nibble bytes): d * code + m
+struct Q41 {
+  static constexpr int kQt = 3, kTs = 160, kAlign = 16, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t w[10]; };
+  struct Group { const uint32_t* q; float d, m; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) { Run r; ld.words<10, 8>(40 * t, r.w); return r; }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    const uint32_t h = r.w[5 * grp];
+    return Group{r.w + 5 * grp + 1, f16_bits_to_float(h & 0xFFFF), f16_bits_to_float(h >> 16)};
+  }
+  TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) { nibble_octet(g.q[q], p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) { return fmaf_(g.m, xsum, fmaf_(g.d, acc, out)); }
+};
+
+// Q5_0 (22 B: d, 32 fifth bits, 16 nibble bytes): d * (code - 16)
+struct Q50 {
+  static constexpr int kQt = 6, kTs = 176, kAlign = 16, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t q[8], h[2]; float d[2]; };
+  struct Group { const uint32_t* q; uint32_t h; float d; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    uint32_t w[11];
+    ld.words<11, 4>(44 * t, w);
+    r.d[0] = f16_bits_to_float(w[0] & 0xFFFF);
+    r.h[0] = funnel16(w[0], w[1]);
+    r.d[1] = f16_bits_to_float(w[5] >> 16);
+    r.h[1] = w[6];
+    for (int i = 0; i < 4; i++) { r.q[i] = funnel16(w[1 + i], w[2 + i]); r.q[4 + i] = w[7 + i]; }
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) { return Group{r.q + 4 * grp, r.h[grp], r.d[grp]}; }
+  TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) { nibble5_octet(g.q[q], g.h >> (4 * q), p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
+    return fmaf_(g.d, fmaf_(-16.0f, xsum, acc), out);
+  }
+};
+
+// Q5_1 (24 B: d, m, 32 fifth bits, 16 nibble bytes): d * code + m
+struct Q51 {
+  static constexpr int kQt = 7, kTs = 192, kAlign = 16, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t w[12]; };
+  struct Group { const uint32_t* q; uint32_t h; float d, m; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) { Run r; ld.words<12, 16>(48 * t, r.w); return r; }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    const uint32_t h = r.w[6 * grp];
+    return Group{r.w + 6 * grp + 2, r.w[6 * grp + 1], f16_bits_to_float(h & 0xFFFF), f16_bits_to_float(h >> 16)};
+  }
+  TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) { nibble5_octet(g.q[q], g.h >> (4 * q), p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) { return fmaf_(g.m, xsum, fmaf_(g.d, acc, out)); }
+};
+
+// MXFP4 (17 B: an exponent byte e, 16 nibble bytes): 2^(e - 128) * value, codes value + 12.  Blocks have no alignment: the
+// run's 34 bytes start at 2 t (mod 4) and its blocks at bytes 0 and 17.  The scale reaches down to 2^-128 and meets sums
+// staged times 2^-37: it is carried times 2^37, so that no product leaves the float32 range sooner than the result does.
+struct MXFP4 {
+  static constexpr int kQt = 39, kTs = 136, kAlign = 8, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 1, kKv = 2, kScaleExp = 37;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t q[8]; float d[2]; };
+  struct Group { const uint32_t* q; float d; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static float scale(uint32_t e) {
+    const uint32_t bits = e < 2 ? 0x00200000u << e : (e - 1) << 23;
+#if TF_DEVICE
+    return mulf(__uint_as_float(bits), 0x1p37f);
+#else
+    float d;
+    memcpy(&d, &bits, 4);
+    return mulf(d, 0x1p37f);
+#endif
+  }
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    uint32_t v[8], tail;
+    ld.words<8, 2>(34 * t, v);
+    tail = ld.u16(34 * t + 32);
+    r.d[0] = scale(v[0] & 0xFF);
+    r.d[1] = scale((v[4] >> 8) & 0xFF);
+    for (int i = 0; i < 4; i++) r.q[i] = prmt(v[i], v[i + 1], 0x4321u);
+    for (int i = 0; i < 4; i++) r.q[4 + i] = funnel16(v[4 + i], i == 3 ? tail : v[5 + i]);
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) { return Group{r.q + 4 * grp, r.d[grp]}; }
+  TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) { lookup_octet(tb, g.q[q], p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
+    return fmaf_(g.d, fmaf_(-12.0f, xsum, acc), out);
+  }
+};
+
+// NVFP4 (36 B per 64 weights: four UE4M3 scales, 32 nibble bytes): group s = 16 weights, elements 16 s + j (low nibble of
+// byte 8 s + j) and 16 s + 8 + j (high nibble), codes value + 12.  A superblock is four blocks, run t is block t.
+struct NVFP4 {
+  static constexpr int kQt = 40, kTs = 144, kAlign = 16, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 1, kKv = 2;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kTableBytes = 0;
+  struct Run { uint32_t w[9]; };
+  struct Group { const uint32_t* q; float d; };
+  TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 16 * (oo >> 1) + 4 * (oo & 1); b = a + 8; }
+  TF_HD static int x_exp(int, int) { return 0; }
+  TF_HD static Run load_run(const BlockLd& ld, int t) { Run r; ld.words<9, 4>(36 * t, r.w); return r; }
+  TF_HD static float scale(uint32_t x) {       // half the UE4M3 value; 0 and 0x7F stand for 0
+    const int ex = (int)(x >> 3) & 15;
+    const float man = u2f(x & 7);
+    const float raw = ex == 0 ? mulf(man, 0x1p-9f) : mulf(8.0f + man, u2f(1u << ex) * 0x1p-10f);
+    return (x == 0 || x == 0x7F) ? 0.0f : mulf(raw, 0.5f);
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    return Group{r.w + 1 + 2 * grp, scale((r.w[0] >> (8 * grp)) & 0xFF)};
+  }
+  TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) { lookup_octet(tb, g.q[q], p); }
+  TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
+    return fmaf_(g.d, fmaf_(-12.0f, xsum, acc), out);
   }
 };
 

@@ -119,7 +119,7 @@ def fused_matmul(x: torch.Tensor, w: QuantizedArray, *, out_dtype=torch.bfloat16
         key = (int(w.qtype), n_rows, k_dim, m)
         need = _ws_need.get(key)
         if need is None:
-            need = _ws_need[key] = L.ggq_workspace_bytes(*key)
+            need = _ws_need[key] = L.ggq_scratch_bytes(*key)
         ws = _backend.workspace(dev, need, stream)
         _lib.check(fn(key[0], data.data_ptr(), n_rows, k_dim, x_ptr, m, y.data_ptr(),
                       _backend.dtype_code(out_dtype), ws.data_ptr() if ws is not None else None,

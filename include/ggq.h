@@ -104,6 +104,11 @@ int32_t ggq_gemv_max_batch(void);
  * kernels that need none where there is one, and return GGQ_INVALID_VALUE otherwise. */
 size_t ggq_workspace_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M);
 
+/* The scratch with which every kernel ggq_gemv / ggq_gemm may choose can run, never less than ggq_workspace_bytes: the
+ * legacy, FP4, ternary and Q3_K formats work without any at batches up to 16, two to five times slower than with this much.
+ * Same rules (zero-filled once, 256-byte aligned, one per stream).  No reference counterpart. */
+size_t ggq_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M);
+
 /* y[M, N] = x[M, K] @ W[N, K]^T with W quantized (row-major blocks, N rows of
  * K / block_elems * block_bytes bytes), x bf16, y of y_dtype, 1 <= M <= ggq_gemv_max_batch().
  * Weights are applied at full float32 precision (exact integer codes times float32

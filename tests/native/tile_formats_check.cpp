@@ -2,6 +2,8 @@
 // blocks, the A-operand registers, the activation map and the fold of a format must reproduce the
 // decoded weights (given in a file written by the Python test from the CPU decoders).
 //
+// (a superblock is 256 weights: one block, or eight / four consecutive blocks of the 32- and 64-element formats)
+//
 // usage: tile_formats_check <qtype> <blocks.bin> <decoded_f32.bin> <table.bin> <n_blocks>
 #include <cmath>
 #include <cstdio>
@@ -76,7 +78,7 @@ int check(const std::vector<uint8_t>& blocks, const float* want, const Tables& t
         for (int e = 0; e < 256; e++) {
           if (!in_group[e]) continue;
           if (in_sum[e] != 1) { fprintf(stderr, "weight %d enters the group's sum of x %d times\n", e, in_sum[e]); return 1; }
-          const float got = F::fold(raw, (float)acc[e], 1.0f, 0.0f);
+          const float got = std::ldexp(F::fold(raw, (float)acc[e], 1.0f, 0.0f), -ScaleExpOf<F>::value);
           const float ref = want[(size_t)b * 256 + e];
           seen++;
           if (!(got == ref) && !(std::isnan(got) && std::isnan(ref))) {
@@ -100,7 +102,7 @@ int main(int argc, char** argv) {
   const float* want = reinterpret_cast<const float*>(dec.data());
   Tables tb{};
   tb.grid = table.data();
-  if (qt == IQ4XS::kQt) memcpy(tb.kv, table.data(), 16);
+  if (table.size() == 16) memcpy(tb.kv, table.data(), 16);
   switch (qt) {
     case Q4K::kQt: return check<Q4K>(blocks, want, tb, nb);
     case Q2K::kQt: return check<Q2K>(blocks, want, tb, nb);
@@ -114,6 +116,17 @@ int main(int argc, char** argv) {
     case IQ3S::kQt: return check<IQ3S>(blocks, want, tb, nb);
     case IQ1S::kQt: return check<IQ1S>(blocks, want, tb, nb);
     case IQ1M::kQt: return check<IQ1M>(blocks, want, tb, nb);
+    case Q3K::kQt: return check<Q3K>(blocks, want, tb, nb);
+    case TQ10::kQt: return check<TQ10>(blocks, want, tb, nb);
+    case TQ20::kQt: return check<TQ20>(blocks, want, tb, nb);
+    case Q80::kQt: return check<Q80>(blocks, want, tb, nb);
+    case Q40::kQt: return check<Q40>(blocks, want, tb, nb);
+    case Q41::kQt: return check<Q41>(blocks, want, tb, nb);
+    case Q50::kQt: return check<Q50>(blocks, want, tb, nb);
+    case Q51::kQt: return check<Q51>(blocks, want, tb, nb);
+    case IQ4NL::kQt: return check<IQ4NL>(blocks, want, tb, nb);
+    case MXFP4::kQt: return check<MXFP4>(blocks, want, tb, nb);
+    case NVFP4::kQt: return check<NVFP4>(blocks, want, tb, nb);
   }
   fprintf(stderr, "no tile format for qtype %d\n", qt);
   return 2;

@@ -7,6 +7,7 @@ import subprocess
 
 import numpy as np
 import pytest
+from gguf.constants import GGML_QUANT_SIZES
 from gguf.constants import GGMLQuantizationType as QT
 
 from gguf_jax_b200 import _lib, synth
@@ -14,7 +15,8 @@ from oracle import oracle as O
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SRC = os.path.join(ROOT, "tests", "native", "tile_formats_check.cpp")
-TILE_QTYPES = [QT.Q4_K, QT.Q5_K, QT.Q6_K, QT.Q2_K, QT.IQ4_XS, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT.IQ3_XXS, QT.IQ3_S, QT.IQ1_S, QT.IQ1_M]
+TILE_QTYPES = [QT.Q4_K, QT.Q5_K, QT.Q6_K, QT.Q2_K, QT.IQ4_XS, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT.IQ3_XXS, QT.IQ3_S, QT.IQ1_S, QT.IQ1_M,
+               QT.Q3_K, QT.TQ1_0, QT.TQ2_0, QT.Q8_0, QT.Q4_0, QT.Q4_1, QT.Q5_0, QT.Q5_1, QT.IQ4_NL, QT.MXFP4, QT.NVFP4]
 _TAB_OFFSET = {QT.IQ2_XXS: (0, 2048), QT.IQ2_XS: (2048, 4096), QT.IQ2_S: (6144, 8192), QT.IQ3_XXS: (14336, 1024),
                QT.IQ3_S: (15360, 2048), QT.IQ1_S: (17408, 16384), QT.IQ1_M: (17408, 16384)}
 
@@ -30,9 +32,11 @@ def checker(tmp_path_factory):
 def kernel_table(qtype) -> bytes:
     """The lookup table as the kernel holds it in shared memory."""
     blob = _lib.tables_blob()
-    if qtype == QT.IQ4_XS:
+    if qtype in (QT.IQ4_XS, QT.IQ4_NL):
         kv = blob[33792:33808].view(np.int8).astype(np.int16) + 128
         return kv.astype(np.uint8).tobytes()
+    if qtype in (QT.MXFP4, QT.NVFP4):
+        return (blob[33808:33824].view(np.int8) + 12).astype(np.uint8).tobytes()
     if qtype not in _TAB_OFFSET:
         return b"\0" * 16
     off, size = _TAB_OFFSET[qtype]
@@ -44,8 +48,8 @@ def kernel_table(qtype) -> bytes:
 
 @pytest.mark.parametrize("qtype", TILE_QTYPES, ids=lambda t: t.name)
 def test_operands_reproduce_the_decoded_weights(qtype, checker, tmp_path):
-    n_blocks = 96
-    blocks = synth.random_blocks(qtype, n_blocks, seed=int(qtype))
+    n_blocks = 96                                   # superblocks of 256 weights
+    blocks = synth.random_blocks(qtype, n_blocks * (256 // GGML_QUANT_SIZES[qtype][0]), seed=int(qtype))
     dense = O.c_dequantize(blocks, qtype).astype(np.float32)
     O.assert_bitwise_equal(dense, O.ref_dequantize(blocks, qtype), qtype.name)
     (tmp_path / "b.bin").write_bytes(blocks.tobytes())

@@ -118,3 +118,35 @@ def test_low_bit_sweep_shape_sampled_rows(qtype):
         if got16.size >= 512:
             assert O.rel_l2(got16, ref) <= 2e-3, (qtype.name, m)
         np.testing.assert_allclose(got16, ref, rtol=1e-2, atol=1e-2 * np.abs(ref).max())
+
+
+TILE_SMALL_BLOCKS = [QT.Q8_0, QT.Q4_0, QT.Q4_1, QT.Q5_0, QT.Q5_1, QT.IQ4_NL, QT.MXFP4, QT.NVFP4, QT.Q3_K, QT.TQ1_0, QT.TQ2_0]
+
+
+@pytest.mark.parametrize("qtype", TILE_SMALL_BLOCKS, ids=lambda t: t.name)
+def test_formats_of_small_blocks_at_tile_edges(qtype):
+    """Same bar as above (float32 sums in another order) for the legacy, FP4, ternary and Q3_K formats: one and several
+    16-row tiles with and without a remainder, one superblock and several chunks, every number of passes."""
+    for n, k in [(1, 2048), (16, 2048), (200, 2048), (1100, 6144), (4100, 4096)]:
+        wb = synth.make_weight_bytes(n, k, qtype, seed=n)
+        w = on_device(wb, qtype, n, k)
+        for m in (1, 2, 3, 8, 9, 16):
+            xb = synth.make_x(m, k, seed=m)
+            ref = O.c_matmul(O.bf16_bits(xb), wb, qtype)
+            got = kernels.fused_matmul(to_x(xb), w, out_dtype=torch.float32).cpu().numpy()
+            assert O.rel_l2(got, ref) <= 2e-5, (qtype.name, n, k, m)
+
+
+@pytest.mark.parametrize("qtype", TILE_SMALL_BLOCKS + [QT.Q2_K, QT.IQ4_XS], ids=lambda t: t.name)
+def test_non_finite_activations_give_what_the_decoded_weights_give(qtype):
+    """An infinite activation times the decoded weights: infinities keep their sign, and only weights that are exactly
+    zero (or infinities that cancel) give NaN."""
+    n, k = 40, 2048
+    wb = synth.make_weight_bytes(n, k, qtype, seed=5)
+    dense = O.ref_dequantize(wb, qtype).astype(np.float32)
+    xb = synth.make_x(2, k, seed=5)
+    xb[1, 300] = -np.inf
+    got = kernels.fused_matmul(to_x(xb), on_device(wb, qtype, n, k), out_dtype=torch.float32).cpu().numpy()
+    assert np.isfinite(got[0]).all()
+    want = np.where(dense[:, 300] == 0, np.nan, -np.sign(dense[:, 300]) * np.inf)
+    assert np.array_equal(got[1], want, equal_nan=True), qtype.name
