@@ -85,4 +85,5 @@ def workspace(device_index: int, nbytes: int, stream: int | None = None) -> torc
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", device_index))
         _workspaces[key] = ws
+        _lib.native().set_scratch(key[0], key[1], ws)
     return ws

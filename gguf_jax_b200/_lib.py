@@ -6,6 +6,7 @@ is raised to the caller.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 
@@ -91,6 +92,28 @@ def lib() -> ctypes.CDLL:
                     fn.argtypes = args
                 _lib = L
     return _lib
+
+
+NATIVE_PATH = os.path.join(_HERE, "_native.so")
+_native_module = None
+
+
+def native():
+    """The native call path (csrc/torch_call.cpp), bound to the loaded library's entry points."""
+    global _native_module
+    if _native_module is None:
+        with _lock:
+            if _native_module is None:
+                L = lib()
+                if not os.path.exists(NATIVE_PATH):
+                    raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m gguf_jax_b200.build`.")
+                spec = importlib.util.spec_from_file_location("_native", NATIVE_PATH)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_fused_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info)
+                module.bind(*[ctypes.cast(f, ctypes.c_void_p).value for f in entries], int(L.ggq_gemv_max_batch()))
+                _native_module = module
+    return _native_module
 
 
 def check(status: int) -> None:

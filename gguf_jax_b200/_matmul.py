@@ -69,6 +69,13 @@ def fused_batch_limit(w: QuantizedArray) -> int:
     return hit[1](w) if hit is not None and len(w.shape) == 2 else 0
 
 
+def _native_matmul(*args):
+    """First call: load the native module, then be replaced by its function."""
+    global _native_matmul
+    _native_matmul = _lib.native().fast_matmul
+    return _native_matmul(*args)
+
+
 def _validate(x: torch.Tensor, w) -> None:
     if not isinstance(w, QuantizedArray):
         raise TypeError(f"expected a QuantizedArray weight, got {type(w).__name__}")
@@ -94,6 +101,11 @@ def matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None
     served by the fused route only (see :func:`gguf_jax_b200.kernels.fused_matmul`), without
     gradients; anything the fused route does not take raises ``ValueError``.
     """
+    if out is None and w.__class__ is QuantizedArray:
+        # the common call (device activations, no gradient, batch within the fused route) is one native function
+        y = _native_matmul(x, w.data, w.qtype, w.shape, force_fused)
+        if y is not None:
+            return y
     _validate(x, w)
     route = None
     hit = _fused().get(w.qtype)

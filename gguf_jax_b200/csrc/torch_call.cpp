@@ -1,0 +1,142 @@
+// The eager call path of `matmul` as one native function: what gguf_jax_b200/_matmul.py and kernels.py do for the common
+// call (device activations, no gradient, batch within the fused route) without the interpreter in between.
+//
+// A decode step is a chain of products of 4 to 40 us, so the host's time per call is what such a step takes once it is
+// above the kernels': measured on B200, seven products of a 1B-shaped layer took 122 us through the Python path (17 us a
+// call) for 37 us of kernels; through here they take 51 us (7 us a call).  `fast_matmul` returns None for every call that is not the common one, and the Python path,
+// which stays the reference for behaviour and errors, takes it.
+//
+// The library's entry points are handed over as addresses (bind), so that this module follows whichever
+// libggq_b200.so the binding has loaded.  All state is guarded by the interpreter lock.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
+#include <ATen/core/grad_mode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+
+#include <array>
+#include <cstdint>
+#include <map>
+#include <utility>
+
+namespace {
+
+using LaunchFn = int32_t (*)(int32_t, const void*, int64_t, int64_t, const void*, int32_t, void*, int32_t, void*, size_t, void*);
+using LimitFn = int32_t (*)(int32_t, int64_t, int64_t);
+using BytesFn = size_t (*)(int32_t, int64_t, int64_t, int32_t);
+using CodeFn = int32_t (*)(int32_t);
+using InfoFn = int32_t (*)(int32_t, int32_t*, int32_t*);
+
+LaunchFn g_gemv = nullptr, g_gemm = nullptr;
+LimitFn g_limit = nullptr;
+BytesFn g_bytes = nullptr;
+CodeFn g_fused = nullptr;
+InfoFn g_info = nullptr;
+int g_gemv_max = 0;
+constexpr int kBf16 = 1;                 // GGQ_BF16
+
+// scratch per (device, stream): the tensors _backend.workspace hands out (never destroyed: the allocator may be gone by then)
+auto& g_scratch = *new std::map<std::pair<int, uintptr_t>, at::Tensor>();
+
+// What the library answers for a shape, remembered in a small direct-mapped table.
+struct Shape {
+  int64_t n = 0, k = 0;
+  int32_t qtype = -1, m = -1;
+  int32_t limit = 0;
+  size_t scratch = 0, payload = 0;
+};
+std::array<Shape, 1024> g_shapes;
+
+const Shape* shape_of(int32_t qtype, int64_t n, int64_t k, int32_t m) {
+  uint64_t h = (uint64_t)n * 0x9E3779B97F4A7C15ull ^ (uint64_t)k * 0xC2B2AE3D27D4EB4Full ^ (uint64_t)m * 0x165667B19E3779F9ull ^ (uint64_t)qtype << 32;
+  Shape& s = g_shapes[(h >> 40) % g_shapes.size()];
+  if (s.qtype != qtype || s.n != n || s.k != k || s.m != m) {
+    int32_t elems = 0, bytes = 0;
+    if (!g_fused(qtype) || g_info(qtype, &elems, &bytes) != 0 || k <= 0 || k % elems) return nullptr;
+    s = Shape{n, k, qtype, m, g_limit(qtype, n, k), g_bytes(qtype, n, k, m), (size_t)(n * (k / elems)) * (size_t)bytes};
+  }
+  return &s;
+}
+
+// fast_matmul(x, payload, qtype, shape, force_fused) -> Tensor or None (not the common case)
+PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 5 || !g_gemv || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1]) || !PyTuple_CheckExact(args[3]) ||
+      PyTuple_GET_SIZE(args[3]) != 2)
+    Py_RETURN_NONE;
+  const at::Tensor& x = THPVariable_Unpack(args[0]);
+  const at::Tensor& w = THPVariable_Unpack(args[1]);
+  // plain strided CUDA tensors on the current device only; whatever wraps, records or transforms takes the Python path
+  if (!x.defined() || !w.defined() || !x.is_cuda() || !w.is_cuda() || x.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kByte ||
+      x.layout() != at::kStrided || w.layout() != at::kStrided || x.dim() < 1 || x.device() != w.device() || !w.is_contiguous() ||
+      at::isTensorSubclassLike(x) || at::isTensorSubclassLike(w) || x.is_conj() || x.is_neg() || w.is_neg() ||
+      c10::impl::TorchDispatchModeTLS::any_modes_set() || torch::jit::tracer::isTracing() || x._fw_grad(0).defined() ||
+      (x.requires_grad() && at::GradMode::is_enabled()))
+    Py_RETURN_NONE;
+  const int64_t n = PyLong_AsLongLong(PyTuple_GET_ITEM(args[3], 0)), k = PyLong_AsLongLong(PyTuple_GET_ITEM(args[3], 1));
+  const long qtype = PyLong_AsLong(args[2]);
+  if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+  const int dev = x.device().index();
+  if (n <= 0 || k <= 0 || x.size(-1) != k || dev != c10::cuda::current_device()) Py_RETURN_NONE;
+  const int64_t m = x.numel() / k;
+  if (m < 1 || m > 65536) Py_RETURN_NONE;
+  const Shape* s = shape_of((int32_t)qtype, n, k, (int32_t)m);
+  if (!s || (m > s->limit && args[4] != Py_True) || (size_t)w.numel() != s->payload) Py_RETURN_NONE;
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev);
+  const auto it = g_scratch.find({dev, (uintptr_t)stream.stream()});
+  // no scratch yet on this stream (its first call also uploads the code books), or one that has to grow
+  if (it == g_scratch.end() || (size_t)it->second.numel() < s->scratch) Py_RETURN_NONE;
+  const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+  c10::SmallVector<int64_t, 6> sizes(x.sizes().begin(), x.sizes().end());
+  sizes.back() = n;
+  at::Tensor y = at::empty(sizes, x.options().requires_grad(false));
+  const int32_t rc = (m <= g_gemv_max ? g_gemv : g_gemm)((int32_t)qtype, w.data_ptr(), n, k, xc.data_ptr(), (int32_t)m, y.data_ptr(), kBf16,
+                                                         it->second.data_ptr(), (size_t)it->second.numel(), stream.stream());
+  if (rc != 0) Py_RETURN_NONE;         // the Python path repeats the call and raises its error
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// bind(gemv, gemm, fused_batch_limit, scratch_bytes, has_fused, type_info, gemv_max_batch): entry point addresses
+PyObject* bind(PyObject*, PyObject* args) {
+  unsigned long long gemv, gemm, limit, bytes, fused, info;
+  int max_batch;
+  if (!PyArg_ParseTuple(args, "KKKKKKi", &gemv, &gemm, &limit, &bytes, &fused, &info, &max_batch)) return nullptr;
+  g_gemv = (LaunchFn)(uintptr_t)gemv;
+  g_gemm = (LaunchFn)(uintptr_t)gemm;
+  g_limit = (LimitFn)(uintptr_t)limit;
+  g_bytes = (BytesFn)(uintptr_t)bytes;
+  g_fused = (CodeFn)(uintptr_t)fused;
+  g_info = (InfoFn)(uintptr_t)info;
+  g_gemv_max = max_batch;
+  Py_RETURN_NONE;
+}
+
+// set_scratch(device, stream, tensor): the scratch of a stream, as _backend.workspace (re)allocates it
+PyObject* set_scratch(PyObject*, PyObject* args) {
+  HANDLE_TH_ERRORS
+  int dev;
+  unsigned long long stream;
+  PyObject* t;
+  if (!PyArg_ParseTuple(args, "iKO", &dev, &stream, &t)) return nullptr;
+  if (!THPVariable_Check(t)) { PyErr_SetString(PyExc_TypeError, "set_scratch: a tensor is wanted"); return nullptr; }
+  g_scratch[{dev, (uintptr_t)stream}] = THPVariable_Unpack(t);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"fast_matmul", (PyCFunction)(void (*)())fast_matmul, METH_FASTCALL, "x @ w.T by the fused kernels, or None"},
+    {"bind", bind, METH_VARARGS, "hand over the library's entry points"},
+    {"set_scratch", set_scratch, METH_VARARGS, "register a stream's scratch"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module_def); }
