@@ -48,9 +48,11 @@ __device__ __forceinline__ uint2 ld8(const uint8_t* p) {
     const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
     return make_uint2(GGQ_LD(q), GGQ_LD(q + 1));
   } else if constexpr (ALIGN >= 2) {
-    const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
-    return make_uint2((uint32_t)GGQ_LD(q) | ((uint32_t)GGQ_LD(q + 1) << 16),
-                      (uint32_t)GGQ_LD(q + 2) | ((uint32_t)GGQ_LD(q + 3) << 16));
+    // the two or three aligned words that hold the bytes (never one that holds none of them)
+    const uint32_t sh = ((uintptr_t)p & 2) * 8;
+    const uint32_t* q = reinterpret_cast<const uint32_t*>((uintptr_t)p & ~(uintptr_t)3);
+    const uint32_t a = GGQ_LD(q), b = GGQ_LD(q + 1), c = sh ? GGQ_LD(q + 2) : 0u;
+    return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh));
   } else {
     return make_uint2(ld32(p), ld32(p + 4));
   }

@@ -1,0 +1,84 @@
+"""The native call path of `matmul` against the Python path it stands for: same results for every form of activations, and the
+forms it must leave alone (gradients, host memory, transforms, subclasses, shapes and batches outside the fused route)."""
+import pytest
+import torch
+from gguf.constants import GGMLQuantizationType as QT
+
+import gguf_jax_b200 as gj
+from gguf_jax_b200 import _lib, kernels, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def native(x, w, force=False):
+    return _lib.native().fast_matmul(x, w.data, w.qtype, w.shape, force)
+
+
+@pytest.fixture(scope="module")
+def weight():
+    w = synth.make_weight(96, 2048, QT.Q4_K, seed=1, device="cuda")
+    x = torch.randn((16, 2048), device="cuda").bfloat16()
+    for m in (1, 2, 16):
+        gj.matmul(x[:m], w)            # the stream's scratch
+    return w, x
+
+
+def test_takes_the_common_call(weight):
+    w, x = weight
+    for a in (x[:1], x[3], x.reshape(2, 2, 4, 2048), x[:6:2], x.T.contiguous().T[:5]):
+        got = native(a, w)
+        want = kernels.fused_matmul(a, w)
+        assert got.shape == want.shape == (*a.shape[:-1], 96) and got.dtype == torch.bfloat16 and got.is_contiguous()
+        assert torch.equal(got, want) and torch.equal(gj.matmul(a, w), want)
+    with torch.inference_mode():
+        assert native(x[:2], w).is_inference()
+    with torch.no_grad():
+        assert not native(x[:2].requires_grad_(True), w).requires_grad
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert native(x[:2], w) is None                 # no scratch on this stream yet: the Python path makes it
+        first = gj.matmul(x[:2], w)
+        second = native(x[:2], w)
+    torch.cuda.synchronize()
+    assert torch.equal(first, second) and torch.equal(first, kernels.fused_matmul(x[:2], w))
+
+
+def test_leaves_everything_else_to_the_python_path(weight):
+    w, x = weight
+
+    class Sub(torch.Tensor):
+        pass
+
+    assert native(x.clone().requires_grad_(True), w) is None
+    assert native(x.float(), w) is None and native(x.cpu(), w) is None
+    assert native(x[:, :1024], w) is None and native(x[:0], w) is None
+    assert native(x.as_subclass(Sub), w) is None
+    assert native(x, synth.make_weight(96, 2048, QT.Q4_K, seed=1, device="cuda").astype(torch.float32)) is not None   # fused: w.dtype plays no part
+    big = torch.randn((64, 2048), device="cuda").bfloat16()
+    assert native(big, synth.make_weight(96, 2048, QT.Q8_0, seed=1, device="cuda")) is None         # above its limit: dense route
+    for bad in (object(), None, [x]):
+        assert native(bad, w) is None
+    with pytest.raises(ValueError):
+        gj.matmul(x[:, :1024], w)
+    with pytest.raises(TypeError):
+        gj.matmul(x, w.data)
+    x2 = x.clone().requires_grad_(True)
+    gj.matmul(x2, w).float().sum().backward()
+    assert x2.grad is not None and x2.grad.shape == x2.shape
+
+
+def test_under_capture(weight):
+    w, x = weight
+    want = gj.matmul(x[:4], w)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        gj.matmul(x[:4], w)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = gj.matmul(x[:4], w)
+    y.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
