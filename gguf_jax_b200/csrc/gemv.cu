@@ -61,6 +61,19 @@ static bool tile_scratch_is_optional(int qtype) {
          qtype != QT_IQ3_XXS && qtype != QT_IQ3_S && qtype != QT_IQ1_S && qtype != QT_IQ1_M;
 }
 
+// Where the tiled kernel and the kernels it replaces (streaming at batch 1, one MMA launch for 2..16 rows) cross, for the
+// formats of tile_scratch_is_optional and for rows that are not 16-byte aligned.  The tiled kernel starts at 6 us (batch 1) to 13 us
+// (batch 8; a larger batch is two launches) and grows slowly; the others start at 5 and 10 to 20 us and grow with their
+// decoding.  Measured on B200, us, others / tiled: batch 1, 1024 x 4096 Q8_0 5.5 / 6.2, Q4_0 5.4 / 6.3, 14336 x 4096 25.8 /
+// 19.7, 31.2 / 15.4; batch 8, 1024 x 4096 Q8_0 10.1 / 12.9, Q4_0 17.1 / 12.9; batch 16, 14336 x 4096 Q8_0 54.8 / 58.3, TQ2_0 60.6 /
+// 52.9, Q4_0 92 / 53, IQ4_NL 104 / 67, 5003 x 2816 IQ2_XS 25.7 / 29.2, Q2_K 22.7 / 27.0.
+static bool tile_pays(int qtype, int64_t weights, int M) {
+  if (M == 1) return weights >= (8 << 20);
+  if (M <= 4) return true;
+  if (M <= 8) return qtype != QT_Q8_0 || weights >= (10 << 20);
+  return weights >= (qtype == QT_Q8_0 ? 80 << 20 : qtype == QT_TQ2_0 ? 32 << 20 : 16 << 20);
+}
+
 static size_t tile_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
   const int tmax = gemv_tile_max_batch(qtype);
   return tmax && M <= kGemvMaxBatch && K % 256 == 0 ? gemv_tile_workspace_bytes(qtype, N, K, M < tmax ? M : tmax) : 0;
@@ -147,7 +160,11 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   // the batch-major kernel takes the larger weights (Q4_K 8192 x 28672: 68 / 77 us at batch 8 / 16 against
   // 100 / 153 us) and the integer-code MMA kernel (gemv_mma.cu) the smaller ones (see wide_pays).
   const bool k_quant = is_k_quant(qtype);
-  const bool tile_first = !k_quant || (M >= 2 && M <= 4) || (M == 1 && m1_tiled);
+  // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them
+  const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
+  const int64_t weights = N * K;
+  const bool tile_first = k_quant ? (M >= 2 && M <= 4) || (M == 1 && (odd_rows ? tile_pays(qtype, weights, 1) : m1_tiled))
+                                  : (!odd_rows && !tile_scratch_is_optional(qtype)) || tile_pays(qtype, weights, M);
   const int tile_max = gemv_tile_max_batch(qtype);
   const int tile_m = M < tile_max ? M : tile_max;
   const size_t tile_need = tile_max ? gemv_tile_workspace_bytes(qtype, N, K, tile_m) : 0;

@@ -73,6 +73,7 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
         g.spu = g.chunk_sb / nb;
         g.C = (SB + g.chunk_sb - 1) / g.chunk_sb;
         g.RT = (int)((N + 15) / 16);
+        g.row_skew = (int)((int64_t)SB * fi.ts % 16);
         g.S = (int64_t)g.C * g.RT * g.spu;
         const int64_t units = (int64_t)g.C * g.RT;
         g.W = (int)std::min<int64_t>((int64_t)sm_count * kWarps, units);
@@ -138,7 +139,7 @@ bool gemv_tile_applicable(int qtype, int64_t N, int64_t K, int M, const void* w,
   tile::FormatInfo fi;
   if (!tile::format_of(qtype, &fi)) return false;
   if (M < 1 || M > gemv_tile_max_batch(qtype) || K <= 0 || K % 256 || N < 1 || N > (1ll << 24)) return false;
-  if ((K / 256 * fi.ts) % 16 || (uintptr_t)w % 16 || (uintptr_t)x % 16 || (K * 2) % 16) return false;
+  if ((uintptr_t)w % 16 || (uintptr_t)x % 16 || (K * 2) % 16) return false;
   if (N * (K / 256 * fi.ts) >= (1ll << 31)) return false;      // block offsets are 32-bit inside a row; rows are 64-bit
   tile::Geo geo;
   return tile::plan(fi, N, K, M, 148, 0, 0, &geo);

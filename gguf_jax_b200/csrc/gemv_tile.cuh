@@ -19,7 +19,9 @@
 // copies, one to five steps ahead of the one it is multiplying; consecutive steps of a warp are
 // consecutive bytes of the same 16 rows.  There is no block-wide barrier after the prologue.  Blocks
 // of most formats are only 2-byte aligned, so a step copies the 16-byte aligned window around its
-// bytes; rows must start 16-byte aligned (K / 256 * block bytes a multiple of 16).
+// bytes.  Where the rows are whole multiples of 16 bytes apart all rows of a step have the same offset in
+// their windows; otherwise (K / 256 * block bytes not a multiple of 16: Q6_K at K = 2816, the IQ2 formats at
+// most K) every row has its own, found by the copying and by the reading lanes from the row number.
 //
 // Arithmetic.  mma.sync.m16n8k16 with exact integer codes as bf16 operands (tile_formats.cuh).
 // The eight B columns are four lane-run channels x two batch rows: column 2t carries batch row
@@ -60,6 +62,7 @@ struct Geo {
   int x_row_bytes;       // staged bytes per batch row and chunk, padded to 64 (mod 128)
   int xs_row_floats;     // sums per batch row and chunk
   int off_x, off_xs, off_zero, off_tab, off_misc, total;
+  int row_skew;          // bytes by which consecutive rows differ modulo 16 (0: rows 16-byte aligned)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -212,30 +215,45 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
       const int nbh = min(nb, SB - sb0);
       if (nbh > 0) {
         const int boff = sb0 * F::kTs;
-        const int pieces = ((boff & 15) + nbh * F::kTs + 15) >> 4;
         const int row0 = rt_i * 16;
-        const uint8_t* src0 = w + (boff & ~15) + 16 * kl;
         const uint32_t dst0 = my_ring + slot_i * geo.slot_bytes + hl * pitch + 16 * kl;
-        // a half-warp copies one row: lane kl takes pieces kl, kl + 16 (and kl + 32 where a step can be
-        // wider than 512 bytes); predicated single instructions, no loops, so the warp stays converged
-        const bool q0 = kl < pieces, q1 = kl + 16 < pieces, q2 = kl + 32 < pieces;
         constexpr bool kWide = 14 + 4 * F::kTs + 15 > 512;
-        if (row0 + 16 <= N) {
-          const uint8_t* src = src0 + (int64_t)(row0 + hl) * row_bytes;
+        if (geo.row_skew != 0) {
+          // rows at different offsets of their windows: as below, with the window worked out per row (a copied piece holds
+          // at least one byte of the row, so nothing behind the 16-byte boundary after the tensor's end is read)
 #pragma unroll
           for (int i = 0; i < 8; i++) {
-            if (q0) cp_async16(dst0 + i * (2 * pitch), src);
-            if (q1) cp_async16(dst0 + i * (2 * pitch) + 256, src + 256);
-            if (kWide && q2) cp_async16(dst0 + i * (2 * pitch) + 512, src + 512);
-            src += 2 * row_bytes;
+            const int row = min(row0 + 2 * i + hl, N - 1);
+            const uint8_t* p = w + (int64_t)row * row_bytes + boff;
+            const int skew = (int)((uintptr_t)p & 15), pieces = (skew + nbh * F::kTs + 15) >> 4;
+            const uint8_t* src = p - skew + 16 * kl;
+            if (kl < pieces) cp_async16(dst0 + i * (2 * pitch), src);
+            if (kl + 16 < pieces) cp_async16(dst0 + i * (2 * pitch) + 256, src + 256);
+            if (kWide && kl + 32 < pieces) cp_async16(dst0 + i * (2 * pitch) + 512, src + 512);
           }
-        } else {            // last, ragged row tile: rows past the end repeat row N - 1 (multiplied, never stored)
+        } else {
+          const int pieces = ((boff & 15) + nbh * F::kTs + 15) >> 4;
+          const uint8_t* src0 = w + (boff & ~15) + 16 * kl;
+          // a half-warp copies one row: lane kl takes pieces kl, kl + 16 (and kl + 32 where a step can be
+          // wider than 512 bytes); predicated single instructions, no loops, so the warp stays converged
+          const bool q0 = kl < pieces, q1 = kl + 16 < pieces, q2 = kl + 32 < pieces;
+          if (row0 + 16 <= N) {
+            const uint8_t* src = src0 + (int64_t)(row0 + hl) * row_bytes;
 #pragma unroll
-          for (int i = 0; i < 8; i++) {
-            const uint8_t* src = src0 + (int64_t)min(row0 + 2 * i + hl, N - 1) * row_bytes;
-            if (q0) cp_async16(dst0 + i * (2 * pitch), src);
-            if (q1) cp_async16(dst0 + i * (2 * pitch) + 256, src + 256);
-            if (kWide && q2) cp_async16(dst0 + i * (2 * pitch) + 512, src + 512);
+            for (int i = 0; i < 8; i++) {
+              if (q0) cp_async16(dst0 + i * (2 * pitch), src);
+              if (q1) cp_async16(dst0 + i * (2 * pitch) + 256, src + 256);
+              if (kWide && q2) cp_async16(dst0 + i * (2 * pitch) + 512, src + 512);
+              src += 2 * row_bytes;
+            }
+          } else {            // last, ragged row tile: rows past the end repeat row N - 1 (multiplied, never stored)
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              const uint8_t* src = src0 + (int64_t)min(row0 + 2 * i + hl, N - 1) * row_bytes;
+              if (q0) cp_async16(dst0 + i * (2 * pitch), src);
+              if (q1) cp_async16(dst0 + i * (2 * pitch) + 256, src + 256);
+              if (kWide && q2) cp_async16(dst0 + i * (2 * pitch) + 512, src + 512);
+            }
           }
         }
       }
@@ -294,17 +312,19 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
   }
   __syncthreads();
 
-  // Stage the activations of chunk c into buffer cb: destination order [block][run t][octet][8 values],
-  // 16 bytes per octet, so a lane's run of a block is 128 contiguous bytes.
+  // Stage the activations of batch rows m_lo .. m_hi - 1 of chunk c into buffer cb, scaled by 2^S: destination order
+  // [block][run t][octet][8 values], 16 bytes per octet, so a lane's run of a block is 128 contiguous bytes.  All rows
+  // together are dealt to the threads (row by row took eight dependent rounds of loads at eight rows and kept 32 to
+  // 128 of the 512 threads busy where chunks are short: 1024 x 4096 Q8_0 at 8 rows 17.2 us).
   constexpr uint32_t kRunBytes = F::kOct * 16;          // staged activations of one lane run
   constexpr uint32_t kRunStride = kRunBytes + 16;
-  auto stage_pass = [&](int cb, int c, int m, int S) -> float {
-    const int n_oct = geo.chunk_sb * (4 * F::kOct);
-    uint4* xv = reinterpret_cast<uint4*>(smem + geo.off_x + (cb * XR + m) * geo.x_row_bytes);
-    float* xs = reinterpret_cast<float*>(smem + geo.off_xs) + (cb * XR + m) * geo.xs_row_floats;
+  const int n_oct = geo.chunk_sb * (4 * F::kOct);       // octets per row and chunk: a multiple of 32, so a warp has one row
+  auto stage_rows = [&](int cb, int c, int m_lo, int m_hi, int S, bool track) {
     const float sum_scale = pow2f(S - 133);
-    float amax = 0.f;
-    for (int o = tid; o < n_oct; o += kThreads) {
+    for (int idx = tid; idx < (m_hi - m_lo) * n_oct; idx += kThreads) {
+      const int m = m_lo + idx / n_oct, o = idx % n_oct;
+      uint8_t* xv = smem + geo.off_x + (cb * XR + m) * geo.x_row_bytes;
+      float* xs = reinterpret_cast<float*>(smem + geo.off_xs) + (cb * XR + m) * geo.xs_row_floats;
       const int blk = o / (4 * F::kOct), tt = (o / F::kOct) & 3, oo = o % F::kOct;
       int qa, qb;
       F::src_quads(tt, oo, qa, qb);
@@ -326,14 +346,17 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
       uint4 o4;
       if (F::kPairOrder == 0) o4 = make_uint4(pack_bf16(a0 * up, a2 * up), pack_bf16(a1 * up, a3 * up),
                                                pack_bf16(b0 * up, b2 * up), pack_bf16(b1 * up, b3 * up));
-      else o4 = make_uint4(pack_bf16(a0 * up, a1 * up), pack_bf16(b0 * up, b1 * up),
-                           pack_bf16(a2 * up, a3 * up), pack_bf16(b2 * up, b3 * up));
+      else o4 = make_uint4(pack_bf16(a0 * up, b0 * up), pack_bf16(a1 * up, b1 * up),
+                           pack_bf16(a2 * up, b2 * up), pack_bf16(a3 * up, b3 * up));
       // a run takes kRunBytes + 16 bytes and a batch row 64 (mod 128) bytes, so that the eight lanes that
       // read activations at once (four runs x two batch rows) hit eight different 16-byte bank groups
-      *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(xv) + (blk * 4 + tt) * kRunStride + oo * 16) = o4;
+      *reinterpret_cast<uint4*>(xv + (blk * 4 + tt) * kRunStride + oo * 16) = o4;
       float sum = ((a0 + a1) + (a2 + a3)) + ((b0 + b1) + (b2 + b3));
       const float asum = ((fabsf(a0) + fabsf(a1)) + (fabsf(a2) + fabsf(a3))) + ((fabsf(b0) + fabsf(b1)) + (fabsf(b2) + fabsf(b3)));
-      amax = fmaxf(amax, asum);
+      if (track && m < M) {                              // non-negative floats order like integers
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(asum));
+        if (lane == 0) atomicMax(&misc[cb * 16 + 8 + m], (int)top);
+      }
       if constexpr (F::kSums) {
         if ((oo & (F::kGroupOct - 1)) >= F::kSumOct) sum = 0.f;      // second plane of a two-plane format: same weights again
         if (F::kGroupOct >= 2) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
@@ -342,22 +365,17 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
         if ((oo & (F::kGroupOct - 1)) == 0) xs[o / F::kGroupOct] = sum * sum_scale;
       }
     }
-    return amax;
   };
   // Optimistic scale 2^96: right whenever the largest |x| of a chunk lies in about [2^-30, 2^24); a row
   // outside that range is staged a second time with a scale that puts its largest magnitude near 2^120.
-  for (int c = c_lo; c <= c_hi; c++)
-    for (int m = 0; m < XR; m++) {
-      const float amax = stage_pass(c - c_lo, c, m, 96);
-      if (m < M) atomicMax(&misc[(c - c_lo) * 16 + 8 + m], (int)__float_as_uint(amax));   // non-negative floats order like integers
-    }
+  for (int c = c_lo; c <= c_hi; c++) stage_rows(c - c_lo, c, 0, XR, 96, true);
   __syncthreads();
   for (int c = c_lo; c <= c_hi; c++)
     for (int m = 0; m < M; m++) {
       const int emax = min((misc[(c - c_lo) * 16 + 8 + m] >> 23) & 0xFF, 254);   // biased exponent of the largest octet sum of |x|
       if (emax > 156 || (emax < 97 && emax > 0)) {
         const int S = max(8, min(120, 247 - emax));
-        stage_pass(c - c_lo, c, m, S);
+        stage_rows(c - c_lo, c, m, m + 1, S, false);
         if (tid == 0) misc[(c - c_lo) * 16 + m] = S;
       }
     }
@@ -425,7 +443,13 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
       const int sb0 = c * geo.chunk_sb + k * nb;
       const int nbh = min(nb, SB - sb0);
       const int cb = c - c_lo;
-      const uint32_t tile = my_ring + slot * geo.slot_bytes + g * pitch + ((sb0 * F::kTs) & 15);
+      // offsets of the blocks of rows g and g + 8 in their windows (the copy side's min() with N - 1 included)
+      const uint32_t tile = my_ring + slot * geo.slot_bytes + g * pitch;
+      uint32_t skew0 = (sb0 * F::kTs) & 15, skew1 = skew0;
+      if (geo.row_skew != 0) {
+        skew0 = (sb0 * F::kTs + min(rt * 16 + g, N - 1) * geo.row_skew) & 15;
+        skew1 = (sb0 * F::kTs + min(rt * 16 + g + 8, N - 1) * geo.row_skew) & 15;
+      }
       const uint32_t xr0 = x_lane + cb * x_buf + (k * nb) * x_blk;
       const uint32_t xs0 = xs_base + (uint32_t)(((cb * XR) * geo.xs_row_floats + (k * nb * 4 + t) * kGroups) * 4);
       if constexpr (kQ4kM1) {
@@ -433,12 +457,12 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
           const uint32_t xa0 = q4k_x_lane + cb * x_buf + (k * nb) * x_blk;
           const uint32_t xsa0 = xs0;           // the run's two sub-block sums: xs[(blk * 4 + t) * 2 + {0, 1}]
           for (int blk = 0; blk < nbh; blk++)
-            q4k_block_m1(tile + blk * F::kTs, tile + blk * F::kTs + 8 * pitch, t, q4k_lane, xa0 + blk * x_blk, x_oct,
+            q4k_block_m1(tile + skew0 + blk * F::kTs, tile + skew1 + blk * F::kTs + 8 * pitch, t, q4k_lane, xa0 + blk * x_blk, x_oct,
                          xsa0 + blk * (4 * kGroups * 4), out[0][0], out[0][2]);
         }
       }
       for (int blk = 0; blk < (q4k_fast ? 0 : nbh); blk++) {
-        const tf::BlockLd ld0{tile + blk * F::kTs}, ld1{tile + blk * F::kTs + 8 * pitch};
+        const tf::BlockLd ld0{tile + skew0 + blk * F::kTs}, ld1{tile + skew1 + blk * F::kTs + 8 * pitch};
         const typename F::Run run0 = F::load_run(ld0, t), run1 = F::load_run(ld1, t);
         const uint32_t xr = xr0 + blk * x_blk;
         const uint32_t xsb = xs0 + blk * (4 * kGroups * 4);

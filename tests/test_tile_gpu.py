@@ -150,3 +150,18 @@ def test_non_finite_activations_give_what_the_decoded_weights_give(qtype):
     assert np.isfinite(got[0]).all()
     want = np.where(dense[:, 300] == 0, np.nan, -np.sign(dense[:, 300]) * np.inf)
     assert np.array_equal(got[1], want, equal_nan=True), qtype.name
+
+
+@pytest.mark.parametrize("qtype", [QT.Q6_K, QT.Q2_K, QT.Q3_K, QT.IQ4_XS, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT.IQ3_XXS, QT.IQ3_S, QT.IQ1_S,
+                                   QT.IQ1_M, QT.TQ1_0, QT.TQ2_0, QT.MXFP4], ids=lambda t: t.name)
+def test_rows_at_every_offset_of_a_16_byte_piece(qtype):
+    """K = 256 times an odd number: consecutive rows start at different offsets modulo 16 for these formats.  Enough weights
+    for the tiled kernel at batch 1 and above 8 too (its rules count weights), the last row tile ragged."""
+    for n, k in [(3005, 11 * 256), (7001, 5 * 256)]:
+        wb = synth.make_weight_bytes(n, k, qtype, seed=n)
+        w = on_device(wb, qtype, n, k)
+        rows = np.unique(np.concatenate([np.arange(40), np.random.default_rng(2).choice(n, 200), np.arange(n - 30, n)]))
+        for m in (1, 2, 4, 8):
+            xb = synth.make_x(m, k, seed=m)
+            got = kernels.fused_matmul(to_x(xb), w, out_dtype=torch.float32).cpu().numpy()[:, rows]
+            assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb[rows], qtype)) <= 2e-5, (qtype.name, n, k, m)
