@@ -163,7 +163,11 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them
   const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
   const int64_t weights = N * K;
-  const bool tile_first = k_quant ? (M >= 2 && M <= 4) || (M == 1 && (odd_rows ? tile_pays(qtype, weights, 1) : m1_tiled))
+  // K-quants below 6 M weights at 2..4 rows: the MMA kernel (2048 x 2048 Q4_K 4.7 us against the tiled kernel's 6.7 / 8.3 at
+  // 2 / 4 rows; 8192 x 2048 9.3 against 8.3 / 9.8)
+  const bool small_batch = k_quant && M >= 2 && M <= 4 && weights < (6 << 20) && gemv_mma_applicable(ti, N, K, M);
+  if (small_batch) tuned = nullptr;
+  const bool tile_first = k_quant ? (M >= 2 && M <= 4 && !small_batch) || (M == 1 && (odd_rows ? tile_pays(qtype, weights, 1) : m1_tiled))
                                   : (!odd_rows && !tile_scratch_is_optional(qtype)) || tile_pays(qtype, weights, M);
   const int tile_max = gemv_tile_max_batch(qtype);
   const int tile_m = M < tile_max ? M : tile_max;
@@ -171,7 +175,9 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const bool tile_ok = tile_first && tile_need && workspace && workspace_bytes >= tile_need && (uintptr_t)workspace % 256 == 0 &&
                        sm_count_of(dev) > 0 && gemv_tile_applicable(qtype, N, K, tile_m, w, x_bf16);
   static const int wide_min = [] { const char* e = getenv("GGQ_WIDE_MIN"); return e ? atoi(e) : 5; }();
-  const bool wide_ok = k_quant && M >= wide_min && wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes) && workspace && (uintptr_t)workspace % 256 == 0 && sm_count_of(dev) > 0 &&
+  // (rows that are not 16-byte aligned: the MMA kernel reads them with 2-byte loads; 5003 x 2816 Q6_K at 5 / 16 rows 21.3 / 25.2 us
+  // there, 18.0 / 19.8 here; 1024 x 5376 13.0 / 14.6 there, 20.0 / 21.0 here)
+  const bool wide_ok = k_quant && M >= wide_min && (odd_rows ? weights >= (12ll << 20) : wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes)) && workspace && (uintptr_t)workspace % 256 == 0 && sm_count_of(dev) > 0 &&
                        workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, M, sm_count_of(dev)) &&
                        gemv_wide_applicable(qtype, N, K, M, w, x_bf16);
   if (wide_ok) {
@@ -296,7 +302,7 @@ extern "C" int32_t ggq_gemm_sharded(int32_t qtype, const void* w, int64_t N_loca
   cudaGetDevice(&dev);
   const int slice = gemv_wide_max_batch();
   const int first = M < slice ? M : slice;
-  if (!is_k_quant(qtype) || !gemv_wide_applicable(qtype, N_local, K, first, w, x_bf16))
+  if (!is_k_quant(qtype) || (K / ti->block_elems * ti->block_bytes) % 16 || !gemv_wide_applicable(qtype, N_local, K, first, w, x_bf16))
     return fail(GGQ_UNSUPPORTED, "ggq_gemm_sharded: only Q4_K / Q5_K / Q6_K weights with K a multiple of 256 and 16-byte aligned rows "
                 "publish batches to peers; use ggq_gemm plus an all-gather for qtype %d, K=%lld", qtype, (long long)K);
   const size_t need = gemv_wide_workspace_bytes(qtype, N_local, K, first, sm_count_of(dev));
@@ -431,7 +437,8 @@ extern "C" int32_t ggq_gemm(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const int sms = sm_count_of(dev);
   const bool ws_ok = workspace && (uintptr_t)workspace % 256 == 0;
   const int slice_m = M < wide_slice ? M : wide_slice;
-  const bool can_wide = ws_ok && gemv_wide_applicable(qtype, N, K, slice_m, w, x_bf16) &&
+  const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
+  const bool can_wide = ws_ok && (M <= wide_slice || !odd_rows) && gemv_wide_applicable(qtype, N, K, slice_m, w, x_bf16) &&
                         workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, slice_m, sms);
   const bool can_bf16w = ws_ok && gemm_bf16w_applicable(qtype, N, K, M) &&
                          workspace_bytes >= gemm_bf16w_workspace_bytes(qtype, N, K, M, sms);

@@ -134,6 +134,7 @@ struct Geo {
   int xstage_bytes;           // XR * (512 + kOffBytes)
   int off_x, total;
   int tma;                    // weight slots arrive as TMA boxes (one per warp and step) instead of cp.async copies
+  int row_skew;               // bytes by which consecutive rows differ modulo 16 (0: rows 16-byte aligned; else cp.async copies)
   int vec_store;              // 2-byte outputs whose 8-row runs are 16-byte aligned: stored as 16-byte vectors
 };
 
@@ -353,8 +354,10 @@ __device__ __forceinline__ void block_q5k(uint32_t blk0, uint32_t blk1, int g, i
 // Q6_K: sixteen groups of 16 weights, one MMA each; codes 0..63 = nibble | two bits of qh << 4, the -32 rides on the
 // offset MMAs (A = the int8 scales as sign-magnitude codes, B = three-term sums of x).  A 210-byte block is only
 // 2-byte aligned: MIS = 1 when the block sits at 2 (mod 4), then a word is two aligned loads and a byte permute.
+// MIS = 2: not known, each row has its own (rows that are not 16-byte aligned).
 template <int MIS>
 __device__ __forceinline__ uint32_t ldw(uint32_t a) {
+  if (MIS == 2) return __funnelshift_r(lds_u32(a & ~3u), lds_u32((a & ~3u) + 4), (a & 2u) << 3);
   if (MIS) return __byte_perm(lds_u32(a - 2), lds_u32(a + 2), 0x5432);
   return lds_u32(a);
 }
@@ -432,11 +435,12 @@ __device__ __forceinline__ void block_q6k(uint32_t blk0, uint32_t blk1, int g, i
 }
 
 template <class F, int NT>
-__device__ __forceinline__ void block_mul(uint32_t blk0, uint32_t blk1, int g, int t, uint32_t xs, float (&out)[NT][4]) {
+__device__ __forceinline__ void block_mul(uint32_t blk0, uint32_t blk1, int g, int t, uint32_t xs, float (&out)[NT][4], bool odd_rows) {
   if constexpr (F::kQt == QT_Q4_K) block_q4k<NT>(blk0, blk1, g, t, xs, out);
   else if constexpr (F::kQt == QT_Q5_K) block_q5k<NT>(blk0, blk1, g, t, xs, out);
   else {
-    if (blk0 & 2) block_q6k<NT, 1>(blk0, blk1, g, t, xs, out);
+    if (odd_rows) block_q6k<NT, 2>(blk0, blk1, g, t, xs, out);
+    else if (blk0 & 2) block_q6k<NT, 1>(blk0, blk1, g, t, xs, out);
     else block_q6k<NT, 0>(blk0, blk1, g, t, xs, out);
   }
 }
@@ -490,6 +494,15 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
         if (lane == 0)
           tma_box_load(my_ring + w_slot * geo.wslot_bytes, &w_map, ((w_k * F::kTs) & ~15) >> 2, row0, my_bars + 8 * w_slot,
                        (uint32_t)geo.wslot_bytes);
+      } else if (geo.row_skew != 0 && row0 < N) {
+        // rows at different offsets of their windows (a copied piece holds at least one byte of its row)
+        const uint32_t dst0 = my_ring + w_slot * geo.wslot_bytes + hl * F::kPitch + 16 * kl;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const uint8_t* p = w + (int64_t)min(row0 + 2 * i + hl, N - 1) * row_bytes + w_k * F::kTs;
+          const int skew = (int)((uintptr_t)p & 15);
+          if (16 * kl < skew + F::kTs) cp_async16(dst0 + i * (2 * F::kPitch), p - skew + 16 * kl);
+        }
       } else if (row0 < N) {
         const int boff = w_k * F::kTs;
         const int pieces = ((boff & 15) + F::kTs + 15) >> 4;
@@ -610,8 +623,13 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
     if (tma) { tma_box_wait(my_bars + 8 * slot, ring_round & 1, status, lane); __syncwarp(); }
     const int row0 = rb * kBlockRows + warp * 16;
     if (row0 < N) {
-      const uint32_t blk0 = my_ring + slot * geo.wslot_bytes + g * F::kPitch + ((k * F::kTs) & 15);
-      block_mul<F, NT>(blk0, blk0 + 8 * F::kPitch, g, t, x_ring + slot * geo.xstage_bytes, out);
+      const uint32_t base = my_ring + slot * geo.wslot_bytes + g * F::kPitch;
+      uint32_t skew0 = (k * F::kTs) & 15, skew1 = skew0;
+      if (geo.row_skew != 0) {
+        skew0 = (k * F::kTs + min(row0 + g, N - 1) * geo.row_skew) & 15;
+        skew1 = (k * F::kTs + min(row0 + g + 8, N - 1) * geo.row_skew) & 15;
+      }
+      block_mul<F, NT>(base + skew0, base + skew1 + 8 * F::kPitch, g, t, x_ring + slot * geo.xstage_bytes, out, geo.row_skew != 0);
     }
     if (++slot == depth) { slot = 0; ++ring_round; }
 
@@ -686,6 +704,7 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, Geo* geo) {
   g.SB = (int)(K / 256);
   g.RB = (int)((N + kBlockRows - 1) / kBlockRows);
   g.S = (int64_t)g.RB * g.SB;
+  g.row_skew = (int)((int64_t)g.SB * fi.ts % 16);
   g.wslot_bytes = 16 * fi.pitch;
   g.xstage_bytes = XR * (512 + fi.off_bytes);
   const int per_depth = kWarps * g.wslot_bytes + g.xstage_bytes;
@@ -752,7 +771,7 @@ bool gemv_wide_applicable(int qtype, int64_t N, int64_t K, int M, const void* w,
   wide::FormatInfo fi;
   if (!wide::format_of(qtype, &fi)) return false;
   if (M < 1 || M > wide::kMaxBatch || K <= 0 || K % 256 || N < 1 || N > (1ll << 24)) return false;
-  if ((K / 256 * fi.ts) % 16 || (uintptr_t)w % 16 || (uintptr_t)x % 16) return false;
+  if ((uintptr_t)w % 16 || (uintptr_t)x % 16) return false;
   if (N * (K / 256 * fi.ts) >= (1ll << 40)) return false;
   wide::Geo geo;
   return wide::plan(fi, N, K, M, &geo);
@@ -792,7 +811,7 @@ cudaError_t gemv_wide(int qtype, const uint8_t* w, int64_t N, int64_t K, const v
   const bool want_tma = !(tma_env && tma_env[0] == '0');
   CUtensorMap w_map;
   memset(&w_map, 0, sizeof(w_map));
-  geo.tma = want_tma && make_weight_map(&w_map, w, N, K / 256 * fi.ts, fi.pitch / 4) ? 1 : 0;
+  geo.tma = want_tma && geo.row_skew == 0 && make_weight_map(&w_map, w, N, K / 256 * fi.ts, fi.pitch / 4) ? 1 : 0;
   // 16-byte output stores: 2-byte outputs, and every run of 8 rows of a column starts on a 16-byte boundary
   bool vec = y_dtype == GGQ_BF16 || y_dtype == GGQ_F16;
   if (pp.world == 0) {

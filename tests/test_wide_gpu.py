@@ -161,3 +161,16 @@ def test_benchmark_shape_sampled_rows(qtype):
         got = kernels.fused_matmul(x, w, out_dtype=torch.float32)
         ref = O.c_matmul(O.bf16_bits(x.float().cpu().numpy()), rows, qtype)
         assert O.rel_l2(got[:, idx].cpu().numpy(), ref) <= 2e-5, (qtype.name, m)
+
+
+@pytest.mark.parametrize("n,k", [(5003, 11 * 256), (130, 3 * 256), (4100, 13 * 256)])
+def test_rows_that_are_not_16_byte_aligned(n, k):
+    """Q6_K with K no multiple of 2048: every row at its own offset of its copied window; same bar as above, and the refusal of
+    such rows where results go to peers stays."""
+    wb = synth.make_weight_bytes(n, k, QT.Q6_K, seed=n)
+    w = gj.QuantizedArray.from_bytes(wb, QT.Q6_K, shape=(n, k), device="cuda")
+    for m in (5, 8, 16, 17, 32):
+        xb = synth.make_x(m, k, seed=m)
+        x = torch.from_numpy(xb).cuda().to(torch.bfloat16)
+        got = kernels.fused_matmul(x, w, out_dtype=torch.float32).cpu().numpy()
+        assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb, QT.Q6_K)) <= 2e-5, (n, k, m)
