@@ -267,30 +267,48 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
 
   // ---- shared-memory tables (immutable inputs: may be read before the previous kernel has finished)
   tf::Tables tb{};
-  tb.grid = smem_base + geo.off_tab;
-  if constexpr (F::kTableBytes > 0) {
-    uint32_t* dst = reinterpret_cast<uint32_t*>(smem + geo.off_tab);
-    if constexpr (F::kQt == QT_IQ1_S || F::kQt == QT_IQ1_M) {
-      // int8 grid {-1, 0, 1} -> code bytes 8 * grid + 9
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(tab + TAB_IQ1);
-      for (int i = tid; i < F::kTableBytes / 4; i += kThreads) {
-        const uint32_t v = __ldg(src + i);
-        const uint32_t neg = (v >> 7) & 0x01010101u, pos = v & ~(v >> 7) & 0x01010101u;    // per byte: 0xFF / 0x01
-        dst[i] = 0x09090909u - 8u * neg + 8u * pos;
+  if constexpr (F::kTableBytes > 0 && tf::KvOf<F>::value == 0) {
+    // kCopies interleaved copies of every entry; a thread writes 16-byte pieces (2 or 4 copies, which are the same)
+    constexpr int kEW = F::kEntryBytes / 4, kPieces = F::kEntryBytes * F::kCopies / 16;
+    constexpr int kOff = F::kQt == QT_IQ1_S || F::kQt == QT_IQ1_M ? TAB_IQ1 : F::kQt == QT_IQ2_XXS ? TAB_IQ2_XXS :
+                         F::kQt == QT_IQ2_XS ? TAB_IQ2_XS : F::kQt == QT_IQ2_S ? TAB_IQ2_S : F::kQt == QT_IQ3_XXS ? TAB_IQ3_XXS : TAB_IQ3_S;
+    tb.grid = smem_base + geo.off_tab + (lane % F::kCopies) * F::kEntryBytes;
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(tab + kOff);
+    uint4* dst = reinterpret_cast<uint4*>(smem + geo.off_tab);
+    for (int i = tid; i < F::kEntries * kPieces; i += kThreads) {
+      const int e = i / kPieces;
+      uint32_t v[2] = {__ldg(src + e * kEW), __ldg(src + e * kEW + (kEW - 1))};
+      if constexpr (F::kQt == QT_IQ1_S || F::kQt == QT_IQ1_M) {
+        // int8 grid {-1, 0, 1} -> code bytes 8 * grid + 9
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const uint32_t neg = (v[h] >> 7) & 0x01010101u, pos = v[h] & ~(v[h] >> 7) & 0x01010101u;    // per byte: 0xFF / 0x01
+          v[h] = 0x09090909u - 8u * neg + 8u * pos;
+        }
       }
-    } else {
-      constexpr int kOff = F::kQt == QT_IQ2_XXS ? TAB_IQ2_XXS : F::kQt == QT_IQ2_XS ? TAB_IQ2_XS :
-                           F::kQt == QT_IQ2_S ? TAB_IQ2_S : F::kQt == QT_IQ3_XXS ? TAB_IQ3_XXS : TAB_IQ3_S;
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(tab + kOff);
-      for (int i = tid; i < F::kTableBytes / 4; i += kThreads) dst[i] = __ldg(src + i);
+      dst[i] = make_uint4(v[0], v[1], v[0], v[1]);
+    }
+    if constexpr (F::kSignTable) {
+      constexpr int kGridBytes = F::kEntries * F::kEntryBytes * F::kCopies;
+      tb.sign = smem_base + geo.off_tab + kGridBytes + (lane % tf::kSignCopies) * 8;
+      uint4* sd = reinterpret_cast<uint4*>(smem + geo.off_tab + kGridBytes);
+      for (int i = tid; i < (1 << F::kSignBits) * (tf::kSignCopies / 2); i += kThreads) {
+        const uint32_t bits = tf::sign_bits_of(F::kSignBits, (uint32_t)i / (tf::kSignCopies / 2));
+        const uint32_t s0 = tf::spread_signs4(bits), s1 = tf::spread_signs4(bits >> 4);
+        sd[i] = make_uint4(s0, s1, s0, s1);
+      }
     }
   }
   if constexpr (tf::KvOf<F>::value != 0) {
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(tab + (tf::KvOf<F>::value == 1 ? TAB_KV_IQ4 : TAB_KV_MXFP4));
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t v = __ldg(src + i);
-      tb.kv[i] = tf::KvOf<F>::value == 1 ? v ^ 0x80808080u : __vadd4(v, 0x0C0C0C0Cu);     // int8 + 128 or + 12, per byte
+    // byte b -> (code of its low nibble, code of its high nibble), kByteTableCopies copies of each
+    constexpr int kBias = tf::KvOf<F>::value == 1 ? 128 : 12;
+    const int8_t* kv = reinterpret_cast<const int8_t*>(tab + (tf::KvOf<F>::value == 1 ? TAB_KV_IQ4 : TAB_KV_MXFP4));
+    tb.grid = smem_base + geo.off_tab + (lane % tf::kByteTableCopies) * 4;
+    uint4* dst = reinterpret_cast<uint4*>(smem + geo.off_tab);
+    for (int i = tid; i < 256 * (tf::kByteTableCopies / 4); i += kThreads) {
+      const int e = i / (tf::kByteTableCopies / 4);
+      const uint32_t v = (uint32_t)(__ldg(kv + (e & 15)) + kBias) | (uint32_t)(__ldg(kv + (e >> 4)) + kBias) << 16;
+      dst[i] = make_uint4(v, v, v, v);
     }
   }
   if (tid < 16) reinterpret_cast<uint32_t*>(smem + geo.off_zero)[tid] = 0;
@@ -463,11 +481,17 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
       }
       for (int blk = 0; blk < (q4k_fast ? 0 : nbh); blk++) {
         const tf::BlockLd ld0{tile + skew0 + blk * F::kTs}, ld1{tile + skew1 + blk * F::kTs + 8 * pitch};
-        const typename F::Run run0 = F::load_run(ld0, t), run1 = F::load_run(ld1, t);
+        constexpr bool kLean = MP == 4 && tf::SignBitsOf<F>::value != 0;
+        typename F::Run run0, run1;
+        if constexpr (!kLean) { run0 = F::load_run(ld0, t); run1 = F::load_run(ld1, t); }
         const uint32_t xr = xr0 + blk * x_blk;
         const uint32_t xsb = xs0 + blk * (4 * kGroups * 4);
         auto do_group = [&](int grp) {
-          const typename F::Group g0 = F::load_group(ld0, run0, t, grp), g1 = F::load_group(ld1, run1, t, grp);
+          auto load = [&](const tf::BlockLd& ld, const typename F::Run& run) -> typename F::Group {
+            if constexpr (kLean) return F::load_group_lean(ld, t, grp);
+            else return F::load_group(ld, run, t, grp);
+          };
+          const typename F::Group g0 = load(ld0, run0), g1 = load(ld1, run1);
           const uint32_t xg = xr + grp * (F::kGroupOct * x_oct);
           float acc[MP][4], acc2[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -475,8 +499,8 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
 #pragma unroll
           for (int q = 0; q < F::kGroupOct; q++) {
             uint32_t p0[4], p1[4];
-            F::octet(g0, q, tb, p0);
-            F::octet(g1, q, tb, p1);
+            if constexpr (kLean) { F::template octet<false>(g0, q, tb, p0); F::template octet<false>(g1, q, tb, p1); }
+            else { F::octet(g0, q, tb, p0); F::octet(g1, q, tb, p1); }
 #pragma unroll
             for (int p = 0; p < MP; p++) {
               const uint4 xv = tf::lds_v4(xg + q * x_oct + p * x_pass);
@@ -503,7 +527,7 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
             out[p][3] = F::fold(g1, acc[p][3], s1, out[p][3]);
           }
         };
-        if constexpr (F::kUnrollGroups) {
+        if constexpr (F::kUnrollGroups && !kLean) {
 #pragma unroll
           for (int grp = 0; grp < kGroups; grp++) do_group(grp);
         } else {

@@ -24,8 +24,8 @@
 //                       kSumOct octets (all of them, or the first plane of a two-plane format)
 //   kPairOrder          0: an octet is 8 consecutive weights e..e+7 entering as (e, e+2), (e+1, e+3),
 //                          (e+4, e+6), (e+5, e+7)    [byte pairs (0,2), (1,3) of two words]
-//                       1: an octet is two quads a..a+3, b..b+3 entering as (a, a+1), (b, b+1),
-//                          (a+2, a+3), (b+2, b+3)     [nibble pairs of one word]
+//                       1: an octet is two quads a..a+3, b..b+3 entering as (a, b), (a+1, b+1),
+//                          (a+2, b+2), (a+3, b+3)     [the two nibbles of each byte of a word]
 //   src_quads(t, oo)    first weight of the octet's two quads
 //   x_exp(t, oo)        exponent e <= 0: the octet's activations are staged times 2^e
 //   kAlign              alignment of every block when rows start 16-byte aligned: gcd(kTs, 16)
@@ -34,9 +34,12 @@
 //                       groups are loaded one at a time inside a real loop (keeps the loop body small)
 //   Run, load_run(ld, t)             what is read once per run and row
 //   Group, load_group(ld, run, t, grp)   the raw fields and the scale of group grp of the run
-//   kKv                 16-entry code book held in registers (Tables::kv): absent / 0 none, 1 IQ4 values + 128,
+//   kKv                 16-entry code book behind a table of its byte pairs: absent / 0 none, 1 IQ4 values + 128,
 //                       2 MXFP4 values + 12
 //   kScaleExp           the group scales carry 2^kScaleExp (taken back out of the row sums; 0 where the trait is absent)
+//   load_group_lean(ld, t, grp)   the group straight from the block, nothing kept for the run (absent: load_run only).  At
+//                       four passes the registers and, for the signs, the shared-memory pipe are what is short: there the
+//                       groups are loaded one at a time inside a real loop and octet<false> works the signs out
 //   octet(group, q, tab, p)   the four A-operand registers of octet q of the group: p[0], p[1] = first
 //                       MMA (k-slot pairs 2t.. and 2t+8..), p[2], p[3] = second MMA
 //   fold(group, acc, xsum, out) -> float   out + the group's contribution given acc = sum(code * x)
@@ -130,7 +133,7 @@ TF_HD uint32_t pair13(uint32_t w) { return prmt(w, 0u, 0x4341u); }
 TF_HD uint32_t pair02s(uint32_t w, uint32_t s) { return prmt(w, s, 0x6240u); }
 TF_HD uint32_t pair13s(uint32_t w, uint32_t s) { return prmt(w, s, 0x7351u); }
 // Four sign bits (bit j of `nib`, j = 0..3) spread to 0x80 in byte j.
-TF_HD uint32_t spread_signs4(uint32_t nib) { return ((nib & 15u) * 0x00204081u) << 7 & 0x80808080u; }
+TF_HD uint32_t spread_signs4(uint32_t nib) { return ((nib & 15u) * 0x10204080u) & 0x80808080u; }
 // ksigns[i] = i | parity(i) << 7 (gguf/quants.py IQ2_XXS.ksigns)
 TF_HD uint32_t ksigns(uint32_t i7) { return i7 | ((popc(i7) & 1u) << 7); }
 
@@ -152,6 +155,20 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t a) {
 struct BlockLd {
   uint32_t p;        // shared-window address of the block's first byte
   __device__ __forceinline__ uint32_t u16(int off) const { return lds_u16(p + off); }
+  // Sixteen bytes at an even address as two aligned 16-byte loads and a shift by their offset in the piece (selects, no
+  // branch): 8 shared-memory wavefronts per warp where the five word loads of words<4, 2> take 20 with the rows' banks
+  // four apart.
+  __device__ __forceinline__ void words16(int off, uint32_t (&out)[4]) const {
+    const uint32_t a = p + off, base = a & ~15u;
+    const uint4 x = lds_v4(base), y = lds_v4(base + 16);
+    const bool two = a & 8, one = a & 4;
+    const uint32_t v0 = two ? x.z : x.x, v1 = two ? x.w : x.y, v2 = two ? y.x : x.z, v3 = two ? y.y : x.w, v4 = two ? y.z : y.x,
+                   v5 = two ? y.w : y.y;
+    const uint32_t w0 = one ? v1 : v0, w1 = one ? v2 : v1, w2 = one ? v3 : v2, w3 = one ? v4 : v3, w4 = one ? v5 : v4;
+    const uint32_t sh = (a & 2u) << 3;
+    out[0] = __funnelshift_r(w0, w1, sh); out[1] = __funnelshift_r(w1, w2, sh);
+    out[2] = __funnelshift_r(w2, w3, sh); out[3] = __funnelshift_r(w3, w4, sh);
+  }
   template <int NW, int A>
   __device__ __forceinline__ void words(int off, uint32_t (&out)[NW]) const {
     const uint32_t a = p + off;
@@ -182,13 +199,14 @@ struct BlockLd {
 };
 // Per-CTA lookup tables in shared memory.
 struct Tables {
-  uint32_t grid;           // shared-window address of the format's grid: 8 (IQ1, IQ2) or 4 (IQ3) code bytes per entry
-  uint32_t kv[4];          // sixteen unsigned codes, four per register (formats with kKv)
+  uint32_t grid;           // shared-window address of this lane's copy of the format's grid: 8 (IQ1, IQ2) or 4 (IQ3) code bytes per entry
+  uint32_t sign;           // shared-window address of this lane's copy of the sign table (formats with kSignBits)
 };
 #else
 struct BlockLd {
   const uint8_t* p;
   uint32_t u16(int off) const { uint16_t v; memcpy(&v, p + off, 2); return v; }
+  void words16(int off, uint32_t (&out)[4]) const { memcpy(out, p + off, 16); }
   template <int NW, int A>
   void words(int off, uint32_t (&out)[NW]) const {
     for (int i = 0; i < NW; i++) memcpy(&out[i], p + off + 4 * i, 4);
@@ -203,20 +221,24 @@ struct NoRun {};
 // Optional members of a format.
 template <class F, class = void> struct KvOf { static constexpr int value = 0; };
 template <class F> struct KvOf<F, decltype((void)F::kKv)> { static constexpr int value = F::kKv; };
+template <class F, class = void> struct SignBitsOf { static constexpr int value = 0; };
+template <class F> struct SignBitsOf<F, decltype((void)F::kSignBits)> { static constexpr int value = F::kSignBits; };
 template <class F, class = void> struct ScaleExpOf { static constexpr int value = 0; };
 template <class F> struct ScaleExpOf<F, decltype((void)F::kScaleExp)> { static constexpr int value = F::kScaleExp; };
 
-// Sixteen-entry lookup of the four nibbles held in the low 16 bits of `sel`: result bytes in nibble
-// order (byte0.lo, byte0.hi, byte1.lo, byte1.hi).
-TF_HD uint32_t lookup4(const Tables& tb, uint32_t sel) {
-  const uint32_t s7 = sel & 0x7777u;
-  const uint32_t lo = prmt(tb.kv[0], tb.kv[1], s7), hi = prmt(tb.kv[2], tb.kv[3], s7);
-  return prmt(lo, hi, ((sel >> 1) & 0x4444u) | 0x3210u);
-}
-// An octet from one word of eight table nibbles (pair order 1: low nibbles a.., high nibbles b..).
+// An octet from one word of eight code-book nibbles (pair order 1).  A byte's two codes, one in each half of a word, are
+// already an A-operand register: on the device a table of the 256 bytes gives it with one load (32 interleaved
+// copies: a lane has its own bank), where four byte permutes, a blend and the widening of each code took seventeen
+// instructions of the half-rate integer pipe per octet.
+constexpr int kByteTableCopies = 32, kByteTableBytes = 256 * 4 * kByteTableCopies;
 TF_HD void lookup_octet(const Tables& tb, uint32_t w, uint32_t (&p)[4]) {
-  const uint32_t c0 = lookup4(tb, w), c1 = lookup4(tb, w >> 16);
-  p[0] = pair02(c0); p[1] = pair13(c0); p[2] = pair02(c1); p[3] = pair13(c1);
+#if TF_DEVICE
+#pragma unroll
+  for (int j = 0; j < 4; j++) p[j] = lds_u32(tb.grid + 4 * kByteTableCopies * ((w >> (8 * j)) & 0xFF));
+#else
+  const uint8_t* kv = reinterpret_cast<const uint8_t*>(tb.kv);
+  for (int j = 0; j < 4; j++) p[j] = kv[(w >> (8 * j)) & 15] | (uint32_t)kv[(w >> (8 * j + 4)) & 15] << 16;
+#endif
 }
 // An octet from one word of eight plain nibbles (pair order 0: the four low nibbles, then the four high ones).
 TF_HD void nibble_octet(uint32_t w, uint32_t (&p)[4]) {
@@ -416,15 +438,15 @@ struct Q6K {
 // =============================================================================================
 // IQ4_XS  (136 B: d, scales_h, 4 scales_l bytes, 128 nibble bytes)
 // sub-block j (32 weights): low nibbles of qs[16 j ..+16) are weights 0-15, high nibbles 16-31;
-// weight = d * (ls - 32) * kvalues[nibble].  Codes are kvalues + 128 (1..241), looked up with byte
-// permutes from four registers; the fold takes the 128 * sum(x) back out.
+// weight = d * (ls - 32) * kvalues[nibble].  Codes are kvalues + 128 (1..241), looked up two at a time in the
+// table of byte pairs; the fold takes the 128 * sum(x) back out.
 // run t = sub-blocks 2t, 2t+1 = groups 0, 1; octet q of a group = word q of the sub-block: its four
 // low nibbles (weights 4q..4q+3) and four high nibbles (16+4q..): MMA 1 takes the first two bytes
 // of the word, MMA 2 the last two (pair order 1).
 struct IQ4XS {
   static constexpr int kQt = 23, kTs = 136, kAlign = 8, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 1, kKv = 1;
   static constexpr bool kSums = true, kUnrollGroups = false;
-  static constexpr int kTableBytes = 0;
+  static constexpr int kTableBytes = kByteTableBytes;
   typedef NoRun Run;
   struct Group { uint32_t q[4]; float dl; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) {
@@ -452,23 +474,46 @@ struct IQ4XS {
 // =============================================================================================
 // Grid formats.  Common shape: an octet is one 8-byte grid entry (IQ2, IQ1) or two 4-byte entries
 // (IQ3) of unsigned code bytes, times eight sign bits.
-template <int ENTRY_BYTES>
+// The grid is held kCopies times, entry by entry interleaved, and a lane reads copy lane % kCopies: with 16 copies of
+// 8-byte entries (32 of 4-byte ones) every lane of a half-warp (warp) has its own banks and a look-up takes the two (one)
+// wavefronts it must; random entries of a single copy collided 3 ways on average, and the shared-memory pipe was what
+// these formats waited for.  Fewer copies where 64 KB would not hold them.
+template <int ENTRY_BYTES, int COPIES>
 TF_HD void grid_words(const Tables& tb, uint32_t i0, uint32_t i1, uint32_t& w0, uint32_t& w1) {
 #if TF_DEVICE
   if (ENTRY_BYTES == 8) {
-    const uint2 v = lds_v2(tb.grid + 8 * i0);
+    const uint2 v = lds_v2(tb.grid + 8 * COPIES * i0);
     w0 = v.x; w1 = v.y;
   } else {
-    w0 = lds_u32(tb.grid + 4 * i0);
-    w1 = lds_u32(tb.grid + 4 * i1);
+    w0 = lds_u32(tb.grid + 4 * COPIES * i0);
+    w1 = lds_u32(tb.grid + 4 * COPIES * i1);
   }
 #else
   if (ENTRY_BYTES == 8) { memcpy(&w0, tb.grid + 8 * i0, 4); memcpy(&w1, tb.grid + 8 * i0 + 4, 4); }
   else { memcpy(&w0, tb.grid + 4 * i0, 4); memcpy(&w1, tb.grid + 4 * i1, 4); }
 #endif
 }
-TF_HD void signed_octet(uint32_t w0, uint32_t w1, uint32_t signs8, uint32_t (&p)[4]) {
-  const uint32_t s0 = spread_signs4(signs8), s1 = spread_signs4(signs8 >> 4);
+// Sign bytes (0x80: negative) of an octet.  On the device they come from a table of 128 (seven-bit indices with a parity
+// bit) or 256 (plain bits) 8-byte entries, kept in interleaved copies like the grid: a shift, a mask and a load
+// where the parity, its merge and the spreading of eight bits took a dozen instructions of the half-rate integer pipe.
+// IQ2_S, whose grid has room for eight copies only, is faster without (8192 x 28672 at 1 / 4 rows 50.6 / 61.1 us, with 52.3 / 67.1).
+constexpr int kSignCopies = 16;
+TF_HD constexpr int sign_table_bytes(int bits) { return bits ? (1 << bits) * 8 * kSignCopies : 0; }
+TF_HD uint32_t sign_bits_of(int bits, uint32_t i) { return bits == 7 ? ksigns(i) : i; }
+template <int BITS, bool TABLE>
+TF_HD void sign_words(const Tables& tb, uint32_t i, uint32_t& s0, uint32_t& s1) {
+#if TF_DEVICE
+  if (TABLE) {
+    const uint2 v = lds_v2(tb.sign + 8 * kSignCopies * i);
+    s0 = v.x; s1 = v.y;
+    return;
+  }
+#endif
+  (void)tb;
+  const uint32_t b = sign_bits_of(BITS, i);
+  s0 = spread_signs4(b); s1 = spread_signs4(b >> 4);
+}
+TF_HD void signed_octet(uint32_t w0, uint32_t w1, uint32_t s0, uint32_t s1, uint32_t (&p)[4]) {
   p[0] = pair02s(w0, s0); p[1] = pair13s(w0, s0); p[2] = pair02s(w1, s1); p[3] = pair13s(w1, s1);
 }
 TF_HD void plain_octet(uint32_t w0, uint32_t w1, uint32_t (&p)[4]) {
@@ -478,23 +523,34 @@ TF_HD void plain_octet(uint32_t w0, uint32_t w1, uint32_t (&p)[4]) {
 // IQ2_XXS (66 B: d, 8 x {4 index bytes, u32 = 4 x 7-bit sign index | 4-bit scale << 28}); group = one of them
 struct IQ2XXS {
   static constexpr int kQt = 16, kTs = 66, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kSums = false, kUnrollGroups = false;
-  static constexpr int kTableBytes = 256 * 8;
-  typedef NoRun Run;
-  struct Group { uint32_t q[2]; float db; };
+  static constexpr bool kSums = false, kUnrollGroups = true;
+  static constexpr int kEntries = 256, kEntryBytes = 8, kCopies = 16, kSignBits = 7;
+  static constexpr bool kSignTable = true;
+  static constexpr int kTableBytes = kEntries * kEntryBytes * kCopies + sign_table_bytes(kSignTable ? kSignBits : 0);
+  struct Run { uint32_t q[4]; float d4; };
+  struct Group { uint32_t q, aux; float db; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
   TF_HD static int x_exp(int, int) { return 0; }
-  TF_HD static Run load_run(const BlockLd&, int) { return Run{}; }
-  TF_HD static Group load_group(const BlockLd& ld, const Run&, int t, int grp) {
-    Group g;
-    ld.words<2, 2>(2 + 16 * t + 8 * grp, g.q);
-    g.db = mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.5f + u2f(g.q[1] >> 28)), 0.25f);
-    return g;
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    ld.words16(2 + 16 * t, r.q);
+    r.d4 = mulf(f16_bits_to_float(ld.u16(0)), 0.25f);
+    return r;
   }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    return Group{r.q[2 * grp], r.q[2 * grp + 1], mulf(r.d4, 0.5f + u2f(r.q[2 * grp + 1] >> 28))};
+  }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    uint32_t q[2];
+    ld.words<2, 2>(2 + 16 * t + 8 * grp, q);
+    return Group{q[0], q[1], mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(q[1] >> 28))};
+  }
+  template <bool SIGN_TABLE = true>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
-    uint32_t w0, w1;
-    grid_words<8>(tb, (g.q[0] >> (8 * q)) & 0xFF, 0, w0, w1);
-    signed_octet(w0, w1, ksigns((g.q[1] >> (7 * q)) & 127), p);
+    uint32_t w0, w1, s0, s1;
+    grid_words<8, kCopies>(tb, (g.q >> (8 * q)) & 0xFF, 0, w0, w1);
+    sign_words<kSignBits, SIGN_TABLE>(tb, (g.aux >> (7 * q)) & 127, s0, s1);
+    signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
 };
@@ -502,25 +558,35 @@ struct IQ2XXS {
 // IQ2_XS (74 B: d, 32 x u16 = 9-bit grid index | 7-bit sign index << 9, 8 scale bytes of two nibbles)
 struct IQ2XS {
   static constexpr int kQt = 17, kTs = 74, kAlign = 2, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
-  static constexpr bool kSums = false, kUnrollGroups = false;
-  static constexpr int kTableBytes = 512 * 8;
-  typedef NoRun Run;
+  static constexpr bool kSums = false, kUnrollGroups = true;
+  static constexpr int kEntries = 512, kEntryBytes = 8, kCopies = 16, kSignBits = 7;
+  static constexpr bool kSignTable = true;
+  static constexpr int kTableBytes = kEntries * kEntryBytes * kCopies + sign_table_bytes(kSignTable ? kSignBits : 0);
+  struct Run { uint32_t q[4], sc; float d4; };
   struct Group { uint32_t q; float db; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
   TF_HD static int x_exp(int, int) { return 0; }
-  TF_HD static Run load_run(const BlockLd&, int) { return Run{}; }
-  TF_HD static Group load_group(const BlockLd& ld, const Run&, int t, int grp) {
-    Group g;
-    g.q = ld.u16(2 + 16 * t + 4 * grp) | (ld.u16(4 + 16 * t + 4 * grp) << 16);
-    const uint32_t sc = (ld.u16(66 + 2 * t) >> (4 * grp)) & 15;
-    g.db = mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.5f + u2f(sc)), 0.25f);
-    return g;
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    ld.words16(2 + 16 * t, r.q);
+    r.sc = ld.u16(66 + 2 * t);
+    r.d4 = mulf(f16_bits_to_float(ld.u16(0)), 0.25f);
+    return r;
   }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    return Group{r.q[grp], mulf(r.d4, 0.5f + u2f((r.sc >> (4 * grp)) & 15))};
+  }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    const uint32_t q = ld.u16(2 + 16 * t + 4 * grp) | (ld.u16(4 + 16 * t + 4 * grp) << 16);
+    const uint32_t sc = (ld.u16(66 + 2 * t) >> (4 * grp)) & 15;
+    return Group{q, mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(sc))};
+  }
+  template <bool SIGN_TABLE = true>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
-    const uint32_t q16 = (g.q >> (16 * q)) & 0xFFFF;
-    uint32_t w0, w1;
-    grid_words<8>(tb, q16 & 511, 0, w0, w1);
-    signed_octet(w0, w1, ksigns(q16 >> 9), p);
+    uint32_t w0, w1, s0, s1;
+    grid_words<8, kCopies>(tb, (g.q >> (16 * q)) & 511, 0, w0, w1);
+    sign_words<kSignBits, SIGN_TABLE>(tb, (g.q >> (16 * q + 9)) & 127, s0, s1);
+    signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
 };
@@ -528,27 +594,39 @@ struct IQ2XS {
 // IQ2_S (82 B: d, 32 index bytes, 32 sign bytes, 8 bytes of 2 high index bits, 8 scale bytes)
 struct IQ2S {
   static constexpr int kQt = 22, kTs = 82, kAlign = 2, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
-  static constexpr bool kSums = false, kUnrollGroups = false;
-  static constexpr int kTableBytes = 1024 * 8;
-  typedef NoRun Run;
+  static constexpr bool kSums = false, kUnrollGroups = true;
+  static constexpr int kEntries = 1024, kEntryBytes = 8, kCopies = 8, kSignBits = 8;
+  static constexpr bool kSignTable = false;
+  static constexpr int kTableBytes = kEntries * kEntryBytes * kCopies + sign_table_bytes(kSignTable ? kSignBits : 0);
+  struct Run { uint32_t qs[2], sg[2], qh, sc; float d4; };
   struct Group { uint32_t qs, sg, qh; float db; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
   TF_HD static int x_exp(int, int) { return 0; }
-  TF_HD static Run load_run(const BlockLd&, int) { return Run{}; }
-  TF_HD static Group load_group(const BlockLd& ld, const Run&, int t, int grp) {
-    Group g;
-    g.qs = ld.u16(2 + 8 * t + 2 * grp);
-    g.sg = ld.u16(34 + 8 * t + 2 * grp);
-    g.qh = ld.u16(66 + 2 * t) >> (4 * grp);
-    const uint32_t sc = (ld.u16(74 + 2 * t) >> (4 * grp)) & 15;
-    g.db = mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.5f + u2f(sc)), 0.25f);
-    return g;
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    ld.words<2, 2>(2 + 8 * t, r.qs);
+    ld.words<2, 2>(34 + 8 * t, r.sg);
+    r.qh = ld.u16(66 + 2 * t);
+    r.sc = ld.u16(74 + 2 * t);
+    r.d4 = mulf(f16_bits_to_float(ld.u16(0)), 0.25f);
+    return r;
   }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    const int sh = 16 * (grp & 1);
+    return Group{r.qs[grp >> 1] >> sh, r.sg[grp >> 1] >> sh, r.qh >> (4 * grp), mulf(r.d4, 0.5f + u2f((r.sc >> (4 * grp)) & 15))};
+  }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    const uint32_t sc = (ld.u16(74 + 2 * t) >> (4 * grp)) & 15;
+    return Group{ld.u16(2 + 8 * t + 2 * grp), ld.u16(34 + 8 * t + 2 * grp), ld.u16(66 + 2 * t) >> (4 * grp),
+                 mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(sc))};
+  }
+  template <bool SIGN_TABLE = true>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t idx = ((g.qs >> (8 * q)) & 0xFF) | (((g.qh >> (2 * q)) & 3) << 8);
-    uint32_t w0, w1;
-    grid_words<8>(tb, idx, 0, w0, w1);
-    signed_octet(w0, w1, (g.sg >> (8 * q)) & 0xFF, p);
+    uint32_t w0, w1, s0, s1;
+    grid_words<8, kCopies>(tb, idx, 0, w0, w1);
+    sign_words<kSignBits, SIGN_TABLE>(tb, (g.sg >> (8 * q)) & 0xFF, s0, s1);
+    signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
 };
@@ -556,27 +634,37 @@ struct IQ2S {
 // IQ3_XXS (98 B: d, 64 index bytes (one per 4 weights), 8 x u32 = 4 x 7-bit sign index | scale << 28)
 struct IQ3XXS {
   static constexpr int kQt = 18, kTs = 98, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kSums = false, kUnrollGroups = false;
-  static constexpr int kTableBytes = 256 * 4;
-  typedef NoRun Run;
+  static constexpr bool kSums = false, kUnrollGroups = true;
+  static constexpr int kEntries = 256, kEntryBytes = 4, kCopies = 32, kSignBits = 7;
+  static constexpr bool kSignTable = true;
+  static constexpr int kTableBytes = kEntries * kEntryBytes * kCopies + sign_table_bytes(kSignTable ? kSignBits : 0);
+  struct Run { uint32_t q[4], aux[2]; float d2; };
   struct Group { uint32_t q[2], aux; float db; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
   TF_HD static int x_exp(int, int) { return 0; }
-  TF_HD static Run load_run(const BlockLd&, int) { return Run{}; }
-  TF_HD static Group load_group(const BlockLd& ld, const Run&, int t, int grp) {
-    Group g;
-    ld.words<2, 2>(2 + 16 * t + 8 * grp, g.q);
-    uint32_t a[1];
-    ld.words<1, 2>(66 + 8 * t + 4 * grp, a);
-    g.aux = a[0];
-    g.db = mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.5f + u2f(g.aux >> 28)), 0.5f);
-    return g;
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    ld.words16(2 + 16 * t, r.q);
+    ld.words<2, 2>(66 + 8 * t, r.aux);
+    r.d2 = mulf(f16_bits_to_float(ld.u16(0)), 0.5f);
+    return r;
   }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    return Group{{r.q[2 * grp], r.q[2 * grp + 1]}, r.aux[grp], mulf(r.d2, 0.5f + u2f(r.aux[grp] >> 28))};
+  }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    uint32_t q[2], aux[1];
+    ld.words<2, 2>(2 + 16 * t + 8 * grp, q);
+    ld.words<1, 2>(66 + 8 * t + 4 * grp, aux);
+    return Group{{q[0], q[1]}, aux[0], mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.5f), 0.5f + u2f(aux[0] >> 28))};
+  }
+  template <bool SIGN_TABLE = true>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
-    const uint32_t q16 = (g.q[q >> 1] >> (16 * (q & 1))) & 0xFFFF;
-    uint32_t w0, w1;
-    grid_words<4>(tb, q16 & 0xFF, q16 >> 8, w0, w1);
-    signed_octet(w0, w1, ksigns((g.aux >> (7 * q)) & 127), p);
+    const uint32_t q16 = g.q[q >> 1] >> (16 * (q & 1));
+    uint32_t w0, w1, s0, s1;
+    grid_words<4, kCopies>(tb, q16 & 0xFF, (q16 >> 8) & 0xFF, w0, w1);
+    sign_words<kSignBits, SIGN_TABLE>(tb, (g.aux >> (7 * q)) & 127, s0, s1);
+    signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
 };
@@ -584,31 +672,42 @@ struct IQ3XXS {
 // IQ3_S (110 B: d, 64 index bytes, 8 bytes of ninth index bits, 32 sign bytes, 4 scale bytes of two nibbles)
 struct IQ3S {
   static constexpr int kQt = 21, kTs = 110, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kSums = false, kUnrollGroups = false;
-  static constexpr int kTableBytes = 512 * 4;
-  typedef NoRun Run;
+  static constexpr bool kSums = false, kUnrollGroups = true;
+  static constexpr int kEntries = 512, kEntryBytes = 4, kCopies = 16, kSignBits = 8;
+  static constexpr bool kSignTable = true;
+  static constexpr int kTableBytes = kEntries * kEntryBytes * kCopies + sign_table_bytes(kSignTable ? kSignBits : 0);
+  struct Run { uint32_t q[4], sg[2], qh, sc; float d; };
   struct Group { uint32_t q[2], sg, qh; float db; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
   TF_HD static int x_exp(int, int) { return 0; }
-  TF_HD static Run load_run(const BlockLd&, int) { return Run{}; }
-  TF_HD static Group load_group(const BlockLd& ld, const Run&, int t, int grp) {
-    Group g;
-    ld.words<2, 2>(2 + 16 * t + 8 * grp, g.q);
-    uint32_t s[1];
-    ld.words<1, 2>(74 + 8 * t + 4 * grp, s);
-    g.sg = s[0];
-    g.qh = ld.u16(66 + 2 * t) >> (8 * grp);
-    const uint32_t sc = (ld.u16(106 + (t & 2)) >> (8 * (t & 1) + 4 * grp)) & 15;
-    g.db = mulf(f16_bits_to_float(ld.u16(0)), u2f(1 + 2 * sc));
-    return g;
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    ld.words16(2 + 16 * t, r.q);
+    ld.words<2, 2>(74 + 8 * t, r.sg);
+    r.qh = ld.u16(66 + 2 * t);
+    r.sc = ld.u16(106 + (t & 2)) >> (8 * (t & 1));
+    r.d = f16_bits_to_float(ld.u16(0));
+    return r;
   }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    return Group{{r.q[2 * grp], r.q[2 * grp + 1]}, r.sg[grp], r.qh >> (8 * grp), mulf(r.d, u2f(1 + 2 * ((r.sc >> (4 * grp)) & 15)))};
+  }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    uint32_t q[2], sg[1];
+    ld.words<2, 2>(2 + 16 * t + 8 * grp, q);
+    ld.words<1, 2>(74 + 8 * t + 4 * grp, sg);
+    const uint32_t sc = (ld.u16(106 + (t & 2)) >> (8 * (t & 1) + 4 * grp)) & 15;
+    return Group{{q[0], q[1]}, sg[0], ld.u16(66 + 2 * t) >> (8 * grp), mulf(f16_bits_to_float(ld.u16(0)), u2f(1 + 2 * sc))};
+  }
+  template <bool SIGN_TABLE = true>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
-    const uint32_t q16 = (g.q[q >> 1] >> (16 * (q & 1))) & 0xFFFF;
+    const uint32_t q16 = g.q[q >> 1] >> (16 * (q & 1));
     const uint32_t i0 = (q16 & 0xFF) | (((g.qh >> (2 * q)) & 1) << 8);
-    const uint32_t i1 = (q16 >> 8) | (((g.qh >> (2 * q + 1)) & 1) << 8);
-    uint32_t w0, w1;
-    grid_words<4>(tb, i0, i1, w0, w1);
-    signed_octet(w0, w1, (g.sg >> (8 * q)) & 0xFF, p);
+    const uint32_t i1 = ((q16 >> 8) & 0xFF) | (((g.qh >> (2 * q + 1)) & 1) << 8);
+    uint32_t w0, w1, s0, s1;
+    grid_words<4, kCopies>(tb, i0, i1, w0, w1);
+    sign_words<kSignBits, SIGN_TABLE>(tb, (g.sg >> (8 * q)) & 0xFF, s0, s1);
+    signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
 };
@@ -619,25 +718,33 @@ struct IQ3S {
 // fold removes the 9 and the factor 8:  (dl / 8) * (sum(code x) - 9 sum(x)).
 struct IQ1S {
   static constexpr int kQt = 19, kTs = 50, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kSums = true, kUnrollGroups = false;
-  static constexpr int kTableBytes = 2048 * 8;
-  typedef NoRun Run;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kEntries = 2048, kEntryBytes = 8, kCopies = 4, kSignBits = 0;
+  static constexpr bool kSignTable = false;
+  static constexpr int kTableBytes = kEntries * kEntryBytes * kCopies + sign_table_bytes(kSignTable ? kSignBits : 0);
+  struct Run { uint32_t qs[2], qh[1]; float d8; };
   struct Group { uint32_t qs, qh, dlt; float dl8; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
   TF_HD static int x_exp(int, int) { return 0; }
-  TF_HD static Run load_run(const BlockLd&, int) { return Run{}; }
-  TF_HD static Group load_group(const BlockLd& ld, const Run&, int t, int grp) {
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
+    ld.words<2, 2>(2 + 8 * t, r.qs);
+    ld.words<1, 2>(34 + 4 * t, r.qh);
+    r.d8 = mulf(f16_bits_to_float(ld.u16(0)), 0.125f);
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
     Group g;
-    g.qs = ld.u16(2 + 8 * t + 4 * grp) | (ld.u16(4 + 8 * t + 4 * grp) << 16);
-    g.qh = ld.u16(34 + 4 * t + 2 * grp);
+    g.qs = r.qs[grp];
+    g.qh = r.qh[0] >> (16 * grp);
     g.dlt = (g.qh & 0x8000) ? 0xFEFEFEFFu : 0x01010101u;      // -1 / +1 in every byte
-    g.dl8 = mulf(mulf(f16_bits_to_float(ld.u16(0)), u2f(2 * ((g.qh >> 12) & 7) + 1)), 0.125f);
+    g.dl8 = mulf(r.d8, u2f(2 * ((g.qh >> 12) & 7) + 1));
     return g;
   }
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t idx = ((g.qs >> (8 * q)) & 0xFF) | (((g.qh >> (3 * q)) & 7) << 8);
     uint32_t w0, w1;
-    grid_words<8>(tb, idx, 0, w0, w1);
+    grid_words<8, kCopies>(tb, idx, 0, w0, w1);
     plain_octet(w0 + g.dlt, w1 + g.dlt, p);
   }
   TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
@@ -649,29 +756,33 @@ struct IQ1S {
 // a nibble of the f16 super-scale << 12)
 struct IQ1M {
   static constexpr int kQt = 29, kTs = 56, kAlign = 8, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
-  static constexpr bool kSums = true, kUnrollGroups = false;
-  static constexpr int kTableBytes = 2048 * 8;
-  typedef NoRun Run;
+  static constexpr bool kSums = true, kUnrollGroups = true;
+  static constexpr int kEntries = 2048, kEntryBytes = 8, kCopies = 4, kSignBits = 0;
+  static constexpr bool kSignTable = false;
+  static constexpr int kTableBytes = kEntries * kEntryBytes * kCopies + sign_table_bytes(kSignTable ? kSignBits : 0);
+  struct Run { uint32_t qs[2], qh[1], w; float d8; };
   struct Group { uint32_t qs, qh; float dl8; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 8 * oo; b = a + 4; }
   TF_HD static int x_exp(int, int) { return 0; }
-  TF_HD static Run load_run(const BlockLd&, int) { return Run{}; }
-  TF_HD static Group load_group(const BlockLd& ld, const Run&, int t, int grp) {
-    Group g;
-    g.qs = ld.u16(8 * t + 2 * grp);
-    g.qh = (ld.u16(32 + 4 * t + (grp & 2)) >> (8 * (grp & 1))) & 0xFF;
+  TF_HD static Run load_run(const BlockLd& ld, int t) {
+    Run r;
     uint32_t sc[2];
+    ld.words<2, 8>(8 * t, r.qs);
+    ld.words<1, 4>(32 + 4 * t, r.qh);
     ld.words<2, 8>(48, sc);
     const uint32_t dbits = ((sc[0] >> 12) & 0x000F) | ((sc[0] >> 24) & 0x00F0) | ((sc[1] >> 4) & 0x0F00) | ((sc[1] >> 16) & 0xF000);
-    const uint32_t w = (sc[t >> 1] >> (16 * (t & 1))) & 0xFFFF;
-    g.dl8 = mulf(mulf(f16_bits_to_float(dbits), u2f(2 * ((w >> (3 * grp)) & 7) + 1)), 0.125f);
-    return g;
+    r.w = ((t & 2) ? sc[1] : sc[0]) >> (16 * (t & 1));
+    r.d8 = mulf(f16_bits_to_float(dbits), 0.125f);
+    return r;
+  }
+  TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
+    return Group{r.qs[grp >> 1] >> (16 * (grp & 1)), r.qh[0] >> (8 * grp), mulf(r.d8, u2f(2 * ((r.w >> (3 * grp)) & 7) + 1))};
   }
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t n = (g.qh >> (4 * q)) & 15;
     const uint32_t idx = ((g.qs >> (8 * q)) & 0xFF) | ((n & 7) << 8);
     uint32_t w0, w1;
-    grid_words<8>(tb, idx, 0, w0, w1);
+    grid_words<8, kCopies>(tb, idx, 0, w0, w1);
     const uint32_t dlt = (n & 8) ? 0xFEFEFEFFu : 0x01010101u;
     plain_octet(w0 + dlt, w1 + dlt, p);
   }
@@ -846,7 +957,7 @@ struct Q40 {
 
 // IQ4_NL (18 B, laid out as Q4_0): nibbles select one of sixteen values, codes value + 128
 struct IQ4NL : Q40 {
-  static constexpr int kQt = 20, kPairOrder = 1, kKv = 1;
+  static constexpr int kQt = 20, kPairOrder = 1, kKv = 1, kTableBytes = kByteTableBytes;
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) { lookup_octet(tb, g.q[q], p); }
   TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
     return fmaf_(g.d, fmaf_(-128.0f, xsum, acc), out);
@@ -922,7 +1033,7 @@ struct Q51 {
 struct MXFP4 {
   static constexpr int kQt = 39, kTs = 136, kAlign = 8, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 1, kKv = 2, kScaleExp = 37;
   static constexpr bool kSums = true, kUnrollGroups = true;
-  static constexpr int kTableBytes = 0;
+  static constexpr int kTableBytes = kByteTableBytes;
   struct Run { uint32_t q[8]; float d[2]; };
   struct Group { const uint32_t* q; float d; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
@@ -960,7 +1071,7 @@ struct MXFP4 {
 struct NVFP4 {
   static constexpr int kQt = 40, kTs = 144, kAlign = 16, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 1, kKv = 2;
   static constexpr bool kSums = true, kUnrollGroups = true;
-  static constexpr int kTableBytes = 0;
+  static constexpr int kTableBytes = kByteTableBytes;
   struct Run { uint32_t w[9]; };
   struct Group { const uint32_t* q; float d; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 16 * (oo >> 1) + 4 * (oo & 1); b = a + 8; }

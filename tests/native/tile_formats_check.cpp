@@ -51,6 +51,18 @@ int check(const std::vector<uint8_t>& blocks, const float* want, const Tables& t
       const typename F::Run run = F::load_run(ld, t);
       for (int grp = 0; grp < F::kOct / F::kGroupOct; grp++) {
         const typename F::Group raw = F::load_group(ld, run, t, grp);
+        if constexpr (SignBitsOf<F>::value != 0) {       // the lean loader must give the same group
+          const typename F::Group lean = F::load_group_lean(ld, t, grp);
+          for (int q = 0; q < F::kGroupOct; q++) {
+            uint32_t pa[4], pb[4];
+            F::octet(raw, q, tb, pa);
+            F::template octet<false>(lean, q, tb, pb);
+            if (memcmp(pa, pb, sizeof(pa)) || F::fold(raw, 3.0f, 1.0f, 0.5f) != F::fold(lean, 3.0f, 1.0f, 0.5f)) {
+              fprintf(stderr, "block %d run %d group %d: the lean loader differs\n", b, t, grp);
+              return 1;
+            }
+          }
+        }
         // one-hot activations, one weight at a time: the group's accumulator receives code * x from every
         // octet the weight appears in (one, or one per plane), the sum of x is 1
         std::vector<double> acc(256, 0.0);
@@ -66,7 +78,7 @@ int check(const std::vector<uint8_t>& blocks, const float* want, const Tables& t
               const uint32_t reg = pr[2 * m + h];
               int e0, e1;
               if (F::kPairOrder == 0) { e0 = (m ? qb : qa) + h; e1 = e0 + 2; }
-              else { e0 = (h ? qb : qa) + 2 * m; e1 = e0 + 1; }
+              else { e0 = qa + 2 * m + h; e1 = qb + 2 * m + h; }
               acc[e0] += code_of(reg & 0xFFFF) * xs;
               acc[e1] += code_of(reg >> 16) * xs;
               in_group[e0]++; in_group[e1]++;
