@@ -74,14 +74,17 @@ def staging(device_index: int, nbytes: int, stream: int | None = None) -> torch.
     return buf
 
 
-def workspace(device_index: int, nbytes: int, stream: int | None = None) -> torch.Tensor | None:
+def workspace(device_index: int, nbytes: int, stream: int | None = None, least: int | None = None) -> torch.Tensor | None:
     """Zero-filled scratch for the fused kernels, one per (device, stream), grown on demand.
     The kernels leave it zeroed, so it is cleared only when (re)allocated.  ``stream``: the current stream's
-    handle if the caller already has it."""
-    if nbytes == 0:
-        return None
+    handle if the caller already has it.  ``least``: what the call cannot do without; a capturing stream gets no more than
+    that newly allocated (its zero fill would only happen on replay)."""
     key = (device_index, stream_ptr(device_index) if stream is None else stream)
     ws = _workspaces.get(key)
+    if least is not None and least < nbytes and (ws is None or ws.numel() < nbytes) and torch.cuda.is_current_stream_capturing():
+        nbytes = least
+    if nbytes == 0:
+        return None
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", device_index))
         _workspaces[key] = ws

@@ -110,7 +110,8 @@ def native():
                 spec = importlib.util.spec_from_file_location("_native", NATIVE_PATH)
                 module = importlib.util.module_from_spec(spec)
                 spec.loader.exec_module(module)
-                entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_fused_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info)
+                entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_fused_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info,
+                           L.ggq_dequant)
                 module.bind(*[ctypes.cast(f, ctypes.c_void_p).value for f in entries], int(L.ggq_gemv_max_batch()))
                 _native_module = module
     return _native_module

@@ -3,8 +3,10 @@
 //
 // A decode step is a chain of products of 4 to 40 us, so the host's time per call is what such a step takes once it is
 // above the kernels': measured on B200, seven products of a 1B-shaped layer took 122 us through the Python path (17 us a
-// call) for 37 us of kernels; through here they take 51 us (7 us a call).  `fast_matmul` returns None for every call that is not the common one, and the Python path,
-// which stays the reference for behaviour and errors, takes it.
+// call) for 37 us of kernels; through here they take 51 us (7 us a call).  `fast_matmul` returns None for every call that
+// is not the common one, and the Python path, which stays the reference for behaviour and errors, takes it.
+//
+// The dense route (decode, library GEMM) is two launches for which the Python path spent 50 us; here 15 to 20.
 //
 // The library's entry points are handed over as addresses (bind), so that this module follows whichever
 // libggq_b200.so the binding has loaded.  All state is guarded by the interpreter lock.
@@ -30,6 +32,7 @@ using LaunchFn = int32_t (*)(int32_t, const void*, int64_t, int64_t, const void*
 using LimitFn = int32_t (*)(int32_t, int64_t, int64_t);
 using BytesFn = size_t (*)(int32_t, int64_t, int64_t, int32_t);
 using CodeFn = int32_t (*)(int32_t);
+using DequantFn = int32_t (*)(int32_t, const void*, int64_t, void*, int32_t, void*);
 using InfoFn = int32_t (*)(int32_t, int32_t*, int32_t*);
 
 LaunchFn g_gemv = nullptr, g_gemm = nullptr;
@@ -37,6 +40,7 @@ LimitFn g_limit = nullptr;
 BytesFn g_bytes = nullptr;
 CodeFn g_fused = nullptr;
 InfoFn g_info = nullptr;
+DequantFn g_dequant = nullptr;
 int g_gemv_max = 0;
 constexpr int kBf16 = 1;                 // GGQ_BF16
 
@@ -49,6 +53,7 @@ struct Shape {
   int32_t qtype = -1, m = -1;
   int32_t limit = 0;
   size_t scratch = 0, payload = 0;
+  int64_t blocks = 0;
 };
 std::array<Shape, 1024> g_shapes;
 
@@ -58,15 +63,16 @@ const Shape* shape_of(int32_t qtype, int64_t n, int64_t k, int32_t m) {
   if (s.qtype != qtype || s.n != n || s.k != k || s.m != m) {
     int32_t elems = 0, bytes = 0;
     if (!g_fused(qtype) || g_info(qtype, &elems, &bytes) != 0 || k <= 0 || k % elems) return nullptr;
-    s = Shape{n, k, qtype, m, g_limit(qtype, n, k), g_bytes(qtype, n, k, m), (size_t)(n * (k / elems)) * (size_t)bytes};
+    s = Shape{n, k, qtype, m, g_limit(qtype, n, k), g_bytes(qtype, n, k, m), (size_t)(n * (k / elems)) * (size_t)bytes, n * (k / elems)};
   }
   return &s;
 }
 
-// fast_matmul(x, payload, qtype, shape, force_fused) -> Tensor or None (not the common case)
+// fast_matmul(x, payload, qtype, shape, force_fused, dense_budget) -> Tensor or None (not the common case)
+// dense_budget: bytes a dense copy may take at 4 bytes per weight, 0 where it would not be the built-in bf16 decode
 PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 5 || !g_gemv || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1]) || !PyTuple_CheckExact(args[3]) ||
+  if (nargs != 6 || !g_gemv || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1]) || !PyTuple_CheckExact(args[3]) ||
       PyTuple_GET_SIZE(args[3]) != 2)
     Py_RETURN_NONE;
   const at::Tensor& x = THPVariable_Unpack(args[0]);
@@ -86,14 +92,23 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t m = x.numel() / k;
   if (m < 1 || m > 65536) Py_RETURN_NONE;
   const Shape* s = shape_of((int32_t)qtype, n, k, (int32_t)m);
-  if (!s || (m > s->limit && args[4] != Py_True) || (size_t)w.numel() != s->payload) Py_RETURN_NONE;
+  if (!s || (size_t)w.numel() != s->payload) Py_RETURN_NONE;
   const auto stream = c10::cuda::getCurrentCUDAStream(dev);
+  c10::SmallVector<int64_t, 6> sizes(x.sizes().begin(), x.sizes().end());
+  sizes.back() = n;
+  if (m > s->limit && args[4] != Py_True) {
+    // the dense route in one piece: decode to bf16, library GEMM (rows of the result on 16-byte boundaries)
+    const double budget = PyFloat_AsDouble(args[5]);
+    if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+    if (n % 8 || 4.0 * (double)n * (double)k > budget) Py_RETURN_NONE;
+    const at::Tensor dense = at::empty({n, k}, x.options().requires_grad(false));
+    if (g_dequant((int32_t)qtype, w.data_ptr(), s->blocks, dense.data_ptr(), kBf16, stream.stream()) != 0) Py_RETURN_NONE;
+    return THPVariable_Wrap(at::mm(x.reshape({m, k}), dense.t()).view(sizes));
+  }
   const auto it = g_scratch.find({dev, (uintptr_t)stream.stream()});
   // no scratch yet on this stream (its first call also uploads the code books), or one that has to grow
   if (it == g_scratch.end() || (size_t)it->second.numel() < s->scratch) Py_RETURN_NONE;
   const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
-  c10::SmallVector<int64_t, 6> sizes(x.sizes().begin(), x.sizes().end());
-  sizes.back() = n;
   at::Tensor y = at::empty(sizes, x.options().requires_grad(false));
   const int32_t rc = (m <= g_gemv_max ? g_gemv : g_gemm)((int32_t)qtype, w.data_ptr(), n, k, xc.data_ptr(), (int32_t)m, y.data_ptr(), kBf16,
                                                          it->second.data_ptr(), (size_t)it->second.numel(), stream.stream());
@@ -102,17 +117,18 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(gemv, gemm, fused_batch_limit, scratch_bytes, has_fused, type_info, gemv_max_batch): entry point addresses
+// bind(gemv, gemm, fused_batch_limit, scratch_bytes, has_fused, type_info, dequant, gemv_max_batch): entry point addresses
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long gemv, gemm, limit, bytes, fused, info;
+  unsigned long long gemv, gemm, limit, bytes, fused, info, dequant;
   int max_batch;
-  if (!PyArg_ParseTuple(args, "KKKKKKi", &gemv, &gemm, &limit, &bytes, &fused, &info, &max_batch)) return nullptr;
+  if (!PyArg_ParseTuple(args, "KKKKKKKi", &gemv, &gemm, &limit, &bytes, &fused, &info, &dequant, &max_batch)) return nullptr;
   g_gemv = (LaunchFn)(uintptr_t)gemv;
   g_gemm = (LaunchFn)(uintptr_t)gemm;
   g_limit = (LimitFn)(uintptr_t)limit;
   g_bytes = (BytesFn)(uintptr_t)bytes;
   g_fused = (CodeFn)(uintptr_t)fused;
   g_info = (InfoFn)(uintptr_t)info;
+  g_dequant = (DequantFn)(uintptr_t)dequant;
   g_gemv_max = max_batch;
   Py_RETURN_NONE;
 }

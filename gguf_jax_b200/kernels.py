@@ -28,7 +28,7 @@ __all__ = [
 LOWBIT_TYPES = (QT.Q2_K, QT.IQ1_S, QT.IQ1_M, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT.IQ3_XXS, QT.IQ3_S)
 
 
-_ws_need: dict[tuple[int, int, int, int], int] = {}
+_ws_need: dict[tuple[int, int, int, int], tuple[int, int]] = {}      # scratch: for every kernel, for those that need one
 _cap: list[int] = []
 
 
@@ -119,8 +119,8 @@ def fused_matmul(x: torch.Tensor, w: QuantizedArray, *, out_dtype=torch.bfloat16
         key = (int(w.qtype), n_rows, k_dim, m)
         need = _ws_need.get(key)
         if need is None:
-            need = _ws_need[key] = L.ggq_scratch_bytes(*key)
-        ws = _backend.workspace(dev, need, stream)
+            need = _ws_need[key] = (L.ggq_scratch_bytes(*key), L.ggq_workspace_bytes(*key))
+        ws = _backend.workspace(dev, need[0], stream, need[1])
         _lib.check(fn(key[0], data.data_ptr(), n_rows, k_dim, x_ptr, m, y.data_ptr(),
                       _backend.dtype_code(out_dtype), ws.data_ptr() if ws is not None else None,
                       ws.numel() if ws is not None else 0, stream))

@@ -35,6 +35,9 @@ __all__ = [
 DequantFn = Callable[[torch.Tensor, Any], torch.Tensor]
 
 _DEQUANT: dict[GGMLQuantizationType, DequantFn] = {}
+_builtins: dict[GGMLQuantizationType, DequantFn] = {}
+# Types whose decoder is the caller's own: their dense weights are what that decoder says they are.
+_replaced: set[GGMLQuantizationType] = set()
 
 
 def register_dequant(qtype: GGMLQuantizationType, fn: DequantFn, *, override: bool = False) -> None:
@@ -47,6 +50,7 @@ def register_dequant(qtype: GGMLQuantizationType, fn: DequantFn, *, override: bo
     if qtype in _DEQUANT and not override:
         raise ValueError(f"dequant kernel for {qtype.name} already registered")
     _DEQUANT[qtype] = fn
+    (_replaced.discard if _builtins.get(qtype) is fn else _replaced.add)(qtype)
 
 
 def supported_types() -> list[GGMLQuantizationType]:
@@ -77,7 +81,8 @@ def _builtin(qtype: GGMLQuantizationType) -> DequantFn:
 # passthroughs it special-cases, as in the reference (tests/test_bitwise.py:104-110).
 for _qt in (*_ref._type_traits.keys(), GGMLQuantizationType.F16, GGMLQuantizationType.F32):
     if _qt not in _DEQUANT:
-        register_dequant(_qt, _builtin(_qt))
+        _builtins[_qt] = _builtin(_qt)
+        register_dequant(_qt, _builtins[_qt])
 
 
 def dequantize_blocks(blocks: torch.Tensor, qtype: GGMLQuantizationType, dtype=torch.float32) -> torch.Tensor:

@@ -5,13 +5,13 @@ import torch
 from gguf.constants import GGMLQuantizationType as QT
 
 import gguf_jax_b200 as gj
-from gguf_jax_b200 import _lib, kernels, synth
+from gguf_jax_b200 import _lib, kernels, quants, synth
 
 pytestmark = pytest.mark.gpu
 
 
-def native(x, w, force=False):
-    return _lib.native().fast_matmul(x, w.data, w.qtype, w.shape, force)
+def native(x, w, force=False, budget=1 << 29):
+    return _lib.native().fast_matmul(x, w.data, w.qtype, w.shape, force, budget)
 
 
 @pytest.fixture(scope="module")
@@ -56,7 +56,8 @@ def test_leaves_everything_else_to_the_python_path(weight):
     assert native(x.as_subclass(Sub), w) is None
     assert native(x, synth.make_weight(96, 2048, QT.Q4_K, seed=1, device="cuda").astype(torch.float32)) is not None   # fused: w.dtype plays no part
     big = torch.randn((64, 2048), device="cuda").bfloat16()
-    assert native(big, synth.make_weight(96, 2048, QT.Q8_0, seed=1, device="cuda")) is None         # above its limit: dense route
+    assert native(big, w, budget=0) is None and native(big, w, budget=4 * 96 * 2048 - 1) is None    # dense, but not in one piece here
+    assert native(big, synth.make_weight(97, 2048, QT.Q8_0, seed=1, device="cuda")) is None         # rows of the result not 16-byte aligned
     for bad in (object(), None, [x]):
         assert native(bad, w) is None
     with pytest.raises(ValueError):
@@ -66,6 +67,25 @@ def test_leaves_everything_else_to_the_python_path(weight):
     x2 = x.clone().requires_grad_(True)
     gj.matmul(x2, w).float().sum().backward()
     assert x2.grad is not None and x2.grad.shape == x2.shape
+
+
+def test_dense_route_in_one_piece():
+    for qtype in (QT.Q4_K, QT.Q8_0, QT.IQ3_S, QT.MXFP4):
+        w = synth.make_weight(96, 2048, qtype, seed=2, device="cuda")
+        x = torch.randn((2, 40, 2048), device="cuda").bfloat16()
+        want = gj.dequant_matmul(x, w)
+        got = native(x, w)
+        assert got.shape == (2, 40, 96) and got.is_contiguous()
+        assert torch.equal(got, want) and torch.equal(gj.matmul(x, w), want)
+        assert gj.matmul(x, w.astype(torch.float32)).dtype == torch.float32          # another dense dtype: the Python path
+    saved = quants._DEQUANT[QT.Q8_0]
+    try:
+        gj.register_dequant(QT.Q8_0, lambda b, d: torch.ones((b.shape[0], 32), dtype=d, device=b.device), override=True)
+        w = synth.make_weight(96, 2048, QT.Q8_0, seed=2, device="cuda")
+        assert torch.equal(gj.matmul(x, w), gj.dequant_matmul(x, w)) and not torch.equal(gj.matmul(x, w), native(x, w))
+    finally:
+        gj.register_dequant(QT.Q8_0, saved, override=True)
+    assert torch.equal(gj.matmul(x, w), native(x, w))
 
 
 def test_under_capture(weight):
@@ -82,3 +102,20 @@ def test_under_capture(weight):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+def test_first_call_of_a_stream_under_capture_takes_no_scratch_it_can_do_without():
+    w = synth.make_weight(14336, 2048, QT.Q8_0, seed=4, device="cuda")
+    x = torch.randn((2, 2048), device="cuda").bfloat16()
+    want = gj.matmul(x, w)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = gj.matmul(x, w)
+    graph.replay()
+    with torch.cuda.stream(stream):
+        z = gj.matmul(x, w)
+    torch.cuda.synchronize()
+    assert torch.equal(z, want)
+    assert ((y.double() - want.double()).norm() / want.double().norm()).item() <= 2 ** -8      # another kernel's summation order
