@@ -61,17 +61,19 @@ static bool tile_scratch_is_optional(int qtype) {
          qtype != QT_IQ3_XXS && qtype != QT_IQ3_S && qtype != QT_IQ1_S && qtype != QT_IQ1_M;
 }
 
-// Where the tiled kernel and the kernels it replaces (streaming at batch 1, one MMA launch for 2..16 rows) cross, for the
-// formats of tile_scratch_is_optional and for rows that are not 16-byte aligned.  The tiled kernel starts at 6 us (batch 1) to 13 us
-// (batch 8; a larger batch is two launches) and grows slowly; the others start at 5 and 10 to 20 us and grow with their
-// decoding.  Measured on B200, us, others / tiled: batch 1, 1024 x 4096 Q8_0 5.5 / 6.2, Q4_0 5.4 / 6.3, 14336 x 4096 25.8 /
-// 19.7, 31.2 / 15.4; batch 8, 1024 x 4096 Q8_0 10.1 / 12.9, Q4_0 17.1 / 12.9; batch 16, 14336 x 4096 Q8_0 54.8 / 58.3, TQ2_0 60.6 /
-// 52.9, Q4_0 92 / 53, IQ4_NL 104 / 67, 5003 x 2816 IQ2_XS 25.7 / 29.2, Q2_K 22.7 / 27.0.
+// Where the tiled kernel and the two it competes with (streaming at batch 1, one MMA launch for 2..16 rows) cross, for every format
+// but the K-quants with kernels of their own.  The tiled kernel starts at 7 us (batch 1, 2) to 12 us (batch 8; a larger batch
+// is two launches) and grows slowly with the weight; the others start at 4 and 7 us and grow with their decoding.  Measured on B200,
+// us, other / tiled, at 2 / 8 / 16 / 56 / 128 M weights (M = 2^20):
+//   batch 1    Q4_0 4.4/7.0 6.3/7.6 9.8/8.5 27/17 52/27     Q8_0 4.4/7.3 6.4/7.8 9.8/10.0 27/21 51/35    IQ2_XS 5.1/7.8 7.9/9.7 11.9/11.1 32/20
+//   batch 4    Q4_0 7.0/8.5 11.6/10.4 13.8/10.4 40/19       IQ3_S 7.8/9.8 13.4/11.6 17.3/12.7 49/26
+//   batch 8    Q4_0 7.0/11.7 11.2/14.5 13.8/14.5 40/28      IQ4_XS 6.3/13.8 11.2/18.4 15.2/17.2 44/32 107/58
+//   batch 16   Q4_0 7.0/22 11.1/27 15.3/27 47/55 106/102    IQ2_XS 7.6/25 12.4/34 15.8/30 46/64 140/115   Q3_K 8.3/24 14.5/29 19/34 56/77 224/130
 static bool tile_pays(int qtype, int64_t weights, int M) {
-  if (M == 1) return weights >= (8 << 20);
-  if (M <= 4) return true;
-  if (M <= 8) return qtype != QT_Q8_0 || weights >= (10 << 20);
-  return weights >= (qtype == QT_Q8_0 ? 80 << 20 : qtype == QT_TQ2_0 ? 32 << 20 : 16 << 20);
+  static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
+  if (always) return true;
+  const int64_t from = M == 1 ? (qtype == QT_Q8_0 ? 16 : 12) : M <= 4 ? 4 : M <= 8 ? 18 : 96;
+  return weights >= from << 20;
 }
 
 static size_t tile_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
@@ -156,7 +158,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   }
   static const bool m1_tiled = [] { const char* e = getenv("GGQ_Q4K_M1_TILED"); return e && e[0] == '1'; }();
   // Q4_K / Q5_K / Q6_K keep their batch-1 kernels; the tiled kernel takes their batches 2..4 (Q4_K 8192 x 28672:
-  // 36 / 49 us at batch 2 / 4) and every batch of the formats that have nothing better; from five batch rows on
+  // 36 / 49 us at batch 2 / 4) and the other formats where tile_pays says so; from five batch rows on
   // the batch-major kernel takes the larger weights (Q4_K 8192 x 28672: 68 / 77 us at batch 8 / 16 against
   // 100 / 153 us) and the integer-code MMA kernel (gemv_mma.cu) the smaller ones (see wide_pays).
   const bool k_quant = is_k_quant(qtype);
@@ -168,7 +170,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const bool small_batch = k_quant && M >= 2 && M <= 4 && weights < (6 << 20) && gemv_mma_applicable(ti, N, K, M);
   if (small_batch) tuned = nullptr;
   const bool tile_first = k_quant ? (M >= 2 && M <= 4 && !small_batch) || (M == 1 && (odd_rows ? tile_pays(qtype, weights, 1) : m1_tiled))
-                                  : (!odd_rows && !tile_scratch_is_optional(qtype)) || tile_pays(qtype, weights, M);
+                                  : tile_pays(qtype, weights, M);
   const int tile_max = gemv_tile_max_batch(qtype);
   const int tile_m = M < tile_max ? M : tile_max;
   const size_t tile_need = tile_max ? gemv_tile_workspace_bytes(qtype, N, K, tile_m) : 0;
