@@ -229,7 +229,7 @@ template <class F> struct ScaleExpOf<F, decltype((void)F::kScaleExp)> { static c
 // An octet from one word of eight code-book nibbles (pair order 1).  A byte's two codes, one in each half of a word, are
 // already an A-operand register: on the device a table of the 256 bytes gives it with one load (32 interleaved
 // copies: a lane has its own bank), where four byte permutes, a blend and the widening of each code took seventeen
-// instructions of the half-rate integer pipe per octet.
+// instructions of the half-rate integer pipe per octet (IQ4_XS 8192 x 28672 at batch 1: 59.8 -> 51.0 us).
 constexpr int kByteTableCopies = 32, kByteTableBytes = 256 * 4 * kByteTableCopies;
 TF_HD void lookup_octet(const Tables& tb, uint32_t w, uint32_t (&p)[4]) {
 #if TF_DEVICE
@@ -477,7 +477,8 @@ struct IQ4XS {
 // The grid is held kCopies times, entry by entry interleaved, and a lane reads copy lane % kCopies: with 16 copies of
 // 8-byte entries (32 of 4-byte ones) every lane of a half-warp (warp) has its own banks and a look-up takes the two (one)
 // wavefronts it must; random entries of a single copy collided 3 ways on average, and the shared-memory pipe was what
-// these formats waited for.  Fewer copies where 64 KB would not hold them.
+// these formats waited for.  Fewer copies where 64 KB would not hold them.  With the sign table and runs read at once,
+// 8192 x 28672 at batch 1 / 4: IQ2_XS 58.0 / 75.8 -> 48.0 / 60.4 us, IQ3_XXS 59.6 / 71.6 -> 51.0 / 63.4, IQ1_M 67.2 / 79.1 -> 46.0 / 62.7.
 template <int ENTRY_BYTES, int COPIES>
 TF_HD void grid_words(const Tables& tb, uint32_t i0, uint32_t i1, uint32_t& w0, uint32_t& w1) {
 #if TF_DEVICE
@@ -891,9 +892,9 @@ struct TQ10 {
 
 // =============================================================================================
 // Formats that ran on kernels decoding byte by byte to float32 before (streaming at batch 1, three bf16 terms per weight above).
-// Measured on B200, 14336 x 4096, us at batch 1 / 4 / 8 / 16, before -> here: Q8_0 26 / 55 / 57 / 55 -> 20 / 23 / 34 / 66,
-// Q4_0 31 / 86 / 87 / 92 -> 16 / 20 / 30 / 60, Q5_1 38 / 131 / 133 / 137 -> 18 / 22 / 38 / 75, MXFP4 36 / 90 / 92 / 98 ->
-// 24 / 26 / 36 / 69, Q3_K 43 / 102 / 102 / 97 -> 21 / 25 / 41 / 81, TQ1_0 68 / 91 / 92 / 98 -> 24 / 30 / 40 / 79.
+// Measured on B200, 14336 x 4096, us at batch 1 / 4 / 8, before -> here: Q8_0 26 / 55 / 57 -> 20 / 22 / 30, Q4_0 31 / 86 / 87 -> 16 /
+// 19 / 27, Q5_1 38 / 131 / 133 -> 18 / 21 / 35, MXFP4 36 / 90 / 92 -> 21 / 23 / 34, Q3_K 42 / 102 / 102 -> 21 / 24 / 39, TQ1_0
+// 68 / 92 / 92 -> 23 / 28 / 36.
 //
 // The 32-element formats: eight blocks make a superblock (kTs = 8 x block bytes), run t = blocks 2 t and 2 t + 1
 // = groups 0 and 1.  The run is read as aligned words; the block that starts two bytes into a word is shifted.

@@ -14,7 +14,7 @@
 //     jax.ffi.register_ffi_target("ggq_gemv", jax.ffi.pycapsule(lib.ggq_ffi_gemv), platform="CUDA")
 //     y = jax.ffi.ffi_call("ggq_gemv", jax.ShapeDtypeStruct((M, N), jnp.bfloat16))(
 //             w.data, x2d, workspace, qtype=np.int32(int(w.qtype)))
-// `workspace` is a uint8 device array of ggq_workspace_bytes(...) bytes, zero-filled once and passed
+// `workspace` is a uint8 device array of ggq_scratch_bytes(...) bytes, zero-filled once and passed
 // to every call (the kernels leave it zeroed); XLA owns it like any other operand.
 #include <cuda_runtime_api.h>
 

@@ -119,11 +119,11 @@ size_t ggq_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M);
  * Which kernel runs (all give the same product to float32 rounding; none is a CPU path):
  *   Q4_K / Q5_K / Q6_K at M = 1 and M = 5..16: the per-format kernels (integer codes fed to
  *     mma.sync as exact bf16 values, scales applied to the float32 accumulators);
- *   Q4_K / Q5_K / Q6_K at M = 2..4, and Q2_K, IQ4_XS, IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S,
- *     IQ1_S, IQ1_M at every M: the tiled kernel (same arithmetic; warps own contiguous ranges of
- *     16-row x K-chunk steps; needs K % 256 == 0, rows of a multiple of 16 bytes and the workspace; serves M in slices of 8);
- *   everything else (the 32-element formats, float formats, shapes the above do not take): the
- *     streaming kernels that decode a block in registers and multiply it at once.
+ *   Q4_K / Q5_K / Q6_K at M = 2..4, and every other block format on larger weights: the tiled kernel (same
+ *     arithmetic; warps own contiguous ranges of 16-row x K-chunk steps; needs K % 256 == 0 and the scratch of
+ *     ggq_scratch_bytes; serves M in slices of 8);
+ *   everything else (small weights, no scratch, shapes the above do not take): the streaming and MMA kernels
+ *     that decode a block in registers and multiply it at once.
  * Launches are programmatic dependents: a kernel may begin to read `w` (only `w`) while the
  * previous launch of this library on the same stream is still finishing.  So `w` must not be an
  * output of that previous launch; x, y and the workspace carry no such restriction.  The weight
