@@ -546,7 +546,7 @@ struct IQ2XXS {
     ld.words<2, 2>(2 + 16 * t + 8 * grp, q);
     return Group{q[0], q[1], mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(q[1] >> 28))};
   }
-  template <bool SIGN_TABLE = true>
+  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     uint32_t w0, w1, s0, s1;
     grid_words<8, kCopies>(tb, (g.q >> (8 * q)) & 0xFF, 0, w0, w1);
@@ -582,7 +582,7 @@ struct IQ2XS {
     const uint32_t sc = (ld.u16(66 + 2 * t) >> (4 * grp)) & 15;
     return Group{q, mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(sc))};
   }
-  template <bool SIGN_TABLE = true>
+  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     uint32_t w0, w1, s0, s1;
     grid_words<8, kCopies>(tb, (g.q >> (16 * q)) & 511, 0, w0, w1);
@@ -621,7 +621,7 @@ struct IQ2S {
     return Group{ld.u16(2 + 8 * t + 2 * grp), ld.u16(34 + 8 * t + 2 * grp), ld.u16(66 + 2 * t) >> (4 * grp),
                  mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(sc))};
   }
-  template <bool SIGN_TABLE = true>
+  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t idx = ((g.qs >> (8 * q)) & 0xFF) | (((g.qh >> (2 * q)) & 3) << 8);
     uint32_t w0, w1, s0, s1;
@@ -659,7 +659,7 @@ struct IQ3XXS {
     ld.words<1, 2>(66 + 8 * t + 4 * grp, aux);
     return Group{{q[0], q[1]}, aux[0], mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.5f), 0.5f + u2f(aux[0] >> 28))};
   }
-  template <bool SIGN_TABLE = true>
+  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t q16 = g.q[q >> 1] >> (16 * (q & 1));
     uint32_t w0, w1, s0, s1;
@@ -700,7 +700,7 @@ struct IQ3S {
     const uint32_t sc = (ld.u16(106 + (t & 2)) >> (8 * (t & 1) + 4 * grp)) & 15;
     return Group{{q[0], q[1]}, sg[0], ld.u16(66 + 2 * t) >> (8 * grp), mulf(f16_bits_to_float(ld.u16(0)), u2f(1 + 2 * sc))};
   }
-  template <bool SIGN_TABLE = true>
+  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t q16 = g.q[q >> 1] >> (16 * (q & 1));
     const uint32_t i0 = (q16 & 0xFF) | (((g.qh >> (2 * q)) & 1) << 8);

@@ -141,7 +141,7 @@ def test_formats_of_small_blocks_at_tile_edges(qtype):
 def test_non_finite_activations_give_what_the_decoded_weights_give(qtype):
     """An infinite activation times the decoded weights: infinities keep their sign, and only weights that are exactly
     zero (or infinities that cancel) give NaN."""
-    n, k = 40, 2048
+    n, k = 2056, 2048
     wb = synth.make_weight_bytes(n, k, qtype, seed=5)
     dense = O.ref_dequantize(wb, qtype).astype(np.float32)
     xb = synth.make_x(2, k, seed=5)
