@@ -139,18 +139,22 @@ struct Geo {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Prepare kernel: one CTA per staged batch column (columns >= M are zero-filled).
+// Prepare kernel: `parts` CTAs per staged batch column (columns >= M are zero-filled).  The multiply kernel waits for it, so
+// its length counts, and one CTA per column walked the column in dependent rounds of loads.  Every CTA of a column finds
+// the column's largest magnitude itself, from the L2 and eight loads at a time, and stages its share of the pieces.  Whole
+// product on B200, one CTA per column / up to eight: Q4_K 8192 x 28672 60.2 / 56.1 us at 8 rows and 68.9 / 65.1 at 16;
+// Q4_K 4096 x 14336 39.2 / 37.9 and Q6_K 14336 x 4096 40.2 / 38.5 at 32; 4096 x 4096 the same (16.2).
 //   xp[sb][q][col][t]   kPiece bytes: activations * 2^(S + x_exp), permuted (0,2,1,3[,4,6,5,7]) to the A registers' pairing
 //   xo[sb][col][...]    kOffBytes: the group sums of x (times 2^S), three bf16 terms each, in offset-MMA order
 //   S_col[col]          the column's power-of-two exponent
 template <class F, int XR>
 __global__ void __launch_bounds__(256)
 prepare_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int K, int M, uint8_t* __restrict__ xp, uint8_t* __restrict__ xo,
-               int* __restrict__ S_col, const PeerPublish pp, int* __restrict__ status) {
+               int* __restrict__ S_col, const int parts, const PeerPublish pp, int* __restrict__ status) {
   __shared__ int s_max;
   pdl_wait();            // x may be the previous kernel's output, and the previous launch may still read the staged copy
   pdl_trigger();         // the multiply kernel may start fetching weights
-  const int col = blockIdx.x, tid = threadIdx.x;
+  const int col = blockIdx.x / parts, part = blockIdx.x - col * parts, tid = threadIdx.x;
   // row-sharded: x is what the peers stored during the previous exchange; wait (bounded) for all of their flags
   peer_wait_previous(pp, tid, status);
   if (pp.world > 0 && pp.wait_previous) __syncthreads();
@@ -160,24 +164,29 @@ prepare_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int K, int M, u
   if (tid == 0) s_max = 0;
   __syncthreads();
   float amax = 0.f;
-  if (real)
+  if (real) {
+#pragma unroll 8
     for (int i = tid; i < K / 8; i += 256) {
       const uint4 v = __ldcg(reinterpret_cast<const uint4*>(xr) + i);
       const float s = (fabsf(bf16lo(v.x)) + fabsf(bf16hi(v.x))) + (fabsf(bf16lo(v.y)) + fabsf(bf16hi(v.y))) +
                       (fabsf(bf16lo(v.z)) + fabsf(bf16hi(v.z))) + (fabsf(bf16lo(v.w)) + fabsf(bf16hi(v.w)));
       amax = fmaxf(amax, s);
     }
-  atomicMax(&s_max, (int)__float_as_uint(amax));
+  }
+  const uint32_t wmax = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(amax));      // non-negative floats order like integers
+  if ((tid & 31) == 0) atomicMax(&s_max, (int)wmax);
   __syncthreads();
   // 2^96 suits any octet sum of |x| in about [2^-30, 2^30); otherwise put the largest near 2^120
   const int emax = min((s_max >> 23) & 0xFF, 254);
   const int S = (emax > 156 || (emax < 97 && emax > 0)) ? max(8, min(120, 247 - emax)) : 96;
-  if (tid == 0) S_col[col] = S;
+  if (tid == 0 && part == 0) S_col[col] = S;
   constexpr int kE = F::kPiece / 2;                       // elements per piece: 8 or 4
   constexpr int kPiecesPerSum = F::kSumLen / kE;          // pieces (consecutive t) that make one scale group: 4
   static_assert(kPiecesPerSum == 4, "a scale group is the four lane groups of one MMA group");
   const int n_pieces = SB * F::kGroups * 4;
-  for (int o = tid; o < (n_pieces + 255) / 256 * 256; o += 256) {
+  // a part is a whole number of rounds of 256 pieces (a scale group is four consecutive ones)
+  const int rounds = (n_pieces + 255) / 256, r_begin = rounds * part / parts, r_end = rounds * (part + 1) / parts;
+  for (int o = r_begin * 256 + tid; o < r_end * 256; o += 256) {
     const bool in = o < n_pieces;
     const int sb = o / (F::kGroups * 4), q = (o / 4) % F::kGroups, t = o & 3;
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -743,8 +752,9 @@ static cudaError_t launch(const Geo& geo, int grid, cudaStream_t st, const uint8
     attr_done[dev].store(true, std::memory_order_release);
   }
   constexpr int XR = 8 * NT;
-  cudaError_t err = launch_pdl(prepare_kernel<F, XR>, XR, 256, 0, st, (const __nv_bfloat16*)x, ldx, K, M, ws + l.xp, ws + l.xo,
-                               reinterpret_cast<int*>(ws + l.scol), pp, status);
+  const int rounds = (K / 256 * F::kGroups * 4 + 255) / 256, parts = std::min(8, rounds);
+  cudaError_t err = launch_pdl(prepare_kernel<F, XR>, XR * parts, 256, 0, st, (const __nv_bfloat16*)x, ldx, K, M, ws + l.xp, ws + l.xo,
+                               reinterpret_cast<int*>(ws + l.scol), parts, pp, status);
   if (err != cudaSuccess) return err;
   err = launch_pdl(gemv_wide_kernel<F, NT>, grid, kThreads, (size_t)geo.total, st, w, N, K, (const uint8_t*)(ws + l.xp),
                    (const uint8_t*)(ws + l.xo), reinterpret_cast<const int*>(ws + l.scol), M, y, y_dtype,
