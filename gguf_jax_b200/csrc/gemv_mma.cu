@@ -113,7 +113,10 @@ gemv_mma_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16
     for (int ww = 0; ww < kWarps; ww++) sum += red[ww][c][i][ln];
     const int row = n0 + (ln >> 2) + 8 * (i >> 1);
     const int m = 8 * c + 2 * (ln & 3) + (i & 1);
-    if (row < N && m < M) store_out(y, y_dtype, (int64_t)m * N + row, sum);
+    if (row < N && m < M) {
+      if (!(fabsf(sum) <= 3.402823466e38f)) sum = exact_dot<QT>(w + row * row_bytes, x + (int64_t)m * K, K, tab);
+      store_out(y, y_dtype, (int64_t)m * N + row, sum);
+    }
   }
 }
 

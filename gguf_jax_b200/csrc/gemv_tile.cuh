@@ -154,23 +154,6 @@ __device__ __forceinline__ void q4k_block_m1(uint32_t blk0, uint32_t blk1, int t
   out1 = fmaf(dlb, hi[3], out1); out1 = fmaf(dmb, sx1, out1);
 }
 
-// One output element the plain way: float32 weights of the block decoders times the activations, in order.  The code sums
-// of the kernel below subtract multiples of sum(x), so an activation or a scale that is infinite (or a sum that leaves the
-// float32 range on the way) makes them NaN where the product of the decoded weights is not: such an element is
-// recomputed here.  One lane walks the row; nothing else ever calls it.
-template <int QT>
-__device__ __noinline__ float exact_dot(const uint8_t* wrow, const __nv_bfloat16* xrow, int K, const uint8_t* tab) {
-  constexpr int BS = block_elems_of(QT), TS = block_bytes_of(QT);
-  float acc = 0.f;
-  for (int e = 0; e < K; e += 8) {
-    float v[8];
-    Dec<QT>::run(wrow + (int64_t)(e / BS) * TS, (e % BS) >> 3, tab, v);
-#pragma unroll
-    for (int i = 0; i < 8; i++) acc = fmaf(v[i], __bfloat162float(xrow[e + i]), acc);
-  }
-  return acc;
-}
-
 template <class F, int MP>
 __global__ void __launch_bounds__(kThreads, 1)
 gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,

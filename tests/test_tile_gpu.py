@@ -137,11 +137,12 @@ def test_formats_of_small_blocks_at_tile_edges(qtype):
             assert O.rel_l2(got, ref) <= 2e-5, (qtype.name, n, k, m)
 
 
-@pytest.mark.parametrize("qtype", TILE_SMALL_BLOCKS + [QT.Q2_K, QT.IQ4_XS], ids=lambda t: t.name)
-def test_non_finite_activations_give_what_the_decoded_weights_give(qtype):
+@pytest.mark.parametrize("n", [40, 2056])
+@pytest.mark.parametrize("qtype", TILE_SMALL_BLOCKS + [QT.Q2_K, QT.IQ4_XS, QT.IQ2_XS, QT.IQ1_S], ids=lambda t: t.name)
+def test_non_finite_activations_give_what_the_decoded_weights_give(qtype, n):
     """An infinite activation times the decoded weights: infinities keep their sign, and only weights that are exactly
-    zero (or infinities that cancel) give NaN."""
-    n, k = 2056, 2048
+    zero (or infinities that cancel) give NaN.  40 rows go to the MMA kernel, 2056 to the tiled one."""
+    k = 2048
     wb = synth.make_weight_bytes(n, k, qtype, seed=5)
     dense = O.ref_dequantize(wb, qtype).astype(np.float32)
     xb = synth.make_x(2, k, seed=5)
