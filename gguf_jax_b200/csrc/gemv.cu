@@ -157,7 +157,8 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
     else if (qtype == QT_Q6_K && gemv_q6k_applicable(N, K, 1, w, x_bf16)) tuned = gemv_q6k;
   }
   static const bool m1_tiled = [] { const char* e = getenv("GGQ_Q4K_M1_TILED"); return e && e[0] == '1'; }();
-  // Q4_K / Q5_K / Q6_K keep their batch-1 kernels; the tiled kernel takes their batches 2..4 (Q4_K 8192 x 28672:
+  // Q4_K / Q5_K / Q6_K keep their batch-1 kernels; the tiled kernel takes their batches 2..4 whatever the size (it scales each
+  // row and keeps any magnitude; the integer-code MMA kernel keeps about 2^-50 to 2^62; Q4_K 8192 x 28672:
   // 36 / 49 us at batch 2 / 4) and the other formats where tile_pays says so; from five batch rows on
   // the batch-major kernel takes the larger weights (Q4_K 8192 x 28672: 68 / 77 us at batch 8 / 16 against
   // 100 / 153 us) and the integer-code MMA kernel (gemv_mma.cu) the smaller ones (see wide_pays).
@@ -165,11 +166,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them
   const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
   const int64_t weights = N * K;
-  // K-quants below 6 M weights at 2..4 rows: the MMA kernel (2048 x 2048 Q4_K 4.7 us against the tiled kernel's 6.7 / 8.3 at
-  // 2 / 4 rows; 8192 x 2048 9.3 against 8.3 / 9.8)
-  const bool small_batch = k_quant && M >= 2 && M <= 4 && weights < (6 << 20) && gemv_mma_applicable(ti, N, K, M);
-  if (small_batch) tuned = nullptr;
-  const bool tile_first = k_quant ? (M >= 2 && M <= 4 && !small_batch) || (M == 1 && (odd_rows ? tile_pays(qtype, weights, 1) : m1_tiled))
+  const bool tile_first = k_quant ? (M >= 2 && M <= 4) || (M == 1 && (odd_rows ? tile_pays(qtype, weights, 1) : m1_tiled))
                                   : tile_pays(qtype, weights, M);
   const int tile_max = gemv_tile_max_batch(qtype);
   const int tile_m = M < tile_max ? M : tile_max;

@@ -153,6 +153,20 @@ def test_non_finite_activations_give_what_the_decoded_weights_give(qtype, n):
     assert np.array_equal(got[1], want, equal_nan=True), qtype.name
 
 
+@pytest.mark.parametrize("exponent", [-90, 90])
+@pytest.mark.parametrize("qtype", [QT.Q4_K, QT.Q5_K, QT.Q6_K], ids=lambda t: t.name)
+def test_activations_far_from_one_on_small_weights(qtype, exponent):
+    """Activations around 2^-90 and 2^90 at 2..4 rows: the tiled kernel scales each row by a power of two, so the result is the
+    ordinary one times that power, to the same 2e-5 (the MMA kernel of the larger batches keeps about 2^-50 to 2^62)."""
+    n, k = 200, 2048
+    wb = synth.make_weight_bytes(n, k, qtype, seed=9)
+    w = on_device(wb, qtype, n, k)
+    for m in (2, 3, 4):
+        xb = synth.make_x(m, k, seed=m)
+        got = kernels.fused_matmul(to_x(xb) * 2.0 ** exponent, w, out_dtype=torch.float32).cpu().numpy().astype(np.float64)
+        assert O.rel_l2(np.ldexp(got, -exponent), O.c_matmul(O.bf16_bits(xb), wb, qtype)) <= 2e-5, (qtype.name, m)
+
+
 @pytest.mark.parametrize("qtype", [QT.Q6_K, QT.Q2_K, QT.Q3_K, QT.IQ4_XS, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT.IQ3_XXS, QT.IQ3_S, QT.IQ1_S,
                                    QT.IQ1_M, QT.TQ1_0, QT.TQ2_0, QT.MXFP4], ids=lambda t: t.name)
 def test_rows_at_every_offset_of_a_16_byte_piece(qtype):
