@@ -168,6 +168,15 @@ def _promoted_mm(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 # to kernels an order of magnitude slower (8655 x 27136 at 1336 rows: 5.8 ms against 0.6 ms for 8656).
 _ROW_ELEMS = 8
 
+# Padding costs an allocation and one or two launches more per product, 25 us of host time each.  Below this many operations the
+# slow kernels finish in less (2445 x 1792 at 508 rows, forward and backward: 192 us unpadded, 246 us padded, both bound by
+# the host); above, they are what the call waits for.
+_PAD_FROM_OPS = 1 << 35
+
+
+def _pads(rows: int, w: QuantizedArray) -> bool:
+    return w.shape[0] % _ROW_ELEMS != 0 and 2 * rows * w.shape[0] * w.shape[1] >= _PAD_FROM_OPS
+
 
 def _plain(t: torch.Tensor) -> bool:
     """An ordinary tensor outside every transform, trace and dispatch mode: results may be written in place."""
@@ -180,7 +189,7 @@ def _materialized_forward(x: torch.Tensor, w: QuantizedArray, count: int) -> tor
     n_out = w.shape[0]
     x2 = x.reshape(-1, w.shape[1])
     y = None
-    if (count > 1 or n_out % _ROW_ELEMS) and _plain(x):
+    if _plain(x) and (count > 1 or _pads(x2.shape[0], w)):
         # every slab's product goes straight to its columns of the result; slab and row boundaries are multiples of
         # _ROW_ELEMS (a result whose rows are not is copied once at the end).  Slabs are rounded down, so that none
         # exceeds the budget; one of all rows stays whole.
@@ -208,7 +217,7 @@ def _input_cotangent(g: torch.Tensor, w: QuantizedArray, count: int) -> torch.Te
     """``g (..., N) @ w (N, K)``: the slabs cut the contraction, so their products add up (in
     float32 when there is more than one)."""
     g2 = g.reshape(-1, w.shape[0])
-    if w.shape[0] % _ROW_ELEMS:         # rows of the left operand on 16-byte boundaries
+    if _pads(g2.shape[0], w):           # rows of the left operand on 16-byte boundaries
         g2 = torch.nn.functional.pad(g2, (0, -w.shape[0] % _ROW_ELEMS))[:, :w.shape[0]]
     if count == 1:
         (_, dense), = _slabs(w, 1)

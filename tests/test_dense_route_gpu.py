@@ -38,6 +38,19 @@ def test_products_and_gradients_of_any_row_count(n, slab_rows):
     assert gj.dequant_matmul(x[:0], w, block_bytes=budget).shape == (0, n)
 
 
+def test_padded_rows_of_a_large_product():
+    """Enough operations for the padded rows of the result and of the gradient."""
+    m, n, k = 2048, 2049, 4096
+    w = synth.make_weight(n, k, QT.Q5_1, seed=1, device="cuda")
+    dense = w.dequantize()
+    x = torch.randn((m, k), device="cuda").bfloat16().requires_grad_(True)
+    g = torch.randn((m, n), device="cuda").bfloat16()
+    y = gj.dequant_matmul(x, w, block_bytes=None)
+    (dx,) = torch.autograd.grad(y, x, g)
+    assert y.shape == (m, n) and y.is_contiguous()
+    assert rel(y, x.double() @ dense.double().T) <= 2 ** -8 and rel(dx, g.double() @ dense.double()) <= 2 ** -8
+
+
 def test_transforms_take_the_general_way():
     w = synth.make_weight(100, 512, QT.Q5_1, seed=3, device="cuda")
     x = torch.randn((4, 6, 512), device="cuda")
