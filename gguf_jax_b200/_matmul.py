@@ -179,8 +179,10 @@ def _pads(rows: int, w: QuantizedArray) -> bool:
 
 
 def _plain(t: torch.Tensor) -> bool:
-    """An ordinary tensor outside every transform, trace and dispatch mode: results may be written in place."""
+    """An ordinary tensor outside every transform, trace, dispatch mode and autocast region (which casts ``matmul`` but no product
+    with ``out=``): results may be written in place."""
     return (type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and t.device.type in ("cuda", "cpu") and not torch.is_autocast_enabled(t.device.type)
             and torch._C._len_torch_dispatch_stack() == 0 and torch.autograd.forward_ad._current_level < 0
             and not torch.jit.is_tracing() and not (t.requires_grad and torch.is_grad_enabled()))
 

@@ -1,0 +1,51 @@
+"""The materializing route's choice between products written in place and the general way, on the CPU: a registered decoder makes
+dense weights there, so that autocast, transforms, traces and modes can be tried without a device.  The in-place products
+and the padded rows must be indistinguishable from one product of the whole dense weight."""
+import gguf
+import numpy as np
+import pytest
+import torch
+from gguf.constants import GGMLQuantizationType as QT
+
+import gguf_jax_b200 as gj
+from gguf_jax_b200 import _matmul as mm
+from gguf_jax_b200 import quants, synth
+
+K = 128
+IN_SLABS = 4 * K * 32           # a budget of 32 rows
+
+
+@pytest.fixture(autouse=True)
+def decoder_on_the_cpu():
+    saved = quants._DEQUANT[QT.Q8_0]
+
+    def decode(blocks, dtype):
+        return torch.from_numpy(np.asarray(gguf.quants.dequantize(blocks.numpy(), QT.Q8_0))).to(dtype)
+
+    gj.register_dequant(QT.Q8_0, decode, override=True)
+    yield
+    gj.register_dequant(QT.Q8_0, saved, override=True)
+
+
+def case(n, m=6, seed=1):
+    w = synth.make_weight(n, K, QT.Q8_0, seed=seed, device="cpu")
+    return w, torch.randn((m, K), generator=torch.Generator().manual_seed(seed))
+
+
+# one slab; several slabs; one slab whose rows are padded (the size rule set aside)
+FORMS = [(96, None, False), (96, IN_SLABS, False), (100, IN_SLABS, False), (100, None, True)]
+
+
+@pytest.mark.parametrize("n,budget,padded", FORMS)
+@pytest.mark.parametrize("train", [False, True])
+@pytest.mark.parametrize("x_dtype,cast_to", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.float16)], ids=str)
+def test_autocast_decides_the_dtype_whatever_the_shape(n, budget, padded, train, x_dtype, cast_to, monkeypatch):
+    if padded:
+        monkeypatch.setattr(mm, "_PAD_FROM_OPS", 0)
+    w, x = case(n)
+    x = x.to(x_dtype).requires_grad_(train)
+    with torch.autocast("cpu", dtype=cast_to):
+        y = gj.dequant_matmul(x, w, block_bytes=budget)
+        want = torch.matmul(x.detach(), w.dequantize().T)
+    assert want.dtype == cast_to and y.dtype == cast_to
+    assert torch.allclose(y.float(), want.float(), rtol=2 ** -7, atol=2 ** -7 * want.abs().max().item())
