@@ -23,6 +23,7 @@ from typing import Callable
 import torch
 from gguf.constants import GGML_QUANT_SIZES
 from gguf.constants import GGMLQuantizationType as QT
+from torch.utils._device import DeviceContext
 
 from . import _backend, _lib, kernels, quants
 from .array import QuantizedArray
@@ -101,7 +102,7 @@ def matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None
     served by the fused route only (see :func:`gguf_jax_b200.kernels.fused_matmul`), without
     gradients; anything the fused route does not take raises ``ValueError``.
     """
-    if out is None and w.__class__ is QuantizedArray:
+    if out is None and w.__class__ is QuantizedArray and not _function_modes():
         # the common call (device activations, no gradient; fused, or dense in one piece by the built-in bf16 decoder) is one
         # native function
         budget = DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes
@@ -178,13 +179,20 @@ def _pads(rows: int, w: QuantizedArray) -> bool:
     return w.shape[0] % _ROW_ELEMS != 0 and 2 * rows * w.shape[0] * w.shape[1] >= _PAD_FROM_OPS
 
 
+def _function_modes() -> bool:
+    """A ``TorchFunctionMode`` is active that may want to see the operations (``torch.device`` as a context only adds a device
+    to factory calls, and every call here names its own)."""
+    depth = torch._C._len_torch_function_stack()
+    return depth > 0 and any(type(torch._C._get_function_stack_at(i)) is not DeviceContext for i in range(depth))
+
+
 def _plain(t: torch.Tensor) -> bool:
-    """An ordinary tensor outside every transform, trace, dispatch mode and autocast region (which casts ``matmul`` but no product
+    """An ordinary tensor outside every transform, trace, mode and autocast region (which casts ``matmul`` but no product
     with ``out=``): results may be written in place."""
     return (type(t) in (torch.Tensor, torch.nn.Parameter) and not torch._C._functorch.is_functorch_wrapped_tensor(t)
             and t.device.type in ("cuda", "cpu") and not torch.is_autocast_enabled(t.device.type)
-            and torch._C._len_torch_dispatch_stack() == 0 and torch.autograd.forward_ad._current_level < 0
-            and not torch.jit.is_tracing() and not (t.requires_grad and torch.is_grad_enabled()))
+            and torch._C._len_torch_dispatch_stack() == 0 and not _function_modes()
+            and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing() and not (t.requires_grad and torch.is_grad_enabled()))
 
 
 def _materialized_forward(x: torch.Tensor, w: QuantizedArray, count: int) -> torch.Tensor:

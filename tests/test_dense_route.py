@@ -49,3 +49,30 @@ def test_autocast_decides_the_dtype_whatever_the_shape(n, budget, padded, train,
         want = torch.matmul(x.detach(), w.dequantize().T)
     assert want.dtype == cast_to and y.dtype == cast_to
     assert torch.allclose(y.float(), want.float(), rtol=2 ** -7, atol=2 ** -7 * want.abs().max().item())
+
+
+class Recorder(torch.overrides.TorchFunctionMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func)
+        return func(*args, **(kwargs or {}))
+
+
+def test_function_modes_see_the_operations(monkeypatch):
+    w, x = case(96)
+    with Recorder() as mode:
+        y = gj.dequant_matmul(x, w, block_bytes=IN_SLABS)
+    assert torch.matmul in mode.seen and torch.mm not in mode.seen
+    assert torch.allclose(y, x @ w.dequantize(torch.float32).T, rtol=2 ** -7, atol=0.1)
+    # the native call path has no operations a mode could see: it is not asked, except under the mode that only sets the device
+    monkeypatch.setattr(mm, "_native_matmul", lambda *a: "native")
+    with Recorder(), pytest.raises(RuntimeError):
+        gj.matmul(x, w)                       # the general path, which refuses host memory
+    assert gj.matmul(x, w) == "native"
+    with torch.device("cpu"):
+        assert gj.matmul(x, w) == "native"
+        with Recorder(), pytest.raises(RuntimeError):
+            gj.matmul(x, w)
