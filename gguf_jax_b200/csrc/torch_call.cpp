@@ -91,12 +91,14 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (n <= 0 || k <= 0 || x.size(-1) != k || dev != c10::cuda::current_device()) Py_RETURN_NONE;
   const int64_t m = x.numel() / k;
   if (m < 1 || m > 65536) Py_RETURN_NONE;
+  const int force = PyObject_IsTrue(args[4]);      // any truth value, as in the Python path
+  if (force < 0) { PyErr_Clear(); Py_RETURN_NONE; }
   const Shape* s = shape_of((int32_t)qtype, n, k, (int32_t)m);
   if (!s || (size_t)w.numel() != s->payload) Py_RETURN_NONE;
   const auto stream = c10::cuda::getCurrentCUDAStream(dev);
   c10::SmallVector<int64_t, 6> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = n;
-  if (m > s->limit && args[4] != Py_True) {
+  if (m > s->limit && !force) {
     // the dense route in one piece: decode to bf16, library GEMM (rows of the result on 16-byte boundaries)
     const double budget = PyFloat_AsDouble(args[5]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }

@@ -1,5 +1,6 @@
 """The native call path of `matmul` against the Python path it stands for: same results for every form of activations, and the
 forms it must leave alone (gradients, host memory, transforms, subclasses, shapes and batches outside the fused route)."""
+import numpy as np
 import pytest
 import torch
 from gguf.constants import GGMLQuantizationType as QT
@@ -119,3 +120,17 @@ def test_first_call_of_a_stream_under_capture_takes_no_scratch_it_can_do_without
     torch.cuda.synchronize()
     assert torch.equal(z, want)
     assert ((y.double() - want.double()).norm() / want.double().norm()).item() <= 2 ** -8      # another kernel's summation order
+
+
+def test_force_fused_is_any_truth_value():
+    """Above the cap: the fused kernel (float32 weights) for whatever is true, the dense route (weights rounded to bf16) otherwise."""
+    w = synth.make_weight(96, 2048, QT.Q8_0, seed=6, device="cuda")
+    x = torch.randn((40, 2048), device="cuda").bfloat16()
+    fused, dense = kernels.fused_matmul(x, w), gj.dequant_matmul(x, w)
+    assert not torch.equal(fused, dense)
+    for value in (True, 1, np.True_, "yes"):
+        assert torch.equal(gj.matmul(x, w, force_fused=value), fused), value
+    for value in (False, 0, np.False_, None):
+        assert torch.equal(gj.matmul(x, w, force_fused=value), dense), value
+    with pytest.raises(ValueError):
+        gj.matmul(x, w, force_fused=np.array([1, 0]))
