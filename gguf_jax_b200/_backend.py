@@ -11,8 +11,6 @@ import torch
 from . import _lib
 
 _DTYPE_CODE = {torch.float32: _lib.GGQ_F32, torch.bfloat16: _lib.GGQ_BF16, torch.float16: _lib.GGQ_F16}
-_workspaces: dict[tuple[int, int], torch.Tensor] = {}
-_stagings: dict[tuple[int, int], torch.Tensor] = {}
 
 
 def canon_dtype(dtype) -> torch.dtype:
@@ -63,30 +61,64 @@ def stream_ptr(device_index: int) -> int:
     return torch.cuda.current_stream(device_index).cuda_stream
 
 
+def _capture_id(stream: int) -> int:
+    """Identity of the CUDA graph capture that the stream takes part in, 0 outside any."""
+    return _lib.native().capture_id(stream)
+
+
+class _Buffers:
+    """One device buffer per (device, stream), grown on demand: the calls of a stream are ordered, so one serves them all.
+
+    A buffer that is first allocated under a CUDA graph capture belongs to that capture alone: it is the graph's memory and its
+    zero fill runs on replay, so no other graph and no call outside may take it for a cleared one."""
+
+    def __init__(self, smallest: int, zeroed: bool, publish: bool):
+        self.smallest, self.zeroed, self.publish = smallest, zeroed, publish
+        self.current: dict[tuple[int, int], torch.Tensor] = {}
+        self.of_capture: dict[tuple[int, int], tuple[int, torch.Tensor]] = {}
+
+    def _new(self, device_index: int, nbytes: int) -> torch.Tensor:
+        make = torch.zeros if self.zeroed else torch.empty
+        return make(max(nbytes, self.smallest), dtype=torch.uint8, device=torch.device("cuda", device_index))
+
+    def get(self, device_index: int, nbytes: int, stream: int, least: int | None = None) -> torch.Tensor | None:
+        """At least ``nbytes``; under capture, where none is that large yet, ``least`` will do."""
+        key = (device_index, stream)
+        buf = self.current.get(key)
+        capture = _capture_id(stream)
+        if capture:
+            own = self.of_capture.get(key)
+            if own is not None and own[0] == capture and own[1].numel() >= nbytes:
+                return own[1]
+            if least is not None and least < nbytes and (buf is None or buf.numel() < nbytes):
+                return self.get(device_index, least, stream)
+            if buf is not None and buf.numel() >= nbytes > 0:
+                return buf
+            if nbytes > 0:
+                buf = self._new(device_index, nbytes)
+                self.of_capture[key] = (capture, buf)
+                return buf
+        if nbytes == 0:
+            return None
+        if buf is None or buf.numel() < nbytes:
+            buf = self.current[key] = self._new(device_index, nbytes)
+            if self.publish:
+                _lib.native().set_scratch(key[0], key[1], buf)
+        return buf
+
+
+_workspaces = _Buffers(1 << 20, zeroed=True, publish=True)
+_stagings = _Buffers(1 << 16, zeroed=False, publish=False)
+
+
 def staging(device_index: int, nbytes: int, stream: int | None = None) -> torch.Tensor:
-    """Device buffer that receives host-resident activations, one per (device, stream), grown on demand.
-    Calls on one stream are ordered, so one buffer serves them all.  ``stream``: the current stream's handle if
-    the caller already has it."""
-    key = (device_index, stream_ptr(device_index) if stream is None else stream)
-    buf = _stagings.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = _stagings[key] = torch.empty(max(nbytes, 1 << 16), dtype=torch.uint8, device=torch.device("cuda", device_index))
-    return buf
+    """Device buffer that receives host-resident activations.  ``stream``: the current stream's handle if the caller already
+    has it."""
+    return _stagings.get(device_index, nbytes, stream_ptr(device_index) if stream is None else stream)
 
 
 def workspace(device_index: int, nbytes: int, stream: int | None = None, least: int | None = None) -> torch.Tensor | None:
-    """Zero-filled scratch for the fused kernels, one per (device, stream), grown on demand.
-    The kernels leave it zeroed, so it is cleared only when (re)allocated.  ``stream``: the current stream's
-    handle if the caller already has it.  ``least``: what the call cannot do without; a capturing stream gets no more than
-    that newly allocated (its zero fill would only happen on replay)."""
-    key = (device_index, stream_ptr(device_index) if stream is None else stream)
-    ws = _workspaces.get(key)
-    if least is not None and least < nbytes and (ws is None or ws.numel() < nbytes) and torch.cuda.is_current_stream_capturing():
-        nbytes = least
-    if nbytes == 0:
-        return None
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", device_index))
-        _workspaces[key] = ws
-        _lib.native().set_scratch(key[0], key[1], ws)
-    return ws
+    """Zero-filled scratch for the fused kernels.  The kernels leave it zeroed, so it is cleared only when (re)allocated.
+    ``stream``: the current stream's handle if the caller already has it.  ``least``: what the call cannot do without; a
+    capturing stream gets no more than that newly allocated."""
+    return _workspaces.get(device_index, nbytes, stream_ptr(device_index) if stream is None else stream, least)

@@ -148,9 +148,20 @@ PyObject* set_scratch(PyObject*, PyObject* args) {
   END_HANDLE_TH_ERRORS
 }
 
+// capture_id(stream): identity of the graph capture the stream takes part in, 0 outside any
+PyObject* capture_id(PyObject*, PyObject* arg) {
+  const unsigned long long handle = PyLong_AsUnsignedLongLong(arg);
+  if (PyErr_Occurred()) return nullptr;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)(uintptr_t)handle, &status, &id) != cudaSuccess) (void)cudaGetLastError();
+  return PyLong_FromUnsignedLongLong(status == cudaStreamCaptureStatusNone ? 0 : id);
+}
+
 PyMethodDef methods[] = {
     {"fast_matmul", (PyCFunction)(void (*)())fast_matmul, METH_FASTCALL, "x @ w.T by the fused kernels, or None"},
     {"bind", bind, METH_VARARGS, "hand over the library's entry points"},
+    {"capture_id", capture_id, METH_O, "the graph capture a stream takes part in, or 0"},
     {"set_scratch", set_scratch, METH_VARARGS, "register a stream's scratch"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

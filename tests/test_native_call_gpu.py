@@ -134,3 +134,28 @@ def test_force_fused_is_any_truth_value():
         assert torch.equal(gj.matmul(x, w, force_fused=value), dense), value
     with pytest.raises(ValueError):
         gj.matmul(x, w, force_fused=np.array([1, 0]))
+
+
+def test_two_graphs_captured_on_a_cold_stream_replay_in_any_order():
+    """K-quants cannot do without scratch: each capture that finds none on its stream takes its own, cleared on every replay."""
+    w = synth.make_weight(4096, 6144, QT.Q4_K, seed=7, device="cuda")
+    xs = [torch.randn((m, 6144), device="cuda").bfloat16() for m in (3, 12)]
+    want = [gj.matmul(x, w) for x in xs]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graphs, results = [], []
+    for x in xs:
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], stream=stream):
+            results.append([gj.matmul(x, w), gj.matmul(x, w)])
+    with torch.cuda.stream(stream):
+        eager = gj.matmul(xs[1], w)                    # before either graph has run
+    torch.cuda.synchronize()
+    assert torch.equal(eager, want[1])
+    for i in (1, 0, 1):
+        for y in results[i]:
+            y.zero_()
+        graphs[i].replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want[i]) for y in results[i]), i
+        assert torch.equal(gj.matmul(xs[i], w), want[i])
