@@ -69,12 +69,16 @@ def _capture_id(stream: int) -> int:
 class _Buffers:
     """One device buffer per (device, stream), grown on demand: the calls of a stream are ordered, so one serves them all.
 
-    A buffer that is first allocated under a CUDA graph capture belongs to that capture alone: it is the graph's memory and its
-    zero fill runs on replay, so no other graph and no call outside may take it for a cleared one."""
+    CUDA graphs keep the addresses they were captured with.  So a buffer that a capture has been given stays allocated when a
+    larger one takes its place (which is then at least twice as large: those kept never add up to more than the current
+    one).  And a buffer that is first allocated under capture belongs to that capture alone: it is the graph's memory and
+    its zero fill runs on replay, so no other graph and no call outside may take it for a cleared one."""
 
     def __init__(self, smallest: int, zeroed: bool, publish: bool):
         self.smallest, self.zeroed, self.publish = smallest, zeroed, publish
         self.current: dict[tuple[int, int], torch.Tensor] = {}
+        self.in_graphs: set[tuple[int, int]] = set()               # keys whose current buffer a capture was given
+        self.kept: dict[tuple[int, int], list[torch.Tensor]] = {}
         self.of_capture: dict[tuple[int, int], tuple[int, torch.Tensor]] = {}
 
     def _new(self, device_index: int, nbytes: int) -> torch.Tensor:
@@ -93,6 +97,7 @@ class _Buffers:
             if least is not None and least < nbytes and (buf is None or buf.numel() < nbytes):
                 return self.get(device_index, least, stream)
             if buf is not None and buf.numel() >= nbytes > 0:
+                self.in_graphs.add(key)
                 return buf
             if nbytes > 0:
                 buf = self._new(device_index, nbytes)
@@ -101,6 +106,10 @@ class _Buffers:
         if nbytes == 0:
             return None
         if buf is None or buf.numel() < nbytes:
+            if key in self.in_graphs:
+                self.in_graphs.discard(key)
+                self.kept.setdefault(key, []).append(buf)
+                nbytes = max(nbytes, 2 * buf.numel())
             buf = self.current[key] = self._new(device_index, nbytes)
             if self.publish:
                 _lib.native().set_scratch(key[0], key[1], buf)

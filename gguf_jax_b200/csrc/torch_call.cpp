@@ -17,6 +17,7 @@
 #include <ATen/core/grad_mode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
@@ -110,6 +111,8 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const auto it = g_scratch.find({dev, (uintptr_t)stream.stream()});
   // no scratch yet on this stream (its first call also uploads the code books), or one that has to grow
   if (it == g_scratch.end() || (size_t)it->second.numel() < s->scratch) Py_RETURN_NONE;
+  // a graph that is being captured keeps the scratch's address: the Python path notes that
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) Py_RETURN_NONE;
   const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
   at::Tensor y = at::empty(sizes, x.options().requires_grad(false));
   const int32_t rc = (m <= g_gemv_max ? g_gemv : g_gemm)((int32_t)qtype, w.data_ptr(), n, k, xc.data_ptr(), (int32_t)m, y.data_ptr(), kBf16,

@@ -159,3 +159,25 @@ def test_two_graphs_captured_on_a_cold_stream_replay_in_any_order():
         torch.cuda.synchronize()
         assert all(torch.equal(y, want[i]) for y in results[i]), i
         assert torch.equal(gj.matmul(xs[i], w), want[i])
+
+
+def test_a_graph_replays_after_the_streams_scratch_has_grown():
+    small, big = synth.make_weight(4096, 6144, QT.Q4_K, seed=8, device="cuda"), synth.make_weight(8192, 28672, QT.Q4_K, seed=9, device="cuda")
+    x, xb = (torch.randn((12, k), device="cuda").bfloat16() for k in (6144, 28672))
+    want = gj.matmul(x, small)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        gj.matmul(x, small)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = gj.matmul(x, small)
+    with torch.cuda.stream(stream):
+        grown = gj.matmul(xb, big, force_fused=True)
+        others = [torch.full((1 << 20,), 7, device="cuda") for _ in range(64)]         # whatever the allocator has free
+        y.zero_()
+        graph.replay()
+        again = gj.matmul(xb, big, force_fused=True)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and torch.equal(grown, again)
+    assert all(bool((t == 7).all()) for t in others)

@@ -1,5 +1,8 @@
-"""The scratch and staging buffers of the host path around CUDA graphs, with the device calls replaced: which buffer a call gets and when it
-is cleared.  CPU only."""
+"""The scratch and staging buffers of the host path around CUDA graphs, with the device calls replaced: which buffer a call gets, when it
+is cleared, and that no buffer a graph may write goes back to the allocator.  CPU only."""
+import gc
+import weakref
+
 import pytest
 import torch
 
@@ -61,6 +64,31 @@ def test_a_capture_uses_the_streams_scratch_where_it_is_large_enough(device):
     big = _backend.workspace(0, 9 * MB, 11)
     assert big.numel() >= 9 * MB and _backend.workspace(0, 9 * MB, 11, 1 * MB) is big
     assert len(device.cleared) == 2
+
+
+@pytest.mark.parametrize("get", [lambda n: _backend.workspace(0, n, 11, n), lambda n: _backend.staging(0, n, 11)], ids=["workspace", "staging"])
+def test_a_buffer_a_graph_uses_outlives_its_replacement(device, get):
+    first = weakref.ref(get(2 * MB))
+    get(3 * MB)
+    gc.collect()
+    device.native_scratch.clear()
+    assert first() is None                                            # no graph knows it
+    seen, size = [], 4 * MB
+    for capture in range(1, 41):
+        device.capture = capture
+        buf = get(size)
+        seen.append(weakref.ref(buf))
+        device.capture = 0
+        size += 1 * MB
+        buf = get(size)
+    del buf
+    device.native_scratch.clear()
+    gc.collect()
+    current = get(1)
+    in_graphs = [r() for r in seen[1:]]                               # (the first was the capture's own)
+    assert all(t is not None for t in in_graphs)
+    kept = {t.data_ptr(): t.numel() for t in in_graphs if t is not current}
+    assert 0 < sum(kept.values()) < current.numel()                   # bounded by the size of the current one
 
 
 def test_staging_first_taken_by_a_capture_is_not_used_outside(device):
