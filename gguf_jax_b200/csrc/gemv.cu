@@ -172,7 +172,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const int tile_m = M < tile_max ? M : tile_max;
   const size_t tile_need = tile_max ? gemv_tile_workspace_bytes(qtype, N, K, tile_m) : 0;
   const bool tile_ok = tile_first && tile_need && workspace && workspace_bytes >= tile_need && (uintptr_t)workspace % 256 == 0 &&
-                       sm_count_of(dev) > 0 && gemv_tile_applicable(qtype, N, K, tile_m, w, x_bf16);
+                       sm_count_of(dev) > 0 && gemv_tile_applicable(qtype, N, K, tile_m, w, x_bf16, sm_count_of(dev));
   static const int wide_min = [] { const char* e = getenv("GGQ_WIDE_MIN"); return e ? atoi(e) : 5; }();
   // (rows that are not 16-byte aligned: the MMA kernel reads them with 2-byte loads; 5003 x 2816 Q6_K at 5 / 16 rows 21.3 / 25.2 us
   // there, 18.0 / 19.8 here; 1024 x 5376 13.0 / 14.6 there, 20.0 / 21.0 here)

@@ -135,14 +135,17 @@ int gemv_tile_max_batch(int qtype) {
   return qtype == QT_Q6_K ? 4 : tile::kMaxBatch;
 }
 
-bool gemv_tile_applicable(int qtype, int64_t N, int64_t K, int M, const void* w, const void* x) {
+// Every 16-row tile has an arrival counter in the counter area that the kernels share.
+static bool counters_fit(int64_t N) { return kWsCounterOffset + (size_t)((N + 15) / 16) * sizeof(int) <= kWsGemmPartialOffset; }
+
+bool gemv_tile_applicable(int qtype, int64_t N, int64_t K, int M, const void* w, const void* x, int sm_count) {
   tile::FormatInfo fi;
   if (!tile::format_of(qtype, &fi)) return false;
-  if (M < 1 || M > gemv_tile_max_batch(qtype) || K <= 0 || K % 256 || N < 1 || N > (1ll << 24)) return false;
+  if (M < 1 || M > gemv_tile_max_batch(qtype) || K <= 0 || K % 256 || N < 1 || !counters_fit(N)) return false;
   if ((uintptr_t)w % 16 || (uintptr_t)x % 16 || (K * 2) % 16) return false;
   if (N * (K / 256 * fi.ts) >= (1ll << 31)) return false;      // block offsets are 32-bit inside a row; rows are 64-bit
   tile::Geo geo;
-  return tile::plan(fi, N, K, M, 148, 0, 0, &geo);
+  return tile::plan(fi, N, K, M, sm_count, 0, 0, &geo);
 }
 
 // Scratch: one arrival counter per 16-row tile in the counter area every kernel shares, and two
@@ -150,7 +153,7 @@ bool gemv_tile_applicable(int qtype, int64_t N, int64_t K, int M, const void* w,
 // the plan may pick.
 size_t gemv_tile_workspace_bytes(int qtype, int64_t N, int64_t K, int M) {
   tile::FormatInfo fi;
-  if (!tile::format_of(qtype, &fi) || M < 1 || M > tile::kMaxBatch) return 0;
+  if (!tile::format_of(qtype, &fi) || M < 1 || M > tile::kMaxBatch || !counters_fit(N)) return 0;
   const int64_t RT = (N + 15) / 16;
   const int chunk = tile::min_chunk_sb(N, K);
   const int64_t C = (K / 256 + chunk - 1) / chunk;
@@ -168,7 +171,7 @@ cudaError_t gemv_tile(int qtype, const uint8_t* w, int64_t N, int64_t K, const v
   if (!plan(fi, N, K, M, sm_count, forced_nb(), forced_chunk(), &geo) && !plan(fi, N, K, M, sm_count, 0, 0, &geo))
     return cudaErrorInvalidValue;
   if (!ws || ws_bytes < gemv_tile_workspace_bytes(qtype, N, K, M) || (uintptr_t)ws % 256) return cudaErrorInvalidValue;
-  if (kWsCounterOffset + (size_t)geo.RT * sizeof(int) > kWsGemmPartialOffset) return cudaErrorInvalidValue;
+  if (!counters_fit(N)) return cudaErrorInvalidValue;
   static const bool debug = env_int("GGQ_TILE_DEBUG") != 0;     // prints the plan of every launch (a tuning aid)
   if (debug)
     fprintf(stderr, "gemv_tile qtype %d N=%lld K=%lld M=%d: nb=%d chunk=%d spu=%d C=%d RT=%d S=%lld W=%d depth=%d pitch=%d xbufs=%d smem=%d\n",

@@ -90,3 +90,13 @@ def test_workspace_sizes(built_lib):
     assert big == 0 or big >= (4 << 20) + 2 * 64 * 1024 * 4
     # many row tiles: one K range per tile, no scratch
     assert built_lib.ggq_workspace_bytes(int(QT.Q8_0), 148 * 128 * 4, 1024, 64) == 0
+
+
+def test_tiled_kernel_leaves_weights_with_more_row_tiles_than_counters(built_lib):
+    """The counter area holds 1015808 row tiles of 16 rows: beyond, the formats that need no scratch ask for none, so that
+    ggq_gemv goes to the kernels that use none."""
+    rows = ((4 << 20) - (128 << 10)) // 4 * 16
+    for qt in (QT.TQ1_0, QT.TQ2_0, QT.Q3_K):
+        for m in (1, 2):
+            assert built_lib.ggq_scratch_bytes(int(qt), rows, 256, m) > 4 << 20
+            assert built_lib.ggq_scratch_bytes(int(qt), rows + 1, 256, m) == built_lib.ggq_workspace_bytes(int(qt), rows + 1, 256, m) == 0

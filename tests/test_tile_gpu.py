@@ -180,3 +180,16 @@ def test_rows_at_every_offset_of_a_16_byte_piece(qtype):
             xb = synth.make_x(m, k, seed=m)
             got = kernels.fused_matmul(to_x(xb), w, out_dtype=torch.float32).cpu().numpy()[:, rows]
             assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb[rows], qtype)) <= 2e-5, (qtype.name, n, k, m)
+
+
+def test_more_row_tiles_than_arrival_counters():
+    """16252928 rows fill the counter area; a call beyond runs on the kernels without counters, also where scratch is at hand."""
+    n, k, qtype = 16252928 + 40, 256, QT.TQ1_0
+    w = synth.make_weight_on_device(n, k, qtype, seed=1, device="cuda")
+    rows = np.unique(np.concatenate([np.arange(50), np.random.default_rng(4).choice(n, 300), np.arange(n - 90, n)]))
+    wb = w.data[torch.from_numpy(rows).cuda()].cpu().numpy()
+    gj.matmul(to_x(synth.make_x(2, 4096, seed=1)), synth.make_weight(4096, 4096, QT.Q4_K, seed=1, device="cuda"))      # the stream has scratch
+    for m in (1, 2):
+        xb = synth.make_x(m, k, seed=m)
+        got = kernels.fused_matmul(to_x(xb), w, out_dtype=torch.float32)[:, torch.from_numpy(rows).cuda()].cpu().numpy()
+        assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb, qtype)) <= 2e-5, m
