@@ -7,8 +7,11 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
+import itertools
 import os
+import sys
 import threading
+import warnings
 
 import numpy as np
 
@@ -94,7 +97,35 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
-NATIVE_PATH = os.path.join(_HERE, "_native.so")
+def native_path() -> str:
+    """File of the native call path.  It is compiled against one Python's and one torch's C++ interface, so both are in its name:
+    a build for another one is not loaded."""
+    import torch
+
+    return os.path.join(_HERE, f"_native-{sys.implementation.cache_tag}-torch{torch.__version__}.so")
+
+
+class _PythonPath:
+    """In place of the native module where none was built for this Python and torch: every call takes the Python path, which
+    launches the same kernels."""
+
+    @staticmethod
+    def fast_matmul(*_):
+        return None
+
+    @staticmethod
+    def set_scratch(*_):
+        return None
+
+    @staticmethod
+    def capture_id(stream: int) -> int:
+        import torch
+
+        # not known which capture: no two calls are taken for the same one
+        return next(_capture_ids) if torch.cuda.is_current_stream_capturing() else 0
+
+
+_capture_ids = itertools.count(1)
 _native_module = None
 
 
@@ -105,14 +136,18 @@ def native():
         with _lock:
             if _native_module is None:
                 L = lib()
-                if not os.path.exists(NATIVE_PATH):
-                    raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m gguf_jax_b200.build`.")
-                spec = importlib.util.spec_from_file_location("_native", NATIVE_PATH)
-                module = importlib.util.module_from_spec(spec)
-                spec.loader.exec_module(module)
-                entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_fused_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info,
-                           L.ggq_dequant)
-                module.bind(*[ctypes.cast(f, ctypes.c_void_p).value for f in entries], int(L.ggq_gemv_max_batch()))
+                path = native_path()
+                try:
+                    spec = importlib.util.spec_from_file_location("_native", path)
+                    module = importlib.util.module_from_spec(spec)
+                    spec.loader.exec_module(module)
+                except ImportError as e:
+                    warnings.warn(f"matmul takes its slower Python call path: {e} (build it with `python -m gguf_jax_b200.build`)")
+                    module = _PythonPath
+                else:
+                    entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_fused_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info,
+                               L.ggq_dequant)
+                    module.bind(*[ctypes.cast(f, ctypes.c_void_p).value for f in entries], int(L.ggq_gemv_max_batch()))
                 _native_module = module
     return _native_module
 

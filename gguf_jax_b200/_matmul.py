@@ -73,8 +73,12 @@ def fused_batch_limit(w: QuantizedArray) -> int:
 def _native_matmul(*args):
     """First call: load the native module, then be replaced by its function."""
     global _native_matmul
-    _native_matmul = _lib.native().fast_matmul
-    return _native_matmul(*args)
+    try:
+        fn = _lib.native().fast_matmul
+    except RuntimeError:            # no library: the Python path says so, behind its checks of the arguments
+        return None
+    _native_matmul = fn
+    return fn(*args)
 
 
 def _validate(x: torch.Tensor, w) -> None:

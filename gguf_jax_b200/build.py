@@ -14,7 +14,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "libggq_b200.so")
-NATIVE = os.path.join(HERE, "_native.so")      # the native call path (csrc/torch_call.cpp)
 
 SOURCES = ["capi.cu", "dequant.cu", "gemv.cu", "gemv_generic.cu", "gemv_stream.cu", "gemv_q4k.cu", "gemv_q5k.cu", "gemv_q6k.cu", "gemm_tcgen05.cu", "gemv_mma.cu", "gemv_tile.cu", "gemv_tile_k.cu", "gemv_tile_iq.cu", "gemv_tile_b32.cu", "gemv_wide.cu", "gemm_codes.cu", "gemm_bf16w.cu"]
 
@@ -75,24 +74,27 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_native(force: bool = False) -> str:
-    """Compile csrc/torch_call.cpp, the native call path of ``matmul``, into _native.so next to the library."""
+    """Compile csrc/torch_call.cpp, the native call path of ``matmul``, next to the library; the file's name says for which
+    Python and torch."""
     import sysconfig
 
     import torch
     from torch.utils import cpp_extension
 
-    src = os.path.join(CSRC, "torch_call.cpp")
-    if force or _stale(NATIVE, [src]):
+    from gguf_jax_b200 import _lib
+
+    src, native = os.path.join(CSRC, "torch_call.cpp"), _lib.native_path()
+    if force or _stale(native, [src]):
         cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
         torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
         include = [sysconfig.get_paths()["include"], *cpp_extension.include_paths("cuda")]
         cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", *[f"-I{d}" for d in include],
-               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", src, "-o", NATIVE, f"-L{torch_lib}",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", src, "-o", native, f"-L{torch_lib}",
                "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{torch_lib}"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"torch_call.cpp failed to compile:\n{r.stdout}\n{r.stderr}")
-    return NATIVE
+    return native
 
 
 def build_xla_ffi(verbose: bool = False) -> str | None:
