@@ -9,7 +9,8 @@
 // The dense route (decode, library GEMM) is two launches for which the Python path spent 50 us; here 15 to 20.
 //
 // The library's entry points are handed over as addresses (bind), so that this module follows whichever
-// libggq_b200.so the binding has loaded.  All state is guarded by the interpreter lock.
+// libggq_b200.so the binding has loaded.  All state is guarded by the interpreter lock, which is not held while
+// memory is allocated and kernels are launched: either may wait for the device, and other threads run meanwhile.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -58,6 +59,11 @@ struct Shape {
 };
 std::array<Shape, 1024> g_shapes;
 
+struct WithoutGil {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 const Shape* shape_of(int32_t qtype, int64_t n, int64_t k, int32_t m) {
   uint64_t h = (uint64_t)n * 0x9E3779B97F4A7C15ull ^ (uint64_t)k * 0xC2B2AE3D27D4EB4Full ^ (uint64_t)m * 0x165667B19E3779F9ull ^ (uint64_t)qtype << 32;
   Shape& s = g_shapes[(h >> 40) % g_shapes.size()];
@@ -76,8 +82,7 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (nargs != 6 || !g_gemv || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1]) || !PyTuple_CheckExact(args[3]) ||
       PyTuple_GET_SIZE(args[3]) != 2)
     Py_RETURN_NONE;
-  const at::Tensor& x = THPVariable_Unpack(args[0]);
-  const at::Tensor& w = THPVariable_Unpack(args[1]);
+  const at::Tensor x = THPVariable_Unpack(args[0]), w = THPVariable_Unpack(args[1]);
   // plain strided CUDA tensors on the current device only; whatever wraps, records or transforms takes the Python path
   if (!x.defined() || !w.defined() || !x.is_cuda() || !w.is_cuda() || x.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kByte ||
       x.layout() != at::kStrided || w.layout() != at::kStrided || x.dim() < 1 || x.device() != w.device() || !w.is_contiguous() ||
@@ -94,29 +99,42 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (m < 1 || m > 65536) Py_RETURN_NONE;
   const int force = PyObject_IsTrue(args[4]);      // any truth value, as in the Python path
   if (force < 0) { PyErr_Clear(); Py_RETURN_NONE; }
-  const Shape* s = shape_of((int32_t)qtype, n, k, (int32_t)m);
-  if (!s || (size_t)w.numel() != s->payload) Py_RETURN_NONE;
+  const Shape* known = shape_of((int32_t)qtype, n, k, (int32_t)m);
+  if (!known || (size_t)w.numel() != known->payload) Py_RETURN_NONE;
+  const Shape s = *known;                  // another thread may take its place in the table
   const auto stream = c10::cuda::getCurrentCUDAStream(dev);
   c10::SmallVector<int64_t, 6> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = n;
-  if (m > s->limit && !force) {
+  if (m > s.limit && !force) {
     // the dense route in one piece: decode to bf16, library GEMM (rows of the result on 16-byte boundaries)
     const double budget = PyFloat_AsDouble(args[5]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
     if (n % 8 || 4.0 * (double)n * (double)k > budget) Py_RETURN_NONE;
-    const at::Tensor dense = at::empty({n, k}, x.options().requires_grad(false));
-    if (g_dequant((int32_t)qtype, w.data_ptr(), s->blocks, dense.data_ptr(), kBf16, stream.stream()) != 0) Py_RETURN_NONE;
-    return THPVariable_Wrap(at::mm(x.reshape({m, k}), dense.t()).view(sizes));
+    at::Tensor y;
+    {
+      WithoutGil no_gil;
+      const at::Tensor dense = at::empty({n, k}, x.options().requires_grad(false));
+      if (g_dequant((int32_t)qtype, w.data_ptr(), s.blocks, dense.data_ptr(), kBf16, stream.stream()) == 0)
+        y = at::mm(x.reshape({m, k}), dense.t()).view(sizes);
+    }
+    if (!y.defined()) Py_RETURN_NONE;
+    return THPVariable_Wrap(std::move(y));
   }
   const auto it = g_scratch.find({dev, (uintptr_t)stream.stream()});
   // no scratch yet on this stream (its first call also uploads the code books), or one that has to grow
-  if (it == g_scratch.end() || (size_t)it->second.numel() < s->scratch) Py_RETURN_NONE;
+  if (it == g_scratch.end() || (size_t)it->second.numel() < s.scratch) Py_RETURN_NONE;
   // a graph that is being captured keeps the scratch's address: the Python path notes that
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) Py_RETURN_NONE;
-  const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
-  at::Tensor y = at::empty(sizes, x.options().requires_grad(false));
-  const int32_t rc = (m <= g_gemv_max ? g_gemv : g_gemm)((int32_t)qtype, w.data_ptr(), n, k, xc.data_ptr(), (int32_t)m, y.data_ptr(), kBf16,
-                                                         it->second.data_ptr(), (size_t)it->second.numel(), stream.stream());
+  const at::Tensor scratch = it->second;
+  at::Tensor y;
+  int32_t rc;
+  {
+    WithoutGil no_gil;
+    const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+    y = at::empty(sizes, x.options().requires_grad(false));
+    rc = (m <= g_gemv_max ? g_gemv : g_gemm)((int32_t)qtype, w.data_ptr(), n, k, xc.data_ptr(), (int32_t)m, y.data_ptr(), kBf16,
+                                             scratch.data_ptr(), (size_t)scratch.numel(), stream.stream());
+  }
   if (rc != 0) Py_RETURN_NONE;         // the Python path repeats the call and raises its error
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS

@@ -1,5 +1,8 @@
 """The native call path of `matmul` against the Python path it stands for: same results for every form of activations, and the
 forms it must leave alone (gradients, host memory, transforms, subclasses, shapes and batches outside the fused route)."""
+import threading
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -181,3 +184,35 @@ def test_a_graph_replays_after_the_streams_scratch_has_grown():
     torch.cuda.synchronize()
     assert torch.equal(y, want) and torch.equal(grown, again)
     assert all(bool((t == 7).all()) for t in others)
+
+
+@pytest.mark.parametrize("m", [1, 40], ids=["fused", "dense"])
+def test_other_threads_run_while_a_call_waits_for_the_device(m):
+    """A launch waits once about a thousand are queued behind a busy kernel (a second here).  A thread that only looks at the clock
+    must not be held up for that long."""
+    w = synth.make_weight(96, 2048, QT.Q4_K, seed=10, device="cuda")
+    x = torch.randn((m, 2048), device="cuda").bfloat16()
+    gj.matmul(x, w)
+    torch.cuda.synchronize()
+    stop, gaps = threading.Event(), [0.0]
+
+    def watch():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps[0] = max(gaps[0], now - last)
+            last = now
+
+    watcher = threading.Thread(target=watch)
+    watcher.start()
+    start = time.perf_counter()
+    torch.cuda._sleep(2_000_000_000)               # about a second at 1.9 GHz
+    for _ in range(3000):
+        gj.matmul(x, w)
+    issued = time.perf_counter() - start
+    stop.set()
+    watcher.join()
+    torch.cuda.synchronize()
+    assert issued > 0.5, "the queue never filled: nothing was tested"
+    assert gaps[0] < 0.25, gaps[0]
