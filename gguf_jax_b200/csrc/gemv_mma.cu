@@ -18,6 +18,7 @@
 // in practice bound by the decode + split instruction count (about 10 per weight).
 #include "ggq_decode.cuh"
 #include "gemv.cuh"
+#include "recompute.cuh"
 
 namespace ggq {
 namespace mmav {
@@ -76,6 +77,9 @@ gemv_mma_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16
 #pragma unroll
     for (int i = 0; i < 4; i++) acc[c][i] = 0.f;
 
+  // four steps' loads in flight, stated: how far the compiler unrolled by itself changed with unrelated code behind the loop
+  // (Q2_K 4096 x 4096 at 16 rows between 18.5 and 23.1 us)
+#pragma unroll 4
   for (int s = warp; s < n_steps; s += kWarps) {
     const int e = 32 * s + 8 * t;                       // this lane's eight weights of the step
     const int64_t boff = (int64_t)(e / BS) * TS;
@@ -113,10 +117,10 @@ gemv_mma_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16
     for (int ww = 0; ww < kWarps; ww++) sum += red[ww][c][i][ln];
     const int row = n0 + (ln >> 2) + 8 * (i >> 1);
     const int m = 8 * c + 2 * (ln & 3) + (i & 1);
-    if (row < N && m < M) {
-      if (!(fabsf(sum) <= 3.402823466e38f)) sum = exact_dot<QT>(w + row * row_bytes, x + (int64_t)m * K, K, tab);
-      store_out(y, y_dtype, (int64_t)m * N + row, sum);
-    }
+    const bool mine = row < N && m < M;
+    if (mine) store_out(y, y_dtype, (int64_t)m * N + row, sum);
+    const bool bad = mine && not_finite(sum);
+    if (__any_sync(0xFFFFFFFFu, bad)) recompute<QT>(bad, row, m, w, row_bytes, N, x, K, tab, y, y_dtype);
   }
 }
 

@@ -36,6 +36,7 @@
 
 #include "gemv.cuh"
 #include "ggq_decode.cuh"
+#include "recompute.cuh"
 #include "tile_formats.cuh"
 
 namespace ggq {
@@ -391,12 +392,11 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
   constexpr int kGroups = F::kOct / F::kGroupOct;
   const int total_steps = geo.C * spu;            // arrivals that complete a row tile
 
-  auto emit = [&](int row, int m, float val) {
-    if (pp.world == 0) {
-      if (!(fabsf(val) <= 3.402823466e38f)) val = exact_dot<F::kQt>(w + row * row_bytes, x + (int64_t)m * K, K, tab);
-      store_out(y, y_dtype, (int64_t)m * N + row, val);
-    }
-    else peer_emit(pp, y, y_dtype, row, val, out_tag);
+  // stores an output; true if it has to be recomputed
+  auto emit = [&](int row, int m, float val) -> bool {
+    if (pp.world != 0) { peer_emit(pp, y, y_dtype, row, val, out_tag); return false; }
+    store_out(y, y_dtype, (int64_t)m * N + row, val);
+    return not_finite(val);
   };
   // Completion of a row tile: whoever brings its step count to C * spu adds the 2 C slots in order.
   int pend_rt = -1, pend_steps = 0, pend_old = 0;
@@ -416,10 +416,16 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
         }
       }
       const int idx0 = lane * kPer;
+      uint32_t bad = 0;
 #pragma unroll
       for (int i = 0; i < kPer; i++) {
         const int row = pend_rt * 16 + (idx0 + i) / XR, m = (idx0 + i) % XR;
-        if (row < N && m < M) emit(row, m, sum[i]);
+        if (row < N && m < M) bad |= (uint32_t)emit(row, m, sum[i]) << i;
+      }
+      if (__any_sync(0xFFFFFFFFu, bad)) {
+#pragma unroll 1
+        for (int i = 0; i < kPer; i++)
+          recompute<F::kQt>((bad >> i) & 1, pend_rt * 16 + (idx0 + i) / XR, (idx0 + i) % XR, w, row_bytes, N, x, K, tab, y, y_dtype);
       }
       if (lane == 0) counters[pend_rt] = 0;
     }
@@ -539,15 +545,21 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
           }
         }
         if (geo.C == 1 && whole) {
+          uint32_t bad = 0;
           if (t == 0) {
 #pragma unroll
             for (int p = 0; p < MP; p++) {
 #pragma unroll
               for (int q = 0; q < 4; q++) {
                 const int row = rt * 16 + g + 8 * (q >> 1), m = 2 * p + (q & 1);
-                if (row < N && m < M) emit(row, m, v[p][q]);
+                if (row < N && m < M) bad |= (uint32_t)emit(row, m, v[p][q]) << (4 * p + q);
               }
             }
+          }
+          if (__any_sync(0xFFFFFFFFu, bad)) {
+#pragma unroll 1
+            for (int i = 0; i < 4 * MP; i++)
+              recompute<F::kQt>((bad >> i) & 1, rt * 16 + g + 8 * ((i & 3) >> 1), 2 * (i >> 2) + (i & 1), w, row_bytes, N, x, K, tab, y, y_dtype);
           }
         } else {
           float* sl = slots + (((int64_t)c * RT + rt) * 2) * 16 * XR;

@@ -463,23 +463,5 @@ inline bool dispatch_block_qtype(int qtype, F&& f) {
   }
 }
 
-// One output element the plain way: float32 weights of the block decoders times the activations, in order.  The kernels on
-// the tensor cores take a weight apart (into codes and multiples of sum(x), or into three bf16 terms of which the last are
-// often zero), so an activation or a scale that is infinite, or a sum that leaves the float32 range on the way, makes
-// their result NaN where the product of the decoded weights is not: such an element is recomputed here.  One lane walks the
-// row; nothing else ever calls it.
-template <int QT>
-__device__ __noinline__ float exact_dot(const uint8_t* wrow, const __nv_bfloat16* xrow, int K, const uint8_t* tab) {
-  constexpr int BS = block_elems_of(QT), TS = block_bytes_of(QT);
-  float acc = 0.f;
-  for (int e = 0; e < K; e += 8) {
-    float v[8];
-    Dec<QT>::run(wrow + (int64_t)(e / BS) * TS, (e % BS) >> 3, tab, v);
-#pragma unroll
-    for (int i = 0; i < 8; i++) acc = fmaf(v[i], __bfloat162float(xrow[e + i]), acc);
-  }
-  return acc;
-}
-
 }  // inline namespace
 }  // namespace ggq

@@ -193,3 +193,38 @@ def test_more_row_tiles_than_arrival_counters():
         xb = synth.make_x(m, k, seed=m)
         got = kernels.fused_matmul(to_x(xb), w, out_dtype=torch.float32)[:, torch.from_numpy(rows).cuda()].cpu().numpy()
         assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb, qtype)) <= 2e-5, m
+
+
+@pytest.mark.parametrize("n", [40, 2056])
+@pytest.mark.parametrize("qtype", TILE_SMALL_BLOCKS + [QT.Q2_K, QT.IQ4_XS, QT.IQ2_XS, QT.IQ1_S], ids=lambda t: t.name)
+def test_a_nan_activation_stays_in_its_batch_row(qtype, n):
+    k, m = 2048, 9
+    wb = synth.make_weight_bytes(n, k, qtype, seed=6)
+    xb = synth.make_x(m, k, seed=6)
+    xb[3, 1999] = xb[8, 0] = np.nan
+    got = kernels.fused_matmul(to_x(xb), on_device(wb, qtype, n, k), out_dtype=torch.float32).cpu().numpy()
+    assert np.isnan(got[[3, 8]]).all()
+    rest = [r for r in range(m) if r not in (3, 8)]
+    assert O.rel_l2(got[rest], O.c_matmul(O.bf16_bits(xb[rest]), wb, qtype)) <= 2e-5, qtype.name
+
+
+@pytest.mark.parametrize("qtype,n,k,m", [(QT.IQ3_S, 14336, 4096, 4), (QT.Q8_0, 14336, 4096, 16), (QT.Q4_K, 14336, 4096, 4)], ids=str)
+def test_a_batch_row_that_is_not_finite_does_not_hold_up_the_others(qtype, n, k, m):
+    """All outputs of a batch row with a NaN are recomputed; one lane per output took 5 to 32 times the whole product."""
+    w = synth.make_weight_on_device(n, k, qtype, seed=1, device="cuda")
+    x = to_x(synth.make_x(m, k, seed=1))
+    bad = x.clone()
+    bad[0, 77] = float("nan")
+    times = []
+    for a in (x, bad):
+        for _ in range(3):
+            gj.matmul(a, w)
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda._sleep(2_000_000)          # so that the calls are queued when the first one starts
+        begin.record()
+        for _ in range(20):
+            gj.matmul(a, w)
+        end.record()
+        end.synchronize()
+        times.append(begin.elapsed_time(end) / 20)
+    assert times[1] <= 3 * times[0], times
