@@ -94,9 +94,14 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
         g.xbufs = bufs;
         const int fixed = bufs * x_rows * (g.x_row_bytes + g.xs_row_floats * 4) + 64 + (fi.table_bytes + 15) / 16 * 16 + 64 * kMaxXBufs;
         const int room = kSmemLimit - fixed;
-        if (span_ok && room >= 2 * kWarps * g.slot_bytes) {
-          g.depth = std::min(kMaxDepth, room / (kWarps * g.slot_bytes));
-          g.off_x = kWarps * g.depth * g.slot_bytes;
+        // a ring of two slots at least; a warp that has a single step fills one (the tables of the grid formats leave no room for
+        // two slots of four superblocks, and the split into smaller steps took longer: IQ2_XXS 8192 x 4096 at 8 rows 24.8 us, 22)
+        const int64_t warp_steps = (g.S + g.W - 1) / g.W;
+        const int fit = room / (kWarps * g.slot_bytes);
+        if (span_ok && fit >= std::min<int64_t>(2, warp_steps)) {
+          g.depth = std::min(kMaxDepth, std::max(2, fit));
+          g.slots = (int)std::min<int64_t>(g.depth, warp_steps);
+          g.off_x = kWarps * g.slots * g.slot_bytes;
           g.off_xs = g.off_x + bufs * x_rows * g.x_row_bytes;
           g.off_zero = g.off_xs + bufs * x_rows * g.xs_row_floats * 4;
           g.off_tab = g.off_zero + 64;
@@ -105,7 +110,7 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
           // time ~ steps of the busiest warp x (blocks per step + a fixed cost per step) + staging + a flush per
           // unit, in units of one block's multiply; the constants are fitted to B200 timings (8192 x 28672:
           // nb = 2 with chunks of 16 superblocks is the fastest split for every format)
-          const double steps = (double)((g.S + g.W - 1) / g.W);
+          const double steps = (double)warp_steps;
           const double cost = steps * (nb + 0.6) * (g.depth >= 3 ? 1.0 : 1.03) + bufs * g.chunk_sb * x_rows * 0.02 + steps / g.spu * 0.6;
           if (cost < best_cost) { best_cost = cost; best = g; }
         }

@@ -57,7 +57,8 @@ struct Geo {
   int C, RT;             // chunks per row, 16-row tiles
   int64_t S;             // warp steps in all = C * RT * spu
   int W;                 // warps that take part (each gets a contiguous range of at least one unit)
-  int depth, pitch, slot_bytes;
+  int depth, pitch, slot_bytes;     // ring: steps in flight, bytes per row and per step
+  int slots;             // slots in memory: depth, or fewer where no warp has that many steps
   int xbufs;             // chunk buffers: the most adjacent chunks the warps of one CTA touch
   int x_rows;            // staged batch rows = 2 * passes (rows >= M are zero)
   int x_row_bytes;       // staged bytes per batch row and chunk, padded to 64 (mod 128)
@@ -155,6 +156,15 @@ __device__ __forceinline__ void q4k_block_m1(uint32_t blk0, uint32_t blk1, int t
   out1 = fmaf(dlb, hi[3], out1); out1 = fmaf(dmb, sx1, out1);
 }
 
+// How the grid's interleaved copies are dealt to the threads: 16-byte pieces (2 or 4 copies of an entry, which are the same).
+template <class F, bool GRID = (F::kTableBytes > 0 && tf::KvOf<F>::value == 0)>
+struct GridFill { static constexpr int kRounds = 1; };
+template <class F>
+struct GridFill<F, true> {
+  static constexpr int kPieces = F::kEntryBytes * F::kCopies / 16, kRounds = F::kEntries * kPieces / kThreads;
+  static_assert(F::kEntries * kPieces % kThreads == 0, "every thread fills the same number of pieces");
+};
+
 template <class F, int MP>
 __global__ void __launch_bounds__(kThreads, 1)
 gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
@@ -189,7 +199,7 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
 
   // ---- copy side
   const uint32_t smem_base = smem_u32(smem);
-  const uint32_t my_ring = smem_base + warp * (depth * geo.slot_bytes);
+  const uint32_t my_ring = smem_base + warp * (geo.slots * geo.slot_bytes);
   const int hl = lane >> 4, kl = lane & 15;
   int issued = 0, slot_i = 0;
   int c_i = c0, rt_i = rt0, k_i = k0;
@@ -247,21 +257,35 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
     }
     cp_async_commit();
   };
-  for (int d = 0; d < depth - 1; d++) issue_next();
 
-  // ---- shared-memory tables (immutable inputs: may be read before the previous kernel has finished)
+  // ---- shared-memory tables (immutable inputs: may be read before the previous kernel has finished).  A thread's share of the grid
+  // is loaded before the first weights are asked for, all of it at once: behind them, and in rounds, the copies of the grid took
+  // longer to set up than they save on smaller weights (6144 x 4096 at batch 1, us: one copy of the grid IQ2_S 12.4, IQ2_XS 13.0;
+  // copies filled behind the weights 14.3, 14.1; this way 11.0, 10.8).
   tf::Tables tb{};
-  if constexpr (F::kTableBytes > 0 && tf::KvOf<F>::value == 0) {
-    // kCopies interleaved copies of every entry; a thread writes 16-byte pieces (2 or 4 copies, which are the same)
-    constexpr int kEW = F::kEntryBytes / 4, kPieces = F::kEntryBytes * F::kCopies / 16;
+  constexpr bool kGrid = F::kTableBytes > 0 && tf::KvOf<F>::value == 0;
+  [[maybe_unused]] uint32_t grid_v[GridFill<F>::kRounds][2];
+  if constexpr (kGrid) {
+    constexpr int kEW = F::kEntryBytes / 4;
     constexpr int kOff = F::kQt == QT_IQ1_S || F::kQt == QT_IQ1_M ? TAB_IQ1 : F::kQt == QT_IQ2_XXS ? TAB_IQ2_XXS :
                          F::kQt == QT_IQ2_XS ? TAB_IQ2_XS : F::kQt == QT_IQ2_S ? TAB_IQ2_S : F::kQt == QT_IQ3_XXS ? TAB_IQ3_XXS : TAB_IQ3_S;
-    tb.grid = smem_base + geo.off_tab + (lane % F::kCopies) * F::kEntryBytes;
     const uint32_t* src = reinterpret_cast<const uint32_t*>(tab + kOff);
+#pragma unroll
+    for (int j = 0; j < GridFill<F>::kRounds; j++) {
+      const int e = (tid + j * kThreads) / GridFill<F>::kPieces;
+      if constexpr (kEW == 2) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(src) + e);
+        grid_v[j][0] = v.x; grid_v[j][1] = v.y;
+      } else grid_v[j][0] = grid_v[j][1] = __ldg(src + e);
+    }
+  }
+  for (int d = 0; d < depth - 1; d++) issue_next();
+  if constexpr (kGrid) {
+    tb.grid = smem_base + geo.off_tab + (lane % F::kCopies) * F::kEntryBytes;
     uint4* dst = reinterpret_cast<uint4*>(smem + geo.off_tab);
-    for (int i = tid; i < F::kEntries * kPieces; i += kThreads) {
-      const int e = i / kPieces;
-      uint32_t v[2] = {__ldg(src + e * kEW), __ldg(src + e * kEW + (kEW - 1))};
+#pragma unroll
+    for (int j = 0; j < GridFill<F>::kRounds; j++) {
+      uint32_t v[2] = {grid_v[j][0], grid_v[j][1]};
       if constexpr (F::kQt == QT_IQ1_S || F::kQt == QT_IQ1_M) {
         // int8 grid {-1, 0, 1} -> code bytes 8 * grid + 9
 #pragma unroll
@@ -270,7 +294,7 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
           v[h] = 0x09090909u - 8u * neg + 8u * pos;
         }
       }
-      dst[i] = make_uint4(v[0], v[1], v[0], v[1]);
+      dst[tid + j * kThreads] = make_uint4(v[0], v[1], v[0], v[1]);
     }
     if constexpr (F::kSignTable) {
       constexpr int kGridBytes = F::kEntries * F::kEntryBytes * F::kCopies;
