@@ -494,7 +494,7 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
       }
       for (int blk = 0; blk < (q4k_fast ? 0 : nbh); blk++) {
         const tf::BlockLd ld0{tile + skew0 + blk * F::kTs}, ld1{tile + skew1 + blk * F::kTs + 8 * pitch};
-        constexpr bool kLean = MP == 4 && tf::SignBitsOf<F>::value != 0;
+        constexpr bool kLean = MP == 4 && tf::LeanOf<F>::value;
         typename F::Run run0, run1;
         if constexpr (!kLean) { run0 = F::load_run(ld0, t); run1 = F::load_run(ld1, t); }
         const uint32_t xr = xr0 + blk * x_blk;

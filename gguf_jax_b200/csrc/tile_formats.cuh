@@ -37,7 +37,7 @@
 //   kKv                 16-entry code book behind a table of its byte pairs: absent / 0 none, 1 IQ4 values + 128,
 //                       2 MXFP4 values + 12
 //   kScaleExp           the group scales carry 2^kScaleExp (taken back out of the row sums; 0 where the trait is absent)
-//   load_group_lean(ld, t, grp)   the group straight from the block, nothing kept for the run (absent: load_run only).  At
+//   kLean, load_group_lean(ld, t, grp)   the group straight from the block, nothing kept for the run (absent: load_run only).  At
 //                       four passes the registers and, for the signs, the shared-memory pipe are what is short: there the
 //                       groups are loaded one at a time inside a real loop and octet<false> works the signs out
 //   octet(group, q, tab, p)   the four A-operand registers of octet q of the group: p[0], p[1] = first
@@ -221,8 +221,8 @@ struct NoRun {};
 // Optional members of a format.
 template <class F, class = void> struct KvOf { static constexpr int value = 0; };
 template <class F> struct KvOf<F, decltype((void)F::kKv)> { static constexpr int value = F::kKv; };
-template <class F, class = void> struct SignBitsOf { static constexpr int value = 0; };
-template <class F> struct SignBitsOf<F, decltype((void)F::kSignBits)> { static constexpr int value = F::kSignBits; };
+template <class F, class = void> struct LeanOf { static constexpr bool value = false; };
+template <class F> struct LeanOf<F, decltype((void)F::kLean)> { static constexpr bool value = F::kLean; };
 template <class F, class = void> struct ScaleExpOf { static constexpr int value = 0; };
 template <class F> struct ScaleExpOf<F, decltype((void)F::kScaleExp)> { static constexpr int value = F::kScaleExp; };
 
@@ -524,6 +524,7 @@ TF_HD void plain_octet(uint32_t w0, uint32_t w1, uint32_t (&p)[4]) {
 // IQ2_XXS (66 B: d, 8 x {4 index bytes, u32 = 4 x 7-bit sign index | 4-bit scale << 28}); group = one of them
 struct IQ2XXS {
   static constexpr int kQt = 16, kTs = 66, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 256, kEntryBytes = 8, kCopies = 16, kSignBits = 7;
   static constexpr bool kSignTable = true;
@@ -559,6 +560,7 @@ struct IQ2XXS {
 // IQ2_XS (74 B: d, 32 x u16 = 9-bit grid index | 7-bit sign index << 9, 8 scale bytes of two nibbles)
 struct IQ2XS {
   static constexpr int kQt = 17, kTs = 74, kAlign = 2, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
+  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 512, kEntryBytes = 8, kCopies = 16, kSignBits = 7;
   static constexpr bool kSignTable = true;
@@ -595,6 +597,7 @@ struct IQ2XS {
 // IQ2_S (82 B: d, 32 index bytes, 32 sign bytes, 8 bytes of 2 high index bits, 8 scale bytes)
 struct IQ2S {
   static constexpr int kQt = 22, kTs = 82, kAlign = 2, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
+  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 1024, kEntryBytes = 8, kCopies = 8, kSignBits = 8;
   static constexpr bool kSignTable = false;
@@ -635,6 +638,7 @@ struct IQ2S {
 // IQ3_XXS (98 B: d, 64 index bytes (one per 4 weights), 8 x u32 = 4 x 7-bit sign index | scale << 28)
 struct IQ3XXS {
   static constexpr int kQt = 18, kTs = 98, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 256, kEntryBytes = 4, kCopies = 32, kSignBits = 7;
   static constexpr bool kSignTable = true;
@@ -673,6 +677,7 @@ struct IQ3XXS {
 // IQ3_S (110 B: d, 64 index bytes, 8 bytes of ninth index bits, 32 sign bytes, 4 scale bytes of two nibbles)
 struct IQ3S {
   static constexpr int kQt = 21, kTs = 110, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 512, kEntryBytes = 4, kCopies = 16, kSignBits = 8;
   static constexpr bool kSignTable = true;
@@ -719,6 +724,7 @@ struct IQ3S {
 // fold removes the 9 and the factor 8:  (dl / 8) * (sum(code x) - 9 sum(x)).
 struct IQ1S {
   static constexpr int kQt = 19, kTs = 50, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
+  static constexpr bool kLean = true;
   static constexpr bool kSums = true, kUnrollGroups = true;
   static constexpr int kEntries = 2048, kEntryBytes = 8, kCopies = 4, kSignBits = 0;
   static constexpr bool kSignTable = false;
@@ -742,6 +748,17 @@ struct IQ1S {
     g.dl8 = mulf(r.d8, u2f(2 * ((g.qh >> 12) & 7) + 1));
     return g;
   }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    uint32_t qs[1];
+    ld.words<1, 2>(2 + 8 * t + 4 * grp, qs);
+    Group g;
+    g.qs = qs[0];
+    g.qh = ld.u16(34 + 4 * t + 2 * grp);
+    g.dlt = (g.qh & 0x8000) ? 0xFEFEFEFFu : 0x01010101u;
+    g.dl8 = mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.125f), u2f(2 * ((g.qh >> 12) & 7) + 1));
+    return g;
+  }
+  template <bool = false>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t idx = ((g.qs >> (8 * q)) & 0xFF) | (((g.qh >> (3 * q)) & 7) << 8);
     uint32_t w0, w1;

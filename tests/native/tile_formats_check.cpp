@@ -51,7 +51,7 @@ int check(const std::vector<uint8_t>& blocks, const float* want, const Tables& t
       const typename F::Run run = F::load_run(ld, t);
       for (int grp = 0; grp < F::kOct / F::kGroupOct; grp++) {
         const typename F::Group raw = F::load_group(ld, run, t, grp);
-        if constexpr (SignBitsOf<F>::value != 0) {       // the lean loader must give the same group
+        if constexpr (LeanOf<F>::value) {       // the lean loader must give the same group
           const typename F::Group lean = F::load_group_lean(ld, t, grp);
           for (int q = 0; q < F::kGroupOct; q++) {
             uint32_t pa[4], pb[4];
