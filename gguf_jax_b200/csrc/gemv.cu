@@ -62,18 +62,24 @@ static bool tile_scratch_is_optional(int qtype) {
 }
 
 // Where the tiled kernel and the two it competes with (streaming at batch 1, one MMA launch for 2..16 rows) cross, for every format
-// but the K-quants with kernels of their own.  The tiled kernel starts at 7 us (batch 1, 2) to 12 us (batch 8; a larger batch
-// is two launches) and grows slowly with the weight; the others start at 4 and 7 us and grow with their decoding.  Measured on B200,
-// us, other / tiled, at 2 / 8 / 16 / 56 / 128 M weights (M = 2^20):
-//   batch 1    Q4_0 4.4/7.0 6.3/7.6 9.8/8.5 27/17 52/27     Q8_0 4.4/7.3 6.4/7.8 9.8/10.0 27/21 51/35    IQ2_XS 5.1/7.8 7.9/9.7 11.9/11.1 32/20
-//   batch 4    Q4_0 7.0/8.5 11.6/10.4 13.8/10.4 40/19       IQ3_S 7.8/9.8 13.4/11.6 17.3/12.7 49/26
-//   batch 8    Q4_0 7.0/11.7 11.2/14.5 13.8/14.5 40/28      IQ4_XS 6.3/13.8 11.2/18.4 15.2/17.2 44/32 107/58
-//   batch 16   Q4_0 7.0/22 11.1/27 15.3/27 47/55 106/102    IQ2_XS 7.6/25 12.4/34 15.8/30 46/64 140/115   Q3_K 8.3/24 14.5/29 19/34 56/77 224/130
-static bool tile_pays(int qtype, int64_t weights, int M) {
+// but the K-quants with kernels of their own.  The tiled kernel cuts K over the warps of the whole device: it starts at 6 us
+// (batch 1, 2) to 11 us (batch 8; a larger batch is two launches, 20 us) and grows slowly with the weight.  The other two give a CTA
+// a few rows and all of K, so below about one CTA of 16 rows per SM (2368 rows) their time follows K, not the weight:
+// they are compared at K * max(N, 2368) weights; two launches of the tiled kernel with 13 rows or more only pay once the MMA kernel
+// has two CTAs per SM to work through.  Measured on B200 over 20 formats and 56 shapes of 0.25 to 130 M weights; with these
+// lines the kernel picked takes on average 0.2 % (batch 1), 0.2 % (2..4), 0.3 % (5..8), 1 to 1.6 % (9..16) longer than the better one
+// of the two, at worst 13 %, 20 %, 30 % and 71 % (Q5_1 16384 x 4096 at 16 rows).  us, other / tiled:
+//   batch 1    2048x2048 Q4_0 3.9/5.8 IQ2_XS 4.5/6.3   4096x4096 Q4_0 9.9/7.6 IQ2_XS 11.3/8.6 TQ1_0 12.3/10.0   512x14336 Q4_0 14/7.9 MXFP4 19/8.6
+//   batch 4    1024x1024 Q4_0 3.7/6.4 IQ3_S 4.4/7.5   4096x2048 Q4_0 8.0/7.8 IQ3_S 10.1/9.0   512x14336 Q4_0 30/12 Q8_0 46/13 IQ1_M 36/13
+//   batch 8    2048x2048 Q4_0 6.0/10.8 IQ3_S 7.3/10.9   4096x4096 Q4_0 16/13 Q3_K 20/15   512x14336 Q8_0 46/21 TQ1_0 31/22
+//   batch 9    4096x4096 Q4_0 19/21 MXFP4 20/25   8192x4096 Q4_0 30/27 Q8_0 29/38 IQ3_S 40/34   512x14336 Q4_0 37/32 IQ1_M 35/33
+//   batch 16   16384x4096 Q4_0 48/58 Q3_K 61/84   8192x14336 Q4_0 97/91 IQ3_S 135/104   512x14336 IQ2_XS 33/41 Q8_0 47/43
+static bool tile_pays(int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
   if (always) return true;
-  const int64_t from = M == 1 ? (qtype == QT_Q8_0 ? 16 : 12) : M <= 4 ? 4 : M <= 8 ? 18 : 96;
-  return weights >= from << 20;
+  const int64_t rows = M <= 12 ? 2368 : 4736;
+  const int64_t from = M == 1 ? 10 : M <= 4 ? 5 : M <= 8 ? 10 : M <= 12 ? 32 : 72;
+  return K * (N > rows ? N : rows) >= from << 20;
 }
 
 static size_t tile_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
@@ -166,8 +172,8 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them
   const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
   const int64_t weights = N * K;
-  const bool tile_first = k_quant ? (M >= 2 && M <= 4) || (M == 1 && (odd_rows ? tile_pays(qtype, weights, 1) : m1_tiled))
-                                  : tile_pays(qtype, weights, M);
+  const bool tile_first = k_quant ? (M >= 2 && M <= 4) || (M == 1 && (odd_rows ? tile_pays(N, K, 1) : m1_tiled))
+                                  : tile_pays(N, K, M);
   const int tile_max = gemv_tile_max_batch(qtype);
   const int tile_m = M < tile_max ? M : tile_max;
   const size_t tile_need = tile_max ? gemv_tile_workspace_bytes(qtype, N, K, tile_m) : 0;

@@ -76,3 +76,39 @@ def test_function_modes_see_the_operations(monkeypatch):
         assert gj.matmul(x, w) == "native"
         with Recorder(), pytest.raises(RuntimeError):
             gj.matmul(x, w)
+
+
+class Dispatched(torch.utils._python_dispatch.TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(func)
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("n,budget,padded", FORMS)
+def test_transforms_traces_and_modes_take_the_general_way(n, budget, padded, monkeypatch):
+    """Each of these fails, or computes something else, where a product is written into its columns of the result: there is no
+    batching rule and no derivative for a product with ``out=``, and a mode sees another operation."""
+    if padded:
+        monkeypatch.setattr(mm, "_PAD_FROM_OPS", 0)
+    w, x = case(n)
+    x = x.double()
+    dense = w.dequantize().double()
+    product = lambda a: gj.dequant_matmul(a, w, block_bytes=budget)
+    assert torch.allclose(product(x), x @ dense.T)
+    rows = torch.stack([x, 2 * x, -x])
+    assert torch.allclose(torch.func.vmap(product)(rows), rows @ dense.T)
+    assert torch.allclose(torch.func.vmap(product, in_dims=1, out_dims=1)(rows), rows @ dense.T)
+    t = torch.randn_like(x)
+    with torch.autograd.forward_ad.dual_level():
+        y = torch.autograd.forward_ad.unpack_dual(product(torch.autograd.forward_ad.make_dual(x, t)))
+    assert torch.allclose(y.primal, x @ dense.T) and torch.allclose(y.tangent, t @ dense.T)
+    traced = torch.jit.trace(product, (x,), check_trace=False)
+    assert torch.allclose(traced(3 * t), 3 * t @ dense.T)
+    with Dispatched() as mode:
+        y = product(x)
+    assert torch.ops.aten.mm.out not in mode.seen and torch.ops.aten.mm.default in mode.seen
+    assert torch.allclose(y, x @ dense.T)

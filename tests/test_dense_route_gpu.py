@@ -56,6 +56,7 @@ def test_transforms_take_the_general_way():
     x = torch.randn((4, 6, 512), device="cuda")
     dense = w.dequantize().float()
     budget = 4 * 512 * 32
-    mapped = torch.func.vmap(lambda a: gj.dequant_matmul(a, w, block_bytes=None))(x)
-    assert rel(mapped, x @ dense.T) <= 1e-5
+    for block_bytes in (None, budget):              # one slab; several, which plain tensors have written in place
+        mapped = torch.func.vmap(lambda a: gj.dequant_matmul(a, w, block_bytes=block_bytes))(x)
+        assert rel(mapped, x @ dense.T) <= 1e-5
     assert rel(gj.dequant_matmul(x, w, block_bytes=budget), x @ dense.T) <= 1e-5

@@ -1,4 +1,4 @@
-"""The tiled fused multiply (gemv_tile.cu: Q4_K, Q2_K, IQ4_XS and the IQ1/IQ2/IQ3 grid formats, batch 1..16)
+"""The tiled fused multiply (gemv_tile.cu, every block format, batch 1..16) and what takes its place on small weights
 against the CPU oracle on a B200, through the public wrappers / the C ABI.
 
 Bars: float32 output within 2e-5 relative L2 of the oracle's double-accumulated product (i.e. nothing
@@ -171,12 +171,13 @@ def test_activations_far_from_one_on_small_weights(qtype, exponent):
                                    QT.IQ1_M, QT.TQ1_0, QT.TQ2_0, QT.MXFP4], ids=lambda t: t.name)
 def test_rows_at_every_offset_of_a_16_byte_piece(qtype):
     """K = 256 times an odd number: consecutive rows start at different offsets modulo 16 for these formats.  Enough weights
-    for the tiled kernel at batch 1 and above 8 too (its rules count weights), the last row tile ragged."""
-    for n, k in [(3005, 11 * 256), (7001, 5 * 256)]:
+    for the tiled kernel up to batch 8 (its rule asks for 10 M), the last row tile ragged; two slices of such rows run where the
+    rule is off (test_tile_small_gpu.py), other kernels take batches 9 and 16 here."""
+    for n, k in [(5003, 11 * 256), (9001, 5 * 256)]:
         wb = synth.make_weight_bytes(n, k, qtype, seed=n)
         w = on_device(wb, qtype, n, k)
         rows = np.unique(np.concatenate([np.arange(40), np.random.default_rng(2).choice(n, 200), np.arange(n - 30, n)]))
-        for m in (1, 2, 4, 8):
+        for m in (1, 2, 4, 8, 9, 16):
             xb = synth.make_x(m, k, seed=m)
             got = kernels.fused_matmul(to_x(xb), w, out_dtype=torch.float32).cpu().numpy()[:, rows]
             assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb[rows], qtype)) <= 2e-5, (qtype.name, n, k, m)
@@ -208,6 +209,20 @@ def test_a_nan_activation_stays_in_its_batch_row(qtype, n):
     assert O.rel_l2(got[rest], O.c_matmul(O.bf16_bits(xb[rest]), wb, qtype)) <= 2e-5, qtype.name
 
 
+def milliseconds(x, w):
+    """Time of one product among twenty that are queued when the first one starts."""
+    for _ in range(3):
+        gj.matmul(x, w)
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    torch.cuda._sleep(2_000_000)
+    begin.record()
+    for _ in range(20):
+        gj.matmul(x, w)
+    end.record()
+    end.synchronize()
+    return begin.elapsed_time(end) / 20
+
+
 @pytest.mark.parametrize("qtype,n,k,m", [(QT.IQ3_S, 14336, 4096, 4), (QT.Q8_0, 14336, 4096, 16), (QT.Q4_K, 14336, 4096, 4)], ids=str)
 def test_a_batch_row_that_is_not_finite_does_not_hold_up_the_others(qtype, n, k, m):
     """All outputs of a batch row with a NaN are recomputed; one lane per output took 5 to 32 times the whole product."""
@@ -215,16 +230,16 @@ def test_a_batch_row_that_is_not_finite_does_not_hold_up_the_others(qtype, n, k,
     x = to_x(synth.make_x(m, k, seed=1))
     bad = x.clone()
     bad[0, 77] = float("nan")
-    times = []
-    for a in (x, bad):
-        for _ in range(3):
-            gj.matmul(a, w)
-        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        torch.cuda._sleep(2_000_000)          # so that the calls are queued when the first one starts
-        begin.record()
-        for _ in range(20):
-            gj.matmul(a, w)
-        end.record()
-        end.synchronize()
-        times.append(begin.elapsed_time(end) / 20)
+    times = [milliseconds(a, w) for a in (x, bad)]
     assert times[1] <= 3 * times[0], times
+
+
+@pytest.mark.parametrize("m", [1, 4, 8])
+def test_few_long_rows_are_not_left_to_few_ctas(m):
+    """The same number of weights in 512 rows and in 3584: the kernels that give a CTA whole rows took 3.1 to 4.2 times as long for
+    the 512, the tiled kernel takes 1.4 to 2."""
+    times = []
+    for n, k in ((512, 14336), (3584, 2048)):
+        w = synth.make_weight_on_device(n, k, QT.IQ3_S, seed=1, device="cuda")
+        times.append(milliseconds(to_x(synth.make_x(m, k, seed=1)), w))
+    assert times[0] <= 2.6 * times[1], times

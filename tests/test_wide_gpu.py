@@ -165,8 +165,8 @@ def test_benchmark_shape_sampled_rows(qtype):
 
 @pytest.mark.parametrize("n,k", [(5003, 11 * 256), (130, 3 * 256), (4100, 13 * 256)])
 def test_rows_that_are_not_16_byte_aligned(n, k):
-    """Q6_K with K no multiple of 2048: every row at its own offset of its copied window; same bar as above, and the refusal of
-    such rows where results go to peers stays."""
+    """Q6_K with K no multiple of 2048: every row at its own offset of its copied window; same bar as above.  Where results go to
+    peers such rows are refused, before anything is launched."""
     wb = synth.make_weight_bytes(n, k, QT.Q6_K, seed=n)
     w = gj.QuantizedArray.from_bytes(wb, QT.Q6_K, shape=(n, k), device="cuda")
     for m in (5, 8, 16, 17, 32):
@@ -174,3 +174,12 @@ def test_rows_that_are_not_16_byte_aligned(n, k):
         x = torch.from_numpy(xb).cuda().to(torch.bfloat16)
         got = kernels.fused_matmul(x, w, out_dtype=torch.float32).cpu().numpy()
         assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb, QT.Q6_K)) <= 2e-5, (n, k, m)
+    x, m = torch.zeros((8, k), dtype=torch.bfloat16, device="cuda"), 8
+    y, flags = torch.zeros((m, n), dtype=torch.bfloat16, device="cuda"), torch.zeros(3, dtype=torch.int32, device="cuda")
+    ws = torch.zeros(_lib.lib().ggq_workspace_bytes(int(QT.Q6_K), n, k, m), dtype=torch.uint8, device="cuda")
+    pointer = lambda t: (ctypes.c_void_p * 8)(t.data_ptr())
+    args = (pointer(y), pointer(flags), 1, 0, n, _lib.GGQ_BF16, 0, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert _lib.lib().ggq_gemm_sharded(int(QT.Q6_K), w.data.data_ptr(), n, k, x.data_ptr(), k, m, *args) == 4       # GGQ_UNSUPPORTED
+    assert b"16-byte aligned rows" in _lib.lib().ggq_last_error()
+    torch.cuda.synchronize()
+    assert not y.any() and not flags.any()
