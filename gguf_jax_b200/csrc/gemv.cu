@@ -169,11 +169,13 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   // the batch-major kernel takes the larger weights (Q4_K 8192 x 28672: 68 / 77 us at batch 8 / 16 against
   // 100 / 153 us) and the integer-code MMA kernel (gemv_mma.cu) the smaller ones (see wide_pays).
   const bool k_quant = is_k_quant(qtype);
-  // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them
+  // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them; streaming and
+  // MMA kernel against the tiled one cross where they do for the other formats (us, other / tiled: 512 x 1280 at 1 / 2 / 4 rows 3.3/6.5
+  // 4.6/6.6 4.6/8.2, 512 x 5376 8.4/7.4 12.5/7.6 12.9/10.1)
   const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
   const int64_t weights = N * K;
-  const bool tile_first = k_quant ? (M >= 2 && M <= 4) || (M == 1 && (odd_rows ? tile_pays(N, K, 1) : m1_tiled))
-                                  : tile_pays(N, K, M);
+  const bool tile_first = k_quant && !odd_rows ? (M >= 2 && M <= 4) || (M == 1 && m1_tiled)
+                                               : (!k_quant || M <= 4) && tile_pays(N, K, M);
   const int tile_max = gemv_tile_max_batch(qtype);
   const int tile_m = M < tile_max ? M : tile_max;
   const size_t tile_need = tile_max ? gemv_tile_workspace_bytes(qtype, N, K, tile_m) : 0;

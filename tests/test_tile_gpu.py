@@ -6,13 +6,15 @@ but float32 summation order separates them); bf16 output within 2e-3 relative L2
 elementwise rtol = 1e-2, atol = 1e-2 max|ref|; a one-hot activation returns the decoded weight times
 the activation exactly (for activations that are powers of two), at every position of a superblock; a launch
 is deterministic."""
+import os
+
 import numpy as np
 import pytest
 import torch
 from gguf.constants import GGMLQuantizationType as QT
 
 import gguf_jax_b200 as gj
-from gguf_jax_b200 import kernels, synth
+from gguf_jax_b200 import _lib, kernels, synth
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -243,3 +245,33 @@ def test_few_long_rows_are_not_left_to_few_ctas(m):
         w = synth.make_weight_on_device(n, k, QT.IQ3_S, seed=1, device="cuda")
         times.append(milliseconds(to_x(synth.make_x(m, k, seed=1)), w))
     assert times[0] <= 2.6 * times[1], times
+
+
+def microseconds_with_and_without_scratch(qtype, n, k, m):
+    """ggq_gemv with the scratch that lets every kernel run, and without, which leaves the kernels that need none."""
+    L = _lib.lib()
+    w = synth.make_weight_on_device(n, k, qtype, seed=1, device="cuda")
+    x, y = to_x(synth.make_x(m, k, seed=1)), torch.empty((m, n), dtype=torch.bfloat16, device="cuda")
+    ws = torch.zeros(L.ggq_scratch_bytes(int(qtype), n, k, m), dtype=torch.uint8, device="cuda")
+    _lib.ensure_tables(0)
+    best = [float("inf")] * 2
+    for _ in range(6):
+        for i, scratch in enumerate(((ws.data_ptr(), ws.numel()), (None, 0))):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(1_000_000)
+            begin.record()
+            for _ in range(40):
+                _lib.check(L.ggq_gemv(int(qtype), w.data.data_ptr(), n, k, x.data_ptr(), m, y.data_ptr(), _lib.GGQ_BF16, *scratch,
+                                      torch.cuda.current_stream().cuda_stream))
+            end.record()
+            end.synchronize()
+            best[i] = min(best[i], begin.elapsed_time(end) * 25)
+    return best
+
+
+@pytest.mark.skipif(os.environ.get("GGQ_TILE_ALWAYS") == "1", reason="about the size rule, which is off")
+@pytest.mark.parametrize("qtype,n,k,m", [(QT.Q6_K, 512, 1024, 2), (QT.Q6_K, 512, 1024, 4), (QT.Q6_K, 1024, 5 * 256, 3)], ids=str)
+def test_scratch_does_not_slow_small_calls_down(qtype, n, k, m):
+    """Small weights with unaligned rows took the tiled kernel, twice the time of the MMA kernel, where scratch was at hand."""
+    with_scratch, without = microseconds_with_and_without_scratch(qtype, n, k, m)
+    assert with_scratch <= 1.15 * without, (with_scratch, without)
