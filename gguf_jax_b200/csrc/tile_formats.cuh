@@ -39,7 +39,8 @@
 //   kScaleExp           the group scales carry 2^kScaleExp (taken back out of the row sums; 0 where the trait is absent)
 //   kLean, load_group_lean(ld, t, grp)   the group straight from the block, nothing kept for the run (absent: load_run only).  At
 //                       four passes the registers and, for the signs, the shared-memory pipe are what is short: there the
-//                       groups are loaded one at a time inside a real loop and octet<false> works the signs out
+//                       groups are loaded one at a time inside a real loop and octet<false> works the signs out (us at 8 rows, whole runs / group
+//                       by group: Q4_1 14336 x 4096 30.1 / 27.8, Q5_1 37.5 / 31.2, NVFP4 37.3 / 33.6 and 16384 x 8192 69.6 / 58.0)
 //   octet(group, q, tab, p)   the four A-operand registers of octet q of the group: p[0], p[1] = first
 //                       MMA (k-slot pairs 2t.. and 2t+8..), p[2], p[3] = second MMA
 //   fold(group, acc, xsum, out) -> float   out + the group's contribution given acc = sum(code * x)
@@ -987,15 +988,22 @@ struct Q41 {
   static constexpr int kQt = 3, kTs = 160, kAlign = 16, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
   static constexpr bool kSums = true, kUnrollGroups = true;
   static constexpr int kTableBytes = 0;
+  static constexpr bool kLean = true;
   struct Run { uint32_t w[10]; };
-  struct Group { const uint32_t* q; float d, m; };
+  struct Group { uint32_t q[4]; float d, m; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
   TF_HD static int x_exp(int, int) { return 0; }
   TF_HD static Run load_run(const BlockLd& ld, int t) { Run r; ld.words<10, 8>(40 * t, r.w); return r; }
   TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
-    const uint32_t h = r.w[5 * grp];
-    return Group{r.w + 5 * grp + 1, f16_bits_to_float(h & 0xFFFF), f16_bits_to_float(h >> 16)};
+    const uint32_t* w = r.w + 5 * grp;
+    return Group{{w[1], w[2], w[3], w[4]}, f16_bits_to_float(w[0] & 0xFFFF), f16_bits_to_float(w[0] >> 16)};
   }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    uint32_t w[5];
+    ld.words<5, 4>(40 * t + 20 * grp, w);
+    return Group{{w[1], w[2], w[3], w[4]}, f16_bits_to_float(w[0] & 0xFFFF), f16_bits_to_float(w[0] >> 16)};
+  }
+  template <bool = false>
   TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) { nibble_octet(g.q[q], p); }
   TF_HD static float fold(const Group& g, float acc, float xsum, float out) { return fmaf_(g.m, xsum, fmaf_(g.d, acc, out)); }
 };
@@ -1032,15 +1040,22 @@ struct Q51 {
   static constexpr int kQt = 7, kTs = 192, kAlign = 16, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
   static constexpr bool kSums = true, kUnrollGroups = true;
   static constexpr int kTableBytes = 0;
+  static constexpr bool kLean = true;
   struct Run { uint32_t w[12]; };
-  struct Group { const uint32_t* q; uint32_t h; float d, m; };
+  struct Group { uint32_t q[4], h; float d, m; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { nibble_src(t, oo, a, b); }
   TF_HD static int x_exp(int, int) { return 0; }
   TF_HD static Run load_run(const BlockLd& ld, int t) { Run r; ld.words<12, 16>(48 * t, r.w); return r; }
   TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
-    const uint32_t h = r.w[6 * grp];
-    return Group{r.w + 6 * grp + 2, r.w[6 * grp + 1], f16_bits_to_float(h & 0xFFFF), f16_bits_to_float(h >> 16)};
+    const uint32_t* w = r.w + 6 * grp;
+    return Group{{w[2], w[3], w[4], w[5]}, w[1], f16_bits_to_float(w[0] & 0xFFFF), f16_bits_to_float(w[0] >> 16)};
   }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    uint32_t w[6];
+    ld.words<6, 8>(48 * t + 24 * grp, w);
+    return Group{{w[2], w[3], w[4], w[5]}, w[1], f16_bits_to_float(w[0] & 0xFFFF), f16_bits_to_float(w[0] >> 16)};
+  }
+  template <bool = false>
   TF_HD static void octet(const Group& g, int q, const Tables&, uint32_t (&p)[4]) { nibble5_octet(g.q[q], g.h >> (4 * q), p); }
   TF_HD static float fold(const Group& g, float acc, float xsum, float out) { return fmaf_(g.m, xsum, fmaf_(g.d, acc, out)); }
 };
@@ -1090,8 +1105,9 @@ struct NVFP4 {
   static constexpr int kQt = 40, kTs = 144, kAlign = 16, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 1, kKv = 2;
   static constexpr bool kSums = true, kUnrollGroups = true;
   static constexpr int kTableBytes = kByteTableBytes;
+  static constexpr bool kLean = true;
   struct Run { uint32_t w[9]; };
-  struct Group { const uint32_t* q; float d; };
+  struct Group { uint32_t q[2]; float d; };
   TF_HD static void src_quads(int t, int oo, int& a, int& b) { a = 64 * t + 16 * (oo >> 1) + 4 * (oo & 1); b = a + 8; }
   TF_HD static int x_exp(int, int) { return 0; }
   TF_HD static Run load_run(const BlockLd& ld, int t) { Run r; ld.words<9, 4>(36 * t, r.w); return r; }
@@ -1102,8 +1118,15 @@ struct NVFP4 {
     return (x == 0 || x == 0x7F) ? 0.0f : mulf(raw, 0.5f);
   }
   TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
-    return Group{r.w + 1 + 2 * grp, scale((r.w[0] >> (8 * grp)) & 0xFF)};
+    return Group{{r.w[1 + 2 * grp], r.w[2 + 2 * grp]}, scale((r.w[0] >> (8 * grp)) & 0xFF)};
   }
+  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
+    uint32_t w[1], q[2];
+    ld.words<1, 4>(36 * t, w);
+    ld.words<2, 4>(36 * t + 4 + 8 * grp, q);
+    return Group{{q[0], q[1]}, scale((w[0] >> (8 * grp)) & 0xFF)};
+  }
+  template <bool = false>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) { lookup_octet(tb, g.q[q], p); }
   TF_HD static float fold(const Group& g, float acc, float xsum, float out) {
     return fmaf_(g.d, fmaf_(-12.0f, xsum, acc), out);
