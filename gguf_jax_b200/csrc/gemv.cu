@@ -65,20 +65,20 @@ static bool tile_scratch_is_optional(int qtype) {
 // but the K-quants with kernels of their own.  The tiled kernel cuts K over the warps of the whole device: it starts at 6 us
 // (batch 1, 2) to 11 us (batch 8; a larger batch is two launches, 20 us) and grows slowly with the weight.  The other two give a CTA
 // a few rows and all of K, so below about one CTA of 16 rows per SM (2368 rows) their time follows K, not the weight:
-// they are compared at K * max(N, 2368) weights; two launches of the tiled kernel with 13 rows or more only pay once the MMA kernel
-// has two CTAs per SM to work through.  Measured on B200 over 20 formats and 56 shapes of 0.25 to 130 M weights; with these
-// lines the kernel picked takes on average 0.2 % (batch 1), 0.2 % (2..4), 0.3 % (5..8), 1 to 1.6 % (9..16) longer than the better one
-// of the two, at worst 13 %, 20 %, 30 % and 71 % (Q5_1 16384 x 4096 at 16 rows).  us, other / tiled:
-//   batch 1    2048x2048 Q4_0 3.9/5.8 IQ2_XS 4.5/6.3   4096x4096 Q4_0 9.9/7.6 IQ2_XS 11.3/8.6 TQ1_0 12.3/10.0   512x14336 Q4_0 14/7.9 MXFP4 19/8.6
-//   batch 4    1024x1024 Q4_0 3.7/6.4 IQ3_S 4.4/7.5   4096x2048 Q4_0 8.0/7.8 IQ3_S 10.1/9.0   512x14336 Q4_0 30/12 Q8_0 46/13 IQ1_M 36/13
-//   batch 8    2048x2048 Q4_0 6.0/10.8 IQ3_S 7.3/10.9   4096x4096 Q4_0 16/13 Q3_K 20/15   512x14336 Q8_0 46/21 TQ1_0 31/22
-//   batch 9    4096x4096 Q4_0 19/21 MXFP4 20/25   8192x4096 Q4_0 30/27 Q8_0 29/38 IQ3_S 40/34   512x14336 Q4_0 37/32 IQ1_M 35/33
-//   batch 16   16384x4096 Q4_0 48/58 Q3_K 61/84   8192x14336 Q4_0 97/91 IQ3_S 135/104   512x14336 IQ2_XS 33/41 Q8_0 47/43
+// they are compared at K * max(N, 2368) weights; a second launch of the tiled kernel with 5 rows or more only pays once the MMA kernel
+// has two CTAs per SM to work through.  Measured on B200 over 20 formats and 56 shapes of 0.25 to 130 M weights; with these lines the kernel
+// picked takes on average 0.2 % (batch 1..4), 0.3 % (5..8), 0.8 to 1.1 % (9..16) longer than the better one of the two, at worst
+// 13 % (1), 30 % (3: Q4_1 6144 x 1024), 32 % (5: Q5_1 4096 x 8192), 60 % (9: Q3_K 1024 x 14336).  us, other / tiled:
+//   batch 1    2048x2048 Q4_0 4.0/5.8 IQ2_XS 4.6/6.3   4096x4096 Q4_0 9.7/7.6 IQ2_XS 11.1/8.6 TQ1_0 12.1/9.9   512x14336 Q4_0 14/8.0 MXFP4 19/8.4
+//   batch 4    1024x1024 Q4_0 3.4/6.6 IQ3_S 3.9/7.5   4096x2048 Q4_0 8.4/7.8 IQ3_S 9.7/9.0   512x14336 Q4_0 24/13 Q8_0 31/13 IQ1_M 27/13
+//   batch 8    2048x2048 Q4_0 5.6/10.8 IQ3_S 6.0/11.0   4096x4096 Q4_0 16/13 Q3_K 20/15   512x14336 Q8_0 31/23 TQ1_0 30/22
+//   batch 9    4096x4096 Q4_0 17/21 MXFP4 20/24   8192x4096 Q4_0 29/27 Q8_0 30/37 IQ3_S 42/33   512x14336 Q4_0 26/32 IQ1_M 28/33
+//   batch 16   16384x4096 Q4_0 47/58 Q3_K 62/83   8192x14336 Q4_0 96/90 IQ3_S 139/104   512x14336 IQ2_XS 27/42 Q8_0 32/43
 static bool tile_pays(int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
   if (always) return true;
   const int64_t rows = M <= 12 ? 2368 : 4736;
-  const int64_t from = M == 1 ? 10 : M <= 4 ? 5 : M <= 8 ? 10 : M <= 12 ? 32 : 72;
+  const int64_t from = M == 1 ? 10 : M <= 4 ? 6 : M <= 8 ? 10 : M <= 12 ? 36 : 72;
   return K * (N > rows ? N : rows) >= from << 20;
 }
 
@@ -171,7 +171,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const bool k_quant = is_k_quant(qtype);
   // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them; streaming and
   // MMA kernel against the tiled one cross where they do for the other formats (us, other / tiled: 512 x 1280 at 1 / 2 / 4 rows 3.3/6.5
-  // 4.6/6.6 4.6/8.2, 512 x 5376 8.4/7.4 12.5/7.6 12.9/10.1)
+  // 4.6/6.6 4.6/8.2, 512 x 5376 8.4/7.4 12.5/7.6 12.9/10.1, 4096 x 1280 4.9/6.9 6.3/7.1 6.5/8.6)
   const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
   const int64_t weights = N * K;
   const bool tile_first = k_quant && !odd_rows ? (M >= 2 && M <= 4) || (M == 1 && m1_tiled)
@@ -206,7 +206,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
                   (uint8_t*)y + (size_t)m * N * y_item, y_dtype, workspace, workspace_bytes, sm_count_of(dev),
                   device_status_word_if_any(dev), st, nullptr);   // the bounded waits for the TMA boxes report there once the word exists (ggq_init)
   } else if (gemv_mma_applicable(ti, N, K, M) && M >= kMmaMinBatch) {
-    err = gemv_mma(ti, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, tab, st);
+    err = gemv_mma(ti, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, tab, sm_count_of(dev), st);
   } else if (gemv_stream_applicable(ti, N, K, M, w, x_bf16)) {
     err = gemv_stream(ti, (const uint8_t*)w, N, K, x_bf16, y, y_dtype, tab, st);
   } else {

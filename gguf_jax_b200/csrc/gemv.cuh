@@ -303,7 +303,7 @@ int32_t gemv_q4k_static(const void* w, int64_t N, int64_t K, const void* x, void
 // of the decoded weights (gemv_mma.cu).
 bool gemv_mma_applicable(const TypeInfo* ti, int64_t N, int64_t K, int M);
 cudaError_t gemv_mma(const TypeInfo* ti, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y,
-                     int y_dtype, const uint8_t* tab, cudaStream_t st);
+                     int y_dtype, const uint8_t* tab, int sm_count, cudaStream_t st);
 
 // Larger batches: tcgen05 / TMEM tensor-core kernel with tf32 operands (gemm_tcgen05.cu).
 bool gemm_applicable(const TypeInfo* ti, int64_t N, int64_t K, int M);

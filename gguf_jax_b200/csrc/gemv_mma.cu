@@ -57,10 +57,10 @@ __device__ __forceinline__ void split3(const float* v, uint32_t (&layer)[3][4]) 
   }
 }
 
-template <int QT, int NCG>   // NCG column groups of 8 batch rows
-__global__ void __launch_bounds__(kThreads)
-gemv_mma_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
-                void* __restrict__ y, int y_dtype, const uint8_t* __restrict__ tab) {
+// NCG column groups of 8 batch rows; UNROLL steps' loads in flight
+template <int QT, int NCG, int UNROLL>
+__device__ __forceinline__ void multiply(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
+                                         void* __restrict__ y, int y_dtype, const uint8_t* __restrict__ tab) {
   constexpr int BS = block_elems_of(QT), TS = block_bytes_of(QT);
   __shared__ float red[kWarps][NCG][4][32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -77,9 +77,7 @@ gemv_mma_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16
 #pragma unroll
     for (int i = 0; i < 4; i++) acc[c][i] = 0.f;
 
-  // four steps' loads in flight, stated: how far the compiler unrolled by itself changed with unrelated code behind the loop
-  // (Q2_K 4096 x 4096 at 16 rows between 18.5 and 23.1 us)
-#pragma unroll 4
+#pragma unroll UNROLL
   for (int s = warp; s < n_steps; s += kWarps) {
     const int e = 32 * s + 8 * t;                       // this lane's eight weights of the step
     const int64_t boff = (int64_t)(e / BS) * TS;
@@ -122,6 +120,30 @@ gemv_mma_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16
     const bool bad = mine && not_finite(sum);
     if (__any_sync(0xFFFFFFFFu, bad)) recompute<QT>(bad, row, m, w, row_bytes, N, x, K, tab, y, y_dtype);
   }
+}
+
+// A warp's loads wait for memory, so what counts is how many are in flight: steps unrolled times warps on the SM.  Both are
+// stated, since what the compiler chooses by itself changes with unrelated code behind the loop.  Up to two CTAs per SM there are
+// registers for four steps; with more CTAs they are better spent on a third or fourth CTA.  Measured on B200 against one kernel with
+// neither stated, mean of 20 formats: 1024 x 14336 0.68 of the time, 2048 x 2048 0.84, 4096 x 4096 0.94; 5003 x 2816 and 14336 x 4096, which
+// take 1.10 and 1.07 with four steps and two CTAs, 1.00 at 8 rows with two steps and 1.01 at 16 with four steps and three CTAs.
+template <int QT, int NCG>
+__global__ void __launch_bounds__(kThreads, 2)
+gemv_mma_few_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
+                    void* __restrict__ y, int y_dtype, const uint8_t* __restrict__ tab) {
+  multiply<QT, NCG, 4>(w, N, K, x, M, y, y_dtype, tab);
+}
+template <int QT>
+__global__ void __launch_bounds__(kThreads)
+gemv_mma_8_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
+                  void* __restrict__ y, int y_dtype, const uint8_t* __restrict__ tab) {
+  multiply<QT, 1, 2>(w, N, K, x, M, y, y_dtype, tab);
+}
+template <int QT>
+__global__ void __launch_bounds__(kThreads, 3)
+gemv_mma_16_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
+                   void* __restrict__ y, int y_dtype, const uint8_t* __restrict__ tab) {
+  multiply<QT, 2, 4>(w, N, K, x, M, y, y_dtype, tab);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -385,11 +407,11 @@ gemv_mma_q6k_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bflo
 
 template <int QT>
 static cudaError_t launch(const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype,
-                          const uint8_t* tab, cudaStream_t st) {
+                          const uint8_t* tab, int sm_count, cudaStream_t st) {
   const unsigned grid = (unsigned)((N + 15) / 16);
-  const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
-  if (M <= 8) gemv_mma_kernel<QT, 1><<<grid, kThreads, 0, st>>>(w, (int)N, (int)K, xb, M, y, y_dtype, tab);
-  else gemv_mma_kernel<QT, 2><<<grid, kThreads, 0, st>>>(w, (int)N, (int)K, xb, M, y, y_dtype, tab);
+  const bool few = grid <= 2u * (unsigned)sm_count;
+  auto* kernel = M <= 8 ? (few ? gemv_mma_few_kernel<QT, 1> : gemv_mma_8_kernel<QT>) : (few ? gemv_mma_few_kernel<QT, 2> : gemv_mma_16_kernel<QT>);
+  kernel<<<grid, kThreads, 0, st>>>(w, (int)N, (int)K, (const __nv_bfloat16*)x, M, y, y_dtype, tab);
   return cudaPeekAtLastError();
 }
 
@@ -401,7 +423,7 @@ bool gemv_mma_applicable(const TypeInfo* ti, int64_t N, int64_t K, int M) {
 }
 
 cudaError_t gemv_mma(const TypeInfo* ti, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y,
-                     int y_dtype, const uint8_t* tab, cudaStream_t st) {
+                     int y_dtype, const uint8_t* tab, int sm_count, cudaStream_t st) {
   if ((ti->qtype == QT_Q4_K || ti->qtype == QT_Q5_K) && K % 256 == 0 && (uintptr_t)w % 16 == 0) {
     const unsigned grid = (unsigned)((N + 15) / 16);
     const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
@@ -420,7 +442,7 @@ cudaError_t gemv_mma(const TypeInfo* ti, const uint8_t* w, int64_t N, int64_t K,
     return cudaPeekAtLastError();
   }
   cudaError_t err = cudaErrorInvalidValue;
-  dispatch_block_qtype(ti->qtype, [&]<int QT>() { err = mmav::launch<QT>(w, N, K, x, M, y, y_dtype, tab, st); });
+  dispatch_block_qtype(ti->qtype, [&]<int QT>() { err = mmav::launch<QT>(w, N, K, x, M, y, y_dtype, tab, sm_count, st); });
   return err;
 }
 
