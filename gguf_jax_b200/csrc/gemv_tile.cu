@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <numeric>
 
 namespace ggq {
 namespace tile {
@@ -81,7 +82,10 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
         g.x_row_bytes = g.chunk_sb * 4 * (16 * fi.oct + 16);
         g.x_row_bytes += (64 - g.x_row_bytes % 128 + 128) % 128;      // 64 (mod 128): see the staging
         g.xs_row_floats = fi.sums ? g.chunk_sb * 4 * fi.sum_groups : 0;
-        const int pieces = (14 + nb * fi.ts + 15) / 16;
+        // a block starts at a multiple of gcd(ts, 16) bytes in its 16-byte aligned window (ts a multiple of 16: at its start; with room for
+        // the largest offset there all the same, Q8_0's ring did not fit next to eight batch rows and large weights had no plan:
+        // 8192 x 12288 at 8 rows 65 to 84 us on the MMA kernel, 43 here)
+        const int pieces = (16 - std::gcd(fi.ts, 16) + nb * fi.ts + 15) / 16;
         if (pieces > 48) { if (whole_k) break; continue; }     // three 16-byte pieces per lane of a half-warp and row
         g.pitch = 16 * pieces;
         if (g.pitch % 32 == 0) g.pitch += 16;          // odd multiple of 16: rows fall into different bank groups

@@ -275,3 +275,16 @@ def test_scratch_does_not_slow_small_calls_down(qtype, n, k, m):
     """Small weights with unaligned rows took the tiled kernel, twice the time of the MMA kernel, where scratch was at hand."""
     with_scratch, without = microseconds_with_and_without_scratch(qtype, n, k, m)
     assert with_scratch <= 1.15 * without, (with_scratch, without)
+
+
+@pytest.mark.parametrize("m", [5, 8])
+def test_q8_0_keeps_the_tiled_kernel_on_large_weights(m):
+    """Its ring of copied blocks fits next to eight staged batch rows also where K is cut into chunks of eight superblocks."""
+    n, k = 8192, 12288
+    with_scratch, without = microseconds_with_and_without_scratch(QT.Q8_0, n, k, m)
+    assert with_scratch <= 0.85 * without, (with_scratch, without)
+    wb = synth.make_weight_bytes(n, k, QT.Q8_0, seed=m)
+    rows = np.sort(np.random.default_rng(3).choice(n, size=64, replace=False))
+    xb = synth.make_x(m, k, seed=m)
+    got = kernels.fused_matmul(to_x(xb), on_device(wb, QT.Q8_0, n, k), out_dtype=torch.float32).cpu().numpy()[:, rows]
+    assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb[rows], QT.Q8_0)) <= 2e-5
