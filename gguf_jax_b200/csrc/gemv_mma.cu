@@ -134,7 +134,7 @@ gemv_mma_few_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bflo
   multiply<QT, NCG, 4>(w, N, K, x, M, y, y_dtype, tab);
 }
 template <int QT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, block_elems_of(QT) == 256 ? 0 : 4)
 gemv_mma_8_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
                   void* __restrict__ y, int y_dtype, const uint8_t* __restrict__ tab) {
   multiply<QT, 1, 2>(w, N, K, x, M, y, y_dtype, tab);
