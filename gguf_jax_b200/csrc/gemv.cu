@@ -183,8 +183,9 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
                        sm_count_of(dev) > 0 && gemv_tile_applicable(qtype, N, K, tile_m, w, x_bf16, sm_count_of(dev));
   static const int wide_min = [] { const char* e = getenv("GGQ_WIDE_MIN"); return e ? atoi(e) : 5; }();
   // (rows that are not 16-byte aligned: the MMA kernel reads them with 2-byte loads; 5003 x 2816 Q6_K at 5 / 16 rows 21.3 / 25.2 us
-  // there, 18.0 / 19.8 here; 1024 x 5376 13.0 / 14.6 there, 20.0 / 21.0 here)
-  const bool wide_ok = k_quant && M >= wide_min && (odd_rows ? weights >= (12ll << 20) : wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes)) && workspace && (uintptr_t)workspace % 256 == 0 && sm_count_of(dev) > 0 &&
+  // there, 18.0 / 19.8 here; 1024 x 5376 13.0 / 14.6 there, 20.0 / 21.0 here; rows of a few superblocks leave its steps too little to
+  // overlap: 16384 x 768 at 5 / 8 / 16 rows 14.2 / 14.6 / 18.4 there, 17.4 / 17.3 / 20.0 here, 28672 x 768 23 / 24 / 29 and 20 / 20 / 21)
+  const bool wide_ok = k_quant && M >= wide_min && (odd_rows ? weights >= (K < 1536 ? 21ll : 12ll) << 20 : wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes)) && workspace && (uintptr_t)workspace % 256 == 0 && sm_count_of(dev) > 0 &&
                        workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, M, sm_count_of(dev)) &&
                        gemv_wide_applicable(qtype, N, K, M, w, x_bf16);
   if (wide_ok) {
