@@ -103,7 +103,10 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
         const int64_t warp_steps = (g.S + g.W - 1) / g.W;
         const int fit = room / (kWarps * g.slot_bytes);
         if (span_ok && fit >= std::min<int64_t>(2, warp_steps)) {
-          g.depth = std::min(kMaxDepth, std::max(2, fit));
+          // (more than two slots of over 4 KB only put more weights in front of the first activations: Q8_0 14336 x 4096 at batch 1 with
+          // two / three / four 19.3 / 19.9 / 19.9 us; smaller slots the same either way)
+          const int most = g.slot_bytes > 4096 ? 2 : kMaxDepth;
+          g.depth = std::min(most, std::max(2, fit));
           g.slots = (int)std::min<int64_t>(g.depth, warp_steps);
           g.off_x = kWarps * g.slots * g.slot_bytes;
           g.off_xs = g.off_x + bufs * x_rows * g.x_row_bytes;
@@ -115,7 +118,7 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
           // unit, in units of one block's multiply; the constants are fitted to B200 timings (8192 x 28672:
           // nb = 2 with chunks of 16 superblocks is the fastest split for every format)
           const double steps = (double)warp_steps;
-          const double cost = steps * (nb + 0.6) * (g.depth >= 3 ? 1.0 : 1.03) + bufs * g.chunk_sb * x_rows * 0.02 + steps / g.spu * 0.6;
+          const double cost = steps * (nb + 0.6) * (g.depth >= std::min(3, most) ? 1.0 : 1.03) + bufs * g.chunk_sb * x_rows * 0.02 + steps / g.spu * 0.6;
           if (cost < best_cost) { best_cost = cost; best = g; }
         }
       }
