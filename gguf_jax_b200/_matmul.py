@@ -203,7 +203,7 @@ def _materialized_forward(x: torch.Tensor, w: QuantizedArray, count: int) -> tor
     n_out = w.shape[0]
     x2 = x.reshape(-1, w.shape[1])
     y = None
-    if _plain(x) and (count > 1 or _pads(x2.shape[0], w)):
+    if (count > 1 or _pads(x2.shape[0], w)) and _plain(x):
         # every slab's product goes straight to its columns of the result; slab and row boundaries are multiples of
         # _ROW_ELEMS (a result whose rows are not is copied once at the end).  Slabs are rounded down, so that none
         # exceeds the budget; one of all rows stays whole.
