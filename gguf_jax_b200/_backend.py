@@ -72,7 +72,8 @@ class _Buffers:
     CUDA graphs keep the addresses they were captured with.  So a buffer that a capture has been given stays allocated when a
     larger one takes its place (which is then at least twice as large: those kept never add up to more than the current
     one).  And a buffer that is first allocated under capture belongs to that capture alone: it is the graph's memory and
-    its zero fill runs on replay, so no other graph and no call outside may take it for a cleared one."""
+    its zero fill runs on replay, so no other graph and no call outside may take it for a cleared one.
+    Graphs captured on a stream that had its buffer share it: their replays must not overlap each other or the stream's calls."""
 
     def __init__(self, smallest: int, zeroed: bool, publish: bool):
         self.smallest, self.zeroed, self.publish = smallest, zeroed, publish

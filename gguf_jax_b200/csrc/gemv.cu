@@ -11,7 +11,7 @@ constexpr int kGemvMaxBatch = 16;
 // From this batch on the tensor-core small-batch kernel beats the per-element FMA kernel.
 constexpr int kMmaMinBatch = 2;
 // Up to this batch the tuned batch-1 kernels are simply launched once per batch row (only where the
-// tiled kernel cannot run: no workspace, or rows that are not 16-byte aligned).
+// tiled kernel cannot run, for want of scratch).
 inline int tuned_max_repeat(int qtype, int64_t weight_bytes) {
   if (qtype == QT_Q6_K) return weight_bytes < (24ll << 20) ? 2 : weight_bytes < (100ll << 20) ? 3 : 4;
   return weight_bytes < (24ll << 20) ? 1 : weight_bytes < (80ll << 20) ? 2 : 3;
@@ -26,17 +26,22 @@ inline bool wide_pays(int qtype, int64_t weight_bytes) {
   return weight_bytes >= (qtype == QT_Q6_K ? (10ll << 20) : (20ll << 20));
 }
 // Above 16 batch rows the choice is between slices of 32 rows through the batch-major kernel and, in the
-// caller, the decode kernel followed by a library GEMM.  One slice wins from about 20 MB on (Q4_K 8192 x 8192:
-// 39 us against 76 us; Q6_K 14336 x 4096: 45 us against 66 us; Q5_K 4096 x 4096, 11.5 MB: 28 us against 23 us,
-// its decoded copy stays in the L2); two slices or more lose, so the router's cap is 32 there and 16 elsewhere.
+// caller, the decode kernel followed by a library GEMM.  One slice wins from about 20 MB on (us, fused / decode and GEMM, on the
+// device: Q4_K 8192 x 8192 36 / 55, Q6_K 14336 x 4096 38 / 50; on smaller weights it loses, their decoded copy stays in the L2:
+// Q5_K 4096 x 4096 22 / 17 and, above Q6_K's line of 10 MB, 4096 x 4096 26 / 16); two slices or more lose, so the router's cap is
+// 32 there and 16 elsewhere.
 // The tcgen05 kernels behind ggq_gemm (integer-code and tf32 operands) are slower than both at every
 // batch measured and are reached only by name, above 128 rows or for the other formats.
 constexpr int kWideRouterBatch = 32;
 // Above 32 rows the bf16-weight tcgen05 kernel (gemm_bf16w.cu; the fallback's own precision) is compared with the same
-// fallback: on the large weights it wins up to 256 rows (Q6_K 14336 x 4096: 52 / 55 / 62 us at 64 / 128 / 256 rows against
-// 67 / 68 / 75 us; Q6_K 4096 x 14336: 54 / 62 / 79 us against 70 / 73 / 80 us), and up to 512 rows where there are enough
-// row tiles to fill the device without cutting K (14336 rows: 78 us against 92 us; 4096 rows: 118 us against 92 us);
-// on weights of a few MB the fallback's library GEMM reads a decoded copy that stays in the L2 and wins from 64 rows on.
+// fallback, up to 256 rows on the large weights and up to 512 where there are enough row tiles to fill the device without
+// cutting K.  us on the device at 64 / 128 / 256 / 512 rows, fused and fallback: Q4_K 14336 x 4096 37 / 39 / 47 / 65 and 47 / 47 / 56 / 73,
+// 4096 x 14336 41 / 48 / 65 / 91 and 52 / 53 / 57 / 73, 8192 x 8192 43 / 49 / 64 / 107 and 56 / 55 / 63 / 74, 28672 x 8192 146 / 171 / 164 / 262 and
+// 186 / 187 / 210 / 270; Q6_K 14336 x 4096 53 / 55 / 62 / 78 and 52 / 51 / 60 / 78, 4096 x 14336 54 / 62 / 79 / 118 and 57 / 57 / 62 / 77, 8192 x 8192 58 /
+// 64 / 79 / 119 and 61 / 59 / 68 / 80.  The caps date from a decode kernel that took 15 us longer on these weights: they still hold for Q4_K
+// and Q5_K but for 256 rows at 4096 x 14336, and lie too high for Q6_K, whose lead ends at 64 rows.  A call through the fallback
+// takes 8 us more of host time, which is what counts where the device does not lag behind.
+// On weights of a few MB the fallback's library GEMM reads a decoded copy that stays in the L2 and wins at every batch above 16.
 constexpr int kGemmRouterBatchWide = 512;      // at least 96 row tiles of 128 rows
 constexpr int kGemmRouterBatch = 256;
 }
@@ -67,8 +72,8 @@ static bool tile_scratch_is_optional(int qtype) {
 // a few rows and all of K, so below about one CTA of 16 rows per SM (2368 rows) their time follows K, not the weight:
 // they are compared at K * max(N, 2368) weights; a second launch of the tiled kernel with 5 rows or more only pays once the MMA kernel
 // has two CTAs per SM to work through.  Measured on B200 over 20 formats and 56 shapes of 0.25 to 130 M weights; with these lines the kernel
-// picked takes on average 0.2 % (batch 1..4), 0.3 % (5..8), 0.8 to 1.1 % (9..16) longer than the better one of the two, at worst
-// 13 % (1), 30 % (3: Q4_1 6144 x 1024), 32 % (5: Q5_1 4096 x 8192), 60 % (9: Q3_K 1024 x 14336).  us, other / tiled:
+// picked takes on average 0.2 % (batch 1..4), 0.3 % (5..8), 0.8 to 0.9 % (9..16) longer than the better one of the two, at worst
+// 13 % (1), 30 % (3: Q4_1 6144 x 1024), 32 % (5: Q5_1 4096 x 8192), 59 % (9).  us, other / tiled:
 //   batch 1    2048x2048 Q4_0 4.0/5.8 IQ2_XS 4.6/6.3   4096x4096 Q4_0 9.7/7.6 IQ2_XS 11.1/8.6 TQ1_0 12.1/9.9   512x14336 Q4_0 14/8.0 MXFP4 19/8.4
 //   batch 4    1024x1024 Q4_0 3.4/6.6 IQ3_S 3.9/7.5   4096x2048 Q4_0 8.4/7.8 IQ3_S 9.7/9.0   512x14336 Q4_0 24/13 Q8_0 31/13 IQ1_M 27/13
 //   batch 8    2048x2048 Q4_0 5.6/10.8 IQ3_S 6.0/11.0   4096x4096 Q4_0 16/13 Q3_K 20/15   512x14336 Q8_0 31/23 TQ1_0 30/22
@@ -78,7 +83,7 @@ static bool tile_pays(int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
   if (always) return true;
   const int64_t rows = M <= 12 ? 2368 : 4736;
-  const int64_t from = M == 1 ? 10 : M <= 4 ? 6 : M <= 8 ? 10 : M <= 12 ? 36 : 72;
+  const int64_t from = M == 1 ? 10 : M <= 4 ? 6 : M <= 8 ? 10 : M <= 10 ? 32 : M <= 12 ? 36 : 72;
   return K * (N > rows ? N : rows) >= from << 20;
 }
 
@@ -166,7 +171,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   // Q4_K / Q5_K / Q6_K keep their batch-1 kernels; the tiled kernel takes their batches 2..4 whatever the size (it scales each
   // row and keeps any magnitude; the integer-code MMA kernel keeps about 2^-50 to 2^62; Q4_K 8192 x 28672:
   // 36 / 49 us at batch 2 / 4) and the other formats where tile_pays says so; from five batch rows on
-  // the batch-major kernel takes the larger weights (Q4_K 8192 x 28672: 68 / 77 us at batch 8 / 16 against
+  // the batch-major kernel takes the larger weights (Q4_K 8192 x 28672: 56 / 65 us at batch 8 / 16 against
   // 100 / 153 us) and the integer-code MMA kernel (gemv_mma.cu) the smaller ones (see wide_pays).
   const bool k_quant = is_k_quant(qtype);
   // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them; streaming and

@@ -139,9 +139,9 @@ TF_HD uint32_t spread_signs4(uint32_t nib) { return ((nib & 15u) * 0x10204080u) 
 TF_HD uint32_t ksigns(uint32_t i7) { return i7 | ((popc(i7) & 1u) << 7); }
 
 // Reads 32-bit words starting at byte offset `off` of a block.  A is the alignment the caller
-// guarantees for that address (16, 8, 4: vector or word loads; 2: aligned word loads plus funnel
-// shifts when the address is 2 (mod 4) -- the branch is the same for every lane of a warp, since
-// rows start 16-byte aligned and all rows of a tile see the block at the same offset).
+// guarantees for that address (16, 8, 4: vector or word loads; 2: aligned words and a funnel shift by
+// 0 or 16 bits, without a branch: lanes of a warp hold different rows, which may start at different
+// offsets modulo 4).
 // On the device a block lives in shared memory and is addressed by its 32-bit shared-window
 // address, so that field offsets fold into the load instructions.
 #if TF_DEVICE
