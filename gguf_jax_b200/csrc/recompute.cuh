@@ -54,6 +54,12 @@ __device__ __noinline__ void recompute(bool bad, int row, int m, const uint8_t* 
     if ((threadIdx.x & 31) == src) store_out(y, y_dtype, (int64_t)mr * N + r, v);
   }
 }
+// An output as it was stored (by a lane of this warp).
+__device__ __forceinline__ float load_out(const void* y, int y_dtype, int64_t idx) {
+  if (y_dtype == GGQ_F32) return reinterpret_cast<const volatile float*>(y)[idx];
+  const uint32_t u = reinterpret_cast<const volatile unsigned short*>(y)[idx];
+  return y_dtype == GGQ_BF16 ? __uint_as_float(u << 16) : __half2float(__ushort_as_half((unsigned short)u));
+}
 __device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 
 }  // namespace ggq
