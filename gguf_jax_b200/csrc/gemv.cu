@@ -87,6 +87,25 @@ static bool tile_pays(int64_t N, int64_t K, int M) {
   return K * (N > rows ? N : rows) >= from << 20;
 }
 
+// The batch kernel (gemv_batch.cu) against what served the call before: from 5 rows on it wins wherever the weight is large enough to fill its
+// CTAs (below, one MMA launch), at 3 and 4 rows against two passes of the tiled kernel only where there are rows enough, at 2 nowhere.
+// us before / here, 700 shapes of 1 to 235 M weights timed: at 5..16 rows on average 0.73 of the time, on the wrong side of these lines at
+// worst 1.15 (Q5_K 1515 x 5888 at 6 rows); at 3, 4 rows 0.92, 1.05:
+//   8 rows   4096x4096 Q4_K 13/9.1 Q5_K 14/9.5 IQ2_XS 13/9.6   2048x8192 Q6_K 23/13   8192x8192 Q4_K 24/17 IQ3_S 37/23   700x28672 Q5_K 51/10
+//   16 rows  8192x2048 Q4_K 14/9.4   8192x8192 IQ3_S 82/30 Q2_K 70/25   14336x4096 Q6_K 30/27   but 1024x4096 Q4_K 7.0/9.7, Q5_K 8.0/10
+//   4 rows   16384x1024 Q4_K 7.9/5.6   14336x4096 Q5_K 28/21 Q6_K 32/24   8192x28672 Q4_K 47/47   but 2560x11520 Q4_K 11/13
+static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
+  static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
+  const int64_t work = K * (N > 2368 ? N : 2368);
+  if (M >= 9) return always || work >= (qtype == QT_Q4_K ? 18ll : qtype == QT_Q5_K ? 14ll : 10ll) << 20;
+  if (M >= 5) return always || work >= (qtype == QT_Q4_K ? 12ll : 10ll) << 20;
+  if (M < 3) return false;
+  if (qtype == QT_Q4_K) return N >= 8192 && K <= 12288;
+  if (qtype == QT_Q5_K) return N >= 2048;
+  if (qtype == QT_Q6_K) return N >= 2048 && N * K >= 6ll << 20;
+  return N >= 10240 && K <= 8192 && N * K >= 14ll << 20;
+}
+
 static size_t tile_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
   const int tmax = gemv_tile_max_batch(qtype);
   return tmax && M <= kGemvMaxBatch && K % 256 == 0 ? gemv_tile_workspace_bytes(qtype, N, K, M < tmax ? M : tmax) : 0;
@@ -181,6 +200,10 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const int64_t weights = N * K;
   const bool tile_first = k_quant && !odd_rows ? (M >= 2 && M <= 4) || (M == 1 && m1_tiled)
                                                : (!k_quant || M <= 4) && tile_pays(N, K, M);
+  // (GGQ_GEMM_KERNEL=wide pins the batch-major kernel here as in ggq_gemm)
+  const char* pin = k_quant ? getenv("GGQ_GEMM_KERNEL") : nullptr;
+  const bool batch_ok = batch_pays(qtype, N, K, M) && !(pin && !strcmp(pin, "wide")) &&
+                        gemv_batch_applicable(qtype, N, K, M, w, x_bf16, sm_count_of(dev));
   const int tile_max = gemv_tile_max_batch(qtype);
   const int tile_m = M < tile_max ? M : tile_max;
   const size_t tile_need = tile_max ? gemv_tile_workspace_bytes(qtype, N, K, tile_m) : 0;
@@ -193,7 +216,9 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const bool wide_ok = k_quant && M >= wide_min && (odd_rows ? weights >= (K < 1536 ? 21ll : 12ll) << 20 : wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes)) && workspace && (uintptr_t)workspace % 256 == 0 && sm_count_of(dev) > 0 &&
                        workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, M, sm_count_of(dev)) &&
                        gemv_wide_applicable(qtype, N, K, M, w, x_bf16);
-  if (wide_ok) {
+  if (batch_ok) {
+    err = gemv_batch(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, sm_count_of(dev), device_status_word_if_any(dev), tab, st);
+  } else if (wide_ok) {
     err = gemv_wide(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, workspace, workspace_bytes, sm_count_of(dev), st, 0, nullptr,
                     device_status_word_if_any(dev));
   } else if (tile_ok) {

@@ -295,6 +295,11 @@ cudaError_t gemv_tile(int qtype, const uint8_t* w, int64_t N, int64_t K, const v
                       const PeerPublish* peers = nullptr);
 int gemv_tile_max_batch(int qtype);     // batch rows per launch (8, Q6_K: 4; 0 if qtype has no tile format)
 
+// Batches of 2 .. 16 rows of the formats with one float scale per 256 weights, without scratch (gemv_batch.cu).
+bool gemv_batch_applicable(int qtype, int64_t N, int64_t K, int M, const void* w, const void* x, int sm_count);
+cudaError_t gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype, int sm_count, int* status,
+                       const uint8_t* tab, cudaStream_t st);
+
 // Same kernel with the scratch in a file-scope device array (no caller buffer); returns a ggq_status.
 int32_t gemv_q4k_static(const void* w, int64_t N, int64_t K, const void* x, void* y, int32_t y_dtype,
                         int sm_count, cudaStream_t st);

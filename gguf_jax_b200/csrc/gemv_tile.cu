@@ -11,10 +11,10 @@ namespace tile {
 // ---------------------------------------------------------------------------------------------
 // host side
 
-struct FormatInfo { int qt, ts, table_bytes, sum_groups, oct; bool sums; };
+struct FormatInfo { int qt, ts, table_bytes, sum_groups, oct; bool sums, four_passes; };
 
 template <class F>
-constexpr FormatInfo info_of() { return {F::kQt, F::kTs, F::kTableBytes, F::kOct / F::kGroupOct, F::kOct, F::kSums}; }
+constexpr FormatInfo info_of() { return {F::kQt, F::kTs, F::kTableBytes, F::kOct / F::kGroupOct, F::kOct, F::kSums, four_passes<F>()}; }
 
 static bool format_of(int qtype, FormatInfo* fi) {
   switch (qtype) {
@@ -139,12 +139,12 @@ static int forced_chunk() { static const int v = env_int("GGQ_TILE_CHUNK"); retu
 
 }  // namespace tile
 
-// Most batch rows one launch takes for qtype (0: not a tile format).  Four passes only pay where decoding
-// dominates; Q6_K, with two planes and 32 MMAs per block and pass, is faster as two launches of two passes.
+// Most batch rows one launch takes for qtype (0: not a tile format): two passes for the formats of the batch kernel, which takes their
+// larger batches, four for the others.
 int gemv_tile_max_batch(int qtype) {
   tile::FormatInfo fi;
   if (!tile::format_of(qtype, &fi)) return 0;
-  return qtype == QT_Q6_K ? 4 : tile::kMaxBatch;
+  return fi.four_passes ? tile::kMaxBatch : 4;
 }
 
 // Every 16-row tile has an arrival counter in the counter area that the kernels share.

@@ -47,6 +47,11 @@ constexpr int kThreads = kWarps * 32;
 constexpr int kSmemLimit = 232448;              // 227 KB opt-in limit per CTA
 constexpr int kMaxDepth = 6;
 constexpr int kMaxBatch = 8;                    // four passes of two batch rows
+// Batches above four: the formats of 32 and 64 weights a block, with a scale each (the others' larger batches go to gemv_batch.cuh).
+template <class F> constexpr bool four_passes() {
+  return F::kQt == QT_Q8_0 || F::kQt == QT_Q4_0 || F::kQt == QT_Q4_1 || F::kQt == QT_Q5_0 || F::kQt == QT_Q5_1 || F::kQt == QT_IQ4_NL ||
+         F::kQt == QT_MXFP4 || F::kQt == QT_NVFP4;
+}
 constexpr int kMaxXBufs = 16;                   // K chunks whose activations a CTA can hold at once
 
 // Launch geometry, computed on the host (plan()) and passed by value.
@@ -662,7 +667,9 @@ static cudaError_t launch_passes(int MP, const Geo& geo, int grid, cudaStream_t 
   switch (MP) {
     case 1: return launch<F, 1>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab);
     case 2: return launch<F, 2>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab);
-    default: return launch<F, 4>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab);
+    default:
+      if constexpr (four_passes<F>()) return launch<F, 4>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab);
+      else return cudaErrorInvalidValue;
   }
 }
 

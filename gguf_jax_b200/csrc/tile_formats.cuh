@@ -38,8 +38,8 @@
 //                       2 MXFP4 values + 12
 //   kScaleExp           the group scales carry 2^kScaleExp (taken back out of the row sums; 0 where the trait is absent)
 //   kLean, load_group_lean(ld, t, grp)   the group straight from the block, nothing kept for the run (absent: load_run only).  At
-//                       four passes the registers and, for the signs, the shared-memory pipe are what is short: there the
-//                       groups are loaded one at a time inside a real loop and octet<false> works the signs out (us at 8 rows, whole runs / group
+//                       four passes the registers are what is short: there the
+//                       groups are loaded one at a time inside a real loop (octet<false>; us at 8 rows, whole runs / group
 //                       by group: Q4_1 14336 x 4096 30.1 / 27.8, Q5_1 37.5 / 31.2, NVFP4 37.3 / 33.6 and 16384 x 8192 69.6 / 58.0)
 //   octet(group, q, tab, p)   the four A-operand registers of octet q of the group: p[0], p[1] = first
 //                       MMA (k-slot pairs 2t.. and 2t+8..), p[2], p[3] = second MMA
@@ -525,7 +525,6 @@ TF_HD void plain_octet(uint32_t w0, uint32_t w1, uint32_t (&p)[4]) {
 // IQ2_XXS (66 B: d, 8 x {4 index bytes, u32 = 4 x 7-bit sign index | 4-bit scale << 28}); group = one of them
 struct IQ2XXS {
   static constexpr int kQt = 16, kTs = 66, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 256, kEntryBytes = 8, kCopies = 16, kSignBits = 7;
   static constexpr bool kSignTable = true;
@@ -543,16 +542,10 @@ struct IQ2XXS {
   TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
     return Group{r.q[2 * grp], r.q[2 * grp + 1], mulf(r.d4, 0.5f + u2f(r.q[2 * grp + 1] >> 28))};
   }
-  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
-    uint32_t q[2];
-    ld.words<2, 2>(2 + 16 * t + 8 * grp, q);
-    return Group{q[0], q[1], mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(q[1] >> 28))};
-  }
-  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     uint32_t w0, w1, s0, s1;
     grid_words<8, kCopies>(tb, (g.q >> (8 * q)) & 0xFF, 0, w0, w1);
-    sign_words<kSignBits, SIGN_TABLE>(tb, (g.aux >> (7 * q)) & 127, s0, s1);
+    sign_words<kSignBits, kSignTable>(tb, (g.aux >> (7 * q)) & 127, s0, s1);
     signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
@@ -561,7 +554,6 @@ struct IQ2XXS {
 // IQ2_XS (74 B: d, 32 x u16 = 9-bit grid index | 7-bit sign index << 9, 8 scale bytes of two nibbles)
 struct IQ2XS {
   static constexpr int kQt = 17, kTs = 74, kAlign = 2, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
-  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 512, kEntryBytes = 8, kCopies = 16, kSignBits = 7;
   static constexpr bool kSignTable = true;
@@ -580,16 +572,10 @@ struct IQ2XS {
   TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
     return Group{r.q[grp], mulf(r.d4, 0.5f + u2f((r.sc >> (4 * grp)) & 15))};
   }
-  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
-    const uint32_t q = ld.u16(2 + 16 * t + 4 * grp) | (ld.u16(4 + 16 * t + 4 * grp) << 16);
-    const uint32_t sc = (ld.u16(66 + 2 * t) >> (4 * grp)) & 15;
-    return Group{q, mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(sc))};
-  }
-  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     uint32_t w0, w1, s0, s1;
     grid_words<8, kCopies>(tb, (g.q >> (16 * q)) & 511, 0, w0, w1);
-    sign_words<kSignBits, SIGN_TABLE>(tb, (g.q >> (16 * q + 9)) & 127, s0, s1);
+    sign_words<kSignBits, kSignTable>(tb, (g.q >> (16 * q + 9)) & 127, s0, s1);
     signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
@@ -598,7 +584,6 @@ struct IQ2XS {
 // IQ2_S (82 B: d, 32 index bytes, 32 sign bytes, 8 bytes of 2 high index bits, 8 scale bytes)
 struct IQ2S {
   static constexpr int kQt = 22, kTs = 82, kAlign = 2, kOct = 8, kGroupOct = 2, kSumOct = 2, kPairOrder = 0;
-  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 1024, kEntryBytes = 8, kCopies = 8, kSignBits = 8;
   static constexpr bool kSignTable = false;
@@ -620,17 +605,11 @@ struct IQ2S {
     const int sh = 16 * (grp & 1);
     return Group{r.qs[grp >> 1] >> sh, r.sg[grp >> 1] >> sh, r.qh >> (4 * grp), mulf(r.d4, 0.5f + u2f((r.sc >> (4 * grp)) & 15))};
   }
-  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
-    const uint32_t sc = (ld.u16(74 + 2 * t) >> (4 * grp)) & 15;
-    return Group{ld.u16(2 + 8 * t + 2 * grp), ld.u16(34 + 8 * t + 2 * grp), ld.u16(66 + 2 * t) >> (4 * grp),
-                 mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.25f), 0.5f + u2f(sc))};
-  }
-  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t idx = ((g.qs >> (8 * q)) & 0xFF) | (((g.qh >> (2 * q)) & 3) << 8);
     uint32_t w0, w1, s0, s1;
     grid_words<8, kCopies>(tb, idx, 0, w0, w1);
-    sign_words<kSignBits, SIGN_TABLE>(tb, (g.sg >> (8 * q)) & 0xFF, s0, s1);
+    sign_words<kSignBits, kSignTable>(tb, (g.sg >> (8 * q)) & 0xFF, s0, s1);
     signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
@@ -639,7 +618,6 @@ struct IQ2S {
 // IQ3_XXS (98 B: d, 64 index bytes (one per 4 weights), 8 x u32 = 4 x 7-bit sign index | scale << 28)
 struct IQ3XXS {
   static constexpr int kQt = 18, kTs = 98, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 256, kEntryBytes = 4, kCopies = 32, kSignBits = 7;
   static constexpr bool kSignTable = true;
@@ -658,18 +636,11 @@ struct IQ3XXS {
   TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
     return Group{{r.q[2 * grp], r.q[2 * grp + 1]}, r.aux[grp], mulf(r.d2, 0.5f + u2f(r.aux[grp] >> 28))};
   }
-  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
-    uint32_t q[2], aux[1];
-    ld.words<2, 2>(2 + 16 * t + 8 * grp, q);
-    ld.words<1, 2>(66 + 8 * t + 4 * grp, aux);
-    return Group{{q[0], q[1]}, aux[0], mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.5f), 0.5f + u2f(aux[0] >> 28))};
-  }
-  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t q16 = g.q[q >> 1] >> (16 * (q & 1));
     uint32_t w0, w1, s0, s1;
     grid_words<4, kCopies>(tb, q16 & 0xFF, (q16 >> 8) & 0xFF, w0, w1);
-    sign_words<kSignBits, SIGN_TABLE>(tb, (g.aux >> (7 * q)) & 127, s0, s1);
+    sign_words<kSignBits, kSignTable>(tb, (g.aux >> (7 * q)) & 127, s0, s1);
     signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
@@ -678,7 +649,6 @@ struct IQ3XXS {
 // IQ3_S (110 B: d, 64 index bytes, 8 bytes of ninth index bits, 32 sign bytes, 4 scale bytes of two nibbles)
 struct IQ3S {
   static constexpr int kQt = 21, kTs = 110, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kLean = true;
   static constexpr bool kSums = false, kUnrollGroups = true;
   static constexpr int kEntries = 512, kEntryBytes = 4, kCopies = 16, kSignBits = 8;
   static constexpr bool kSignTable = true;
@@ -699,21 +669,13 @@ struct IQ3S {
   TF_HD static Group load_group(const BlockLd&, const Run& r, int, int grp) {
     return Group{{r.q[2 * grp], r.q[2 * grp + 1]}, r.sg[grp], r.qh >> (8 * grp), mulf(r.d, u2f(1 + 2 * ((r.sc >> (4 * grp)) & 15)))};
   }
-  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
-    uint32_t q[2], sg[1];
-    ld.words<2, 2>(2 + 16 * t + 8 * grp, q);
-    ld.words<1, 2>(74 + 8 * t + 4 * grp, sg);
-    const uint32_t sc = (ld.u16(106 + (t & 2)) >> (8 * (t & 1) + 4 * grp)) & 15;
-    return Group{{q[0], q[1]}, sg[0], ld.u16(66 + 2 * t) >> (8 * grp), mulf(f16_bits_to_float(ld.u16(0)), u2f(1 + 2 * sc))};
-  }
-  template <bool SIGN_TABLE = kSignTable>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t q16 = g.q[q >> 1] >> (16 * (q & 1));
     const uint32_t i0 = (q16 & 0xFF) | (((g.qh >> (2 * q)) & 1) << 8);
     const uint32_t i1 = ((q16 >> 8) & 0xFF) | (((g.qh >> (2 * q + 1)) & 1) << 8);
     uint32_t w0, w1, s0, s1;
     grid_words<4, kCopies>(tb, i0, i1, w0, w1);
-    sign_words<kSignBits, SIGN_TABLE>(tb, (g.sg >> (8 * q)) & 0xFF, s0, s1);
+    sign_words<kSignBits, kSignTable>(tb, (g.sg >> (8 * q)) & 0xFF, s0, s1);
     signed_octet(w0, w1, s0, s1, p);
   }
   TF_HD static float fold(const Group& g, float acc, float, float out) { return fmaf_(g.db, acc, out); }
@@ -725,7 +687,6 @@ struct IQ3S {
 // fold removes the 9 and the factor 8:  (dl / 8) * (sum(code x) - 9 sum(x)).
 struct IQ1S {
   static constexpr int kQt = 19, kTs = 50, kAlign = 2, kOct = 8, kGroupOct = 4, kSumOct = 4, kPairOrder = 0;
-  static constexpr bool kLean = true;
   static constexpr bool kSums = true, kUnrollGroups = true;
   static constexpr int kEntries = 2048, kEntryBytes = 8, kCopies = 4, kSignBits = 0;
   static constexpr bool kSignTable = false;
@@ -749,17 +710,6 @@ struct IQ1S {
     g.dl8 = mulf(r.d8, u2f(2 * ((g.qh >> 12) & 7) + 1));
     return g;
   }
-  TF_HD static Group load_group_lean(const BlockLd& ld, int t, int grp) {
-    uint32_t qs[1];
-    ld.words<1, 2>(2 + 8 * t + 4 * grp, qs);
-    Group g;
-    g.qs = qs[0];
-    g.qh = ld.u16(34 + 4 * t + 2 * grp);
-    g.dlt = (g.qh & 0x8000) ? 0xFEFEFEFFu : 0x01010101u;
-    g.dl8 = mulf(mulf(f16_bits_to_float(ld.u16(0)), 0.125f), u2f(2 * ((g.qh >> 12) & 7) + 1));
-    return g;
-  }
-  template <bool = false>
   TF_HD static void octet(const Group& g, int q, const Tables& tb, uint32_t (&p)[4]) {
     const uint32_t idx = ((g.qs >> (8 * q)) & 0xFF) | (((g.qh >> (3 * q)) & 7) << 8);
     uint32_t w0, w1;
