@@ -31,7 +31,10 @@ from .array import QuantizedArray
 __all__ = ["dequant_matmul", "fused_batch_limit", "fused_types", "matmul"]
 
 # Byte budget of one dense slab.  The reference's environment knob and default are kept
-# (src/gguf_jax/_matmul.py:39-44); like there, a slab is costed at 4 bytes per weight.
+# (src/gguf_jax/_matmul.py:39-44).  There a slab is costed at 4 bytes per weight, and so it is here under a ``block_bytes`` that the caller
+# gives; under this default it is costed at what it takes, 2 bytes where the weight is decoded to bfloat16, because every slab is a launch of
+# the library GEMM that starts and ends with its tensor cores partly idle (us, 28672 x 8192 Q4_K at 2048 rows, two slabs / one: 935 / 887, in
+# CUDA graphs 842 / 734).
 DEQUANT_BLOCK_BYTES = int(os.environ.get("GGUF_JAX_DEQUANT_BLOCK_BYTES", 512 << 20))
 
 FusedEntry = tuple[Callable[..., torch.Tensor], Callable[[QuantizedArray], int]]
@@ -109,7 +112,7 @@ def matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None
     if out is None and w.__class__ is QuantizedArray and not _function_modes():
         # the common call (device activations, no gradient; fused, or dense in one piece by the built-in bf16 decoder) is one
         # native function
-        budget = DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes
+        budget = 2 * DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes       # of a copy costed at 4 bytes a weight
         y = _native_matmul(x, w.data, w.qtype, w.shape, force_fused,
                            budget if w.dtype is torch.bfloat16 and not quants._replaced else 0)
         if y is not None:
@@ -143,15 +146,17 @@ def dequant_matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | Non
 # ---------------------------------------------------------------------------------------------
 # slabs
 
-def _block_count(out_rows: int, in_features: int, budget: int) -> int:
-    """Number of equal row slabs so that one slab, costed at 4 bytes per weight, fits ``budget``:
+def _block_count(out_rows: int, in_features: int, budget: int, itemsize: int = 4) -> int:
+    """Number of equal row slabs so that one slab of ``itemsize`` bytes per weight fits ``budget``:
     the smallest divisor of ``out_rows`` that is large enough (``out_rows`` itself if none is)."""
-    slabs_wanted = max(1, math.ceil(4 * out_rows * in_features / max(budget, 1)))
+    slabs_wanted = max(1, math.ceil(itemsize * out_rows * in_features / max(budget, 1)))
     return next((d for d in range(slabs_wanted, out_rows) if out_rows % d == 0), out_rows) if slabs_wanted > 1 else 1
 
 
 def _slab_count(w: QuantizedArray, block_bytes: int | None) -> int:
-    return _block_count(w.shape[0], w.shape[1], DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes)
+    if block_bytes is None:
+        return _block_count(w.shape[0], w.shape[1], DEQUANT_BLOCK_BYTES, min(4, w.dtype.itemsize))
+    return _block_count(w.shape[0], w.shape[1], block_bytes)
 
 
 def _slabs(w: QuantizedArray, count: int, rows: int | None = None):
