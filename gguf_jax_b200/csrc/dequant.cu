@@ -6,12 +6,15 @@
 // consecutive threads own consecutive groups, so a warp writes 1 / 2 KiB contiguous.  The block
 // bytes come through the read-only path and are reused by the threads of a superblock out of L1; what the two
 // octets of a thread share (scales, header words) is unpacked once.
+// The kernel is a programmatic dependent of the launch before it, which hides its launch (decode + GEMM of seven weights of 3 to 48 MB at 32
+// rows: 191 -> 183 us).
 //
 // Measured on B200, 14336 x 4096, us to bf16 / float32, eight weights per thread with byte-wise decoders before -> here:
 // Q4_K 41 / 56 -> 27 / 43 (5.7 / 6.2 TB/s read and written), Q5_K 51 / 56 -> 29 / 45, Q2_K 42 / 70 -> 25 / 42, IQ2_XS 59 / 72 ->
 // 27 / 43, IQ1_S 73 / 83 -> 25 / 41, MXFP4 41 / 65 -> 29 / 43, TQ1_0 101 / 103 -> 28 / 45; instructions, not memory, were the bound.
 // The 2-byte aligned formats read their codes as aligned words (four 2-byte loads per octet: Q6_K 39, Q8_0 34, Q3_K 36 us;
 // two or three words: 33, 31, 31; before all of this 46, 34, 55).
+#include "gemv.cuh"
 #include "ggq_decode.cuh"
 
 namespace ggq {
@@ -62,6 +65,8 @@ template <int QT, int BS, int TS, int OUT>
 __global__ void __launch_bounds__(256)
 dequant_kernel(const uint8_t* __restrict__ blocks, int64_t n_groups, void* __restrict__ out,
                const uint8_t* __restrict__ tab, const bool wide) {
+  pdl_trigger();
+  pdl_wait();                   // the launch before this one may still be reading what is about to be written
   constexpr int GPB = BS / 16;  // groups of 16 elements per block
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= n_groups) return;
@@ -97,8 +102,8 @@ static cudaError_t launch_block(const TypeInfo* ti, const uint8_t* blocks, int64
   int64_t n_groups = n_blocks * (BS / 16);
   if (n_groups == 0) return cudaSuccess;
   int64_t grid = (n_groups + 255) / 256;
-  dequant_kernel<QT, BS, TS, OUT><<<(unsigned)grid, 256, 0, st>>>(blocks, n_groups, out, tab, (uintptr_t)out % 32 == 0);
-  return cudaPeekAtLastError();
+  const cudaError_t err = launch_pdl(dequant_kernel<QT, BS, TS, OUT>, (int)grid, 256, 0, st, blocks, n_groups, out, tab, (uintptr_t)out % 32 == 0);
+  return err != cudaSuccess ? err : cudaPeekAtLastError();
 }
 
 template <int OUT>
