@@ -65,7 +65,6 @@ template <int QT, int BS, int TS, int OUT>
 __global__ void __launch_bounds__(256)
 dequant_kernel(const uint8_t* __restrict__ blocks, int64_t n_groups, void* __restrict__ out,
                const uint8_t* __restrict__ tab, const bool wide) {
-  pdl_trigger();
   pdl_wait();                   // the launch before this one may still be reading what is about to be written
   constexpr int GPB = BS / 16;  // groups of 16 elements per block
   const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,6 +75,7 @@ dequant_kernel(const uint8_t* __restrict__ blocks, int64_t n_groups, void* __res
   Dec<QT>::run(blocks + blk * TS, 2 * g, tab, v);
   Dec<QT>::run(blocks + blk * TS, 2 * g + 1, tab, v + 8);
   store16<OUT>(out, gid, v, wide);
+  pdl_trigger();
 }
 
 // F32 / F16 / BF16 "qtypes": widen (or copy) element-wise, bit-exact

@@ -227,7 +227,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
     for (int m0 = 0; m0 < M && err == cudaSuccess; m0 += tile_max) {
       const int mb = M - m0 < tile_max ? M - m0 : tile_max;
       err = gemv_tile(qtype, (const uint8_t*)w, N, K, (const uint8_t*)x_bf16 + (size_t)m0 * K * 2, mb,
-                      (uint8_t*)y + (size_t)m0 * N * y_item, y_dtype, workspace, workspace_bytes, sm_count_of(dev), nullptr, tab,
+                      (uint8_t*)y + (size_t)m0 * N * y_item, y_dtype, workspace, workspace_bytes, sm_count_of(dev), device_status_word_if_any(dev), tab,
                       st, nullptr);
     }
   } else if (tuned) {

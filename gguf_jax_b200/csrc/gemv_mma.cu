@@ -40,15 +40,32 @@ __device__ __forceinline__ uint32_t pack_hi(float a, float b) {
 }
 __device__ __forceinline__ float trunc_bf16(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFF0000u); }
 
-// Start of every kernel here: the next launch may begin to come in, the first 2 KB of the CTA's sixteen rows are asked into the L2, and only then
-// does it wait for the launch before it, so that a chain of these calls of 4 us each does not also pay for every launch (a 1B-shaped layer at
-// 8 rows, four of its seven products here: 66 -> 57 us).  Nothing is read before the wait.
+// Start of every kernel here: the first 2 KB of the CTA's sixteen rows are asked into the L2 while the launch before this one ends; nothing is
+// read before that.  A CTA lets the next launch in only when its main loop is done: CTAs that come in earlier pile up on the few SMs that are
+// free then (a chain of 2048 x 2048 Q4_K at 8 rows 4.5 us a call without overlap, 7.1 let in at the start).
 __device__ __forceinline__ void begin(const uint8_t* w, int64_t row_bytes, int N) {
-  pdl_trigger();
   const int row = blockIdx.x * 16 + (threadIdx.x >> 4);
   const int64_t off = 128 * (threadIdx.x & 15);
   if (row < N && off < row_bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + row * row_bytes + off));
   pdl_wait();
+}
+
+// Launch with room for as many CTAs per SM as an even spread over the device takes, not more: where the launch before this one leaves its SMs
+// one after the other, the CTAs would otherwise all gather on the first few (2048 x 2048 Q4_K behind a batch kernel of 11 us, both: 19.6 -> 16.0 us).
+template <auto Kernel, class... Args>
+static cudaError_t launch_even(unsigned grid, int sm_count, cudaStream_t st, Args... args) {
+  static std::atomic<bool> attr_done[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_done[dev].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 << 10);
+    if (e != cudaSuccess) return e;
+    attr_done[dev].store(true, std::memory_order_release);
+  }
+  const unsigned per_sm = (grid + sm_count - 1) / sm_count;
+  const size_t smem = per_sm <= 2 ? (228 << 10) / (per_sm + 1) : 0;      // (with more there is less to gain and little left for the L1, where the code books are)
+  const cudaError_t err = launch_pdl(Kernel, (int)grid, kThreads, smem, st, args...);
+  return err != cudaSuccess ? err : cudaPeekAtLastError();
 }
 
 // Split eight float32 weights into three exact bf16 layers, packed as the MMA wants them:
@@ -104,7 +121,7 @@ __device__ __forceinline__ void multiply(const uint8_t* __restrict__ w, int N, i
     for (int c = 0; c < NCG; c++) {
       const int m = 8 * c + g;                          // the batch row this lane feeds as B column g
       uint4 xq = make_uint4(0, 0, 0, 0);
-      if (m < M) xq = __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)m * K + e));
+      if (m < M) xq = __ldca(reinterpret_cast<const uint4*>(x + (int64_t)m * K + e));
 #pragma unroll
       for (int l = 0; l < 3; l++) {
         // k-slots (2t, 2t+1) <- weights 0,1 ; (2t+8, 2t+9) <- weights 2,3 ; second MMA: weights 4..7
@@ -113,6 +130,7 @@ __device__ __forceinline__ void multiply(const uint8_t* __restrict__ w, int N, i
       }
     }
   }
+  pdl_trigger();
 #pragma unroll
   for (int c = 0; c < NCG; c++)
 #pragma unroll
@@ -215,7 +233,7 @@ gemv_mma_q45k_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfl
     for (int c = 0; c < NCG; c++) {
       const int m = 8 * c + g;                          // the batch row this lane feeds as B column g
       r.xq[c] = make_uint4(0, 0, 0, 0);
-      if (m < M) r.xq[c] = __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)m * K + (int64_t)b * 256 + 32 * sbk + 8 * t));
+      if (m < M) r.xq[c] = __ldca(reinterpret_cast<const uint4*>(x + (int64_t)m * K + (int64_t)b * 256 + 32 * sbk + 8 * t));
     }
     return r;
   };
@@ -278,6 +296,7 @@ gemv_mma_q45k_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfl
     }
     cur = nxt;
   }
+  pdl_trigger();
 #pragma unroll
   for (int c = 0; c < NCG; c++)
 #pragma unroll
@@ -353,8 +372,8 @@ gemv_mma_q6k_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bflo
       r.xb[cg] = make_uint2(0, 0);
       if (m < M) {
         const __nv_bfloat16* xp = x + (int64_t)m * K + (int64_t)b * 256 + 32 * warp + 4 * t;
-        r.xa[cg] = __ldcg(reinterpret_cast<const uint2*>(xp));
-        r.xb[cg] = __ldcg(reinterpret_cast<const uint2*>(xp + 16));
+        r.xa[cg] = __ldca(reinterpret_cast<const uint2*>(xp));
+        r.xb[cg] = __ldca(reinterpret_cast<const uint2*>(xp + 16));
       }
     }
     return r;
@@ -403,6 +422,7 @@ gemv_mma_q6k_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bflo
     }
     cur = nxt;
   }
+  pdl_trigger();
 #pragma unroll
   for (int cg = 0; cg < NCG; cg++)
 #pragma unroll
@@ -424,9 +444,11 @@ static cudaError_t launch(const uint8_t* w, int64_t N, int64_t K, const void* x,
                           const uint8_t* tab, int sm_count, cudaStream_t st) {
   const unsigned grid = (unsigned)((N + 15) / 16);
   const bool few = grid <= 2u * (unsigned)sm_count;
-  auto* kernel = M <= 8 ? (few ? gemv_mma_few_kernel<QT, 1> : gemv_mma_8_kernel<QT>) : (few ? gemv_mma_few_kernel<QT, 2> : gemv_mma_16_kernel<QT>);
-  const cudaError_t err = launch_pdl(kernel, (int)grid, kThreads, 0, st, w, (int)N, (int)K, (const __nv_bfloat16*)x, M, y, y_dtype, tab);
-  return err != cudaSuccess ? err : cudaPeekAtLastError();
+  const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
+  if (M <= 8 && few) return launch_even<gemv_mma_few_kernel<QT, 1>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype, tab);
+  if (M <= 8) return launch_even<gemv_mma_8_kernel<QT>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype, tab);
+  if (few) return launch_even<gemv_mma_few_kernel<QT, 2>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype, tab);
+  return launch_even<gemv_mma_16_kernel<QT>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype, tab);
 }
 
 }  // namespace mmav
@@ -442,20 +464,16 @@ cudaError_t gemv_mma(const TypeInfo* ti, const uint8_t* w, int64_t N, int64_t K,
     const unsigned grid = (unsigned)((N + 15) / 16);
     const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
     const bool q5 = ti->qtype == QT_Q5_K;
-    cudaError_t err;
-    if (M <= 8 && !q5) err = launch_pdl(mmav::gemv_mma_q45k_kernel<1, false>, (int)grid, mmav::kThreads, 0, st, w, (int)N, (int)K, xb, M, y, y_dtype);
-    else if (!q5) err = launch_pdl(mmav::gemv_mma_q45k_kernel<2, false>, (int)grid, mmav::kThreads, 0, st, w, (int)N, (int)K, xb, M, y, y_dtype);
-    else if (M <= 8) err = launch_pdl(mmav::gemv_mma_q45k_kernel<1, true>, (int)grid, mmav::kThreads, 0, st, w, (int)N, (int)K, xb, M, y, y_dtype);
-    else err = launch_pdl(mmav::gemv_mma_q45k_kernel<2, true>, (int)grid, mmav::kThreads, 0, st, w, (int)N, (int)K, xb, M, y, y_dtype);
-    return err != cudaSuccess ? err : cudaPeekAtLastError();
+    if (M <= 8 && !q5) return mmav::launch_even<mmav::gemv_mma_q45k_kernel<1, false>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype);
+    if (!q5) return mmav::launch_even<mmav::gemv_mma_q45k_kernel<2, false>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype);
+    if (M <= 8) return mmav::launch_even<mmav::gemv_mma_q45k_kernel<1, true>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype);
+    return mmav::launch_even<mmav::gemv_mma_q45k_kernel<2, true>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype);
   }
   if (ti->qtype == QT_Q6_K && K % 256 == 0 && (uintptr_t)w % 2 == 0) {
     const unsigned grid = (unsigned)((N + 15) / 16);
     const __nv_bfloat16* xb = (const __nv_bfloat16*)x;
-    cudaError_t err;
-    if (M <= 8) err = launch_pdl(mmav::gemv_mma_q6k_kernel<1>, (int)grid, mmav::kThreads, 0, st, w, (int)N, (int)K, xb, M, y, y_dtype);
-    else err = launch_pdl(mmav::gemv_mma_q6k_kernel<2>, (int)grid, mmav::kThreads, 0, st, w, (int)N, (int)K, xb, M, y, y_dtype);
-    return err != cudaSuccess ? err : cudaPeekAtLastError();
+    if (M <= 8) return mmav::launch_even<mmav::gemv_mma_q6k_kernel<1>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype);
+    return mmav::launch_even<mmav::gemv_mma_q6k_kernel<2>>(grid, sm_count, st, w, (int)N, (int)K, xb, M, y, y_dtype);
   }
   cudaError_t err = cudaErrorInvalidValue;
   dispatch_block_qtype(ti->qtype, [&]<int QT>() { err = mmav::launch<QT>(w, N, K, x, M, y, y_dtype, tab, sm_count, st); });

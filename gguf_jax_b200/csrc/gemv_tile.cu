@@ -96,7 +96,7 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
         const int bufs = (int)std::min<int64_t>(span, g.C);
         const bool span_ok = bufs <= kMaxXBufs;
         g.xbufs = bufs;
-        const int fixed = bufs * x_rows * (g.x_row_bytes + g.xs_row_floats * 4) + 64 + (fi.table_bytes + 15) / 16 * 16 + 64 * kMaxXBufs;
+        const int fixed = bufs * x_rows * (g.x_row_bytes + g.xs_row_floats * 4) + 64 + (fi.table_bytes + 15) / 16 * 16 + 64 * kMaxXBufs + kWarps * kMaxDepth * 8;
         const int room = kSmemLimit - fixed;
         // a ring of two slots at least; a warp that has a single step fills one (the tables of the grid formats leave no room for
         // two slots of four superblocks, and the split into smaller steps took longer: IQ2_XXS 8192 x 4096 at 8 rows 24.8 us, 22)
@@ -113,12 +113,18 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
           g.off_zero = g.off_xs + bufs * x_rows * g.xs_row_floats * 4;
           g.off_tab = g.off_zero + 64;
           g.off_misc = g.off_tab + (fi.table_bytes + 15) / 16 * 16;
-          g.total = g.off_misc + 64 * kMaxXBufs;
+          g.off_bar = g.off_misc + 64 * kMaxXBufs;
+          g.total = g.off_bar + kWarps * kMaxDepth * 8;
           // time ~ steps of the busiest warp x (blocks per step + a fixed cost per step) + staging + a flush per
           // unit, in units of one block's multiply; the constants are fitted to B200 timings (8192 x 28672:
-          // nb = 2 with chunks of 16 superblocks is the fastest split for every format)
+          // nb = 2 with chunks of 16 superblocks is the fastest split for every format).  Where steps come as TMA boxes, up to four rows, ranges
+          // that end with units save a segment or two, as long as two thirds of the warps have one (us, 8192 x 8192 at batch 1 with units cut /
+          // whole: IQ2_XS 20.2 / 17.8, Q8_0 19.4 / 15.4; over 112 shapes, formats and batches timed with six splits each, the split picked takes
+          // 0.9 % longer than the best of them, without this term 2.5 %)
           const double steps = (double)warp_steps;
-          const double cost = steps * (nb + 0.6) * (g.depth >= std::min(3, most) ? 1.0 : 1.03) + bufs * g.chunk_sb * x_rows * 0.02 + steps / g.spu * 0.6;
+          const bool whole = g.S % ((int64_t)g.W * g.spu) == 0 && g.W >= 0.65 * sm_count * kWarps;
+          const double cost = steps * (nb + 0.6) * (g.depth >= std::min(3, most) ? 1.0 : 1.03) + bufs * g.chunk_sb * x_rows * 0.02 +
+                              steps / g.spu * 0.6 + (g.row_skew == 0 && M <= 4 && !whole ? 2.0 : 0.0);
           if (cost < best_cost) { best_cost = cost; best = g; }
         }
       }
@@ -189,13 +195,17 @@ cudaError_t gemv_tile(int qtype, const uint8_t* w, int64_t N, int64_t K, const v
     fprintf(stderr, "gemv_tile qtype %d N=%lld K=%lld M=%d: nb=%d chunk=%d spu=%d C=%d RT=%d S=%lld W=%d depth=%d pitch=%d xbufs=%d smem=%d\n",
             qtype, (long long)N, (long long)K, M, geo.nb, geo.chunk_sb, geo.spu, geo.C, geo.RT, (long long)geo.S, geo.W, geo.depth,
             geo.pitch, geo.xbufs, geo.total);
+  const int MP = passes_of(M);
   PeerPublish pp = {};
   if (peers) pp = *peers;
   int* counters = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(ws) + kWsCounterOffset);
   float* slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + kWsGemmPartialOffset);
   const int grid = (geo.W + kWarps - 1) / kWarps;
-  const int MP = passes_of(M);
-  const Args a{&geo, grid, MP, st, w, (int)N, (int)K, x, M, y, y_dtype, counters, slots, &pp, status, tab};
+  alignas(64) CUtensorMap map = {};
+  // (us at batch 1 with cp.async / with boxes: 14336 x 4096 Q8_0 19.3 / 17.5, Q4_0 14.9 / 13.0, IQ4_XS 19.3 / 17.3, MXFP4 19.8 / 17.9, Q2_K 14.3 /
+  // 13.3, IQ2_XS 17.9 / 17.6; at four passes, where copies are the least of it, few-row weights were up to 13 % slower with boxes)
+  geo.tma = geo.row_skew == 0 && MP <= 2 && make_weight_map(&map, w, N, K / 256 * fi.ts, geo.pitch / 4);
+  const Args a{&geo, grid, MP, st, w, (int)N, (int)K, x, M, y, y_dtype, counters, slots, &pp, status, tab, &map};
   switch (qtype) {
     case QT_Q4_K: case QT_Q5_K: case QT_Q6_K: case QT_Q2_K: case QT_Q3_K: case QT_TQ1_0: case QT_TQ2_0: return launch_k(qtype, a);
     case QT_IQ4_XS: case QT_IQ2_XXS: case QT_IQ2_XS: case QT_IQ2_S: case QT_IQ3_XXS: case QT_IQ3_S: case QT_IQ1_S: case QT_IQ1_M:

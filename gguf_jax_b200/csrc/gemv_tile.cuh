@@ -15,9 +15,9 @@
 // a launch is deterministic.
 //
 // Data movement.  Sixteen warps per CTA, one persistent CTA per SM.  A warp streams its own steps
-// (16 rows x nb superblocks) through a private ring of shared-memory slots with 16-byte cp.async
-// copies, one to five steps ahead of the one it is multiplying; consecutive steps of a warp are
-// consecutive bytes of the same 16 rows.  There is no block-wide barrier after the prologue.  Blocks
+// (16 rows x nb superblocks) through a private ring of shared-memory slots, one TMA box of 16 rows a step
+// (16-byte cp.async copies where rows are not 16-byte aligned, at four passes, or without a tensor map), one to
+// five steps ahead of the one it is multiplying; consecutive steps of a warp are consecutive bytes of the same 16 rows.  There is no block-wide barrier after the prologue.  Blocks
 // of most formats are only 2-byte aligned, so a step copies the 16-byte aligned window around its
 // bytes.  Where the rows are whole multiples of 16 bytes apart all rows of a step have the same offset in
 // their windows; otherwise (K / 256 * block bytes not a multiple of 16: Q6_K at K = 2816, the IQ2 formats at
@@ -70,6 +70,8 @@ struct Geo {
   int xs_row_floats;     // sums per batch row and chunk
   int off_x, off_xs, off_zero, off_tab, off_misc, total;
   int row_skew;          // bytes by which consecutive rows differ modulo 16 (0: rows 16-byte aligned)
+  int tma;               // steps come as TMA boxes (rows 16-byte aligned, one or two passes), off_bar: a barrier per warp and slot
+  int off_bar;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -170,11 +172,13 @@ struct GridFill<F, true> {
   static_assert(F::kEntries * kPieces % kThreads == 0, "every thread fills the same number of pieces");
 };
 
-template <class F, int MP>
+// kTma: a step is one TMA box (its own instance: the copy plan of the other costs registers, and 2 to 3 % where only it is used).
+template <class F, int MP, bool kTma>
 __global__ void __launch_bounds__(kThreads, 1)
 gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M,
                  void* __restrict__ y, int y_dtype, int* __restrict__ counters, float* __restrict__ slots,
-                 const Geo geo, const PeerPublish pp, int* __restrict__ status, const uint8_t* __restrict__ tab) {
+                 const Geo geo, const PeerPublish pp, int* __restrict__ status, const uint8_t* __restrict__ tab,
+                 const __grid_constant__ CUtensorMap map) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31;
@@ -205,6 +209,8 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
   // ---- copy side
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t my_ring = smem_base + warp * (geo.slots * geo.slot_bytes);
+  const uint32_t my_bars = smem_base + geo.off_bar + warp * (8 * kMaxDepth);
+  if constexpr (kTma) tma_bars_init(my_bars, depth, lane);
   const int hl = lane >> 4, kl = lane & 15;
   int issued = 0, slot_i = 0;
   int c_i = c0, rt_i = rt0, k_i = k0;
@@ -212,7 +218,12 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
     if (issued < n_steps) {
       const int sb0 = c_i * geo.chunk_sb + k_i * nb;
       const int nbh = min(nb, SB - sb0);
-      if (nbh > 0) {
+      if constexpr (kTma) {
+        // one box of 16 rows: the window that starts on the 16-byte boundary before the step's first block; what lies past the last row or
+        // block arrives as zeros
+        if (lane == 0)
+          tma_box_load(my_ring + slot_i * geo.slot_bytes, &map, (int)(((uint32_t)sb0 * F::kTs & ~15u) >> 2), rt_i * 16, my_bars + 8 * slot_i, geo.slot_bytes);
+      } else if (nbh > 0) {
         const int boff = sb0 * F::kTs;
         const int row0 = rt_i * 16;
         const uint32_t dst0 = my_ring + slot_i * geo.slot_bytes + hl * pitch + 16 * kl;
@@ -260,7 +271,7 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
       if (++slot_i == depth) slot_i = 0;
       if (++k_i == spu) { k_i = 0; if (++rt_i == RT) { rt_i = 0; ++c_i; } }
     }
-    cp_async_commit();
+    if constexpr (!kTma) cp_async_commit();
   };
 
   // ---- shared-memory tables (immutable inputs: may be read before the previous kernel has finished).  A thread's share of the grid
@@ -469,12 +480,14 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
 
   if (active) {
     int c = c0, rt = rt0, k = k0, slot = 0, seg_k = k0;
+    uint32_t phase = 0;
     float out[MP][4];
 #pragma unroll
     for (int p = 0; p < MP; p++) out[p][0] = out[p][1] = out[p][2] = out[p][3] = 0.f;
     for (int i = 0; i < n_steps; i++) {
       issue_next();
-      cp_async_wait_pending(depth - 1);
+      if constexpr (kTma) tma_box_wait(my_bars + 8 * slot, phase, status, lane);
+      else cp_async_wait_pending(depth - 1);
       __syncwarp();
       const int sb0 = c * geo.chunk_sb + k * nb;
       const int nbh = min(nb, SB - sb0);
@@ -554,7 +567,7 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
         }
       }
       __syncwarp();          // every lane is done with the slot before a later copy overwrites it
-      if (++slot == depth) slot = 0;
+      if (++slot == depth) { slot = 0; phase ^= 1; }
 
       // ---- end of a unit, or of this warp's range: the segment's 16 x XR sums go to scratch
       if (k == spu - 1 || i == n_steps - 1) {
@@ -636,39 +649,41 @@ gemv_tile_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat1
       }
     }
   }
-  cp_async_wait_pending(0);
+  if constexpr (!kTma) cp_async_wait_pending(0);
   peer_publish(pp, tid, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------------------------
 // launch
 
-template <class F, int MP>
+template <class F, int MP, bool kTma = false>
 static cudaError_t launch(const Geo& geo, int grid, cudaStream_t st, const uint8_t* w, int N, int K, const void* x, int M,
                           void* y, int y_dtype, int* counters, float* slots, const PeerPublish& pp, int* status,
-                          const uint8_t* tab) {
+                          const uint8_t* tab, const CUtensorMap& map) {
   static std::atomic<bool> attr_done[64];   // setting the attribute twice is harmless, so a flag per device suffices
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_done[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(gemv_tile_kernel<F, MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+    cudaError_t e = cudaFuncSetAttribute(gemv_tile_kernel<F, MP, kTma>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
     if (e != cudaSuccess) return e;
     attr_done[dev].store(true, std::memory_order_release);
   }
-  cudaError_t err = launch_pdl(gemv_tile_kernel<F, MP>, grid, kThreads, (size_t)geo.total, st, w, N, K,
-                               (const __nv_bfloat16*)x, M, y, y_dtype, counters, slots, geo, pp, status, tab);
+  cudaError_t err = launch_pdl(gemv_tile_kernel<F, MP, kTma>, grid, kThreads, (size_t)geo.total, st, w, N, K,
+                               (const __nv_bfloat16*)x, M, y, y_dtype, counters, slots, geo, pp, status, tab, map);
   return err != cudaSuccess ? err : cudaPeekAtLastError();
 }
 
 template <class F>
 static cudaError_t launch_passes(int MP, const Geo& geo, int grid, cudaStream_t st, const uint8_t* w, int N, int K,
                                  const void* x, int M, void* y, int y_dtype, int* counters, float* slots,
-                                 const PeerPublish& pp, int* status, const uint8_t* tab) {
+                                 const PeerPublish& pp, int* status, const uint8_t* tab, const CUtensorMap& map) {
+  if (geo.tma && MP == 1) return launch<F, 1, true>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab, map);
+  if (geo.tma && MP == 2) return launch<F, 2, true>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab, map);
   switch (MP) {
-    case 1: return launch<F, 1>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab);
-    case 2: return launch<F, 2>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab);
+    case 1: return launch<F, 1>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab, map);
+    case 2: return launch<F, 2>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab, map);
     default:
-      if constexpr (four_passes<F>()) return launch<F, 4>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab);
+      if constexpr (four_passes<F>()) return launch<F, 4>(geo, grid, st, w, N, K, x, M, y, y_dtype, counters, slots, pp, status, tab, map);
       else return cudaErrorInvalidValue;
   }
 }
@@ -689,10 +704,11 @@ struct Args {
   const PeerPublish* pp;
   int* status;
   const uint8_t* tab;
+  const CUtensorMap* map;
 };
 template <class F>
 static cudaError_t launch_args(const Args& a) {
-  return launch_passes<F>(a.MP, *a.geo, a.grid, a.st, a.w, a.N, a.K, a.x, a.M, a.y, a.y_dtype, a.counters, a.slots, *a.pp, a.status, a.tab);
+  return launch_passes<F>(a.MP, *a.geo, a.grid, a.st, a.w, a.N, a.K, a.x, a.M, a.y, a.y_dtype, a.counters, a.slots, *a.pp, a.status, a.tab, *a.map);
 }
 cudaError_t launch_k(int qtype, const Args& a);
 cudaError_t launch_iq(int qtype, const Args& a);
