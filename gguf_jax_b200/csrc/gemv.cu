@@ -107,13 +107,14 @@ static bool tile_pays(int64_t N, int64_t K, int M) {
 // worst 1.15 (Q5_K 1515 x 5888 at 6 rows); at 3, 4 rows 0.92, 1.05:
 //   8 rows   4096x4096 Q4_K 13/9.1 Q5_K 14/9.5 IQ2_XS 13/9.6   2048x8192 Q6_K 23/13   8192x8192 Q4_K 24/17 IQ3_S 37/23   700x28672 Q5_K 51/10
 //   16 rows  8192x2048 Q4_K 14/9.4   8192x8192 IQ3_S 82/30 Q2_K 70/25   14336x4096 Q6_K 30/27   but 1024x4096 Q4_K 7.0/9.7, Q5_K 8.0/10
-//   4 rows   16384x1024 Q4_K 7.9/5.6   14336x4096 Q5_K 28/21 Q6_K 32/24   8192x28672 Q4_K 47/47   but 2560x11520 Q4_K 11/13
+//   4 rows   1000x768 Q4_K 7.2/3.5   256x1536 Q4_K 6.5/4.4   1000x1024 Q5_K 8.1/4.8   16384x1024 Q4_K 7.9/5.6   14336x4096 Q5_K 28/21 Q6_K 32/24   8192x28672 Q4_K 47/47   but 2560x11520 Q4_K 11/13
 static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
   const int64_t work = K * (N > 2368 ? N : 2368);
   if (M >= 9) return always || work >= (qtype == QT_Q4_K ? 18ll : qtype == QT_Q5_K ? 14ll : 10ll) << 20;
   if (M >= 5) return always || work >= (qtype == QT_Q4_K ? 12ll : 10ll) << 20;
   if (M < 3) return false;
+  if (is_k_quant(qtype) && K <= 2048 && !(qtype == QT_Q6_K && K % 2048)) return true;        // (its rows not 16-byte aligned: the MMA kernel, 1024 x 1024 3.5 / 5.3)
   if (qtype == QT_Q4_K) return N >= 8192 && K <= 12288;
   if (qtype == QT_Q5_K) return N >= 2048;
   if (qtype == QT_Q6_K) return N >= 2048 && N * K >= 6ll << 20;
