@@ -102,7 +102,8 @@ static bool tile_pays(int64_t N, int64_t K, int M) {
 }
 
 // The batch kernel (gemv_batch.cu) against what served the call before: from 5 rows on it wins wherever the weight is large enough to fill its
-// CTAs (below, one MMA launch), at 3 and 4 rows against two passes of the tiled kernel only where there are rows enough, at 2 nowhere.
+// CTAs (below, one MMA launch), at 3 and 4 rows against two passes of the tiled kernel where there are rows enough or,
+// for K-quants, up to 2048 columns (the tiled kernel takes 5.5 to 8 us for those however few the rows), at 2 nowhere.
 // us before / here, 700 shapes of 1 to 235 M weights timed: at 5..16 rows on average 0.73 of the time, on the wrong side of these lines at
 // worst 1.15 (Q5_K 1515 x 5888 at 6 rows); at 3, 4 rows 0.92, 1.05:
 //   8 rows   4096x4096 Q4_K 13/9.1 Q5_K 14/9.5 IQ2_XS 13/9.6   2048x8192 Q6_K 23/13   8192x8192 Q4_K 24/17 IQ3_S 37/23   700x28672 Q5_K 51/10
@@ -114,7 +115,7 @@ static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
   if (M >= 9) return always || work >= (qtype == QT_Q4_K ? 18ll : qtype == QT_Q5_K ? 14ll : 10ll) << 20;
   if (M >= 5) return always || work >= (qtype == QT_Q4_K ? 12ll : 10ll) << 20;
   if (M < 3) return false;
-  if (is_k_quant(qtype) && K <= 2048 && !(qtype == QT_Q6_K && K % 2048)) return true;        // (its rows not 16-byte aligned: the MMA kernel, 1024 x 1024 3.5 / 5.3)
+  if (is_k_quant(qtype) && K <= 2048 && !(qtype == QT_Q6_K && K % 2048)) return true;        // Q6_K rows not 16-byte aligned stay on the MMA kernel: 1024 x 1024 3.5 there / 5.3 here
   if (qtype == QT_Q4_K) return N >= 8192 && K <= 12288;
   if (qtype == QT_Q5_K) return N >= 2048;
   if (qtype == QT_Q6_K) return N >= 2048 && N * K >= 6ll << 20;
