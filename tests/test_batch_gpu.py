@@ -106,3 +106,16 @@ def test_not_finite(qtype):
     assert np.array_equal(got[inf], want[inf].astype(np.float32))
     fin = np.isfinite(want) & (np.abs(want) < 1e38)
     assert np.allclose(got[fin], want[fin], rtol=1e-4, atol=1e-4 * np.abs(want[:1]).max())
+
+
+@pytest.mark.parametrize("qtype", [QT.Q4_K, QT.Q5_K, QT.Q6_K], ids=lambda t: t.name)
+@pytest.mark.parametrize("k", [256, 1792, 2048, 2304])
+def test_three_and_four_rows_around_the_column_limit(qtype, k):
+    # up to 2048 columns the batch kernel takes these (Q6_K at 2048 only), above it the tiled one; the two rows beside them never
+    for n in (1, 17, 300):
+        wb = synth.make_weight_bytes(n, k, qtype, seed=n)
+        for m in (2, 3, 4):
+            xb = synth.make_x(m, k, seed=m)
+            got = product(xb, wb, qtype, n, k).numpy()
+            assert O.rel_l2(got, O.c_matmul(O.bf16_bits(xb), wb, qtype)) <= 2e-5, (n, k, m)
+            assert np.array_equal(got.view(np.uint32), product(xb, wb, qtype, n, k).numpy().view(np.uint32))
