@@ -38,7 +38,6 @@ SIGNATURES = {
                                      ctypes.c_int32, ctypes.c_void_p]),
     "ggq_has_fused": (ctypes.c_int32, [ctypes.c_int32]),
     "ggq_fused_batch_limit": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64]),
-    "ggq_route_batch_limit": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64]),
     "ggq_gemv_max_batch": (ctypes.c_int32, []),
     "ggq_workspace_bytes": (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32]),
     "ggq_scratch_bytes": (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32]),
@@ -146,7 +145,7 @@ def native():
                     warnings.warn(f"matmul takes its slower Python call path: {e} (build it with `python -m gguf_jax_b200.build`)")
                     module = _PythonPath
                 else:
-                    entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_route_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info,
+                    entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_fused_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info,
                                L.ggq_dequant)
                     module.bind(*[ctypes.cast(f, ctypes.c_void_p).value for f in entries], int(L.ggq_gemv_max_batch()))
                 _native_module = module

@@ -68,21 +68,10 @@ def fused_types() -> list[QT]:
 
 
 def fused_batch_limit(w: QuantizedArray) -> int:
-    """Largest flattened batch at which :func:`matmul` multiplies ``w`` without
-    materializing it (0: never).  Above 32 rows, where both routes round the weights to bfloat16, activations on the device take the
-    dense route earlier where that is faster and the copy is small (at most 128 MB, in one slab); ``force_fused`` does not."""
+    """Largest flattened batch at which :func:`matmul` still multiplies ``w`` without
+    materializing it (0: never)."""
     hit = _fused().get(w.qtype)
     return hit[1](w) if hit is not None and len(w.shape) == 2 else 0
-
-
-@functools.lru_cache(maxsize=4096)
-def _route_limit_of(code: int, n: int, k: int) -> int:
-    return int(_lib.lib().ggq_route_batch_limit(code, n, k))
-
-
-def _route_limit(w: QuantizedArray) -> int:
-    """Largest flattened batch of device tensors that :func:`matmul` multiplies fused where the dense copy may be in one piece."""
-    return _route_limit_of(int(w.qtype), *w.shape)
 
 
 def _native_matmul(*args):
@@ -110,7 +99,7 @@ def matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None
     """``x (..., K) @ w(N, K).T -> (..., N)``.
 
     Fused when ``w.qtype`` has a kernel, ``x`` is bfloat16 and the flattened batch does not
-    exceed :func:`fused_batch_limit` (see there for where the dense route is faster); ``force_fused=True`` skips the batch test (the kernels
+    exceed :func:`fused_batch_limit`; ``force_fused=True`` skips the batch test (the kernels
     accept any batch; beyond the limit they are merely slower than materializing).  Everything
     else is materialized under the ``block_bytes`` budget (default
     :data:`DEQUANT_BLOCK_BYTES`).  ``TypeError`` for a weight that is not a
@@ -136,8 +125,6 @@ def matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None
         batch = math.prod(x.shape[:-1])
         if force_fused or batch <= hit[1](w):
             route = hit[0]
-            if not force_fused and out is None and x.is_cuda and batch > _route_limit(w) and _slab_count(w, block_bytes) == 1:
-                route = None            # faster by a dense copy
     if out is not None or not x.is_cuda:
         _backend.require_cuda(w.data, "matmul")
         if route is None:

@@ -57,20 +57,6 @@ extern "C" int32_t ggq_fused_batch_limit(int32_t qtype, int64_t N, int64_t K) {
   return kGemvMaxBatch;
 }
 
-// Where matmul of device tensors changes to decode + library GEMM: between 33 rows and the limit above both round the weights to bf16, so
-// speed decides.  Only weights of up to 2^26 elements (a decoded copy of at most 128 MB, which the L2 mostly holds) in a multiple of 8 rows (the
-// library's kernels for others are slower).  us on the device at 64 / 128 / 192 / 256 / 384 / 512 rows, fused and fallback: Q6_K 4096 x 4096 24 / 30 / 43 / 45 /
-// 50 / 52 and 16 / 16 / 17 / 18 / 20 / 22, 6144 x 6144 41 / 43 / 58 / 58 / 91 / 93 and 33 / 33 / 38 / 38 / 43 / 49, 8192 x 8192 58 / 63 / 77 / 78 / 112 / 129 and 61 / 59 / 64 / 67 /
-// 73 / 81, 14336 x 4096 52 / 54 / 61 / 61 / 76 / 78 and 52 / 52 / 59 / 60 / 67 / 78; Q4_K 6144 x 6144 30 / 36 / 50 / 51 / 81 / 84 and 30 / 30 / 35 / 35 / 40 / 46,
-// 4096 x 14336 40 / 46 / 62 / 64 / 88 / 89 and 52 / 53 / 64 / 58 / 67 / 74, 14336 x 4096 36 / 38 / 45 / 45 / 63 / 64 and 47 / 47 / 54 / 55 / 62 / 73.
-extern "C" int32_t ggq_route_batch_limit(int32_t qtype, int64_t N, int64_t K) {
-  const int32_t limit = ggq_fused_batch_limit(qtype, N, K);
-  if (limit <= kWideRouterBatch || N % 8 || N * K > 1ll << 26) return limit;
-  const bool small = N * K < 45ll << 20, tall = N >= 96 * 128;
-  const int32_t route = qtype == QT_Q6_K ? (small ? 32 : tall ? 256 : 64) : small ? 64 : tall ? limit : 192;
-  return route < limit ? route : limit;
-}
-
 static int sm_count_of(int dev) { return device_sm_count(dev); }
 
 // The formats whose batches up to 16 run without any scratch when none is given (streaming and MMA kernels); the tiled

@@ -140,7 +140,7 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(gemv, gemm, route_batch_limit, scratch_bytes, has_fused, type_info, dequant, gemv_max_batch): entry point addresses
+// bind(gemv, gemm, fused_batch_limit, scratch_bytes, has_fused, type_info, dequant, gemv_max_batch): entry point addresses
 PyObject* bind(PyObject*, PyObject* args) {
   unsigned long long gemv, gemm, limit, bytes, fused, info, dequant;
   int max_batch;

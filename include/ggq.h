@@ -93,10 +93,6 @@ int32_t ggq_has_fused(int32_t qtype);
  * (src/gguf_jax/_matmul.py:60-75, cute/q4_k.py:117-118, cute/lowbit.py:97). */
 int32_t ggq_fused_batch_limit(int32_t qtype, int64_t N, int64_t K);
 
-/* The same for activations and results in device memory and a dense copy of the weight that may be made in one piece: above 32
- * rows, where both routes round the weights to bf16, the faster one may end earlier.  Never above ggq_fused_batch_limit. */
-int32_t ggq_route_batch_limit(int32_t qtype, int64_t N, int64_t K);
-
 /* Largest M served by the small-batch (GEMV) kernel; above it ggq_gemm is used. */
 int32_t ggq_gemv_max_batch(void);
 
