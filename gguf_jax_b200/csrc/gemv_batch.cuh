@@ -145,7 +145,7 @@ __device__ __noinline__ void more_planes(uint32_t blk0, uint32_t blk1, tf::Table
 
 template <class F, int NT>
 __global__ void __launch_bounds__(kThreads, 1)
-gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M, void* __restrict__ y, int y_dtype,
+gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M, void* __restrict__ y, int y_dtype, int ldy,
                   const Geo geo, const uint8_t* __restrict__ tab, int* __restrict__ status, const __grid_constant__ CUtensorMap map) {
   typedef typename F::Base B;
   constexpr int XR = 8 * NT, kXTile = x_tile_bytes<F>(), kXBlock = NT * kXTile;
@@ -499,14 +499,14 @@ gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int row = (tile_lo + tile) * 16 + g + 8 * (i >> 1), m = n * 8 + 2 * t + (i & 1);
-        if (row < N && m < M) { store_out(y, y_dtype, (int64_t)m * N + row, v[n][i]); bad |= not_finite(v[n][i]); }
+        if (row < N && m < M) { store_out(y, y_dtype, (int64_t)m * ldy + row, v[n][i]); bad |= not_finite(v[n][i]); }
       }
     if (__any_sync(0xFFFFFFFFu, bad)) {          // outputs that are not finite
 #pragma unroll 1
       for (int j = 0; j < 4 * NT; j++) {
         const int row = (tile_lo + tile) * 16 + g + 8 * ((j >> 1) & 1), m = (j >> 2) * 8 + 2 * t + (j & 1);
-        const bool again = row < N && m < M && not_finite(load_out(y, y_dtype, (int64_t)m * N + row));
-        recompute<B::kQt>(again, row, m, w, (int64_t)row_bytes, N, x, K, tab, y, y_dtype);
+        const bool again = row < N && m < M && not_finite(load_out(y, y_dtype, (int64_t)m * ldy + row));
+        recompute<B::kQt>(again, row, m, w, (int64_t)row_bytes, ldy, x, K, tab, y, y_dtype);
       }
     }
   }
@@ -523,7 +523,7 @@ struct Args {
   const void* x;
   int M;
   void* y;
-  int y_dtype;
+  int y_dtype, ldy;
   const uint8_t* tab;
   int* status;
   const CUtensorMap* map;
@@ -551,7 +551,7 @@ static cudaError_t launch(const Args& a) {
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.geo->Q > 1 ? 2 : 1;
-  cudaError_t err = cudaLaunchKernelEx(&cfg, gemv_batch_kernel<F, NT>, a.w, a.N, a.K, (const __nv_bfloat16*)a.x, a.M, a.y, a.y_dtype, (const Geo)*a.geo,
+  cudaError_t err = cudaLaunchKernelEx(&cfg, gemv_batch_kernel<F, NT>, a.w, a.N, a.K, (const __nv_bfloat16*)a.x, a.M, a.y, a.y_dtype, a.ldy, (const Geo)*a.geo,
                                        a.tab, a.status, *a.map);
   return err != cudaSuccess ? err : cudaPeekAtLastError();
 }

@@ -1,0 +1,31 @@
+"""The kernels of this library that a call launches, by name, in order: the call is captured into a CUDA graph, which is read and never run."""
+import ctypes
+
+import torch
+
+
+def kernels_of(call):
+    call()                                       # scratch, code books and attributes, which a first call sets up
+    torch.cuda.synchronize()
+    cu = ctypes.CDLL("libcuda.so.1")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    handle, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t()
+    assert cu.cuGraphGetNodes(handle, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert cu.cuGraphGetNodes(handle, nodes, ctypes.byref(count)) == 0
+    names = []
+    for node in nodes:
+        kind, name = ctypes.c_int(), ctypes.c_char_p()
+        assert cu.cuGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        if kind.value != 0:                      # CU_GRAPH_NODE_TYPE_KERNEL
+            continue
+        params = (ctypes.c_uint64 * 16)()        # CUDA_KERNEL_NODE_PARAMS: func first, kern after 7 ints (padded) and two pointers
+        assert cu.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(node), params) == 0
+        func, kern = params[0], params[7]
+        assert (cu.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(func)) if func else
+                cu.cuKernelGetName(ctypes.byref(name), ctypes.c_void_p(kern))) == 0
+        if b"ggq" in name.value:
+            names.append(name.value.decode())
+    return names

@@ -1,11 +1,14 @@
 """Which way a call of `matmul` goes: up to `fused_batch_limit` the fused kernels multiply, whatever dtype the weight decodes to and whoever
-decodes it, and their result is bfloat16; above, the dense copy."""
+decodes it, and their result is bfloat16; above, the dense copy.  And which of the fused kernels takes it."""
+import numpy as np
 import pytest
 import torch
 from gguf.constants import GGMLQuantizationType as QT
 
 import gguf_jax_b200 as gj
 from gguf_jax_b200 import kernels, quants, synth
+from oracle import oracle as O
+from tests.launched import kernels_of
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +44,33 @@ def test_a_registered_decoder_serves_the_dense_route_only():
         assert len(calls) == 1
     finally:
         gj.register_dequant(QT.Q6_K, saved, override=True)
+
+
+# the batch kernel's formats but the K-quants
+LOWBIT = [QT.Q2_K, QT.Q3_K, QT.IQ4_XS, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT.IQ3_XXS, QT.IQ3_S, QT.IQ1_S, QT.IQ1_M, QT.TQ1_0, QT.TQ2_0]
+
+
+@pytest.mark.parametrize("qtype,n,k,m", [(qt, 600_011, 256, 16) for qt in LOWBIT + [QT.Q4_K, QT.Q5_K, QT.Q6_K]] +
+                         [(QT.IQ3_S, 256_000, 2048, 9), (QT.Q2_K, 1_300_003, 256, 5)], ids=str)
+def test_weights_of_very_many_rows_are_cut(qtype, n, k, m):
+    """Too many rows for one launch of the batch kernel, which keeps every tile's sums: parts of rows, each multiplied by it, and the
+    outputs that are not finite computed again in every part.  Same bar as for one launch (test_batch_gpu.py)."""
+    w = synth.make_weight_on_device(n, k, qtype, seed=3, device="cuda")
+    xb = synth.make_x(m, k, seed=m)
+    xb[1, 3] = np.inf
+    x = torch.from_numpy(xb).cuda().to(torch.bfloat16)
+    product = lambda: kernels.fused_matmul(x, w, out_dtype=torch.float32)
+    names = kernels_of(product)
+    assert 2 <= len(names) <= 4 and all("gemv_batch_kernel" in name for name in names), names
+    # the first and last rows, the tiles around every place where the parts may meet, and some rows between
+    tiles = -(-n // 16)
+    cuts = [16 * -(-tiles // parts) * i for parts in (2, 3, 4) for i in range(1, parts)]
+    pick = np.unique(np.clip(np.concatenate([np.arange(16), *[c + np.arange(-17, 18) for c in cuts], n - 1 - np.arange(17),
+                                             np.random.default_rng(0).integers(0, n, 64)]), 0, n - 1))
+    rows = w.data[torch.from_numpy(pick).cuda()].cpu().numpy()
+    got = product()[:, torch.from_numpy(pick).cuda()].cpu().numpy()
+    fine = np.arange(m) != 1
+    assert O.rel_l2(got[fine], O.c_matmul(O.bf16_bits(xb[fine]), rows, qtype)) <= 2e-5
+    column = O.c_dequantize(rows, qtype).reshape(len(pick), k)[:, 3]
+    assert np.array_equal(np.isnan(got[1]), column == 0)
+    assert np.array_equal(got[1][column != 0], np.sign(column[column != 0]) * np.inf)
