@@ -108,6 +108,15 @@ static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
   return N >= 10240 && K <= 8192 && N * K >= 14ll << 20;
 }
 
+// Q6_K takes two products per weight in the batch kernel, and from 9 rows on its activations come in several passes where K is long, the sums of
+// many rows leave little room for the copies, and the batch-major kernel, which streams both, is the faster one.  (Rows that are not 16-byte
+// aligned slow that one down: they stay.)  us at 16 rows, batch-major / batch: 4096 x 16384 35/36, 6144 x 16384 43/47, 4096 x 20480 41/43, 8192 x 28672 86/95;
+// 8192 x 14336 51/50, 10240 x 14336 59/61, 20480 x 10240 74/79; 28672 x 8192 81/80, 32000 x 8192 87/95, 152064 x 8192 359/384; 65536 x 4096 88/84,
+// 128256 x 4096 160/162, 256000 x 2048 161/167.  On the wrong side of these lines: 14336 x 8192 48/50.
+static bool wide_beats_batch(int qtype, int64_t N, int64_t K, int M) {
+  return qtype == QT_Q6_K && M >= 9 && K % 2048 == 0 && N * K >= (K >= 16384 ? 72ll : K > 8192 ? 120ll : K == 8192 ? 240ll : 384ll) << 20;
+}
+
 static size_t tile_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
   const int tmax = gemv_tile_max_batch(qtype);
   return tmax && M <= kGemvMaxBatch && K % 256 == 0 ? gemv_tile_workspace_bytes(qtype, N, K, M < tmax ? M : tmax) : 0;
@@ -218,7 +227,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const bool wide_ok = k_quant && M >= wide_min && (odd_rows ? weights >= (K < 1536 ? 21ll : 12ll) << 20 : wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes)) && workspace && (uintptr_t)workspace % 256 == 0 && sm_count_of(dev) > 0 &&
                        workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, M, sm_count_of(dev)) &&
                        gemv_wide_applicable(qtype, N, K, M, w, x_bf16);
-  if (batch_ok) {
+  if (batch_ok && !(wide_ok && wide_beats_batch(qtype, N, K, M))) {
     err = gemv_batch(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, sm_count_of(dev), device_status_word_if_any(dev), tab, st);
   } else if (wide_ok) {
     err = gemv_wide(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, workspace, workspace_bytes, sm_count_of(dev), st, 0, nullptr,

@@ -74,3 +74,20 @@ def test_weights_of_very_many_rows_are_cut(qtype, n, k, m):
     column = O.c_dequantize(rows, qtype).reshape(len(pick), k)[:, 3]
     assert np.array_equal(np.isnan(got[1]), column == 0)
     assert np.array_equal(got[1][column != 0], np.sign(column[column != 0]) * np.inf)
+
+
+@pytest.mark.parametrize("qtype,n,k,m,kernel", [
+    # Q6_K from 9 rows on: the batch-major kernel from a number of weights on that falls with the columns
+    (QT.Q6_K, 8192, 20480, 9, "wide"), (QT.Q6_K, 8192, 20480, 8, "batch"), (QT.Q6_K, 4096, 16384, 16, "batch"), (QT.Q6_K, 20480, 10240, 16, "wide"),
+    (QT.Q6_K, 32000, 8192, 16, "wide"), (QT.Q6_K, 28672, 8192, 9, "batch"), (QT.Q6_K, 65536, 4096, 16, "batch"),
+    (QT.Q6_K, 8000, 20736, 16, "batch"), (QT.Q5_K, 8192, 20480, 16, "batch"),
+], ids=str)
+def test_kernel_of_a_call(qtype, n, k, m, kernel):
+    w = synth.make_weight_on_device(n, k, qtype, seed=4, device="cuda")
+    xb = synth.make_x(m, k, seed=m)
+    x = torch.from_numpy(xb).cuda().to(torch.bfloat16)
+    product = lambda: kernels.fused_matmul(x, w, out_dtype=torch.float32)
+    names = kernels_of(product)
+    assert any(f"gemv_{kernel}" in name for name in names), names
+    pick = torch.from_numpy(np.random.default_rng(0).choice(n, size=48, replace=False)).cuda()
+    assert O.rel_l2(product()[:, pick].cpu().numpy(), O.c_matmul(O.bf16_bits(xb), w.data[pick].cpu().numpy(), qtype)) <= 2e-5
