@@ -31,12 +31,15 @@ from .array import QuantizedArray
 __all__ = ["dequant_matmul", "fused_batch_limit", "fused_types", "matmul"]
 
 # Byte budget of one dense slab.  The reference's environment knob and default are kept
-# (src/gguf_jax/_matmul.py:39-44).  There a slab is costed at 4 bytes per weight, and so it is here under a ``block_bytes`` that the caller
-# gives; under this default it is costed at what it takes, 2 bytes where the weight is decoded to bfloat16, because every slab is a launch of
+# (src/gguf_jax/_matmul.py:39-44).  There a slab is costed at 4 bytes per weight, and so it is here under a budget that somebody set,
+# ``block_bytes`` or this one; under the default a slab that the GEMM reads as it was decoded (no conversion to the type of ``x``, no
+# autocast) is costed at the 2 bytes a bfloat16 weight takes, because every slab is a launch of
 # the library GEMM that starts and ends with its tensor cores partly idle (us, 28672 x 8192 Q4_K at 2048 rows, two slabs / one: 935 / 887, in
-# CUDA graphs 842 / 734).  Not for weights whose number of rows is no multiple of 8: in one piece the library multiplies them with kernels that
+# CUDA graphs 842 / 734; 17 to 2048 rows of ten weights of 134 to 268 M elements: 0.80 to 1.03 of the time, results equally far from the
+# exact product).  Not for weights whose number of rows is no multiple of 8: in one piece the library multiplies them with kernels that
 # are slower and add partial sums in bfloat16 (9972 x 23552 at 83 rows: 251 / 317 us, 0.0023 / 0.0049 off the exact product).
-DEQUANT_BLOCK_BYTES = int(os.environ.get("GGUF_JAX_DEQUANT_BLOCK_BYTES", 512 << 20))
+_DEFAULT_BLOCK_BYTES = 512 << 20
+DEQUANT_BLOCK_BYTES = int(os.environ.get("GGUF_JAX_DEQUANT_BLOCK_BYTES", _DEFAULT_BLOCK_BYTES))
 
 FusedEntry = tuple[Callable[..., torch.Tensor], Callable[[QuantizedArray], int]]
 
@@ -113,7 +116,9 @@ def matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None
     if out is None and w.__class__ is QuantizedArray and not _function_modes():
         # the common call (device activations, no gradient; fused, or dense in one piece by the built-in bf16 decoder) is one
         # native function
-        budget = 2 * DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes       # of a copy costed at 4 bytes a weight
+        budget = DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes           # of a copy costed at 4 bytes a weight
+        if block_bytes is None and budget == _DEFAULT_BLOCK_BYTES:
+            budget *= 2                 # see there
         y = _native_matmul(x, w.data, w.qtype, w.shape, force_fused,
                            budget if w.dtype is torch.bfloat16 and not quants._replaced else 0)
         if y is not None:
@@ -132,7 +137,7 @@ def matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None
                              f"(bfloat16 x, a fused qtype, batch within fused_batch_limit); got {w.qtype.name}, {x.dtype}, "
                              f"batch {math.prod(x.shape[:-1])}")
         return route(x, w, out=out)
-    return _apply(x, w, route, _slab_count(w, block_bytes))
+    return _apply(x, w, route, _slab_count(x, w, block_bytes))
 
 
 def dequant_matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | None = None) -> torch.Tensor:
@@ -141,7 +146,7 @@ def dequant_matmul(x: torch.Tensor, w: QuantizedArray, *, block_bytes: int | Non
     ``x.dtype`` and ``w.dtype``."""
     if not isinstance(w, QuantizedArray):
         raise TypeError(f"expected a QuantizedArray weight, got {type(w).__name__}")
-    return _apply(x, w, None, _slab_count(w, block_bytes))
+    return _apply(x, w, None, _slab_count(x, w, block_bytes))
 
 
 # ---------------------------------------------------------------------------------------------
@@ -154,10 +159,13 @@ def _block_count(out_rows: int, in_features: int, budget: int, itemsize: int = 4
     return next((d for d in range(slabs_wanted, out_rows) if out_rows % d == 0), out_rows) if slabs_wanted > 1 else 1
 
 
-def _slab_count(w: QuantizedArray, block_bytes: int | None) -> int:
-    if block_bytes is None and w.shape[0] % _ROW_ELEMS == 0:
-        return _block_count(w.shape[0], w.shape[1], DEQUANT_BLOCK_BYTES, min(4, w.dtype.itemsize))
-    return _block_count(w.shape[0], w.shape[1], DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes)
+def _slab_count(x: torch.Tensor, w: QuantizedArray, block_bytes: int | None) -> int:
+    budget = DEQUANT_BLOCK_BYTES if block_bytes is None else block_bytes
+    count = _block_count(w.shape[0], w.shape[1], budget)
+    if (count > 1 and block_bytes is None and budget == _DEFAULT_BLOCK_BYTES and w.shape[0] % _ROW_ELEMS == 0
+            and torch.promote_types(x.dtype, w.dtype) == w.dtype and not torch.is_autocast_enabled(x.device.type)):
+        return _block_count(w.shape[0], w.shape[1], budget, min(4, w.dtype.itemsize))
+    return count
 
 
 def _slabs(w: QuantizedArray, count: int, rows: int | None = None):

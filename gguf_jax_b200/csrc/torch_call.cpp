@@ -15,6 +15,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/TensorSubclassLikeUtils.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/core/grad_mode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -109,7 +110,8 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     // the dense route in one piece: decode to bf16, library GEMM (rows of the result on 16-byte boundaries)
     const double budget = PyFloat_AsDouble(args[5]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
-    if (n % 8 || 4.0 * (double)n * (double)k > budget) Py_RETURN_NONE;
+    // (autocast converts the copy: what then still fits is for the Python path to say)
+    if (n % 8 || (at::autocast::is_autocast_enabled(at::kCUDA) ? 8.0 : 4.0) * (double)n * (double)k > budget) Py_RETURN_NONE;
     at::Tensor y;
     {
       WithoutGil no_gil;

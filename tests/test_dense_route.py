@@ -112,3 +112,33 @@ def test_transforms_traces_and_modes_take_the_general_way(n, budget, padded, mon
         y = product(x)
     assert torch.ops.aten.mm.out not in mode.seen and torch.ops.aten.mm.default in mode.seen
     assert torch.allclose(y, x @ dense.T)
+
+
+@pytest.mark.parametrize("x_dtype,w_dtype,slabs", [
+    (torch.bfloat16, torch.bfloat16, 1), (torch.float16, torch.float16, 1),      # multiplied as decoded: 2 bytes a weight
+    (torch.float32, torch.bfloat16, 2), (torch.float16, torch.bfloat16, 2), (torch.bfloat16, torch.float16, 2),    # converted as well
+    (torch.bfloat16, torch.float32, 2), (torch.float32, torch.float32, 2)], ids=str)
+def test_slabs_are_costed_at_what_they_take(x_dtype, w_dtype, slabs, monkeypatch):
+    """Weights of 64 rows where 32 fit at 4 bytes a weight: under the default budget whole where the GEMM reads the decoded copy itself;
+    under autocast, where the number of rows is no multiple of 8 and under a budget that somebody set, at 4 bytes as ever."""
+    calls = []
+    decode = quants._DEQUANT[QT.Q8_0]
+    monkeypatch.setitem(quants._DEQUANT, QT.Q8_0, lambda blocks, dtype: (calls.append(len(blocks)), decode(blocks, dtype))[1])
+
+    def decoded(n, **kw):
+        calls.clear()
+        w, x = case(n)
+        x = x.to(x_dtype)
+        y = gj.dequant_matmul(x, w.astype(w_dtype), **kw)
+        dense = w.astype(w_dtype).dequantize()
+        del calls[-1]
+        assert torch.allclose(y.double(), x.double() @ dense.double().T, rtol=2 ** -7, atol=0.2)
+        return len(calls)
+
+    monkeypatch.setattr(mm, "DEQUANT_BLOCK_BYTES", IN_SLABS)
+    assert decoded(64) == 2 and decoded(64, block_bytes=IN_SLABS) == 2
+    monkeypatch.setattr(mm, "_DEFAULT_BLOCK_BYTES", IN_SLABS, raising=False)
+    assert decoded(64) == slabs and decoded(64, block_bytes=IN_SLABS) == 2
+    assert decoded(68) >= 3                      # one row more than two slabs of 32 take; never in one
+    with torch.autocast("cpu", dtype=torch.bfloat16):
+        assert decoded(64) == 2

@@ -60,3 +60,24 @@ def test_transforms_take_the_general_way():
         mapped = torch.func.vmap(lambda a: gj.dequant_matmul(a, w, block_bytes=block_bytes))(x)
         assert rel(mapped, x @ dense.T) <= 1e-5
     assert rel(gj.dequant_matmul(x, w, block_bytes=budget), x @ dense.T) <= 1e-5
+
+
+@pytest.mark.parametrize("case", ["float32 x", "autocast", "gradient", "bfloat16"])
+def test_memory_of_a_large_weight(case):
+    """20480 x 8192: 672 MB at 4 bytes a weight, the default budget 537 MB.  Alive at once is one bf16 slab (336 MB whole), and where it is
+    converted its copy: two slabs then, 168 MB each and 336 (to float32) or 168 (to float16) MB more."""
+    n, k, m = 20480, 8192, 64
+    w = synth.make_weight_on_device(n, k, QT.Q8_0, seed=1, device="cuda")
+    x = torch.randn((m, k), device="cuda").to(torch.bfloat16)
+    dtype = torch.float32 if case in ("float32 x", "gradient") else torch.bfloat16
+    x = x.to(dtype).requires_grad_(case == "gradient")
+    gj.matmul(x[:, :k], w)                  # the library's workspace
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    base = torch.cuda.memory_allocated()
+    with torch.autocast("cuda", dtype=torch.float16, enabled=case == "autocast"):
+        y = gj.matmul(x, w)
+    if case == "gradient":
+        torch.autograd.grad(y, x, y.detach())
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - base <= 560 << 20
