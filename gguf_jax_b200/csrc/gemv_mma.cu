@@ -62,7 +62,8 @@ static cudaError_t launch_even(unsigned grid, int sm_count, cudaStream_t st, Arg
     if (e != cudaSuccess) return e;
     attr_done[dev].store(true, std::memory_order_release);
   }
-  const unsigned per_sm = (grid + sm_count - 1) / sm_count;
+  const unsigned sms = sm_count > 0 ? (unsigned)sm_count : 1;            // (0 where the device would not say)
+  const unsigned per_sm = (grid + sms - 1) / sms;
   const size_t smem = per_sm <= 2 ? (228 << 10) / (per_sm + 1) : 0;      // (with more there is less to gain and little left for the L1, where the code books are)
   const cudaError_t err = launch_pdl(Kernel, (int)grid, kThreads, smem, st, args...);
   return err != cudaSuccess ? err : cudaPeekAtLastError();
