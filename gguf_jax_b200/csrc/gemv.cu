@@ -17,11 +17,8 @@ inline int tuned_max_repeat(int qtype, int64_t weight_bytes) {
   return weight_bytes < (24ll << 20) ? 1 : weight_bytes < (80ll << 20) ? 2 : 3;
 }
 inline bool is_k_quant(int qtype) { return qtype == QT_Q4_K || qtype == QT_Q5_K || qtype == QT_Q6_K; }
-// The batch-major kernel (gemv_wide.cu) costs two launches and a partial-sum settle, about 10 us on a weight
-// of a few MB, and then very little per batch row; the integer-code MMA kernel (gemv_mma.cu) starts at 4 us
-// and grows with the weight.  Measured crossover on B200 at 5..16 batch rows: about 20 MB for Q4_K / Q5_K
-// (8192 x 2048 and 4096 x 4096, 9 MB: 10-12 us against 14-18 us; 14336 x 4096, 33 MB: 28-35 us against 24-27 us),
-// about 10 MB for Q6_K (4096 x 4096, 14 MB: 20 us either way).
+// From which size on the batch-major kernel (gemv_wide.cu) takes 17 to 32 batch rows: it costs two launches and a partial-sum
+// settle, about 10 us on a weight of a few MB, and then very little per batch row (against decode + library GEMM, below).
 inline bool wide_pays(int qtype, int64_t weight_bytes) {
   return weight_bytes >= (qtype == QT_Q6_K ? (10ll << 20) : (20ll << 20));
 }
@@ -184,7 +181,7 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
   if (ti->needs_tables && !tab)
     return fail(GGQ_NO_TABLES, "ggq_gemv: call ggq_set_tables(%d, ...) before using qtype %d", dev, qtype);
   cudaStream_t st = (cudaStream_t)stream;
-  cudaError_t err;
+  cudaError_t err = cudaSuccess;
   // The tuned batch-1 kernels (Q4_K, Q5_K, Q6_K).  A few batch rows are served by that many
   // launches of the batch-1 kernel, which is still faster than the small-batch kernel.
   const int y_item = y_dtype == GGQ_F32 ? 4 : 2;
@@ -200,47 +197,53 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
     else if (qtype == QT_Q6_K && gemv_q6k_applicable(N, K, 1, w, x_bf16)) tuned = gemv_q6k;
   }
   static const bool m1_tiled = [] { const char* e = getenv("GGQ_Q4K_M1_TILED"); return e && e[0] == '1'; }();
-  // Q4_K / Q5_K / Q6_K keep their batch-1 kernels; the tiled kernel takes their batches 2..4 whatever the size (it scales each
-  // row and keeps any magnitude; the integer-code MMA kernel keeps about 2^-50 to 2^62; Q4_K 8192 x 28672:
-  // 36 / 49 us at batch 2 / 4) and the other formats where tile_pays says so; from five batch rows on
-  // the batch-major kernel takes the larger weights (Q4_K 8192 x 28672: 56 / 65 us at batch 8 / 16 against
-  // 100 / 153 us) and the integer-code MMA kernel (gemv_mma.cu) the smaller ones (see wide_pays).
+  // Q4_K / Q5_K / Q6_K keep their batch-1 kernels; the tiled kernel takes their batches of 2 (and of 3 and 4 where batch_pays does not hold)
+  // whatever the size (it scales each row and keeps any magnitude; the integer-code MMA kernel keeps about 2^-50 to 2^62) and the other formats
+  // where tile_pays says so; the batch kernel takes what batch_pays says (8192 x 28672 Q4_K at 8 / 16 rows 37 / 51 us), the MMA kernel
+  // the smaller weights.  The batch-major kernel (56 / 65 us) is left with large Q6_K weights and with what the batch kernel has no plan for
+  // (more than 2^31 bytes, or a few hundred thousand columns).
   const bool k_quant = is_k_quant(qtype);
   // rows that are not 16-byte aligned (Q6_K among the K-quants): the batch-1 kernel does not take them; streaming and
   // MMA kernel against the tiled one cross where they do for the other formats (us, other / tiled: 512 x 1280 at 1 / 2 / 4 rows 3.3/6.5
   // 4.6/6.6 4.6/8.2, 512 x 5376 8.4/7.4 12.5/7.6 12.9/10.1, 4096 x 1280 4.9/6.9 6.3/7.1 6.5/8.6)
   const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
-  const int64_t weights = N * K;
   const bool tile_first = k_quant && !odd_rows ? (M >= 2 && M <= 4) || (M == 1 && m1_tiled)
                                                : (!k_quant || M <= 4) && tile_pays(N, K, M);
-  // (GGQ_GEMM_KERNEL=wide pins the batch-major kernel here as in ggq_gemm)
-  const char* pin = k_quant ? getenv("GGQ_GEMM_KERNEL") : nullptr;
-  const bool batch_ok = batch_pays(qtype, N, K, M) && !(pin && !strcmp(pin, "wide")) &&
-                        gemv_batch_applicable(qtype, N, K, M, w, x_bf16, sm_count_of(dev));
-  const int tile_max = gemv_tile_max_batch(qtype);
-  const int tile_m = M < tile_max ? M : tile_max;
-  const size_t tile_need = tile_max ? gemv_tile_workspace_bytes(qtype, N, K, tile_m) : 0;
-  const bool tile_ok = tile_first && tile_need && workspace && workspace_bytes >= tile_need && (uintptr_t)workspace % 256 == 0 &&
-                       sm_count_of(dev) > 0 && gemv_tile_applicable(qtype, N, K, tile_m, w, x_bf16, sm_count_of(dev));
+  const int sms = sm_count_of(dev);
+  const bool workspace_ok = workspace && (uintptr_t)workspace % 256 == 0 && sms > 0;
+  // every kernel is asked only when those before it have declined: what they look at is host time of calls of 5 us
   static const int wide_min = [] { const char* e = getenv("GGQ_WIDE_MIN"); return e ? atoi(e) : 5; }();
-  // (rows that are not 16-byte aligned: the MMA kernel reads them with 2-byte loads; 5003 x 2816 Q6_K at 5 / 16 rows 21.3 / 25.2 us
-  // there, 18.0 / 19.8 here; 1024 x 5376 13.0 / 14.6 there, 20.0 / 21.0 here; rows of a few superblocks leave its steps too little to
-  // overlap: 16384 x 768 at 5 / 8 / 16 rows 14.2 / 14.6 / 18.4 there, 17.4 / 17.3 / 20.0 here, 28672 x 768 23 / 24 / 29 and 20 / 20 / 21)
-  const bool wide_ok = k_quant && M >= wide_min && (odd_rows ? weights >= (K < 1536 ? 21ll : 12ll) << 20 : wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes)) && workspace && (uintptr_t)workspace % 256 == 0 && sm_count_of(dev) > 0 &&
-                       workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, M, sm_count_of(dev)) &&
-                       gemv_wide_applicable(qtype, N, K, M, w, x_bf16);
-  if (batch_ok && !(wide_ok && wide_beats_batch(qtype, N, K, M))) {
-    err = gemv_batch(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, sm_count_of(dev), device_status_word_if_any(dev), tab, st);
-  } else if (wide_ok) {
-    err = gemv_wide(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, workspace, workspace_bytes, sm_count_of(dev), st, 0, nullptr,
+  const bool large = batch_pays(qtype, N, K, M);
+  const auto wide_ok = [&] {
+    return k_quant && M >= wide_min && (large || wide_pays(qtype, N * (K / ti->block_elems) * (int64_t)ti->block_bytes)) && workspace_ok && workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, M, sms) &&
+           gemv_wide_applicable(qtype, N, K, M, w, x_bf16);
+  };
+  const int tile_max = gemv_tile_max_batch(qtype);
+  const auto tile_ok = [&] {
+    const int m = M < tile_max ? M : tile_max;
+    const size_t need = tile_first && tile_max && workspace_ok ? gemv_tile_workspace_bytes(qtype, N, K, m) : 0;
+    return need && workspace_bytes >= need && gemv_tile_applicable(qtype, N, K, m, w, x_bf16, sms);
+  };
+  // (GGQ_GEMM_KERNEL=wide pins the batch-major kernel here as in ggq_gemm, for the tests; read only where it could change anything)
+  const auto wide_first = [&] {
+    if (!k_quant || M < wide_min) return false;
+    if (wide_beats_batch(qtype, N, K, M)) return wide_ok();
+    const char* pin = getenv("GGQ_GEMM_KERNEL");
+    return pin && !strcmp(pin, "wide") && wide_ok();
+  };
+  if (large && !wide_first() &&
+      gemv_batch(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, dev, sms, device_status_word_if_any(dev), tab, st, &err)) {
+    // launched
+  } else if (wide_ok()) {
+    err = gemv_wide(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, workspace, workspace_bytes, sms, st, 0, nullptr,
                     device_status_word_if_any(dev));
-  } else if (tile_ok) {
+  } else if (tile_ok()) {
     // up to tile_max batch rows per launch; a larger batch reads the weight once per tile_max rows
     err = cudaSuccess;
     for (int m0 = 0; m0 < M && err == cudaSuccess; m0 += tile_max) {
       const int mb = M - m0 < tile_max ? M - m0 : tile_max;
       err = gemv_tile(qtype, (const uint8_t*)w, N, K, (const uint8_t*)x_bf16 + (size_t)m0 * K * 2, mb,
-                      (uint8_t*)y + (size_t)m0 * N * y_item, y_dtype, workspace, workspace_bytes, sm_count_of(dev), device_status_word_if_any(dev), tab,
+                      (uint8_t*)y + (size_t)m0 * N * y_item, y_dtype, workspace, workspace_bytes, sms, device_status_word_if_any(dev), tab,
                       st, nullptr);
     }
   } else if (tuned) {

@@ -287,18 +287,18 @@ bool gemv_q5k_applicable(int64_t N, int64_t K, int M, const void* w, const void*
 cudaError_t gemv_q5k(const uint8_t* w, int64_t N, int64_t K, const void* x, void* y, int y_dtype, void* ws,
                      size_t ws_bytes, int sm_count, int* status, cudaStream_t st, const PeerPublish* peers = nullptr);
 
-// Tiled kernel for 1 <= M <= 8 (gemv_tile.cu): Q4_K, Q2_K, IQ4_XS and the IQ1/IQ2/IQ3 grid formats.
+// Tiled kernel (gemv_tile.cu): every format whose blocks make a superblock of 256 weights, K a multiple of 256.
 bool gemv_tile_applicable(int qtype, int64_t N, int64_t K, int M, const void* w, const void* x, int sm_count);
 size_t gemv_tile_workspace_bytes(int qtype, int64_t N, int64_t K, int M);
 cudaError_t gemv_tile(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype,
                       void* ws, size_t ws_bytes, int sm_count, int* status, const uint8_t* tab, cudaStream_t st,
                       const PeerPublish* peers = nullptr);
-int gemv_tile_max_batch(int qtype);     // batch rows per launch (8, Q6_K: 4; 0 if qtype has no tile format)
+int gemv_tile_max_batch(int qtype);     // batch rows per launch (4 for the formats of the batch kernel, 8 for the others; 0 if qtype has no tile format)
 
-// Batches of 2 .. 16 rows of the formats with one float scale per 256 weights, without scratch (gemv_batch.cu).
-bool gemv_batch_applicable(int qtype, int64_t N, int64_t K, int M, const void* w, const void* x, int sm_count);
-cudaError_t gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype, int sm_count, int* status,
-                       const uint8_t* tab, cudaStream_t st);
+// Batches of up to 16 rows of the formats with one float scale per 256 weights, without scratch (gemv_batch.cu).  False, and nothing is
+// launched, where the call has no plan on the device (dev, sm_count); else *err is what the launches returned.
+bool gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype, int dev, int sm_count, int* status,
+                const uint8_t* tab, cudaStream_t st, cudaError_t* err);
 
 // Same kernel with the scratch in a file-scope device array (no caller buffer); returns a ggq_status.
 int32_t gemv_q4k_static(const void* w, int64_t N, int64_t K, const void* x, void* y, int32_t y_dtype,

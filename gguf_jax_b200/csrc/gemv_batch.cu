@@ -37,11 +37,9 @@ static int tiles_of(int M) { return M <= 8 ? 1 : 2; }
 
 // Clusters of Q CTAs, one CTA per SM, that are on the current device at once: a GPC holds whole clusters only, and GPCs differ
 // (148 / 74 / 33 / 15 clusters of 1 / 2 / 4 / 8 on the boxes measured).  Asked once per device.
-static int clusters_of(int sm_count, int Q) {
+static int clusters_of(int dev, int sm_count, int Q) {
   if (Q == 1) return sm_count;
   static std::atomic<int> known[64][4];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); dev = -1; }
   const int slot = Q == 2 ? 0 : Q == 4 ? 1 : 2;
   int n = dev >= 0 && dev < 64 ? known[dev][slot].load(std::memory_order_acquire) : 0;
   if (n == 0) {
@@ -53,7 +51,7 @@ static int clusters_of(int sm_count, int Q) {
 }
 
 // Work split and shared-memory layout for one launch; false if nothing fits.
-static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count, Geo* out) {
+static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int sm_count, Geo* out) {
   const int SB = (int)(K / 256), NT = tiles_of(M), x_block = NT * fi.x_tile;
   Geo best{};
   double best_cost = 1e30;
@@ -69,7 +67,7 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
         g.chunk_sb = g.spu * nb;
         if (P > 1 && Q * (P - 1) * g.chunk_sb >= SB) continue;         // fewer passes do
         g.RT = (int)((N + 15) / 16);
-        g.J = std::min(clusters_of(sm_count, Q), g.RT);
+        g.J = std::min(clusters_of(dev, sm_count, Q), g.RT);
         g.row_skew = (int)((int64_t)SB * fi.ts % 16);
         const int pieces = (16 - std::gcd(fi.ts, 16) + nb * fi.ts + 15) / 16;
         g.pitch = 16 * pieces;
@@ -110,27 +108,23 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count
 // fewest parts of rows that have a plan, a launch each (us at 16 rows, tiled kernel in slices of four rows / here: IQ3_S 256000 x 2048 497 / 149,
 // Q3_K 600000 x 2048 1021 / 317; parts that need not be cut are slower, IQ3_S 152064 x 8192 at 8 rows 258 in one, 270 in two).
 struct Split { Geo geo; int64_t rows = 0; };         // of all parts but the last, which may be shorter
-static bool split(const FormatInfo& fi, int64_t N, int64_t K, int M, int sm_count, Split* out) {
+static bool split(const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int sm_count, Split* out) {
   const int64_t tiles = (N + 15) / 16;
   Geo any;
-  if (!plan(fi, 16, K, M, sm_count, &any)) return false;               // no number of rows has one
+  if (!plan(fi, 16, K, M, dev, sm_count, &any)) return false;               // no number of rows has one
   for (int64_t parts = 1; parts <= tiles; parts++) {
     out->rows = std::min(N, (tiles + parts - 1) / parts * 16);
-    if (plan(fi, out->rows, K, M, sm_count, &out->geo)) return true;
+    if (plan(fi, out->rows, K, M, dev, sm_count, &out->geo)) return true;
   }
   return false;
 }
-static bool plan_of(int qtype, int64_t N, int64_t K, int M, int sm_count, Split* out) {
+static bool plan_of(int qtype, const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int sm_count, Split* out) {
   struct Known { int64_t N = 0, K = 0; int qtype = -1, tiles = 0, sms = 0, dev = 0; bool ok = false; Split split; };
   static thread_local Known table[64];
-  FormatInfo fi;
-  if (!format_of(qtype, &fi)) return false;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); dev = -1; }
   const int tiles = tiles_of(M);
   Known& k = table[((uint64_t)N * 0x9E3779B97F4A7C15ull ^ (uint64_t)K * 0xC2B2AE3D27D4EB4Full ^ (uint64_t)(qtype * 2 + tiles) * 0x165667B19E3779F9ull) >> 58];
   if (k.N != N || k.K != K || k.qtype != qtype || k.tiles != tiles || k.sms != sm_count || k.dev != dev) {
-    k.ok = split(fi, N, K, M, sm_count, &k.split);
+    k.ok = split(fi, N, K, M, dev, sm_count, &k.split);
     k.N = N; k.K = K; k.qtype = qtype; k.tiles = tiles; k.sms = sm_count; k.dev = dev;
   }
   *out = k.split;
@@ -139,22 +133,16 @@ static bool plan_of(int qtype, int64_t N, int64_t K, int M, int sm_count, Split*
 
 }  // namespace batch
 
-bool gemv_batch_applicable(int qtype, int64_t N, int64_t K, int M, const void* w, const void* x, int sm_count) {
-  batch::FormatInfo fi;
-  if (!batch::format_of(qtype, &fi)) return false;
-  if (M < 1 || M > batch::kMaxBatch || K <= 0 || K % 256 || N < 1 || sm_count < 1) return false;
-  if ((uintptr_t)w % 16 || (uintptr_t)x % 16) return false;
-  if (N * (K / 256 * fi.ts) >= (1ll << 31)) return false;      // byte offsets are 32-bit
-  batch::Split split;
-  return batch::plan_of(qtype, N, K, M, sm_count, &split);
-}
-
-cudaError_t gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype, int sm_count, int* status,
-                       const uint8_t* tab, cudaStream_t st) {
+bool gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype, int dev, int sm_count, int* status,
+                const uint8_t* tab, cudaStream_t st, cudaError_t* result) {
   using namespace batch;
   FormatInfo fi;
+  if (!format_of(qtype, &fi)) return false;
+  if (M < 1 || M > kMaxBatch || K <= 0 || K % 256 || N < 1 || sm_count < 1) return false;
+  if ((uintptr_t)w % 16 || (uintptr_t)x % 16) return false;
+  if (N * (K / 256 * fi.ts) >= (1ll << 31)) return false;      // byte offsets are 32-bit
   Split split;
-  if (!format_of(qtype, &fi) || !plan_of(qtype, N, K, M, sm_count, &split)) return cudaErrorInvalidValue;
+  if (!plan_of(qtype, fi, N, K, M, dev, sm_count, &split)) return false;
   const int64_t row_bytes = K / 256 * fi.ts;
   cudaError_t err = cudaSuccess;
   for (int64_t row0 = 0; row0 < N && err == cudaSuccess; row0 += split.rows) {
@@ -171,7 +159,8 @@ cudaError_t gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const 
       default: err = launch_k(qtype, a);
     }
   }
-  return err;
+  *result = err;
+  return true;
 }
 
 }  // namespace ggq
