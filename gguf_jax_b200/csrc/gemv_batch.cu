@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <numeric>
 
 namespace ggq {
@@ -143,6 +144,7 @@ bool gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x
   if (N * (K / 256 * fi.ts) >= (1ll << 31)) return false;      // byte offsets are 32-bit
   Split split;
   if (!plan_of(qtype, fi, N, K, M, dev, sm_count, &split)) return false;
+  static const bool want_tma = [] { const char* e = getenv("GGQ_TILE_TMA"); return !(e && e[0] == '0'); }();      // "0": cp.async, as without an encoder
   const int64_t row_bytes = K / 256 * fi.ts;
   cudaError_t err = cudaSuccess;
   for (int64_t row0 = 0; row0 < N && err == cudaSuccess; row0 += split.rows) {
@@ -152,7 +154,7 @@ bool gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x
     geo.RT = (rows + 15) / 16;
     geo.J = std::min(geo.J, geo.RT);
     alignas(64) CUtensorMap map = {};
-    geo.tma = geo.row_skew == 0 && make_weight_map(&map, wp, rows, row_bytes, geo.pitch / 4);
+    geo.tma = want_tma && geo.row_skew == 0 && make_weight_map(&map, wp, rows, row_bytes, geo.pitch / 4);
     const Args a{&geo, tiles_of(M), st, wp, rows, (int)K, x, M, (uint8_t*)y + row0 * (y_dtype == GGQ_F32 ? 4 : 2), y_dtype, (int)N, tab, status, &map};
     switch (qtype) {
       case QT_IQ4_XS: case QT_IQ2_XXS: case QT_IQ2_XS: case QT_IQ2_S: case QT_IQ3_XXS: case QT_IQ3_S: case QT_IQ1_S: case QT_IQ1_M: err = launch_iq(qtype, a); break;

@@ -204,7 +204,9 @@ cudaError_t gemv_tile(int qtype, const uint8_t* w, int64_t N, int64_t K, const v
   alignas(64) CUtensorMap map = {};
   // (us at batch 1 with cp.async / with boxes: 14336 x 4096 Q8_0 19.3 / 17.5, Q4_0 14.9 / 13.0, IQ4_XS 19.3 / 17.3, MXFP4 19.8 / 17.9, Q2_K 14.3 /
   // 13.3, IQ2_XS 17.9 / 17.6; at four passes, where copies are the least of it, few-row weights were up to 13 % slower with boxes)
-  geo.tma = geo.row_skew == 0 && MP <= 2 && make_weight_map(&map, w, N, K / 256 * fi.ts, geo.pitch / 4);
+  // GGQ_TILE_TMA=0 keeps cp.async, which is also what happens where the driver offers no encoder.
+  static const bool want_tma = [] { const char* e = getenv("GGQ_TILE_TMA"); return !(e && e[0] == '0'); }();
+  geo.tma = want_tma && geo.row_skew == 0 && MP <= 2 && make_weight_map(&map, w, N, K / 256 * fi.ts, geo.pitch / 4);
   const Args a{&geo, grid, MP, st, w, (int)N, (int)K, x, M, y, y_dtype, counters, slots, &pp, status, tab, &map};
   switch (qtype) {
     case QT_Q4_K: case QT_Q5_K: case QT_Q6_K: case QT_Q2_K: case QT_Q3_K: case QT_TQ1_0: case QT_TQ2_0: return launch_k(qtype, a);

@@ -1,4 +1,4 @@
-"""The batch-1 kernels with their weight tiles copied by per-lane cp.async instead of TMA boxes (what they do where the
+"""The batch-1, tiled and batch kernels with their weight tiles copied by per-lane cp.async instead of TMA boxes (what they do where the
 driver offers no tensor-map encoder).  The switch is read once per process, so the check runs in a child process."""
 import os
 import subprocess
@@ -33,3 +33,11 @@ def test_cp_async_copy_path_matches_the_oracle():
     env["PYTHONPATH"] = root + os.pathsep + env.get("PYTHONPATH", "")
     r = subprocess.run([sys.executable, "-c", CHILD], env=env, cwd=root, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "FALLBACK_OK" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_cp_async_copies_of_aligned_rows_in_the_tiled_and_the_batch_kernel():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-m", "pytest", os.path.join(root, "tests", "test_tile_gpu.py"), os.path.join(root, "tests", "test_batch_gpu.py"),
+                        "-q", "-x", "-m", "gpu", "-k", "ragged_shapes or edges_of_tiles"],
+                       env=dict(os.environ, GGQ_TILE_ALWAYS="1", GGQ_TILE_TMA="0"), cwd=root, capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0 and " passed" in r.stdout, r.stdout[-3000:] + r.stderr[-1000:]
