@@ -67,8 +67,8 @@ def test_one_hot_returns_the_weight(qtype):
 @pytest.mark.skipif(not ALWAYS, reason="runs in the child process")
 @pytest.mark.parametrize("qtype", FORMATS, ids=lambda t: t.name)
 def test_magnitudes_over_the_whole_range(qtype):
-    # a block whose activations span 2^-120 .. 2^60: what lies below its largest by more than 2^31 counts as exactly as the rest, which a
-    # row shows whose large activations meet weights that are zero
+    # a block whose activations span 2^-120 .. 2^60; and in the formats that have weights of zero, a row whose large activation meets them: what lies
+    # below it by more than 2^31 counts as exactly as the rest (the next test shows that for every format)
     n, k, m = 48, 1024, 9
     wb = synth.make_weight_bytes(n, k, qtype, seed=11)
     dense = O.c_dequantize(wb, qtype).reshape(n, k).astype(np.float64)
@@ -85,6 +85,28 @@ def test_magnitudes_over_the_whole_range(qtype):
     zero = dense[:, col] == 0
     assert np.all(np.abs(got[0] - want[0])[zero] <= (np.abs(xb[0].astype(np.float64)) @ np.abs(dense).T)[zero] * 1e-5)
     assert not got[1].any()
+
+
+@pytest.mark.skipif(not ALWAYS, reason="runs in the child process")
+@pytest.mark.parametrize("qtype", FORMATS, ids=lambda t: t.name)
+def test_magnitudes_far_below_the_largest_of_their_block(qtype):
+    # in every batch row two neighbouring columns hold 2^30 and -2^30 and everything else is about 2^42 to 2^112 below: in the weight rows whose two
+    # weights are equal the large terms cancel exactly, and what is left is the product of the small ones, the block's own among them
+    n, k, m = 400, 1024, 11
+    wb = synth.make_weight_bytes(n, k, qtype, seed=12)
+    dense = O.c_dequantize(wb, qtype).reshape(n, k).astype(np.float64)
+    pairs = np.argsort((dense[:, 0::4] == dense[:, 1::4]).sum(0))[-m:] * 4      # the pairs with the most equal weights
+    xb = synth.make_x(m, k, seed=6) * np.exp2(-12.0 - 7.0 * np.arange(m))[:, None].astype(np.float32)
+    small = torch.from_numpy(xb).to(torch.bfloat16).double().numpy()
+    for i, c in enumerate(pairs):
+        small[i, c:c + 2] = 0
+        xb[i, c], xb[i, c + 1] = 2.0 ** 30, -2.0 ** 30
+    got = product(xb, wb, qtype, n, k).numpy().astype(np.float64)
+    want, scale = small @ dense.T, np.abs(small) @ np.abs(dense).T
+    for i, c in enumerate(pairs):
+        equal = dense[:, c] == dense[:, c + 1]
+        assert equal.any() and np.all(np.abs(got[i] - want[i])[equal] <= scale[i][equal] * 1e-5), (i, c)
+        assert np.abs(want[i])[equal].max() > 0.01 * scale[i][equal].max()      # far above the bar: a term left out shows
 
 
 @pytest.mark.skipif(not ALWAYS, reason="runs in the child process")
