@@ -134,7 +134,8 @@ def test_repeatable_and_independent_of_other_batch_rows():
 
 
 @pytest.mark.parametrize("qtype", WIDE, ids=lambda t: t.name)
-def test_picked_by_the_small_batch_entry_for_large_weights(qtype):
+def test_the_pin_holds_in_the_small_batch_entry(qtype):
+    # unpinned, ggq_gemv has the batch kernel multiply these; which calls it leaves to this kernel: test_routes_gpu.py
     n, k = BIG
     wb = synth.make_weight_bytes(n, k, qtype, seed=5)
     w = on_device(wb, qtype, n, k)
