@@ -95,9 +95,7 @@ static bool tile_pays(int64_t N, int64_t K, int M) {
 static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
   const int64_t work = K * (N > 2368 ? N : 2368);
-  // (up to 1024 rows the MMA kernel is faster than at 2048: Q4_K at 9 rows, MMA / here, 556 x 8448 11.5/12.5, 1024 x 9216 14/14, 556 x 10240
-  // 13.6/12.4, 2048 x 8192 18.5/12.5)
-  if (M >= 9) return always || work >= (qtype == QT_Q4_K ? (N <= 1024 ? 21ll : 18ll) : qtype == QT_Q5_K ? 14ll : 10ll) << 20;
+  if (M >= 9) return always || work >= (qtype == QT_Q4_K ? 18ll : qtype == QT_Q5_K ? 14ll : 10ll) << 20;
   if (M >= 5) return always || work >= (qtype == QT_Q4_K ? 12ll : 10ll) << 20;
   if (M < 3) return false;
   if (is_k_quant(qtype) && K <= 2048 && !(qtype == QT_Q6_K && K % 2048)) return true;        // Q6_K rows not 16-byte aligned stay on the MMA kernel: 1024 x 1024 3.5 there / 5.3 here
