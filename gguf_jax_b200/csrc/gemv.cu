@@ -68,14 +68,15 @@ static bool tile_scratch_is_optional(int qtype) {
 // (batch 1, 2) to 11 us (batch 8; a larger batch is two launches, 20 us) and grows slowly with the weight.  The other two give a CTA
 // a few rows and all of K, so below about one CTA of 16 rows per SM (2368 rows) their time follows K, not the weight:
 // they are compared at K * max(N, 2368) weights; a second launch of the tiled kernel with 5 rows or more only pays once the MMA kernel
-// has two CTAs per SM to work through.  Measured on B200 over 20 formats and 56 shapes of 0.25 to 130 M weights; with these lines the kernel
+// has two CTAs per SM to work through.  From 5 rows on this is the rule of the formats of 32 and 64 weights a block (the batch kernel has the
+// others).  Measured on B200 over 20 formats and 56 shapes of 0.25 to 130 M weights; with these lines the kernel
 // picked takes on average 0.2 % (batch 1..4), 0.3 % (5..8), 0.8 to 0.9 % (9..16) longer than the better one of the two, at worst
 // 13 % (1), 30 % (3: Q4_1 6144 x 1024), 32 % (5: Q5_1 4096 x 8192), 59 % (9).  us, other / tiled:
 //   batch 1    2048x2048 Q4_0 4.0/5.8 IQ2_XS 4.6/6.3   4096x4096 Q4_0 9.7/7.6 IQ2_XS 11.1/8.6 TQ1_0 12.1/9.9   512x14336 Q4_0 14/8.0 MXFP4 19/8.4
 //   batch 4    1024x1024 Q4_0 3.4/6.6 IQ3_S 3.9/7.5   4096x2048 Q4_0 8.4/7.8 IQ3_S 9.7/9.0   512x14336 Q4_0 24/13 Q8_0 31/13 IQ1_M 27/13
-//   batch 8    2048x2048 Q4_0 5.6/10.8 IQ3_S 6.0/11.0   4096x4096 Q4_0 16/13 Q3_K 20/15   512x14336 Q8_0 31/23 TQ1_0 30/22
-//   batch 9    4096x4096 Q4_0 17/21 MXFP4 20/24   8192x4096 Q4_0 29/27 Q8_0 30/37 IQ3_S 42/33   512x14336 Q4_0 26/32 IQ1_M 28/33
-//   batch 16   16384x4096 Q4_0 47/58 Q3_K 62/83   8192x14336 Q4_0 96/90 IQ3_S 139/104   512x14336 IQ2_XS 27/42 Q8_0 32/43
+//   batch 8    2048x2048 Q4_0 5.6/10.8   4096x4096 Q4_0 16/13   512x14336 Q8_0 31/23
+//   batch 9    4096x4096 Q4_0 17/21 MXFP4 20/24   8192x4096 Q4_0 29/27 Q8_0 30/37   512x14336 Q4_0 26/32
+//   batch 16   16384x4096 Q4_0 47/58   8192x14336 Q4_0 96/90   512x14336 Q8_0 32/43
 static bool tile_pays(int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
   if (always) return true;
@@ -84,13 +85,14 @@ static bool tile_pays(int64_t N, int64_t K, int M) {
   return K * (N > rows ? N : rows) >= from << 20;
 }
 
-// The batch kernel (gemv_batch.cu) against what served the call before: from 5 rows on it wins wherever the weight is large enough to fill its
-// CTAs (below, one MMA launch), at 3 and 4 rows against two passes of the tiled kernel where there are rows enough or,
+// The batch kernel (gemv_batch.cu) against the other kernels: from 5 rows on it wins wherever the weight is large enough to fill its
+// CTAs (below, one MMA launch; for large Q6_K see wide_beats_batch), at 3 and 4 rows against two passes of the tiled kernel where there are rows enough or,
 // for K-quants, up to 2048 columns (the tiled kernel takes 5.5 to 8 us for those however few the rows), at 2 nowhere.
-// us before / here, 700 shapes of 1 to 235 M weights timed: at 5..16 rows on average 0.73 of the time, on the wrong side of these lines at
-// worst 1.15 (Q5_K 1515 x 5888 at 6 rows); at 3, 4 rows 0.92, 1.05:
+// us others / here, 700 shapes of 1 to 235 M weights timed: at 5..16 rows on average 0.73 of the time, on the wrong side of these lines at
+// worst 1.15 (Q5_K 1515 x 5888 at 6 rows); at 3, 4 rows 0.92, 1.05.  Eight formats on seven shapes of 131 to 1245 M weights: 0.31 to 0.95 of
+// the time at 5..16 rows (Q4_K 600000 x 2048 at 9 rows 1.03), 0.58 to 0.98 at 3 and 4 (IQ2_S up to 1.02).
 //   8 rows   4096x4096 Q4_K 13/9.1 Q5_K 14/9.5 IQ2_XS 13/9.6   2048x8192 Q6_K 23/13   8192x8192 Q4_K 24/17 IQ3_S 37/23   700x28672 Q5_K 51/10
-//   16 rows  8192x2048 Q4_K 14/9.4   8192x8192 IQ3_S 82/30 Q2_K 70/25   14336x4096 Q6_K 30/27   but 1024x4096 Q4_K 7.0/9.7, Q5_K 8.0/10
+//   16 rows  8192x2048 Q4_K 14/9.4   8192x8192 IQ3_S 82/30 Q2_K 70/25   14336x4096 Q6_K 30/27   256000x2048 IQ3_S 342/149   but 1024x4096 Q4_K 7.0/9.7, Q5_K 8.0/10
 //   4 rows   1000x768 Q4_K 7.2/3.5   256x1536 Q4_K 6.5/4.4   1000x1024 Q5_K 8.1/4.8   16384x1024 Q4_K 7.9/5.6   14336x4096 Q5_K 28/21 Q6_K 32/24   8192x28672 Q4_K 47/47   but 2560x11520 Q4_K 11/13
 static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes

@@ -1,4 +1,4 @@
-// Fused decode + multiply for 2 .. 16 batch rows per launch on B200: the formats of batch_formats.cuh (one float scale per block of 256).
+// Fused decode + multiply for up to 16 batch rows per launch on B200 (ggq_gemv calls it from 3 on): the formats of batch_formats.cuh (one float scale per block of 256).
 //
 // Arithmetic.  mma.sync.m16n8k16 with float16 operands: A = 16 weight rows x 16 weights as exact integers (group scale times code),
 // B = 16 activations of eight batch rows (one or two column tiles share the decoded A).  The integers of a whole block add up in
@@ -6,7 +6,8 @@
 // on bfloat16 pairs (the 4- or 6-bit mins times the group sums of x, split into three terms of 8 bits).
 // Activations are bfloat16 and are staged as float16 times a power of two that puts the largest magnitude of a batch row and block just
 // below 2^15.  Eight significant bits are exact down to 2^-17, so magnitudes within 2^32 of the block's largest are exact; smaller ones are
-// left out of the staged copy and multiplied in further passes over the block (planes), straight from x: no activation is rounded.
+// left out of the staged copy and multiplied in further passes over the block (planes), straight from x: no activation is rounded.  (Their
+// sums are in units of the block's largest: 2^120 below it they reach the end of the float32 range.)
 //
 // Work split.  A cluster of Q CTAs owns a contiguous range of 16-row tiles, and each of its CTAs a Q-th of K (in P passes, where the
 // activations of one do not fit): the CTA stages its share of the activations once and deals its steps (16 rows x nb blocks, tile by tile)
@@ -16,7 +17,7 @@
 // the cluster's CTAs in a fixed order, and stores the outputs.  No scratch, no counters, no atomics: a launch is deterministic.
 // (Partial sums through global memory, one arrival counter per row tile, took 2 us more on small weights for the fence, the atomic and the
 // read back, and staged more activations per CTA.)
-// What bounds it: 8192 x 8192 Q4_K at 8 rows takes 17 us (4.2 us of HBM): issue slots 47 % busy, the half-rate integer pipe (codes out of
+// What bounds it: 8192 x 8192 Q4_K at 8 rows takes 17 us (5.8 us of HBM): issue slots 47 % busy, the half-rate integer pipe (codes out of
 // bytes) 41 %, the tensor pipe 10 %, four warps per scheduler at 128 registers and no stall above an eighth of the time.  The kernels before it
 // kept groups apart (an MMA for two batch rows, or a pair of them per scale group and column tile, with a scale on every partial sum):
 // us before / here at 8 and 16 rows, Q4_K 23.9 / 17.4, 27.0 / 21.5; IQ3_S 37.3 / 22.7, 82.4 / 30.1; Q6_K 29.9 / 24.6, 33.0 / 30.8; IQ3_S
@@ -178,10 +179,10 @@ gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat
         // the window of the step's blocks that starts on a 16-byte boundary; rows and blocks past the end arrive as zeros
         if (lane == 0) tma_box_load(dst, &map, (int)((boff & ~15u) >> 2), (tile_lo + rt_i) * 16, my_bars + 8 * slot_i, geo.slot_bytes);
       } else {
-        // a half-warp copies a row, lane kl the 16-byte pieces kl, kl + 16, kl + 32 of its window; rows past the end repeat row N - 1
+        // a half-warp copies a row, lane kl the 16-byte pieces kl and kl + 16 of its window; rows past the end repeat row N - 1
         // (multiplied, never stored); a copied piece holds at least one byte of its row
         const int nbh = min(nb, SB - sb0);
-        constexpr bool kWide = 14 + 2 * B::kTs + 15 > 512;
+        static_assert(14 + 2 * B::kTs + 15 <= 512, "two pieces per lane cover a window of two blocks");
 #pragma unroll
         for (int i = 0; i < 8; i++) {
           const uint32_t off = (uint32_t)min((tile_lo + rt_i) * 16 + 2 * i + hl, N - 1) * row_bytes + boff;
@@ -190,7 +191,6 @@ gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat
           const uint32_t to = dst + (2 * i + hl) * pitch + 16 * kl;
           if (kl < pieces) cp_async16(to, src);
           if (kl + 16 < pieces) cp_async16(to + 256, src + 256);
-          if (kWide && kl + 32 < pieces) cp_async16(to + 512, src + 512);
         }
       }
       --to_issue;

@@ -60,7 +60,7 @@ def _check(x: torch.Tensor, w: QuantizedArray, qtypes=None) -> tuple[int, int]:
 
 def fused_matmul(x: torch.Tensor, w: QuantizedArray, *, out_dtype=torch.bfloat16, out: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ w.T`` through the fused kernels, whatever the batch: ``ggq_gemv`` up to
-    ``gemv_max_batch()`` rows (tuned batch-1, tiled, batch-major or small-weight MMA kernel, chosen
+    ``gemv_max_batch()`` rows (tuned batch-1, tiled, batch, batch-major or small-weight MMA kernel, chosen
     by the library per format, batch and weight size), ``ggq_gemm`` above it (Q4_K / Q5_K / Q6_K:
     the batch-major kernel up to 32 rows, then the bf16-weight tcgen05 kernel; other formats: the
     tf32 tcgen05 kernel).
