@@ -104,7 +104,9 @@ static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
   if (qtype == QT_Q4_K) return N >= 8192 && K <= 12288;
   if (qtype == QT_Q5_K) return N >= 2048;
   if (qtype == QT_Q6_K) return N >= 2048 && N * K >= 6ll << 20;
-  return qtype != QT_IQ4_XS && N >= 10240 && K <= 8192 && N * K >= 14ll << 20;       // (two MMAs per weight; tiled / here: 16384 x 8192 34/38, 128256 x 4096 105/118)
+  // (IQ4_XS takes two MMAs per weight here; tiled / here at 4 rows: 18432 x 4608 30/25, 28672 x 2048 20/20, 28672 x 4096 32/33, 16384 x 8192 34/38,
+  // 128256 x 4096 105/118)
+  return N >= 10240 && K <= 8192 && N * K >= 14ll << 20 && (qtype != QT_IQ4_XS || N * K < 96ll << 20);
 }
 
 // Q6_K takes two products per weight in the batch kernel, and from 9 rows on its activations come in several passes where K is long, the sums of

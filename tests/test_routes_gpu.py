@@ -81,8 +81,9 @@ def test_weights_of_very_many_rows_are_cut(qtype, n, k, m):
     (QT.Q6_K, 8192, 20480, 9, "wide"), (QT.Q6_K, 8192, 20480, 8, "batch"), (QT.Q6_K, 4096, 16384, 16, "batch"), (QT.Q6_K, 20480, 10240, 16, "wide"),
     (QT.Q6_K, 32000, 8192, 16, "wide"), (QT.Q6_K, 28672, 8192, 9, "batch"), (QT.Q6_K, 65536, 4096, 16, "batch"),
     (QT.Q6_K, 8000, 20736, 16, "batch"), (QT.Q5_K, 8192, 20480, 16, "batch"),
-    # 3 and 4 rows of the low-bit formats: the batch kernel where there are rows enough, but for IQ4_XS
-    (QT.IQ3_S, 16384, 8192, 4, "batch"), (QT.IQ4_XS, 16384, 8192, 3, "tile"), (QT.IQ4_XS, 32000, 4096, 4, "tile"), (QT.IQ4_XS, 16384, 8192, 5, "batch"),
+    # 3 and 4 rows of the low-bit formats: the batch kernel where there are rows enough, for IQ4_XS up to a size
+    (QT.IQ3_S, 16384, 8192, 4, "batch"), (QT.IQ4_XS, 16384, 8192, 3, "tile"), (QT.IQ4_XS, 32000, 4096, 4, "tile"),
+    (QT.IQ4_XS, 18432, 4608, 4, "batch"), (QT.IQ4_XS, 16384, 8192, 5, "batch"),
 ], ids=str)
 def test_kernel_of_a_call(qtype, n, k, m, kernel):
     w = synth.make_weight_on_device(n, k, qtype, seed=4, device="cuda")
