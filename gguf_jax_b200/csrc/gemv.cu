@@ -110,12 +110,16 @@ static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
 }
 
 // Q6_K takes two products per weight in the batch kernel, and from 9 rows on its activations come in several passes where K is long, the sums of
-// many rows leave little room for the copies, and the batch-major kernel, which streams both, is the faster one.  (Rows that are not 16-byte
-// aligned slow that one down: they stay.)  us at 16 rows, batch-major / batch: 4096 x 16384 35/36, 6144 x 16384 43/47, 4096 x 20480 41/43, 8192 x 28672 86/95;
+// many rows leave little room for the copies, and the batch-major kernel, which streams both, is the faster one.  us at 16 rows, batch-major /
+// batch: 4096 x 16384 35/36, 6144 x 16384 43/47, 4096 x 20480 41/43, 8192 x 28672 86/95;
 // 8192 x 14336 51/50, 10240 x 14336 59/61, 20480 x 10240 74/79; 28672 x 8192 81/80, 32000 x 8192 87/95, 152064 x 8192 359/384; 65536 x 4096 88/84,
-// 128256 x 4096 160/162, 256000 x 2048 161/167.  On the wrong side of these lines: 14336 x 8192 48/50.
+// 128256 x 4096 160/162, 256000 x 2048 161/167.  Rows that are not 16-byte aligned, which slow its copies down: 40000 x 5376 92/85, 32000 x 7424 100/96,
+// 151936 x 3584 209/190; 8192 x 9472 41/44, 12288 x 9472 55/61, 16000 x 14592 100/107, 4096 x 19200 46/48, 10496 x 19200 87/98.  On the wrong side of
+// these lines: 14336 x 8192 48/50, 16384 x 11520 84/82.
 static bool wide_beats_batch(int qtype, int64_t N, int64_t K, int M) {
-  return qtype == QT_Q6_K && M >= 9 && K % 2048 == 0 && N * K >= (K >= 16384 ? 72ll : K > 8192 ? 120ll : K == 8192 ? 240ll : 384ll) << 20;
+  if (qtype != QT_Q6_K || M < 9) return false;
+  if (K % 2048) return K > 8192 && N * K >= 72ll << 20;
+  return N * K >= (K >= 16384 ? 72ll : K > 8192 ? 120ll : K == 8192 ? 240ll : 384ll) << 20;
 }
 
 static size_t tile_scratch_bytes(int32_t qtype, int64_t N, int64_t K, int32_t M) {
