@@ -97,7 +97,11 @@ static bool tile_pays(int64_t N, int64_t K, int M) {
 static bool batch_pays(int qtype, int64_t N, int64_t K, int M) {
   static const bool always = [] { const char* e = getenv("GGQ_TILE_ALWAYS"); return e && e[0] == '1'; }();     // for the tests of small shapes
   const int64_t work = K * (N > 2368 ? N : 2368);
-  if (M >= 9) return always || work >= (qtype == QT_Q4_K ? 18ll : qtype == QT_Q5_K ? 14ll : 10ll) << 20;
+  // (from 65 to 148 row tiles the MMA kernel, a CTA each, takes no longer than with fewer, and a cluster here has several of them: us at 9 rows
+  // with the weights in memory, MMA / here, 2048 x 4608 IQ4_XS 12.1/14.1 TQ1_0 12.4/13.5 Q2_K 11.4/12.1, 2048 x 5120 IQ4_XS 12.7/14.1, 2048 x 5632
+  // 14.4/14.1 and Q2_K 13.4/12.2, 1024 x 4608 IQ4_XS 11.7/11.3 Q2_K 11.1/10.7; in the L2 the MMA kernel takes 2 us less)
+  const bool one_wave = !is_k_quant(qtype) && N > 1024 && N <= 2368;
+  if (M >= 9) return always || work >= (qtype == QT_Q4_K ? 18ll : qtype == QT_Q5_K ? 14ll : one_wave ? 12ll : 10ll) << 20;
   if (M >= 5) return always || work >= (qtype == QT_Q4_K ? 12ll : 10ll) << 20;
   if (M < 3) return false;
   if (is_k_quant(qtype) && K <= 2048 && !(qtype == QT_Q6_K && K % 2048)) return true;        // Q6_K rows not 16-byte aligned stay on the MMA kernel: 1024 x 1024 3.5 there / 5.3 here

@@ -82,6 +82,9 @@ def test_weights_of_very_many_rows_are_cut(qtype, n, k, m):
     (QT.Q6_K, 32000, 8192, 16, "wide"), (QT.Q6_K, 28672, 8192, 9, "batch"), (QT.Q6_K, 65536, 4096, 16, "batch"),
     (QT.Q6_K, 8000, 20736, 16, "wide"), (QT.Q6_K, 12291, 9472, 9, "wide"), (QT.Q6_K, 4096, 14592, 16, "batch"), (QT.Q6_K, 16384, 7424, 16, "batch"),
     (QT.Q5_K, 8192, 20480, 16, "batch"),
+    # 9 rows and more of the low-bit formats with one row tile per SM
+    (QT.IQ4_XS, 2048, 5120, 9, "mma"), (QT.Q2_K, 2368, 4608, 16, "mma"), (QT.TQ1_0, 1025, 4608, 9, "mma"), (QT.TQ1_0, 1024, 4608, 9, "batch"),
+    (QT.IQ4_XS, 2369, 4608, 16, "batch"), (QT.IQ4_XS, 2048, 5632, 9, "batch"), (QT.IQ4_XS, 2048, 5120, 8, "batch"), (QT.Q6_K, 2048, 5120, 9, "batch"),
     # 3 and 4 rows of the low-bit formats: the batch kernel where there are rows enough, for IQ4_XS up to a size
     (QT.IQ3_S, 16384, 8192, 4, "batch"), (QT.IQ4_XS, 16384, 8192, 3, "tile"), (QT.IQ4_XS, 32000, 4096, 4, "tile"),
     (QT.IQ4_XS, 18432, 4608, 4, "batch"), (QT.IQ4_XS, 16384, 8192, 5, "batch"),
