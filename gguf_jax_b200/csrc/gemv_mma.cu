@@ -41,8 +41,10 @@ __device__ __forceinline__ uint32_t pack_hi(float a, float b) {
 __device__ __forceinline__ float trunc_bf16(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFF0000u); }
 
 // Start of every kernel here: the first 2 KB of the CTA's sixteen rows are asked into the L2 while the launch before this one ends; nothing is
-// read before that.  Only where every CTA of the launch is on the device at once (launch_even gives those launches dynamic shared memory): one that
-// comes later has nothing to wait for, and its prefetch is in the way of the others' loads (5632 x 5120 Q5_0 at 11 rows, 352 CTAs, 29.3 -> 28.1 us).
+// read before that.  Where not every CTA of the launch is on the device at once (launch_even gives only those launches dynamic shared memory), one
+// that comes later has nothing to wait for: there only rows that the prefetch covers, but for a line at most, are asked ahead (us at 11 rows without / with,
+// by bytes of a row: 14336 x 1792 Q4_0 1008 22.1/20.6, 8192 x 2560 Q5_1 1920 19.1/18.4, 8192 x 2048 Q8_0 2176 16.6/15.4, 6144 x 4096 Q4_0 2304 21.0/21.3,
+// 6000 x 3072 Q8_0 3264 16.0/16.9, 5632 x 5120 Q5_0 3520 28.1/29.3).
 // A CTA lets the next launch in only when its main loop is done: CTAs that come in earlier pile up on the few SMs that are
 // free then (a chain of 2048 x 2048 Q4_K at 8 rows 4.5 us a call without overlap, 7.1 let in at the start).
 __device__ __forceinline__ void begin(const uint8_t* w, int64_t row_bytes, int N) {
@@ -50,7 +52,7 @@ __device__ __forceinline__ void begin(const uint8_t* w, int64_t row_bytes, int N
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynamic_smem));
   const int row = blockIdx.x * 16 + (threadIdx.x >> 4);
   const int64_t off = 128 * (threadIdx.x & 15);
-  if (dynamic_smem > 0 && row < N && off < row_bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + row * row_bytes + off));
+  if ((dynamic_smem > 0 || row_bytes <= 2048 + 128) && row < N && off < row_bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + row * row_bytes + off));
   pdl_wait();
 }
 
