@@ -108,27 +108,24 @@ static bool plan(const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int
 // tile stay in shared memory until the end, so a weight of very many rows (from 150 to 500 thousand, by format and columns) is cut into the
 // fewest parts of rows that have a plan, a launch each (us at 16 rows, tiled kernel in slices of four rows / here: IQ3_S 256000 x 2048 497 / 149,
 // Q3_K 600000 x 2048 1021 / 317; parts that need not be cut are slower, IQ3_S 152064 x 8192 at 8 rows 258 in one, 270 in two).
-struct Split { Geo geo; int64_t rows = 0; };         // of all parts but the last, which may be shorter
-static bool split(const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int sm_count, Split* out) {
+static bool split(const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int sm_count, Geo* out) {       // the plan of all parts but the last, which may be shorter
   const int64_t tiles = (N + 15) / 16;
   Geo any;
   if (!plan(fi, 16, K, M, dev, sm_count, &any)) return false;               // no number of rows has one
-  for (int64_t parts = 1; parts <= tiles; parts++) {
-    out->rows = std::min(N, (tiles + parts - 1) / parts * 16);
-    if (plan(fi, out->rows, K, M, dev, sm_count, &out->geo)) return true;
-  }
+  for (int64_t parts = 1; parts <= tiles; parts++)
+    if (plan(fi, std::min(N, (tiles + parts - 1) / parts * 16), K, M, dev, sm_count, out)) return true;
   return false;
 }
-static bool plan_of(int qtype, const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int sm_count, Split* out) {
-  struct Known { int64_t N = 0, K = 0; int qtype = -1, tiles = 0, sms = 0, dev = 0; bool ok = false; Split split; };
+static bool plan_of(int qtype, const FormatInfo& fi, int64_t N, int64_t K, int M, int dev, int sm_count, Geo* out) {
+  struct Known { int64_t N = 0, K = 0; int qtype = -1, tiles = 0, sms = 0, dev = 0; bool ok = false; Geo geo; };
   static thread_local Known table[64];
   const int tiles = tiles_of(M);
   Known& k = table[((uint64_t)N * 0x9E3779B97F4A7C15ull ^ (uint64_t)K * 0xC2B2AE3D27D4EB4Full ^ (uint64_t)(qtype * 2 + tiles) * 0x165667B19E3779F9ull) >> 58];
   if (k.N != N || k.K != K || k.qtype != qtype || k.tiles != tiles || k.sms != sm_count || k.dev != dev) {
-    k.ok = split(fi, N, K, M, dev, sm_count, &k.split);
+    k.ok = split(fi, N, K, M, dev, sm_count, &k.geo);
     k.N = N; k.K = K; k.qtype = qtype; k.tiles = tiles; k.sms = sm_count; k.dev = dev;
   }
-  *out = k.split;
+  *out = k.geo;
   return k.ok;
 }
 
@@ -142,20 +139,18 @@ bool gemv_batch(int qtype, const uint8_t* w, int64_t N, int64_t K, const void* x
   if (M < 1 || M > kMaxBatch || K <= 0 || K % 256 || N < 1 || sm_count < 1) return false;
   if ((uintptr_t)w % 16 || (uintptr_t)x % 16) return false;
   if (N * (K / 256 * fi.ts) >= (1ll << 31)) return false;      // byte offsets are 32-bit
-  Split split;
-  if (!plan_of(qtype, fi, N, K, M, dev, sm_count, &split)) return false;
+  Geo part;
+  if (!plan_of(qtype, fi, N, K, M, dev, sm_count, &part)) return false;
   static const bool want_tma = [] { const char* e = getenv("GGQ_TILE_TMA"); return !(e && e[0] == '0'); }();      // "0": cp.async, as without an encoder
-  const int64_t row_bytes = K / 256 * fi.ts;
+  alignas(64) CUtensorMap map = {};
+  Geo geo = part;
+  geo.tma = want_tma && geo.row_skew == 0 && make_weight_map(&map, w, N, K / 256 * fi.ts, geo.pitch / 4);
+  const Args a{&geo, tiles_of(M), st, w, (int)N, (int)K, x, M, y, y_dtype, tab, status, &map};
+  const int tiles = (int)((N + 15) / 16);
   cudaError_t err = cudaSuccess;
-  for (int64_t row0 = 0; row0 < N && err == cudaSuccess; row0 += split.rows) {
-    const uint8_t* wp = w + row0 * row_bytes;          // sixteen rows of any format are a multiple of 16 bytes
-    const int rows = (int)std::min(split.rows, N - row0);
-    Geo geo = split.geo;
-    geo.RT = (rows + 15) / 16;
-    geo.J = std::min(geo.J, geo.RT);
-    alignas(64) CUtensorMap map = {};
-    geo.tma = want_tma && geo.row_skew == 0 && make_weight_map(&map, wp, rows, row_bytes, geo.pitch / 4);
-    const Args a{&geo, tiles_of(M), st, wp, rows, (int)K, x, M, (uint8_t*)y + row0 * (y_dtype == GGQ_F32 ? 4 : 2), y_dtype, (int)N, tab, status, &map};
+  for (; geo.tile0 < tiles && err == cudaSuccess; geo.tile0 += part.RT) {
+    geo.RT = std::min(part.RT, tiles - geo.tile0);
+    geo.J = std::min(part.J, geo.RT);
     switch (qtype) {
       case QT_IQ4_XS: case QT_IQ2_XXS: case QT_IQ2_XS: case QT_IQ2_S: case QT_IQ3_XXS: case QT_IQ3_S: case QT_IQ1_S: case QT_IQ1_M: err = launch_iq(qtype, a); break;
       default: err = launch_k(qtype, a);

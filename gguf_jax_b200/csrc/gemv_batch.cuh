@@ -41,7 +41,7 @@ constexpr int kMaxBatch = 16;
 
 struct Geo {
   int nb, spu, chunk_sb;            // blocks per step, steps per unit (a tile in one pass), blocks per pass
-  int Q, P, J, RT;                  // CTAs per cluster, passes, clusters, 16-row tiles
+  int Q, P, J, RT, tile0;           // CTAs per cluster, passes, clusters, 16-row tiles of the launch and the first of them
   int depth, pitch, slot_bytes;     // ring of a warp
   int off_x, off_sum, off_tab, off_misc, off_bar, total;
   int tma;                          // steps come as TMA boxes
@@ -55,7 +55,7 @@ template <class F> constexpr int x_tile_bytes() { return 4096 + mins_bytes<F>() 
 // Steps of a CTA and pass: T; first step of warp v (0 .. 16), and the warp that has step s.
 __host__ __device__ __forceinline__ int warp_begin(int T, int v) { return T * v / kWarps; }
 __host__ __device__ __forceinline__ int warp_of(int T, int s) { return ((s + 1) * kWarps - 1) / T; }
-__host__ __device__ __forceinline__ int first_tile(const Geo& g, int j) { return (int)((int64_t)g.RT * j / g.J); }
+__host__ __device__ __forceinline__ int first_tile(const Geo& g, int j) { return g.tile0 + (int)((int64_t)g.RT * j / g.J); }
 
 __device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -146,7 +146,7 @@ __device__ __noinline__ void more_planes(uint32_t blk0, uint32_t blk1, tf::Table
 
 template <class F, int NT>
 __global__ void __launch_bounds__(kThreads, 1)
-gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M, void* __restrict__ y, int y_dtype, int ldy,
+gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int M, void* __restrict__ y, int y_dtype,
                   const Geo geo, const uint8_t* __restrict__ tab, int* __restrict__ status, const __grid_constant__ CUtensorMap map) {
   typedef typename F::Base B;
   constexpr int XR = 8 * NT, kXTile = x_tile_bytes<F>(), kXBlock = NT * kXTile;
@@ -499,14 +499,14 @@ gemv_batch_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int row = (tile_lo + tile) * 16 + g + 8 * (i >> 1), m = n * 8 + 2 * t + (i & 1);
-        if (row < N && m < M) { store_out(y, y_dtype, (int64_t)m * ldy + row, v[n][i]); bad |= not_finite(v[n][i]); }
+        if (row < N && m < M) { store_out(y, y_dtype, (int64_t)m * N + row, v[n][i]); bad |= not_finite(v[n][i]); }
       }
     if (__any_sync(0xFFFFFFFFu, bad)) {          // outputs that are not finite
 #pragma unroll 1
       for (int j = 0; j < 4 * NT; j++) {
         const int row = (tile_lo + tile) * 16 + g + 8 * ((j >> 1) & 1), m = (j >> 2) * 8 + 2 * t + (j & 1);
-        const bool again = row < N && m < M && not_finite(load_out(y, y_dtype, (int64_t)m * ldy + row));
-        recompute<B::kQt>(again, row, m, w, (int64_t)row_bytes, ldy, x, K, tab, y, y_dtype);
+        const bool again = row < N && m < M && not_finite(load_out(y, y_dtype, (int64_t)m * N + row));
+        recompute<B::kQt>(again, row, m, w, (int64_t)row_bytes, N, x, K, tab, y, y_dtype);
       }
     }
   }
@@ -523,7 +523,7 @@ struct Args {
   const void* x;
   int M;
   void* y;
-  int y_dtype, ldy;
+  int y_dtype;
   const uint8_t* tab;
   int* status;
   const CUtensorMap* map;
@@ -551,7 +551,7 @@ static cudaError_t launch(const Args& a) {
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.geo->Q > 1 ? 2 : 1;
-  cudaError_t err = cudaLaunchKernelEx(&cfg, gemv_batch_kernel<F, NT>, a.w, a.N, a.K, (const __nv_bfloat16*)a.x, a.M, a.y, a.y_dtype, a.ldy, (const Geo)*a.geo,
+  cudaError_t err = cudaLaunchKernelEx(&cfg, gemv_batch_kernel<F, NT>, a.w, a.N, a.K, (const __nv_bfloat16*)a.x, a.M, a.y, a.y_dtype, (const Geo)*a.geo,
                                        a.tab, a.status, *a.map);
   return err != cudaSuccess ? err : cudaPeekAtLastError();
 }
