@@ -504,7 +504,7 @@ extern "C" int32_t ggq_gemm(int32_t qtype, const void* w, int64_t N, int64_t K, 
   const bool odd_rows = (K / ti->block_elems * ti->block_bytes) % 16 != 0;
   const bool can_wide = ws_ok && (M <= wide_slice || !odd_rows) && gemv_wide_applicable(qtype, N, K, slice_m, w, x_bf16) &&
                         workspace_bytes >= gemv_wide_workspace_bytes(qtype, N, K, slice_m, sms);
-  const bool can_bf16w = ws_ok && gemm_bf16w_applicable(qtype, N, K, M) &&
+  const bool can_bf16w = ws_ok && gemm_bf16w_applicable(qtype, N, K, M) && gemm_bf16w_available() &&
                          workspace_bytes >= gemm_bf16w_workspace_bytes(qtype, N, K, M, sms);
   const bool can_codes = ws_ok && gemm_codes_applicable(qtype, N, K, M) &&
                          workspace_bytes >= gemm_codes_workspace_bytes(qtype, N, K, M, sms);
