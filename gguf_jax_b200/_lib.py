@@ -47,6 +47,11 @@ SIGNATURES = {
     "ggq_gemm": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                   ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32,
                                   ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]),
+    "ggq_rounded_gemm_pays": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32]),
+    "ggq_rounded_gemm_temp": (ctypes.c_size_t, [ctypes.c_int32, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32]),
+    "ggq_rounded_gemm": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
+                                          ctypes.c_void_p, ctypes.c_int32, ctypes.c_void_p, ctypes.c_int32,
+                                          ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]),
     "ggq_gemv_sharded": (ctypes.c_int32, [ctypes.c_int32, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                           ctypes.c_void_p, ctypes.c_int32, ctypes.POINTER(ctypes.c_void_p),
                                           ctypes.POINTER(ctypes.c_void_p), ctypes.c_int32, ctypes.c_int32,
@@ -146,7 +151,7 @@ def native():
                     module = _PythonPath
                 else:
                     entries = (L.ggq_gemv, L.ggq_gemm, L.ggq_fused_batch_limit, L.ggq_scratch_bytes, L.ggq_has_fused, L.ggq_type_info,
-                               L.ggq_dequant)
+                               L.ggq_dequant, L.ggq_rounded_gemm, L.ggq_rounded_gemm_pays, L.ggq_rounded_gemm_temp)
                     module.bind(*[ctypes.cast(f, ctypes.c_void_p).value for f in entries], int(L.ggq_gemv_max_batch()))
                 _native_module = module
     return _native_module

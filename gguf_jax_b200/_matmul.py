@@ -8,7 +8,9 @@ gradient in ``x`` only.  What is behind them is this library's own:
   (small-batch GEMV, or the tcgen05 GEMM above it) and up to which batch is decided by the
   compiled library (``ggq_fused_batch_limit``), per qtype and shape; this module only asks.
 * **materialize** -- the decode kernel writes a dense bf16/f32 copy of ``w`` (all of it, or
-  ``R`` equal row slabs when the copy would exceed a byte budget) and a library GEMM multiplies.
+  ``R`` equal row slabs when the copy would exceed a byte budget) and a library GEMM multiplies.  Where the
+  copy would be bf16 and a kernel that decodes the same weights inside the multiply is faster
+  (``ggq_rounded_gemm_pays``), that kernel stands in for both, with the same weights and sums in another order.
 
 The backward pass is the same for both: ``dx = g @ w`` with ``w`` decoded again slab by slab,
 so only the quantized payload is kept alive between forward and backward.
@@ -213,8 +215,17 @@ def _plain(t: torch.Tensor) -> bool:
             and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing() and not (t.requires_grad and torch.is_grad_enabled()))
 
 
+def _decodes_inside(x: torch.Tensor, w: QuantizedArray) -> bool:
+    """The product of a bfloat16 copy may be taken without one: the copy would be the built-in decoder's, of the type of ``x``, and
+    nothing but the product sees it."""
+    return (x.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and x.is_cuda and kernels.rounded_temp(w, x.numel() // w.shape[1]) >= 0
+            and x.device == w.data.device and not quants._replaced and _plain(x))
+
+
 def _materialized_forward(x: torch.Tensor, w: QuantizedArray, count: int) -> torch.Tensor:
     n_out = w.shape[0]
+    if _decodes_inside(x, w) and (y := kernels.rounded_matmul(x, w)) is not None:
+        return y
     x2 = x.reshape(-1, w.shape[1])
     y = None
     if (count > 1 or _pads(x2.shape[0], w)) and _plain(x):

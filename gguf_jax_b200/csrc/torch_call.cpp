@@ -6,7 +6,8 @@
 // call) for 37 us of kernels; through here they take 40 us (under 6 us a call).  `fast_matmul` returns None for every call that
 // is not the common one, and the Python path, which stays the reference for behaviour and errors, takes it.
 //
-// The dense route (decode, library GEMM) is two launches for which the Python path spent 50 us; here 15 to 20.
+// The dense route (decode, library GEMM) is two launches for which the Python path spent 50 us; here 15 to 20, or one launch that decodes inside
+// the multiply where the library says that it is faster (ggq_rounded_gemm_pays).
 //
 // The library's entry points are handed over as addresses (bind), so that this module follows whichever
 // libggq_b200.so the binding has loaded.  All state is guarded by the interpreter lock, which is not held while
@@ -32,6 +33,8 @@
 namespace {
 
 using LaunchFn = int32_t (*)(int32_t, const void*, int64_t, int64_t, const void*, int32_t, void*, int32_t, void*, size_t, void*);
+using RoundedFn = int32_t (*)(int32_t, const void*, int64_t, int64_t, const void*, int32_t, void*, int32_t, void*, size_t, void*);
+using PaysFn = int32_t (*)(int32_t, int64_t, int64_t, int32_t);
 using LimitFn = int32_t (*)(int32_t, int64_t, int64_t);
 using BytesFn = size_t (*)(int32_t, int64_t, int64_t, int32_t);
 using CodeFn = int32_t (*)(int32_t);
@@ -39,8 +42,10 @@ using DequantFn = int32_t (*)(int32_t, const void*, int64_t, void*, int32_t, voi
 using InfoFn = int32_t (*)(int32_t, int32_t*, int32_t*);
 
 LaunchFn g_gemv = nullptr, g_gemm = nullptr;
+RoundedFn g_rounded = nullptr;
+PaysFn g_rounded_pays = nullptr;
 LimitFn g_limit = nullptr;
-BytesFn g_bytes = nullptr;
+BytesFn g_bytes = nullptr, g_rounded_temp = nullptr;
 CodeFn g_fused = nullptr;
 InfoFn g_info = nullptr;
 DequantFn g_dequant = nullptr;
@@ -57,6 +62,8 @@ struct Shape {
   int32_t limit = 0;
   size_t scratch = 0, payload = 0;
   int64_t blocks = 0;
+  bool rounded = false;                    // the dense route's product decodes inside the multiply, with so much memory of its own
+  size_t rounded_temp = 0;
 };
 std::array<Shape, 1024> g_shapes;
 
@@ -71,7 +78,8 @@ const Shape* shape_of(int32_t qtype, int64_t n, int64_t k, int32_t m) {
   if (s.qtype != qtype || s.n != n || s.k != k || s.m != m) {
     int32_t elems = 0, bytes = 0;
     if (!g_fused(qtype) || g_info(qtype, &elems, &bytes) != 0 || k <= 0 || k % elems) return nullptr;
-    s = Shape{n, k, qtype, m, g_limit(qtype, n, k), g_bytes(qtype, n, k, m), (size_t)(n * (k / elems)) * (size_t)bytes, n * (k / elems)};
+    s = Shape{n, k, qtype, m, g_limit(qtype, n, k), g_bytes(qtype, n, k, m), (size_t)(n * (k / elems)) * (size_t)bytes, n * (k / elems),
+              g_rounded_pays(qtype, n, k, m) != 0, g_rounded_temp(qtype, n, k, m)};
   }
   return &s;
 }
@@ -107,13 +115,24 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   c10::SmallVector<int64_t, 6> sizes(x.sizes().begin(), x.sizes().end());
   sizes.back() = n;
   if (m > s.limit && !force) {
-    // the dense route in one piece: decode to bf16, library GEMM (rows of the result on 16-byte boundaries)
     const double budget = PyFloat_AsDouble(args[5]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
-    // (autocast converts the copy: what then still fits is for the Python path to say)
-    if (n % 8 || (at::autocast::is_autocast_enabled(at::kCUDA) ? 8.0 : 4.0) * (double)n * (double)k > budget) Py_RETURN_NONE;
+    // (autocast converts the copy: its product, and what then still fits, are not these; slabs are the Python path's)
+    const bool autocast = at::autocast::is_autocast_enabled(at::kCUDA);
+    if ((autocast ? 8.0 : 4.0) * (double)n * (double)k > budget) Py_RETURN_NONE;
     at::Tensor y;
-    {
+    if (s.rounded && !autocast && (uintptr_t)w.data_ptr() % 16 == 0 && (!x.is_contiguous() || (uintptr_t)x.data_ptr() % 16 == 0)) {
+      // the weights that the copy would hold, decoded inside the multiply
+      WithoutGil no_gil;
+      const at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+      y = at::empty(sizes, x.options().requires_grad(false));
+      const at::Tensor temp = s.rounded_temp ? at::empty({(int64_t)s.rounded_temp}, w.options().requires_grad(false)) : at::Tensor();
+      if (g_rounded((int32_t)qtype, w.data_ptr(), n, k, xc.data_ptr(), (int32_t)m, y.data_ptr(), kBf16, temp.defined() ? temp.data_ptr() : nullptr,
+                    s.rounded_temp, stream.stream()) != 0)
+        y = at::Tensor();
+    } else {
+      // the dense route in one piece: decode to bf16, library GEMM (rows of the result on 16-byte boundaries)
+      if (n % 8) Py_RETURN_NONE;
       WithoutGil no_gil;
       const at::Tensor dense = at::empty({n, k}, x.options().requires_grad(false));
       if (g_dequant((int32_t)qtype, w.data_ptr(), s.blocks, dense.data_ptr(), kBf16, stream.stream()) == 0)
@@ -142,11 +161,13 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(gemv, gemm, fused_batch_limit, scratch_bytes, has_fused, type_info, dequant, gemv_max_batch): entry point addresses
+// bind(gemv, gemm, fused_batch_limit, scratch_bytes, has_fused, type_info, dequant, rounded_gemm, rounded_gemm_pays, rounded_gemm_temp,
+// gemv_max_batch): entry
+// point addresses
 PyObject* bind(PyObject*, PyObject* args) {
-  unsigned long long gemv, gemm, limit, bytes, fused, info, dequant;
+  unsigned long long gemv, gemm, limit, bytes, fused, info, dequant, rounded, pays, temp;
   int max_batch;
-  if (!PyArg_ParseTuple(args, "KKKKKKKi", &gemv, &gemm, &limit, &bytes, &fused, &info, &dequant, &max_batch)) return nullptr;
+  if (!PyArg_ParseTuple(args, "KKKKKKKKKKi", &gemv, &gemm, &limit, &bytes, &fused, &info, &dequant, &rounded, &pays, &temp, &max_batch)) return nullptr;
   g_gemv = (LaunchFn)(uintptr_t)gemv;
   g_gemm = (LaunchFn)(uintptr_t)gemm;
   g_limit = (LimitFn)(uintptr_t)limit;
@@ -154,6 +175,9 @@ PyObject* bind(PyObject*, PyObject* args) {
   g_fused = (CodeFn)(uintptr_t)fused;
   g_info = (InfoFn)(uintptr_t)info;
   g_dequant = (DequantFn)(uintptr_t)dequant;
+  g_rounded = (RoundedFn)(uintptr_t)rounded;
+  g_rounded_pays = (PaysFn)(uintptr_t)pays;
+  g_rounded_temp = (BytesFn)(uintptr_t)temp;
   g_gemv_max = max_batch;
   Py_RETURN_NONE;
 }

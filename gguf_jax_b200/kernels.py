@@ -29,6 +29,8 @@ LOWBIT_TYPES = (QT.Q2_K, QT.IQ1_S, QT.IQ1_M, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT
 
 
 _ws_need: dict[tuple[int, int, int, int], tuple[int, int]] = {}      # scratch: for every kernel, for those that need one
+_rounded: dict[tuple[int, int, int, int], int] = {}       # what rounded_temp has said
+_ROUNDED_TYPES = (QT.Q4_K, QT.Q5_K, QT.Q6_K)
 _cap: list[int] = []
 
 
@@ -127,6 +129,39 @@ def fused_matmul(x: torch.Tensor, w: QuantizedArray, *, out_dtype=torch.bfloat16
     finally:
         if prev != dev:
             torch.cuda.set_device(prev)
+    return y.reshape(*x.shape[:-1], n_rows)
+
+
+def rounded_temp(w: QuantizedArray, m: int) -> int:
+    """Bytes of memory of its own that :func:`rounded_matmul` takes for ``m`` rows; -1 where a decoded copy and a library GEMM are faster."""
+    if w.qtype not in _ROUNDED_TYPES or len(w.shape) != 2:
+        return -1
+    key = (int(w.qtype), *w.shape, m)
+    temp_bytes = _rounded.get(key)
+    if temp_bytes is None:
+        if len(_rounded) >= 4096:
+            _rounded.clear()
+        L = _lib.lib()
+        pays = 0 < m <= 65536 and L.ggq_rounded_gemm_pays(*key)
+        temp_bytes = _rounded[key] = int(L.ggq_rounded_gemm_temp(*key)) if pays else -1
+    return temp_bytes
+
+
+def rounded_matmul(x: torch.Tensor, w: QuantizedArray) -> torch.Tensor | None:
+    """``x @ w.dequantize(bfloat16).T`` with the weight decoded inside the multiply (``ggq_rounded_gemm``), ``x`` a plain bfloat16 tensor on the
+    device of ``w``, where :func:`rounded_temp` says so; None where memory is not 16-byte aligned."""
+    n_rows, k_dim = w.shape
+    m = x.numel() // k_dim
+    temp_bytes = rounded_temp(w, m)
+    xm, data = x.reshape(m, k_dim).contiguous(), w.data.contiguous()
+    if xm.data_ptr() % 16 or data.data_ptr() % 16:
+        return None
+    dev = _backend.require_cuda(data, f"matmul ({w.qtype.name})")
+    with torch.cuda.device(dev):
+        y = torch.empty((m, n_rows), dtype=torch.bfloat16, device=data.device)
+        temp = torch.empty(temp_bytes, dtype=torch.uint8, device=data.device) if temp_bytes else None
+        _lib.check(_lib.lib().ggq_rounded_gemm(int(w.qtype), data.data_ptr(), n_rows, k_dim, xm.data_ptr(), m, y.data_ptr(), _lib.GGQ_BF16,
+                                               None if temp is None else temp.data_ptr(), temp_bytes, _backend.stream_ptr(dev)))
     return y.reshape(*x.shape[:-1], n_rows)
 
 

@@ -147,6 +147,18 @@ int32_t ggq_gemm(int32_t qtype, const void* w, int64_t N, int64_t K, const void*
                  int32_t M, void* y, int32_t y_dtype, void* workspace,
                  size_t workspace_bytes, void* stream);
 
+/* The product of the materializing route (src/gguf_jax/_matmul.py:141-186: decode W to bf16, then a dense GEMM) without the dense
+ * copy: W is decoded inside the kernel, to the values ggq_dequant gives rounded once to bf16, and multiplied on the tensor cores with
+ * float32 accumulation.  Q4_K / Q5_K / Q6_K, K % 256 == 0, rows of a multiple of 16 bytes, w and x 16-byte aligned; GGQ_UNSUPPORTED
+ * otherwise.  Nothing is kept between calls: calls and captured graphs may overlap on the device like those of a library GEMM.  `temp` is memory of the
+ * call's own (256-byte aligned, any contents) of ggq_rounded_gemm_temp bytes; with less, or none, a plan that needs none runs.  The launch
+ * is a programmatic dependent, see ggq_gemv.
+ * ggq_rounded_gemm_pays: 1 where this is faster than ggq_dequant and a library GEMM (from 17 rows on, up to 2048, most where the weight is large), else 0. */
+int32_t ggq_rounded_gemm_pays(int32_t qtype, int64_t N, int64_t K, int32_t M);
+size_t ggq_rounded_gemm_temp(int32_t qtype, int64_t N, int64_t K, int32_t M);
+int32_t ggq_rounded_gemm(int32_t qtype, const void* w, int64_t N, int64_t K, const void* x_bf16,
+                         int32_t M, void* y, int32_t y_dtype, void* temp, size_t temp_bytes, void* stream);
+
 /* Row-sharded multiply with the exchange fused into the kernel.  No counterpart in the reference
  * (it runs on one device only); it stands where a sharded caller would otherwise follow ggq_gemv
  * with an all-gather.  `w` holds this rank's N_local rows of an (world * N_local, K) weight;

@@ -1,0 +1,88 @@
+"""Products of the dense route whose weight is decoded inside the multiply (ggq_rounded_gemm): which calls take it, and that they give the product of the
+decoded bfloat16 copy.  Bar: float32 sums in another order (1e-5 for K up to 8192, see test_gemm_bf16w_plans_gpu.py) and one bf16 rounding of the result:
+8 significant bits, so half a unit in the last place is 2^-8 of a power of two at most, and errors spread evenly over it have a 2-norm of 2^-8 / sqrt(3)."""
+import pytest
+import torch
+from gguf.constants import GGMLQuantizationType as QT
+
+import gguf_jax_b200 as gj
+from gguf_jax_b200 import _lib, quants, synth
+from tests.launched import kernels_of
+
+pytestmark = pytest.mark.gpu
+
+
+def weight(qtype, n, k, dtype=torch.bfloat16):
+    return synth.make_weight_on_device(n, k, qtype, seed=n, device="cuda").astype(dtype)
+
+
+def inside(call):
+    return [n for n in kernels_of(call) if "gemm_bf16w" in n]
+
+
+@pytest.mark.parametrize("qtype,n,k,m", [(QT.Q5_K, 4096, 4096, 32), (QT.Q4_K, 1003, 4096, 17), (QT.Q6_K, 1024, 4096, 24), (QT.Q4_K, 4096, 4096, 128),
+                                         (QT.Q6_K, 8192, 8192, 300), (QT.Q4_K, 4096, 14336, 512), (QT.Q5_K, 14336, 4096, 1000),
+                                         # tiles cut between ranges, which meet in memory of the call's own
+                                         (QT.Q4_K, 4096, 14336, 768), (QT.Q6_K, 7000, 8192, 768)], ids=str)
+def test_product_of_the_decoded_copy(qtype, n, k, m):
+    w = weight(qtype, n, k)
+    x = torch.randn((2, m // 2, k) if m % 2 == 0 else (m, k), device="cuda").bfloat16()
+    assert m > gj.fused_batch_limit(w)
+    assert (_lib.lib().ggq_rounded_gemm_temp(int(qtype), n, k, m) > 0) == (m == 768)
+    assert len(inside(lambda: gj.matmul(x, w))) == 1
+    y = gj.matmul(x, w)
+    assert y.dtype == torch.bfloat16 and y.shape == (*x.shape[:-1], n)
+    want = x.double() @ w.dequantize().double().T
+    assert ((y.double() - want).norm() / want.norm()).item() <= 2 ** -8 / 3 ** 0.5 + 1e-5
+    assert torch.equal(gj.dequant_matmul(x, w), y) and torch.equal(gj.matmul(x, w, block_bytes=1 << 20), y)
+    strided = torch.stack([x, x], dim=-2)[..., 0, :]
+    assert not strided.is_contiguous() and torch.equal(gj.matmul(strided, w), y)
+    xg = x.clone().requires_grad_(True)
+    yg = gj.matmul(xg, w)
+    assert torch.equal(yg.detach(), y)
+    g = torch.randn_like(y)
+    (dx,) = torch.autograd.grad(yg, xg, g)
+    want = g.double() @ w.dequantize().double()
+    assert ((dx.double() - want).norm() / want.norm()).item() <= 2 ** -8
+
+
+def test_calls_that_keep_the_copy():
+    n, k, m = 4096, 4096, 32
+    w, x = weight(QT.Q5_K, n, k), torch.randn((m, k), device="cuda").bfloat16()
+    y = gj.matmul(x, w)
+    assert inside(lambda: gj.matmul(x, w))
+    other = torch.empty(m * k + 1, device="cuda", dtype=torch.bfloat16)[1:].view(m, k).copy_(x)           # 2 bytes off a 16-byte boundary
+    for name, call in {"rows off 16 bytes": lambda: gj.matmul(other, w), "float32 weights": lambda: gj.matmul(x, w.astype(torch.float32)),
+                       "float16 x": lambda: gj.matmul(x.half(), w), "many rows": lambda: gj.matmul(x.repeat(65, 1), w)[:m]}.items():
+        assert not inside(call), name
+        assert ((call().double() - y.double()).norm() / y.double().norm()).item() <= 2 ** -8, name
+    with torch.autocast("cuda", dtype=torch.float16):
+        assert not inside(lambda: gj.matmul(x, w)) and gj.matmul(x, w).dtype == torch.float16
+    saved, calls = quants._DEQUANT[QT.Q5_K], []
+
+    def decode(blocks, dtype):
+        calls.append(blocks.shape)
+        return saved(blocks, dtype)
+
+    gj.register_dequant(QT.Q5_K, decode, override=True)
+    try:
+        gj.matmul(x, w), gj.dequant_matmul(x, w)
+        assert len(calls) == 2
+    finally:
+        gj.register_dequant(QT.Q5_K, saved, override=True)
+    assert inside(lambda: gj.matmul(x, w))
+
+
+@pytest.mark.parametrize("n,k,m", [(4096, 4096, 40), (4096, 14336, 765)], ids=str)
+def test_calls_on_several_streams_share_nothing(n, k, m):
+    w = weight(QT.Q4_K, n, k)
+    xs = [torch.randn((m + i, k), device="cuda").bfloat16() for i in range(4)]
+    want = [gj.matmul(x, w) for x in xs]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in xs], [[] for _ in xs]
+    for _ in range(10):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(gj.matmul(xs[i], w))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i]) for i in range(len(xs)) for y in got[i])
