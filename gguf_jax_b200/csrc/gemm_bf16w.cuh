@@ -1,0 +1,907 @@
+// The kernel of the fused decode + GEMM with bf16 weights (gemm_bf16w.cu says what it is and what bounds it), its work split and its launch.
+#pragma once
+
+#include "gemv.cuh"
+
+#include <cuda.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+#include <type_traits>
+
+namespace ggq {
+namespace gemmb {
+
+constexpr int kTileN = 128;                  // weight rows per CTA
+constexpr int kStageK = 64;                  // weights per stage: one 128-byte swizzle atom of bf16 per row
+constexpr int kDecodeWarps = 16;
+constexpr int kDecoders = kDecodeWarps * 32;
+constexpr int kThreads = kDecoders + 128;    // + raw copies, B copies, MMA (one warp or two)
+constexpr int kABytes = kTileN * 128;        // 16 KB
+constexpr int kSmemLimit = 232448;
+constexpr uint32_t kSpinLimit = 1u << 22;    // tries (each returns after a short hardware-defined wait)
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// arrival on the barrier at the same shared address in CTA `rank` of the cluster
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tmbarrier.arrive.shared::cluster.b64 _, [a];\n\t}"
+               ::"r"(bar), "r"(rank) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// Bounded wait; returns false (and raises the flags) when it gives up.  (Pausing between tries with nanosleep was
+// measured: the sleeps overshoot and stall the pipeline, up to 2 x slower.)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  if (mbar_try_wait(bar, parity)) return true;
+  if (*abort_flag) return false;
+  for (uint32_t i = 0; i < kSpinLimit; i++) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 255) == 255 && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  if (status) atomicOr(status, STATUS_WAIT_EXPIRED);
+  return false;
+}
+// After a wait that gave up: the last copies into a ring have to land (bounded too) before the shared memory is given back.
+__device__ __forceinline__ void drain(uint32_t full, int slots, int copies) {
+  for (int i = max(0, copies - slots); i < copies; i++)
+    for (uint32_t spin = 0; spin < kSpinLimit && !mbar_try_wait(full + 8 * (i % slots), (i / slots) & 1); spin++) {}
+}
+// Shared-memory matrix descriptor, K-major, 128-byte swizzle: start address / 16 in bits 0-13, leading byte
+// offset (unused for swizzled K-major, 1) in 16-29, stride byte offset (1024 B between 8-row groups) / 16 in
+// 32-45, descriptor version 1 in 46-47, layout type 2 (SWIZZLE_128B) in 61-63.
+__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
+  return (uint64_t)((smem_addr >> 4) & 0x3FFF) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+// Instruction descriptor for kind::f16 with bf16 operands and float32 accumulation, both operands K-major:
+// c_format F32 (bits 4-5 = 1), a / b format BF16 (bits 7-9, 10-12 = 1), N >> 3 in 17-22, M >> 4 in 24-28.
+constexpr uint32_t umma_idesc(int mma_m, int mma_n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(mma_n >> 3) << 17) | ((uint32_t)(mma_m >> 4) << 24);
+}
+template <int CG>
+__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (CG == 1)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// arrival on `bar` (of every CTA of the group) once the MMAs issued so far have completed
+template <int CG>
+__device__ __forceinline__ void umma_commit(uint32_t bar, uint32_t in_cluster) {
+  if constexpr (CG == 1)
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((uint16_t)(3u << (in_cluster & ~1u))) : "memory");
+}
+__device__ __forceinline__ void sts_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void sts_v2(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory"); return v; }
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) { uint32_t v; asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a) : "memory"); return v; }
+__device__ __forceinline__ uint4 lds_v4(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float h2f(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
+// byte SEL of v as a float, exact: the bits 0x4B0000vv are 2^23 + v
+template <int SEL>
+__device__ __forceinline__ float byte_to_float(uint32_t v) {
+  return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440 + SEL)) - 8388608.0f;
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&p);
+}
+// byte SEL of v plus 128 as a float, exact, in one instruction: the bits 0x43vv0000 are 128 + v for v < 128
+template <int SEL>
+__device__ __forceinline__ float byte_plus_128(uint32_t v) {
+  return __uint_as_float(__byte_perm(v, 0x43000000u, 0x7044 + (SEL << 8)));
+}
+// pairs of float32 in one 64-bit register (Blackwell computes on both with one instruction)
+__device__ __forceinline__ uint64_t pair(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint32_t pack_bf16(uint64_t v) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return pack_bf16(a, b);
+}
+// (v & mask) | w
+__device__ __forceinline__ uint32_t and_or(uint32_t v, uint32_t mask, uint32_t w) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(w));
+  return r;
+}
+// float16 pair 1024 + fields minus c (as a pair), exact
+__device__ __forceinline__ uint32_t minus2(uint32_t v, uint32_t c) { uint32_t r; asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(c)); return r; }
+__device__ __forceinline__ float low_half(uint32_t v) { return h2f(v & 0xFFFF); }
+__device__ __forceinline__ float high_half(uint32_t v) { return h2f(v >> 16); }
+
+// ---------------------------------------------------------------------------------------------
+// Formats.  load() takes a warp's share of a superblock out of the raw slot; decode() turns it into weights in the A stages.
+//
+// Q4_K, Q5_K: a warp takes 32 rows (a lane each) of one stage of the superblock: 32 code bytes, whose low nibbles are the stage's first
+// 32 weights and whose high nibbles the other 32; rows are an odd number of 16-byte pieces apart, so eight lanes' 16-byte
+// loads, and their 16-byte stores to the swizzled tile, fall on different banks.
+// weight = fma(code, d * sc, -(dmin * mn)): both products are exact in float32, so this is the decode kernel's float32 value.
+template <bool FIVE>
+struct FQ45 {
+  static constexpr int kTs = FIVE ? 176 : 144, kBoxWords = kTs / 4;
+  static constexpr bool kWholeSuperblock = false;     // a warp fills one stage of a superblock (not all four)
+  static constexpr bool kDirect = false;              // load() brings its bytes to registers
+  struct Raw { uint4 hd, q0, q1, h0, h1; };
+  __device__ static void load(Raw& r, uint32_t slot, int warp, int lane, int) {
+    const int p = warp >> 2;
+    const uint32_t blk = slot + (32 * (warp & 3) + lane) * kTs;
+    r.hd = lds_v4(blk);
+    if constexpr (FIVE) { r.h0 = lds_v4(blk + 16); r.h1 = lds_v4(blk + 32); }
+    r.q0 = lds_v4(blk + (FIVE ? 48 : 16) + 32 * p);
+    r.q1 = lds_v4(blk + (FIVE ? 48 : 16) + 32 * p + 16);
+  }
+  // a: address of the stage's A tile
+  __device__ static void decode(const Raw& r, uint32_t a, int warp, int lane) {
+    const int p = warp >> 2, row = 32 * (warp & 3) + lane;
+    uint32_t sc, mn;                                   // groups 2 p and 2 p + 1: bytes 0, 1
+    if (p < 2) { sc = r.hd.y & 0x3F3F3F3Fu; mn = r.hd.z & 0x3F3F3F3Fu; }
+    else {
+      sc = (r.hd.w & 0x0F0F0F0Fu) | ((r.hd.y >> 2) & 0x30303030u);
+      mn = ((r.hd.w >> 4) & 0x0F0F0F0Fu) | ((r.hd.z >> 2) & 0x30303030u);
+    }
+    if (p & 1) { sc >>= 16; mn >>= 16; }
+    const float d = h2f(r.hd.x & 0xFFFF), nd = -h2f(r.hd.x >> 16);
+    const float s0 = __fmul_rn(d, byte_to_float<0>(sc)), s1 = __fmul_rn(d, byte_to_float<1>(sc));
+    const float o0 = __fmul_rn(nd, byte_to_float<0>(mn)), o1 = __fmul_rn(nd, byte_to_float<1>(mn));
+    const uint64_t a0 = pair(s0, s0), a1 = pair(s1, s1), b0 = pair(o0, o0), b1 = pair(o1, o1), off = pair(-128.0f, -128.0f);
+    const uint32_t dst = a + (row >> 3) * 1024 + (row & 7) * 128, rx = (uint32_t)(row & 7) << 4;
+    // four codes (bytes below 128) -> two words of bf16 pairs
+    auto four = [&](uint32_t c, uint64_t sa, uint64_t sb, uint32_t& w0, uint32_t& w1) {
+      w0 = pack_bf16(fma2(add2(pair(byte_plus_128<0>(c), byte_plus_128<1>(c)), off), sa, sb));
+      w1 = pack_bf16(fma2(add2(pair(byte_plus_128<2>(c), byte_plus_128<3>(c)), off), sa, sb));
+    };
+    // eight bytes of codes: chunk c of the row (low nibbles) and chunk c + 4 (high nibbles)
+    auto put = [&](int c, uint32_t q0, uint32_t q1, uint32_t h0, uint32_t h1) {
+      uint32_t c0 = q0 & 0x0F0F0F0Fu, c1 = q1 & 0x0F0F0F0Fu, c2 = (q0 >> 4) & 0x0F0F0F0Fu, c3 = (q1 >> 4) & 0x0F0F0F0Fu;
+      if constexpr (FIVE) {                            // bit 2 p of a byte: fifth bit of the low nibble's code, bit 2 p + 1: of the high one's
+        h0 >>= 2 * p;
+        h1 >>= 2 * p;
+        c0 = and_or(h0 << 4, 0x10101010u, c0);
+        c1 = and_or(h1 << 4, 0x10101010u, c1);
+        c2 = and_or(h0 << 3, 0x10101010u, c2);
+        c3 = and_or(h1 << 3, 0x10101010u, c3);
+      }
+      uint32_t w[4];
+      four(c0, a0, b0, w[0], w[1]);
+      four(c1, a0, b0, w[2], w[3]);
+      sts_v4(dst + (((uint32_t)c << 4) ^ rx), w[0], w[1], w[2], w[3]);
+      four(c2, a1, b1, w[0], w[1]);
+      four(c3, a1, b1, w[2], w[3]);
+      sts_v4(dst + (((uint32_t)(c + 4) << 4) ^ rx), w[0], w[1], w[2], w[3]);
+    };
+    put(0, r.q0.x, r.q0.y, r.h0.x, r.h0.y);
+    put(1, r.q0.z, r.q0.w, r.h0.z, r.h0.w);
+    put(2, r.q1.x, r.q1.y, r.h1.x, r.h1.y);
+    put(3, r.q1.z, r.q1.w, r.h1.z, r.h1.w);
+  }
+};
+// Q6_K: a block is 210 bytes, 2-byte aligned, at the same offset within its 16-byte piece in every row.  A warp takes eight rows of the whole superblock,
+// four lanes a row, each every fourth word: with rows 15 pieces apart the 32 words of a load lie on 32 banks whatever the
+// offset (words at 2 mod 4 come from two loads), and 16 lanes' 8-byte stores (rows 0, 2, 4, 6 or 1, 3, 5, 7 of the tile's eight) too.
+// Half n (128 weights): lane j takes words j and j + 4 of ql[64 n ..], ql[64 n + 32 ..] and qh[32 n ..]: four weights of each of
+// the half's eight groups of 16.  The 16 float32 scales of a row are worked out once, four by each of its lanes, and meet in
+// the row's raw bytes, which are in registers by then.  weight = a * (q - 32): exact.
+struct FQ6 {
+  static constexpr int kTs = 210, kBoxWords = 60, kPitch = 240;
+  static constexpr bool kWholeSuperblock = true, kDirect = false;
+  struct Raw { uint32_t q[2][6]; uint32_t sc; float d; };
+  __device__ static uint32_t row_of(int lane) { const int rr = lane >> 2; return (uint32_t)(rr < 4 ? 2 * rr : 2 * rr - 7); }
+  __device__ static void load(Raw& r, uint32_t slot, int warp, int lane, int skew) {
+    const uint32_t blk = slot + (8 * warp + row_of(lane)) * kPitch + skew, j4 = 4 * (lane & 3);
+    r.d = h2f(lds_u16(blk + 208));
+    if (skew & 2) {
+      auto word = [&](uint32_t at) { return __byte_perm(lds_u32(blk + at + j4 - 2), lds_u32(blk + at + j4 + 2), 0x5432); };
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int i = 0; i < 6; i++) r.q[n][i] = word((i < 4 ? 64 * n + 32 * (i >> 1) : 128 + 32 * n) + 16 * (i & 1));
+      r.sc = word(192);
+    } else {
+      auto word = [&](uint32_t at) { return lds_u32(blk + at + j4); };
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int i = 0; i < 6; i++) r.q[n][i] = word((i < 4 ? 64 * n + 32 * (i >> 1) : 128 + 32 * n) + 16 * (i & 1));
+      r.sc = word(192);
+    }
+  }
+  // scales of the row into its raw bytes at `tab` (every lane of the warp has loaded its words); then each lane reads all 16
+  __device__ static void scales(const Raw& r, uint32_t tab, int lane) {
+    const uint32_t x = r.sc ^ 0x80808080u;            // int8 + 128
+    const float d = lane & 1 ? r.d * 0.0625f : r.d;    // quarters 2 and 3 (odd words of the scales) take their codes 16-fold, see decode
+    float a[4];
+    a[0] = __fmul_rn(d, byte_to_float<0>(x) - 128.0f);
+    a[1] = __fmul_rn(d, byte_to_float<1>(x) - 128.0f);
+    a[2] = __fmul_rn(d, byte_to_float<2>(x) - 128.0f);
+    a[3] = __fmul_rn(d, byte_to_float<3>(x) - 128.0f);
+    sts_v4(tab + 16 * (lane & 3), __float_as_uint(a[0]), __float_as_uint(a[1]), __float_as_uint(a[2]), __float_as_uint(a[3]));
+  }
+  // half N of the superblock into the tiles at a0 (stage 2 N) and a1 (stage 2 N + 1); s: the half's eight scales
+  template <int N>
+  __device__ static void decode(const Raw& r, const float (&s)[8], uint32_t a0, uint32_t a1, int warp, int lane) {
+    const uint32_t row = row_of(lane), j = lane & 3;
+    const uint32_t dst = 1024 * warp + 128 * row + 8 * (j & 1);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {                     // group of 16: weights 16 i + 4 j .. + 3 of every quarter
+      const uint32_t h = r.q[N][4 + i], h4 = h << 4, h2 = h << 2, g4 = h >> 4, g2 = h >> 6;
+#pragma unroll
+      for (int b = 0; b < 2; b++) {                   // quarters b (low nibbles) and 2 + b (high nibbles, 16 times the code)
+        const uint32_t q = r.q[N][2 * b + i], q8 = q >> 8, he = b ? h2 : h4, ho = b ? g2 : g4;
+        // (v & mask) | 0x64006400 is the float16 pair 1024 + v, wherever below bit 10 the fields lie
+        constexpr uint32_t k1024 = 0x64006400u, k1056 = 0x64206420u, k1536 = 0x66006600u;
+        const uint32_t e0 = minus2(and_or(he, 0x00300030u, and_or(q, 0x000F000Fu, k1024)), k1056), d0 = minus2(and_or(ho, 0x00300030u, and_or(q8, 0x000F000Fu, k1024)), k1056);
+        const uint32_t e1 = minus2(and_or(he, 0x03000300u, and_or(q, 0x00F000F0u, k1024)), k1536), d1 = minus2(and_or(ho, 0x03000300u, and_or(q8, 0x00F000F0u, k1024)), k1536);
+        const float s0 = s[2 * b + i], s1 = s[4 + 2 * b + i];
+        const uint32_t at = dst + (((4 * b + 2 * i + (j >> 1)) ^ row) << 4);
+        sts_v2(a0 + at, pack_bf16(__fmul_rn(low_half(e0), s0), __fmul_rn(low_half(d0), s0)), pack_bf16(__fmul_rn(high_half(e0), s0), __fmul_rn(high_half(d0), s0)));
+        sts_v2(a1 + at, pack_bf16(__fmul_rn(low_half(e1), s1), __fmul_rn(low_half(d1), s1)), pack_bf16(__fmul_rn(high_half(e1), s1), __fmul_rn(high_half(d1), s1)));
+      }
+    }
+  }
+};
+// Eight batch columns of 32 weight rows (a lane each), 2-byte results: the 8 x 8 squares are turned with shuffles, so that a lane stores 16 bytes
+// (rows 8 (lane / 8) .. + 7 of column lane % 8) instead of eight times 2.  at: index of the first element; rows: of the 32 that exist (a multiple of 8).
+__device__ __forceinline__ void store_8x8(void* y, int y_dtype, int64_t at, int64_t N, int cols, int rows, const uint32_t (&v)[8], int lane) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {                        // rows in pairs: lane = 2 r + c has rows 2 r, 2 r + 1 of column 2 i + c
+    const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, lane & 1 ? v[2 * i] : v[2 * i + 1], 1);
+    const float lo = __uint_as_float(lane & 1 ? got : v[2 * i]), hi = __uint_as_float(lane & 1 ? v[2 * i + 1] : got);
+    if (y_dtype == GGQ_BF16) {
+      w[i] = pack_bf16(lo, hi);
+    } else {
+      const __half2 h = __floats2half2_rn(lo, hi);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i += 2) {                     // w[i], w[i + 1]: four rows of column 2 i + lane % 4
+    const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, lane & 2 ? w[i] : w[i + 1], 2);
+    const uint32_t a = lane & 2 ? got : w[i], b = lane & 2 ? w[i + 1] : got;
+    w[i] = a;
+    w[i + 1] = b;
+  }
+  const uint32_t g0 = __shfl_xor_sync(0xFFFFFFFFu, lane & 4 ? w[0] : w[2], 4), g1 = __shfl_xor_sync(0xFFFFFFFFu, lane & 4 ? w[1] : w[3], 4);
+  const uint4 o = lane & 4 ? make_uint4(g0, g1, w[2], w[3]) : make_uint4(w[0], w[1], g0, g1);
+  if ((lane & 7) < cols && 8 * (lane >> 3) < rows)
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(y) + at + (lane & 7) * N + 8 * (lane >> 3)) = o;
+}
+
+// The units of a range, segment by segment (a segment is the part of one tile in the range).  Within a segment the superblocks are taken from a
+// place on that differs from tile to tile, so that the CTAs do not all ask the L2 for the same activations at the same time.
+struct Walk {
+  int SB, left, t, first, len, i, sb;
+  __device__ Walk(int64_t u0, int64_t u1, int SB_) : SB(SB_), left((int)(u1 - u0)), t((int)(u0 / SB_)), first((int)(u0 % SB_)) { segment(); }
+  __device__ void segment() {
+    len = min(SB - first, left);
+    i = 0;
+    sb = len > 1 ? first + (int)(((uint32_t)t * 2654435761u >> 16) % (uint32_t)len) : first;
+  }
+  __device__ bool more() const { return left > 0; }
+  // to the next unit; true where that begins another segment (or nothing is left)
+  __device__ bool next() {
+    left--;
+    if (++sb == first + len) sb = first;
+    if (++i < len) return false;
+    t++;
+    first = 0;
+    segment();
+    return true;
+  }
+};
+
+template <class F, int MT, int CG>
+struct Cfg {
+  static constexpr int kBBytes = MT / CG * 128, kRawBytes = kTileN * F::kBoxWords * 4;
+  static constexpr int kBStages = MT / CG >= 256 ? 3 : MT / CG >= 128 ? 4 : MT / CG >= 64 ? 8 : 12;      // a multiple of kStep, as kAStages
+  // stages the MMA warp takes at once: its waits, fence and commit cost 300 cycles whatever they cover, the MMAs of a stage 64 to 256 up to 128 columns
+  static constexpr int kStep = MT / CG >= 256 ? 1 : 2;
+  static constexpr int kAWanted = MT / CG >= 256 ? 4 : 6;
+  // (a step fewer where two superblocks of raw bytes would not fit: Q8_0)
+  static constexpr int kAStages = kAWanted * kABytes + kBStages * kBBytes + 512 + 1024 + 2 * kRawBytes <= kSmemLimit ? kAWanted : kAWanted - kStep;
+  static constexpr int kFixed = kAStages * kABytes + kBStages * kBBytes + 512 + 1024;
+  static constexpr int kRawFit = (kSmemLimit - kFixed) / kRawBytes, kRawStages = kRawFit > 4 ? 4 : kRawFit;
+  static constexpr int kSmem = kFixed + kRawStages * kRawBytes;
+  static constexpr int kAcc = MT <= 256 ? 2 : 1;                // accumulators in the 512 columns of tensor memory
+  // MMA warps: the issue of a step's MMAs blocks until most of them have run, so with one warp the tensor cores idle through its waits, its commit and its
+  // loop (480 of 1030 cycles per step of 128 weights at 64 columns).  Two warps take the steps in turn, each into an accumulator of its own.
+  static constexpr int kMma = kStep == 2 && CG == 1 ? 2 : 1;
+  static constexpr int kTmemCols = kAcc * kMma * MT;
+  static_assert(kTmemCols >= 32 && kTmemCols <= 512, "tensor memory");
+  static_assert(kRawStages >= 2, "shared memory");
+};
+
+struct Args {
+  int N, K, M, y_dtype, tiles_n, tiles, split;      // tiles_n: row tiles; tiles: times column tiles
+  void* y;
+  int* status;
+  float* partials;
+  int* counters;
+  const uint8_t* tab;      // code books, for the formats that have them
+  const uint8_t* w;
+  int64_t row_bytes;
+};
+
+// four rows of a finished column; vec: N a multiple of 8, so that all four rows exist or none, and y 16-byte aligned
+__device__ __forceinline__ void put_column(const Args& g, int m, int n, const float4& v, bool vec) {
+  const int64_t at = (int64_t)m * g.N + n;
+  const int left = g.N - n;
+  if (vec) {
+    if (left <= 0) return;
+    if (g.y_dtype == GGQ_F32) {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(g.y) + at) = v;
+      return;
+    }
+    uint2 o;
+    if (g.y_dtype == GGQ_BF16) {
+      o = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    } else {
+      const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
+      o = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(g.y) + at) = o;
+    return;
+  }
+  if (left > 0) store_out(g.y, g.y_dtype, at, v.x);
+  if (left > 1) store_out(g.y, g.y_dtype, at + 1, v.y);
+  if (left > 2) store_out(g.y, g.y_dtype, at + 2, v.z);
+  if (left > 3) store_out(g.y, g.y_dtype, at + 3, v.w);
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+  return v;
+}
+
+template <class F, int MT, int CG>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_bf16w_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, const Args g) {
+  using C = Cfg<F, MT, CG>;
+  constexpr int P = C::kStep, kA = C::kAStages / P, kB = C::kBStages / P, kR = C::kRawStages, kAcc = C::kAcc, kMma = C::kMma;     // ring slots of P stages
+  constexpr int kAStep = P * kABytes, kBStep = P * C::kBBytes;
+  extern __shared__ uint8_t smem_raw[];
+  // the swizzle is a function of the address bits: tiles start 1024-byte aligned
+  const uint32_t base = (smem_u32(smem_raw) + 1023) & ~1023u;
+  const uint32_t a_base = base, b_base = a_base + kA * kAStep, raw_base = b_base + kB * kBStep, bars = raw_base + kR * C::kRawBytes;
+  uint8_t* tail = smem_raw + (bars - smem_u32(smem_raw));
+  const uint32_t raw_full = bars, raw_empty = raw_full + 8 * kR, a_full = raw_empty + 8 * kR, a_empty = a_full + 8 * kA,
+                 b_full = a_empty + 8 * kA, b_empty = b_full + 8 * kB, peer_full = b_empty + 8 * kB, acc_full = peer_full + 8 * kA,
+                 acc_empty = acc_full + 8 * kAcc;
+  static_assert(8 * (2 * kR + 3 * kA + 2 * kB + 2 * kAcc) <= 400, "barriers");
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail + 448);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 452);
+  volatile int* last_flag = reinterpret_cast<volatile int*>(tail + 456);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t in_cluster;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(in_cluster));
+  const uint32_t rank = CG == 2 ? in_cluster & 1 : 0;         // within the pair
+  const bool odd_rows = F::kDirect && g.row_bytes % 16 != 0;   // no TMA box: a tensor map's rows are multiples of 16 bytes apart
+  const int SB = g.K / 256, G = gridDim.x / CG, me = blockIdx.x / CG;
+  const int64_t U = (int64_t)g.tiles * SB;
+  // split > 1: a cluster of `split` CTAs (pairs) per tile, a range of K each; else equal ranges of the list of units
+  int64_t u0, u1;
+  if (g.split > 1) {
+    const int64_t t0 = (int64_t)(me / g.split) * SB;
+    const int part = me % g.split;
+    u0 = t0 + SB * part / g.split;
+    u1 = t0 + SB * (part + 1) / g.split;
+  } else {
+    u0 = U * me / G;
+    u1 = U * (me + 1) / G;
+  }
+
+  if (tid == 0) {
+    for (int s = 0; s < kR; s++) { mbar_init(raw_full + 8 * s, F::kDirect && odd_rows ? 32 : 1); mbar_init(raw_empty + 8 * s, kDecodeWarps); }
+    for (int s = 0; s < kA; s++) {
+      mbar_init(a_full + 8 * s, F::kWholeSuperblock ? kDecodeWarps : 4 * P);
+      mbar_init(a_empty + 8 * s, 1);
+      mbar_init(peer_full + 8 * s, 1);
+    }
+    for (int s = 0; s < kB; s++) { mbar_init(b_full + 8 * s, 1); mbar_init(b_empty + 8 * s, 1); }
+    for (int s = 0; s < kAcc; s++) { mbar_init(acc_full + 8 * s, kMma); mbar_init(acc_empty + 8 * s, kDecodeWarps * CG); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  constexpr int kRawWarp = kDecodeWarps, kBWarp = kDecodeWarps + 1, kMmaWarp = kDecodeWarps + 2;
+  if (warp == kMmaWarp) {   // owns the TMEM allocation
+    if constexpr (CG == 1) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)C::kTmemCols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)C::kTmemCols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if constexpr (CG == 2) cluster_sync();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == kRawWarp) {
+    // ------------------------------- raw weight bytes -------------------------------
+    if (odd_rows) {
+      // Eight lanes a row copy the 16-byte aligned window of its superblock (every row at its own offset); rows past the end repeat the last one, which
+      // is never stored.
+      int s = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (Walk at(u0, u1, SB); at.more() && ok; at.next()) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(raw_empty + 8 * s, ph, abort_flag, g.status));
+        if (!ok) break;
+        const int n0 = (at.t % g.tiles_n) * (kTileN * CG) + (int)rank * kTileN;
+        const uint32_t slot = raw_base + s * C::kRawBytes + 16 * (lane & 7) + (lane >> 3) * (F::kBoxWords * 4);
+        const uint32_t mine = 16 * (lane & 7);             // where the lane's piece lies in a window
+        auto copy = [&](int i, const uint8_t* p) {         // row 4 i + lane / 8 of the tile
+          const uint32_t skew = (uint32_t)(uintptr_t)p & 15;
+          const uint8_t* from = p - skew + mine;
+          const uint32_t to = slot + i * (4 * F::kBoxWords * 4);
+          if (mine < skew + F::kTs) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+#pragma unroll
+          for (int more = 128; more < F::kBoxWords * 4; more += 128)
+            if (mine + more < skew + F::kTs) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + more), "l"(from + more) : "memory");
+        };
+        if (n0 + kTileN <= g.N) {
+          const uint8_t* p = g.w + (int64_t)(n0 + (lane >> 3)) * g.row_bytes + (int64_t)at.sb * F::kTs;
+#pragma unroll 8
+          for (int i = 0; i < kTileN / 4; i++, p += 4 * g.row_bytes) copy(i, p);
+        } else {
+          for (int i = 0; i < kTileN / 4; i++) copy(i, g.w + (int64_t)min(n0 + 4 * i + (lane >> 3), g.N - 1) * g.row_bytes + (int64_t)at.sb * F::kTs);
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(raw_full + 8 * s) : "memory");
+        if (++s == kR) { s = 0; ph ^= 1; }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if (lane == 0) {
+      int s = 0, copies = 0;
+      uint32_t ph = 1;                        // parity of the "empty" phase to wait for (the first round passes at once)
+      for (Walk at(u0, u1, SB); at.more(); at.next()) {
+        if (!mbar_wait(raw_empty + 8 * s, ph, abort_flag, g.status)) break;
+        const int row = (at.t % g.tiles_n) * (kTileN * CG) + (int)rank * kTileN;
+        const int word = ((at.sb * F::kTs) & ~15) >> 2;
+        tma_box_load(raw_base + s * C::kRawBytes, &w_map, word, row, raw_full + 8 * s, (uint32_t)C::kRawBytes);
+        copies++;
+        if (++s == kR) { s = 0; ph ^= 1; }
+      }
+      if (*abort_flag) drain(raw_full, kR, copies);
+    }
+  } else if (warp == kBWarp) {
+    // ------------------------------- activations -------------------------------
+    if (lane == 0) {
+      pdl_wait();                             // the launch before may have written them
+      int s = 0, copies = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (Walk at(u0, u1, SB); at.more() && ok; at.next()) {
+        const int t = at.t, sb = at.sb;
+        const int m0 = (t / g.tiles_n) * MT;
+        for (int q = 0; q < 4; q += P) {
+          ok = mbar_wait(b_empty + 8 * s, ph, abort_flag, g.status);
+          if (!ok) break;
+          const uint32_t dst = b_base + s * kBStep, bar = b_full + 8 * s;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)kBStep) : "memory");
+          // CG = 1: one box of MT rows; CG = 2: this CTA's half of the rows of every MMA (of up to 256 columns)
+          constexpr int kMmaN = MT > 256 ? 256 : MT, kBox = kMmaN / CG;
+#pragma unroll
+          for (int i = 0; i < P; i++)
+#pragma unroll
+          for (int h = 0; h < MT / kMmaN; h++)
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                         ::"r"(dst + i * C::kBBytes + h * (kBox * 128)), "l"(&x_map), "r"(sb * 256 + (q + i) * kStageK), "r"(m0 + h * kMmaN + (int)rank * kBox), "r"(bar) : "memory");
+          copies++;
+          if (++s == kB) { s = 0; ph ^= 1; }
+        }
+      }
+      if (*abort_flag) drain(b_full, kB, copies);
+    }
+  } else if (warp >= kMmaWarp) {
+    // ------------------------------- MMA issue -------------------------------
+    // The whole warp walks the loop, also after a wait that gave up (the others then give up at once), and one elected lane issues: the operands
+    // of a tcgen05 instruction are uniform registers.
+    constexpr int kMmaN = MT > 256 ? 256 : MT, kBox = kMmaN / CG;
+    constexpr uint32_t idesc = umma_idesc(kTileN * CG, kMmaN);
+    const uint64_t a_desc0 = umma_desc(a_base), b_desc0 = umma_desc(b_base);
+    const int mw = warp - kMmaWarp;              // takes the steps mw, mw + kMma, ..; a superblock has 4 / P, a multiple of kMma
+    int sa = mw, sb = mw, acc = 0;
+    uint32_t pa = 0, pb = 0, pacc = 1;
+    bool ok = true;
+    for (int64_t u = u0; u < u1 && mw < kMma;) {
+      const int64_t end = min((u / SB + 1) * SB, u1);
+      const int n = (int)(end - u) * (4 / P);
+      if (CG == 1 || rank == 0) {
+        ok &= mbar_wait(acc_empty + 8 * acc, pacc, abort_flag, g.status);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");       // after the epilogue's reads
+      }
+      const uint32_t d = tmem_base + (acc * kMma + mw) * MT;
+      for (int st = mw; st < n; st += kMma) {
+        ok &= mbar_wait(b_full + 8 * sb, pb, abort_flag, g.status);
+        ok &= mbar_wait(a_full + 8 * sa, pa, abort_flag, g.status);
+        if (CG == 2 && rank == 1) {
+          if (lane == 0 && ok) mbar_arrive_remote(peer_full + 8 * sa, in_cluster & ~1u);            // this half of the operands is there
+        } else {
+          if constexpr (CG == 2) ok &= mbar_wait(peer_full + 8 * sa, pa, abort_flag, g.status);
+          const uint64_t ad = a_desc0 + (uint32_t)(sa * (kAStep >> 4)), bd = b_desc0 + (uint32_t)(sb * (kBStep >> 4));
+          if (elect_one() && ok) {
+#pragma unroll
+            for (int kk = 0; kk < P * 4; kk++) {       // four steps of 16 weights per stage
+#pragma unroll
+              for (int h = 0; h < MT / kMmaN; h++)
+                umma_bf16<CG>(d + h * kMmaN, ad + (kk / 4) * (kABytes >> 4) + 2 * (kk % 4), bd + (kk / 4) * (C::kBBytes >> 4) + h * (kBox * 128 >> 4) + 2 * (kk % 4),
+                              idesc, (uint32_t)((st - mw) | kk));
+            }
+            umma_commit<CG>(a_empty + 8 * sa, in_cluster);          // the slots may be refilled once these MMAs have read them
+            umma_commit<CG>(b_empty + 8 * sb, in_cluster);
+            if (st + kMma >= n) umma_commit<CG>(acc_full + 8 * acc, in_cluster);   // and the accumulator is complete
+          }
+          __syncwarp();
+        }
+        static_assert(kMma <= kB && kMma <= kA, "slots");
+        if ((sa += kMma) >= kA) { sa -= kA; pa ^= 1; }
+        if ((sb += kMma) >= kB) { sb -= kB; pb ^= 1; }
+      }
+      if (++acc == kAcc) { acc = 0; pacc ^= 1; }
+      u = end;
+    }
+  } else {
+    // ------------------------------- decode -------------------------------
+    // After a wait that gave up, the rest of the loop runs on (its waits give up at once) on whatever the buffers hold.
+    bool alive = true;
+    int rs = 0, acc = 0;
+    uint32_t rp = 0, pacc = 0;
+    // A slot (in stages) of the warp's next stage, and the parity of its "empty" phase
+    int sa = F::kWholeSuperblock ? 0 : warp >> 2;
+    uint32_t pa = 1;
+    auto next_a = [&](int step) { sa += step; if (sa >= kA * P) { sa -= kA * P; pa ^= 1; } };
+    typename F::Raw raw;
+    Walk at(u0, u1, SB);
+    auto fetch = [&]() {
+      alive &= mbar_wait(raw_full + 8 * rs, rp, abort_flag, g.status);
+      if constexpr (!F::kDirect) F::load(raw, raw_base + rs * C::kRawBytes, warp, lane, (at.sb * F::kTs) & 15);
+    };
+    fetch();
+    for (bool first = true; at.more(); first = false) {
+      const int t = at.t;
+      const bool whole = at.len == SB;
+      for (bool end = false; !end;) {
+        uint32_t skew = (uint32_t)at.sb * F::kTs;
+        if constexpr (F::kDirect) {
+          if (odd_rows) skew += (uint32_t)min((t % g.tiles_n) * (kTileN * CG) + (int)rank * kTileN + F::row_of(warp, lane), g.N - 1) * (uint32_t)(g.row_bytes & 15);
+        }
+        skew &= 15;
+        end = at.next();
+        if constexpr (F::kDirect) {
+          // decoded out of the raw slot, half a superblock (two stages, which are one slot or two) at a time
+          const uint8_t* bytes = smem_raw + (raw_base - smem_u32(smem_raw)) + rs * C::kRawBytes + F::row_of(warp, lane) * (F::kBoxWords * 4) + skew;
+          auto half = [&](auto n) {
+            const int x0 = sa;
+            alive &= mbar_wait(a_empty + 8 * (sa / P), pa, abort_flag, g.status);
+            next_a(1);
+            const int x1 = sa;
+            if (P == 1) alive &= mbar_wait(a_empty + 8 * sa, pa, abort_flag, g.status);
+            next_a(1);
+            F::template decode<decltype(n)::value>(bytes, a_base + x0 * kABytes, a_base + x1 * kABytes, warp, lane, g.tab);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the tensor cores read through the async proxy
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(a_full + 8 * (x0 / P));
+              if (P == 1) mbar_arrive(a_full + 8 * x1);
+            }
+          };
+          half(std::integral_constant<int, 0>{});
+          half(std::integral_constant<int, 1>{});
+          if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
+          if (++rs == kR) { rs = 0; rp ^= 1; }
+          if (at.more()) fetch();
+        } else if constexpr (F::kWholeSuperblock) {
+          const uint32_t tab = raw_base + rs * C::kRawBytes + (8 * warp + F::row_of(lane)) * F::kPitch;
+          __syncwarp();
+          F::scales(raw, tab, lane);
+          __syncwarp();
+          float s0[8], s1[8];
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const uint4 v = lds_v4(tab + 16 * i), w = lds_v4(tab + 32 + 16 * i);
+            s0[4 * i] = __uint_as_float(v.x); s0[4 * i + 1] = __uint_as_float(v.y); s0[4 * i + 2] = __uint_as_float(v.z); s0[4 * i + 3] = __uint_as_float(v.w);
+            s1[4 * i] = __uint_as_float(w.x); s1[4 * i + 1] = __uint_as_float(w.y); s1[4 * i + 2] = __uint_as_float(w.z); s1[4 * i + 3] = __uint_as_float(w.w);
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(raw_empty + 8 * rs);
+          if (++rs == kR) { rs = 0; rp ^= 1; }
+          // half n of the superblock: two stages, which are one slot or two
+          auto half = [&](auto n, const float (&sc)[8]) {
+            const int x0 = sa;
+            alive &= mbar_wait(a_empty + 8 * (sa / P), pa, abort_flag, g.status);
+            next_a(1);
+            const int x1 = sa;
+            if (P == 1) alive &= mbar_wait(a_empty + 8 * sa, pa, abort_flag, g.status);
+            next_a(1);
+            F::template decode<decltype(n)::value>(raw, sc, a_base + x0 * kABytes, a_base + x1 * kABytes, warp, lane);
+            if (decltype(n)::value == 1 && at.more()) fetch();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the tensor cores read through the async proxy
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(a_full + 8 * (x0 / P));
+              if (P == 1) mbar_arrive(a_full + 8 * x1);
+            }
+          };
+          half(std::integral_constant<int, 0>{}, s0);
+          half(std::integral_constant<int, 1>{}, s1);
+        } else {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(raw_empty + 8 * rs);           // the warp's bytes are in its registers
+          if (++rs == kR) { rs = 0; rp ^= 1; }
+          alive &= mbar_wait(a_empty + 8 * (sa / P), pa, abort_flag, g.status);
+          F::decode(raw, a_base + sa * kABytes, warp, lane);
+          const int x = sa;
+          next_a(4);
+          if (at.more()) fetch();                                   // the next bytes are on their way while the stores settle
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the tensor cores read through the async proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive(a_full + 8 * (x / P));
+        }
+      }
+      // ------------------------------- epilogue of the segment -------------------------------
+      if (!at.more() && tid == 0) pdl_trigger();
+      if (first) pdl_wait();            // nothing is written before the launch before has completed
+      const int n0 = (t % g.tiles_n) * (kTileN * CG) + (int)rank * kTileN, m0 = (t / g.tiles_n) * MT;
+      // warp e: TMEM lanes (rows) 32 (e & 3) .. + 31; the columns are split over the four warps of a quarter
+      const int quarter = warp & 3, cpart = warp >> 2;
+      const int row = 32 * quarter + lane, out_row = n0 + row;
+      const bool vec = g.N % 8 == 0 && (uintptr_t)g.y % 16 == 0;
+      const int slot = 2 * me + (first ? 0 : 1);
+      float* mine = g.partials + ((int64_t)slot * CG + rank) * MT * kTileN;
+      alive &= mbar_wait(acc_full + 8 * acc, pacc, abort_flag, g.status);
+      alive = __all_sync(0xFFFFFFFFu, alive);                               // tcgen05.ld needs the whole warp
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // Where the rings are done with (a split tile's range, the last segment), the tile is turned around in their memory, up to 256 columns at a time:
+      // columns of 128 float32 rows, out of which a warp stores a whole column with wide accesses.
+      const bool staged = g.split > 1 || (whole && !at.more());
+      constexpr int kPassCols = MT > 256 ? 256 : MT, kPart = kPassCols / 4;       // columns per pass, of a warp in a pass
+      constexpr int kLd = kPart >= 32 ? 32 / kMma : 8;                            // columns loaded at once
+#pragma unroll 1
+      for (int pass = 0; pass < MT; pass += kPassCols) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < kPart && alive; c0 += kLd) {        // alive: warp-uniform
+          const int col0 = pass + cpart * kPart + c0;
+          if (m0 + col0 >= g.M) break;
+          uint32_t v[kLd / 8][8];
+          const uint32_t taddr = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(acc * kMma * MT + col0);
+          auto load = [&](uint32_t (&d)[kLd / 8][8], uint32_t from) {
+#pragma unroll
+            for (int i = 0; i < kLd / 8; i++)
+              asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                           : "=r"(d[i][0]), "=r"(d[i][1]), "=r"(d[i][2]), "=r"(d[i][3]), "=r"(d[i][4]), "=r"(d[i][5]), "=r"(d[i][6]), "=r"(d[i][7])
+                           : "r"(from + 8 * i));
+          };
+          load(v, taddr);
+          if constexpr (kMma == 2) {
+            uint32_t v2[kLd / 8][8];
+            load(v2, taddr + MT);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < kLd; i++) v[i / 8][i % 8] = __float_as_uint(__uint_as_float(v[i / 8][i % 8]) + __uint_as_float(v2[i / 8][i % 8]));
+          } else {
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          }
+          if (staged) {
+            const uint32_t to = base + ((col0 - pass) * kTileN + row) * 4;
+#pragma unroll
+            for (int i = 0; i < kLd; i++) asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + i * kTileN * 4), "r"(v[i / 8][i % 8]) : "memory");
+          } else if (!whole) {
+            float* to = mine + col0 * kTileN + row;
+#pragma unroll
+            for (int i = 0; i < kLd; i++)
+              if (m0 + col0 + i < g.M) to[i * kTileN] = __uint_as_float(v[i / 8][i % 8]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < kLd / 8; q++) {
+              const int col = col0 + 8 * q;
+              if (vec && g.y_dtype != GGQ_F32) {
+                store_8x8(g.y, g.y_dtype, (int64_t)(m0 + col) * g.N + n0 + 32 * quarter, g.N, g.M - (m0 + col), g.N - (n0 + 32 * quarter), v[q], lane);
+              } else if (out_row < g.N) {
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                  if (m0 + col + i < g.M) store_out(g.y, g.y_dtype, (int64_t)(m0 + col + i) * g.N + out_row, __uint_as_float(v[q][i]));
+              }
+            }
+          }
+        }
+        if (staged && g.split == 1) {
+          // the four warps of these columns
+          asm volatile("bar.sync %0, 128;" ::"r"(2 + cpart) : "memory");
+#pragma unroll 4
+          for (int c = quarter; c < kPart; c += 4) {
+            const int col = pass + cpart * kPart + c;
+            if (m0 + col >= g.M) break;
+            const uint4 v = lds_v4(base + ((col - pass) * kTileN + 4 * lane) * 4);
+            put_column(g, m0 + col, n0 + 4 * lane, make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)), vec);
+          }
+          if (pass + kPassCols < MT) asm volatile("bar.sync %0, 128;" ::"r"(2 + cpart) : "memory");
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {                          // the accumulator is free
+        if (CG == 1 || rank == 0) mbar_arrive(acc_empty + 8 * acc);
+        else mbar_arrive_remote(acc_empty + 8 * acc, in_cluster & ~1u);
+      }
+      if (++acc == kAcc) { acc = 0; pacc ^= 1; }
+      if (!whole && g.split == 1) {
+        // Every decode thread takes part in both barriers, whatever happened above.  (One thread's fence behind the barrier covers the stores of all.)
+        const int c_first = (int)((((int64_t)t * SB + 1) * G - 1) / U), c_last = (int)((((int64_t)(t + 1) * SB) * G - 1) / U);
+        asm volatile("bar.sync 1, %0;" ::"n"(kDecoders) : "memory");
+        if (tid == 0) {
+          __threadfence();
+          int* counter = g.counters + (int64_t)t * CG + rank;
+          const int old = atomicAdd(counter, 1);
+          *last_flag = old == c_last - c_first;
+          if (old == c_last - c_first) *counter = 0;             // nobody else touches it until the next launch
+          __threadfence();
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kDecoders) : "memory");
+        if (*last_flag) {
+          // a lane takes four rows, a warp every sixteenth column; the ranges in K order (the first one's tile may be its second segment)
+          const int64_t slot_step = (int64_t)2 * CG * MT * kTileN;
+          const float* p_first = g.partials + ((int64_t)(2 * c_first + (U * c_first / G < (int64_t)t * SB ? 1 : 0)) * CG + rank) * MT * kTileN + 4 * lane;
+          const float* p_next = g.partials + ((int64_t)(2 * c_first) * CG + rank) * MT * kTileN + 4 * lane;
+#pragma unroll 2
+          for (int col = warp; col < MT && m0 + col < g.M; col += kDecodeWarps) {
+            float4 sum = __ldcg(reinterpret_cast<const float4*>(p_first + col * kTileN));
+#pragma unroll 4
+            for (int c = 1; c <= c_last - c_first; c++) {
+              const float4 v = __ldcg(reinterpret_cast<const float4*>(p_next + c * slot_step + col * kTileN));
+              sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+            }
+            put_column(g, m0 + col, n0 + 4 * lane, sum, vec);
+          }
+        }
+      }
+    }
+  }
+  if (g.split > 1) {
+    // The ranges' tiles are in shared memory (whose rings are done with: no CTA has another tile); every CTA adds a share of the columns, in K order.
+    __syncwarp();
+    cluster_sync();
+    if (warp < kDecodeWarps) {
+      const int t = me / g.split, part = me % g.split, n0 = (t % g.tiles_n) * (kTileN * CG) + (int)rank * kTileN, m0 = (t / g.tiles_n) * MT;
+      const bool vec = g.N % 8 == 0 && (uintptr_t)g.y % 16 == 0;
+      const int cols = min(MT, g.M - m0), c0 = cols * part / g.split, c1 = cols * (part + 1) / g.split;
+      for (int col = c0 + warp; col < c1; col += kDecodeWarps) {
+        const uint32_t at = base + (col * kTileN + 4 * lane) * 4;
+        float4 sum = ld_cluster(at, rank);
+#pragma unroll 4
+        for (int c = 1; c < g.split; c++) {
+          const float4 v = ld_cluster(at, c * CG + rank);
+          sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        put_column(g, m0 + col, n0 + 4 * lane, sum, vec);
+      }
+    }
+  }
+  // common exit: everybody is done with TMEM, and with the shared memory of the other CTAs of a cluster, before it is released
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (CG == 2 || g.split > 1) cluster_sync();
+  if (warp == kMmaWarp) {
+    if constexpr (CG == 1)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)C::kTmemCols) : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)C::kTmemCols) : "memory");
+  }
+}
+
+// Two-dimensional tensor maps: x as bf16 [M rows, K columns] with boxes of 64 columns, 128-byte swizzle; the weight as 32-bit words, boxes of
+// 128 rows; zeros outside.
+static bool make_map(CUtensorMap* map, CUtensorMapDataType type, const void* p, int64_t cols, int64_t rows, int64_t pitch, int box_cols, int box_rows,
+                     CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promotion) {
+  EncodeTiledFn fn = tensor_map_encoder();
+  if (!fn || (uintptr_t)p % 16 || pitch % 16) return false;
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)pitch};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  const cuuint32_t elem[2] = {1, 1};
+  return fn(map, type, 2, const_cast<void*>(p), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promotion,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+struct Plan { int mt, cg, split, groups; int64_t tiles_n, tiles; };      // groups: CTAs or pairs of them
+
+template <class F, int MT, int CG>
+static cudaError_t launch_one(const uint8_t* w, int64_t N, int64_t K, const void* x, int M, void* y, int y_dtype, int* status,
+                              const Plan& p, float* partials, int* counters, const uint8_t* tab, cudaStream_t st) {
+  using C = Cfg<F, MT, CG>;
+  static_assert(C::kSmem <= kSmemLimit, "shared memory");
+  static std::atomic<bool> attr_done[64];   // setting the attribute twice is harmless, so a flag per device suffices
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_done[dev].load(std::memory_order_acquire)) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16w_kernel<F, MT, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
+    if (e != cudaSuccess) return e;
+    attr_done[dev].store(true, std::memory_order_release);
+  }
+  // (a cluster's partial tiles lie where the rings were)
+  if (!partials && p.split == 1 && p.groups != p.tiles) return cudaErrorInvalidValue;
+  if (p.split > 1 && (MT * kTileN * 4 > C::kSmem - 2048 || p.groups != p.tiles * p.split || p.split * 256 > K)) return cudaErrorInvalidValue;
+  alignas(64) CUtensorMap w_map, x_map;
+  const int64_t row_bytes = K / 256 * F::kTs;
+  constexpr int kMmaN = MT > 256 ? 256 : MT;
+  memset(&w_map, 0, sizeof(w_map));
+  if ((!(F::kDirect && row_bytes % 16) && !make_map(&w_map, CU_TENSOR_MAP_DATA_TYPE_UINT32, w, row_bytes / 4, N, row_bytes, F::kBoxWords, kTileN, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B)) ||
+      !make_map(&x_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, x, K, M, K * 2, kStageK, kMmaN / CG, CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B))
+    return cudaErrorInvalidValue;
+  Args a{(int)N, (int)K, M, y_dtype, (int)p.tiles_n, (int)p.tiles, p.split, y, status, partials, counters, tab, w, row_bytes};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(p.groups * CG));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = C::kSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CG * p.split;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CG * p.split > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, gemm_bf16w_kernel<F, MT, CG>, w_map, x_map, a);
+}
+
+// the instances for the formats without kernels of their own, by class (gemm_bf16w_b32.cu, gemm_bf16w_iq.cu)
+struct Call {
+  const uint8_t* w;
+  int64_t N, K;
+  const void* x;
+  int M;
+  void* y;
+  int y_dtype;
+  int* status;
+  Plan plan;
+  float* partials;
+  int* counters;
+  const uint8_t* tab;
+  cudaStream_t st;
+};
+cudaError_t launch_b32(int qtype, const Call& c);
+cudaError_t launch_iq(int qtype, const Call& c);
+
+}  // namespace gemmb
+}  // namespace ggq

@@ -275,13 +275,13 @@ extern "C" int32_t ggq_gemv(int32_t qtype, const void* w, int64_t N, int64_t K, 
 
 // The materializing route's product without the dense copy (include/ggq.h).
 extern "C" int32_t ggq_rounded_gemm_pays(int32_t qtype, int64_t N, int64_t K, int32_t M) {
-  if (!type_info(qtype) || N <= 0 || K <= 0 || M <= 0 || !gemm_bf16w_applicable(qtype, N, K, M) || !gemm_bf16w_available()) return 0;
+  if (!type_info(qtype) || N <= 0 || K <= 0 || M <= 0 || !gemm_bf16w_alone_applicable(qtype, N, K, M) || !gemm_bf16w_available()) return 0;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) { dev = -1; (void)cudaGetLastError(); }
   return gemm_bf16w_beats_dense(qtype, N, K, M, sm_count_of(dev)) ? 1 : 0;
 }
 extern "C" size_t ggq_rounded_gemm_temp(int32_t qtype, int64_t N, int64_t K, int32_t M) {
-  if (!type_info(qtype) || N <= 0 || K <= 0 || M <= 0 || !gemm_bf16w_applicable(qtype, N, K, M)) return 0;
+  if (!type_info(qtype) || N <= 0 || K <= 0 || M <= 0 || !gemm_bf16w_alone_applicable(qtype, N, K, M)) return 0;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) { dev = -1; (void)cudaGetLastError(); }
   return gemm_bf16w_temp_bytes(qtype, N, K, M, sm_count_of(dev));
@@ -292,8 +292,8 @@ extern "C" int32_t ggq_rounded_gemm(int32_t qtype, const void* w, int64_t N, int
   if (!ti) return fail(GGQ_BAD_QTYPE, "ggq_rounded_gemm: qtype %d is not decodable", qtype);
   if (N <= 0 || K <= 0 || K % ti->block_elems || M < 1)
     return fail(GGQ_BAD_SHAPE, "ggq_rounded_gemm: N=%lld K=%lld M=%d (K must be a positive multiple of %d)", (long long)N, (long long)K, M, ti->block_elems);
-  if (!gemm_bf16w_applicable(qtype, N, K, M) || !gemm_bf16w_available())
-    return fail(GGQ_UNSUPPORTED, "ggq_rounded_gemm: qtype %d, N=%lld K=%lld M=%d (Q4_K / Q5_K / Q6_K, K %% 256 == 0, rows of a multiple of 16 bytes)", qtype,
+  if (!gemm_bf16w_alone_applicable(qtype, N, K, M) || !gemm_bf16w_available())
+    return fail(GGQ_UNSUPPORTED, "ggq_rounded_gemm: qtype %d, N=%lld K=%lld M=%d (block formats, K %% 256 == 0)", qtype,
                 (long long)N, (long long)K, M);
   if (y_dtype != GGQ_F32 && y_dtype != GGQ_BF16 && y_dtype != GGQ_F16) return fail(GGQ_BAD_DTYPE, "ggq_rounded_gemm: y_dtype %d", y_dtype);
   if (!w || !x_bf16 || !y) return fail(GGQ_MISALIGNED, "ggq_rounded_gemm: null pointer");
@@ -301,9 +301,11 @@ extern "C" int32_t ggq_rounded_gemm(int32_t qtype, const void* w, int64_t N, int
     return fail(GGQ_MISALIGNED, "ggq_rounded_gemm: w and x must be 16-byte aligned, temp 256-byte");
   int dev = 0;
   cudaGetDevice(&dev);
+  const uint8_t* tab = device_tables(dev);
+  if (ti->needs_tables && !tab) return fail(GGQ_NO_TABLES, "ggq_rounded_gemm: call ggq_set_tables(%d, ...) before using qtype %d", dev, qtype);
   const int sms = sm_count_of(dev);
   const cudaError_t err = gemm_bf16w_alone(qtype, (const uint8_t*)w, N, K, x_bf16, M, y, y_dtype, device_status_word_if_any(dev), temp,
-                                           temp_bytes, sms, (cudaStream_t)stream);
+                                           temp_bytes, tab, sms, (cudaStream_t)stream);
   if (err != cudaSuccess) return fail(GGQ_LAUNCH_FAILED, "ggq_rounded_gemm: %s", cudaGetErrorString(err));
   return GGQ_OK;
 }

@@ -117,9 +117,9 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (m > s.limit && !force) {
     const double budget = PyFloat_AsDouble(args[5]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
-    // (autocast converts the copy: its product, and what then still fits, are not these; slabs are the Python path's)
+    // (autocast converts the copy: its product, and what then still fits, are not these)
     const bool autocast = at::autocast::is_autocast_enabled(at::kCUDA);
-    if ((autocast ? 8.0 : 4.0) * (double)n * (double)k > budget) Py_RETURN_NONE;
+    if (n % 8 || (autocast ? 8.0 : 4.0) * (double)n * (double)k > budget) Py_RETURN_NONE;          // rows of the result off 16 bytes, slabs: the Python path's
     at::Tensor y;
     if (s.rounded && !autocast && (uintptr_t)w.data_ptr() % 16 == 0 && (!x.is_contiguous() || (uintptr_t)x.data_ptr() % 16 == 0)) {
       // the weights that the copy would hold, decoded inside the multiply
@@ -132,7 +132,6 @@ PyObject* fast_matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         y = at::Tensor();
     } else {
       // the dense route in one piece: decode to bf16, library GEMM (rows of the result on 16-byte boundaries)
-      if (n % 8) Py_RETURN_NONE;
       WithoutGil no_gil;
       const at::Tensor dense = at::empty({n, k}, x.options().requires_grad(false));
       if (g_dequant((int32_t)qtype, w.data_ptr(), s.blocks, dense.data_ptr(), kBf16, stream.stream()) == 0)

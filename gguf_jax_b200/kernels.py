@@ -30,7 +30,6 @@ LOWBIT_TYPES = (QT.Q2_K, QT.IQ1_S, QT.IQ1_M, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT
 
 _ws_need: dict[tuple[int, int, int, int], tuple[int, int]] = {}      # scratch: for every kernel, for those that need one
 _rounded: dict[tuple[int, int, int, int], int] = {}       # what rounded_temp has said
-_ROUNDED_TYPES = (QT.Q4_K, QT.Q5_K, QT.Q6_K)
 _cap: list[int] = []
 
 
@@ -134,7 +133,7 @@ def fused_matmul(x: torch.Tensor, w: QuantizedArray, *, out_dtype=torch.bfloat16
 
 def rounded_temp(w: QuantizedArray, m: int) -> int:
     """Bytes of memory of its own that :func:`rounded_matmul` takes for ``m`` rows; -1 where a decoded copy and a library GEMM are faster."""
-    if w.qtype not in _ROUNDED_TYPES or len(w.shape) != 2:
+    if len(w.shape) != 2:
         return -1
     key = (int(w.qtype), *w.shape, m)
     temp_bytes = _rounded.get(key)
@@ -157,6 +156,7 @@ def rounded_matmul(x: torch.Tensor, w: QuantizedArray) -> torch.Tensor | None:
     if xm.data_ptr() % 16 or data.data_ptr() % 16:
         return None
     dev = _backend.require_cuda(data, f"matmul ({w.qtype.name})")
+    _lib.ensure_tables(dev)
     with torch.cuda.device(dev):
         y = torch.empty((m, n_rows), dtype=torch.bfloat16, device=data.device)
         temp = torch.empty(temp_bytes, dtype=torch.uint8, device=data.device) if temp_bytes else None

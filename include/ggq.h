@@ -149,7 +149,7 @@ int32_t ggq_gemm(int32_t qtype, const void* w, int64_t N, int64_t K, const void*
 
 /* The product of the materializing route (src/gguf_jax/_matmul.py:141-186: decode W to bf16, then a dense GEMM) without the dense
  * copy: W is decoded inside the kernel, to the values ggq_dequant gives rounded once to bf16, and multiplied on the tensor cores with
- * float32 accumulation.  Q4_K / Q5_K / Q6_K, K % 256 == 0, rows of a multiple of 16 bytes, w and x 16-byte aligned; GGQ_UNSUPPORTED
+ * float32 accumulation.  Block formats, K % 256 == 0, w and x 16-byte aligned; GGQ_UNSUPPORTED
  * otherwise.  Nothing is kept between calls: calls and captured graphs may overlap on the device like those of a library GEMM.  `temp` is memory of the
  * call's own (256-byte aligned, any contents) of ggq_rounded_gemm_temp bytes; with less, or none, a plan that needs none runs.  The launch
  * is a programmatic dependent, see ggq_gemv.

@@ -23,7 +23,8 @@ def inside(call):
 @pytest.mark.parametrize("qtype,n,k,m", [(QT.Q5_K, 4096, 4096, 32), (QT.Q4_K, 1003, 4096, 17), (QT.Q6_K, 1024, 4096, 24), (QT.Q4_K, 4096, 4096, 128),
                                          (QT.Q6_K, 8192, 8192, 300), (QT.Q4_K, 4096, 14336, 512), (QT.Q5_K, 14336, 4096, 1000),
                                          # tiles cut between ranges, which meet in memory of the call's own
-                                         (QT.Q4_K, 4096, 14336, 768), (QT.Q6_K, 7000, 8192, 768)], ids=str)
+                                         (QT.Q4_K, 4096, 14336, 768), (QT.Q6_K, 7000, 8192, 768),
+                                         (QT.Q8_0, 14336, 4096, 17), (QT.Q5_1, 8192, 8192, 512), (QT.IQ2_XS, 14336, 4096, 100)], ids=str)
 def test_product_of_the_decoded_copy(qtype, n, k, m):
     w = weight(qtype, n, k)
     x = torch.randn((2, m // 2, k) if m % 2 == 0 else (m, k), device="cuda").bfloat16()
@@ -44,6 +45,38 @@ def test_product_of_the_decoded_copy(qtype, n, k, m):
     (dx,) = torch.autograd.grad(yg, xg, g)
     want = g.double() @ w.dequantize().double()
     assert ((dx.double() - want).norm() / want.norm()).item() <= 2 ** -8
+
+
+GENERIC = [QT.Q4_0, QT.Q4_1, QT.Q5_0, QT.Q5_1, QT.Q8_0, QT.IQ4_NL, QT.MXFP4, QT.NVFP4, QT.Q2_K, QT.Q3_K, QT.IQ4_XS, QT.IQ2_XXS, QT.IQ2_XS, QT.IQ2_S, QT.IQ3_XXS, QT.IQ3_S,
+           QT.IQ1_S, QT.IQ1_M, QT.TQ1_0, QT.TQ2_0]
+
+
+@pytest.mark.parametrize("n,k,m", [(33, 4096, 17), (130, 2048, 70), (4700, 2048, 33), (9500, 2048, 33), (4700, 4096, 100), (33, 4096, 257), (6200, 2048, 130),
+                                   (9500, 2048, 200), (1100, 4096, 300), (9500, 2048, 513), (7000, 6144, 300),
+                                   # rows off 16 bytes in the formats whose superblocks are no multiple of it
+                                   (33, 256, 17), (130, 1280, 70), (4700, 1792, 33), (1101, 3328, 300), (9503, 2304, 130), (7001, 2816, 520)], ids=str)
+@pytest.mark.parametrize("qtype", GENERIC + [QT.Q6_K], ids=lambda t: t.name)
+def test_every_format(qtype, n, k, m):
+    """Every block format through the kernel itself, pays or not, with and without memory of the call's own (tiles, pairs, clusters, cut tiles); bit for bit
+    what the decode kernel's weights give, however they are read (byte offsets modulo 16 differ from superblock to superblock)."""
+    L, dev = _lib.lib(), torch.cuda.current_device()
+    _lib.ensure_tables(dev)
+    w = weight(qtype, n, k)
+    x = torch.randn((m, k), device="cuda").bfloat16()
+    want = x.double() @ w.dequantize().double().T
+    for nbytes in {0, L.ggq_rounded_gemm_temp(int(qtype), n, k, m)}:
+        temp = torch.full((max(nbytes, 1),), 255, dtype=torch.uint8, device="cuda")
+        y = torch.full((m, n), float("nan"), device="cuda")
+        for _ in range(2):
+            _lib.check(L.ggq_rounded_gemm(int(qtype), w.data.data_ptr(), n, k, x.data_ptr(), m, y.data_ptr(), _lib.GGQ_F32, temp.data_ptr(), nbytes,
+                                          torch.cuda.current_stream().cuda_stream))
+        assert ((y.double() - want).norm() / want.norm()).item() <= 1e-5
+    onehot = torch.zeros((m, k), device="cuda").bfloat16()
+    cols = torch.randint(0, k, (m,), device="cuda")
+    onehot[torch.arange(m, device="cuda"), cols] = 1
+    _lib.check(L.ggq_rounded_gemm(int(qtype), w.data.data_ptr(), n, k, onehot.data_ptr(), m, y.data_ptr(), _lib.GGQ_F32, None, 0,
+                                  torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y, w.dequantize()[:, cols].T.float())
 
 
 def test_calls_that_keep_the_copy():
