@@ -184,7 +184,7 @@ template <int DEPTH, bool TMA>
 __global__ void __launch_bounds__(kThreads, 1)
 gemv_q6k_m1_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x,
                    void* __restrict__ y, int y_dtype, int* __restrict__ counters, float* __restrict__ partials,
-                   const PeerPublish pp, int* __restrict__ status, const __grid_constant__ CUtensorMap w_map) {
+                   const PeerPublish pp, int* __restrict__ status, const int whole_groups, const __grid_constant__ CUtensorMap w_map) {
   extern __shared__ __align__(128) uint8_t smem[];
   pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -194,7 +194,8 @@ gemv_q6k_m1_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloa
   const int RG = (N + kRowsPerUnit - 1) / kRowsPerUnit;
   const int64_t U = (int64_t)RG * C;
   const int G = gridDim.x, b = blockIdx.x;
-  const int64_t u_begin = U * b / G, u_end = U * (b + 1) / G;
+  const int64_t u_begin = whole_groups ? (int64_t)RG * b / G * C : U * b / G;
+  const int64_t u_end = whole_groups ? (int64_t)RG * (b + 1) / G * C : U * (b + 1) / G;
   const int n_units = (int)(u_end - u_begin);
   const int rg_begin = (int)(u_begin / C), c_begin = (int)(u_begin - (int64_t)rg_begin * C);
 
@@ -487,7 +488,12 @@ cudaError_t gemv_q6k(const uint8_t* w, int64_t N, int64_t K, const void* x, void
   if (ws_bytes < gemv_q4k_workspace_bytes(N, sm_count) || !ws || sm_count > kMaxSmCount) return cudaErrorInvalidValue;
   const int64_t RG = (N + kRowsPerUnit - 1) / kRowsPerUnit;
   const int64_t U = RG * (K / 256 / kSbPerUnit);
-  const int grid = (int)(U < sm_count ? U : sm_count);
+  // Row groups are not cut between CTAs where that lengthens the longest CTA by a chunk at most: a cut costs a fence, an atomic and a read-back
+  // at the end of the launch, 2 to 4 us, a chunk 1 to 2.  us cut / whole: 4096 x 4096 9.1 / 6.6, 8192 x 8192 17.1 / 16.5, 4096 x 14336 16.7 / 14.9, 12288 x
+  // 6144 19.0 / 17.9; two or three chunks longer 2048 x 8192 8.4 / 9.1, 5120 x 8192 13.5 / 15.7.
+  const int64_t C = U / RG, most = (U + sm_count - 1) / sm_count;
+  const bool whole = C > 1 && (RG + sm_count - 1) / sm_count * C <= most + 1;
+  const int grid = (int)(whole ? (RG < sm_count ? RG : sm_count) : U < sm_count ? U : sm_count);
   int depth = 4;
   while (depth > 2 && Smem(depth).total((int)K) > kSmemLimit) depth--;
   const int smem = Smem(depth).total((int)K);
@@ -514,7 +520,7 @@ cudaError_t gemv_q6k(const uint8_t* w, int64_t N, int64_t K, const void* x, void
   static const bool want_tma = [] { const char* e = getenv("GGQ_Q6K_TMA"); return !(e && e[0] == '0'); }();
   const bool tma = want_tma && make_weight_map(&w_map, w, N, K / 256 * kBlockBytes, kSlotPitch / 4);
   cudaError_t err;
-#define GGQ_Q6K_LAUNCH(D, T) launch_pdl(gemv_q6k_m1_kernel<D, T>, grid, kThreads, smem, st, w, (int)N, (int)K, xb, y, y_dtype, counters, partials, pp, status, w_map)
+#define GGQ_Q6K_LAUNCH(D, T) launch_pdl(gemv_q6k_m1_kernel<D, T>, grid, kThreads, smem, st, w, (int)N, (int)K, xb, y, y_dtype, counters, partials, pp, status, whole, w_map)
   if (tma) err = depth == 4 ? GGQ_Q6K_LAUNCH(4, true) : depth == 3 ? GGQ_Q6K_LAUNCH(3, true) : GGQ_Q6K_LAUNCH(2, true);
   else err = depth == 4 ? GGQ_Q6K_LAUNCH(4, false) : depth == 3 ? GGQ_Q6K_LAUNCH(3, false) : GGQ_Q6K_LAUNCH(2, false);
 #undef GGQ_Q6K_LAUNCH
