@@ -18,8 +18,10 @@
 // work) takes row blocks of 128 rows -- warp w the rows 16 w .. 16 w + 15 -- and walks along K one superblock
 // per step; all steps of the launch (row block major) are dealt to the CTAs as equal contiguous ranges.  A row block cut by a range boundary is finished by the last
 // CTA to arrive: each contributor leaves its 128 x M partial sums in one of its two scratch slots,
-// bumps the row block's counter, and the last one adds the slots in CTA order (deterministic).
-// The activations of a step are the same for all warps: a separate launch (prepare kernel) writes
+// bumps the row block's counter, and the last one adds the slots in CTA order (deterministic).  The slots are read four at a time and without
+// the 64-bit divisions that stood between the reads: with 16 contributors (1024 x 4096) that was a third of the launch.  us before / now with
+// both: Q4_K 14336 x 4096 at 17 rows 32.8 / 30.4, Q6_K 14336 x 4096 at 32 37.8 / 36.4, 4096 x 14336 at 32 44.6 / 43.0, 8192 x 28672 at 12 85.5 / 80.3.
+// The activations of a step are the same for all warps: where CTAs have more than kOwnSteps steps a separate launch (prepare kernel) writes
 // them once, already in B-fragment order, and the CTAs copy one superblock's worth per step into a
 // ring in shared memory next to each warp's private ring of raw weight bytes (one TMA box of 16 rows per warp and step on a
 // per-warp mbarrier; per-lane 16-byte cp.async where no tensor-map encoder is to be had).
@@ -128,7 +130,9 @@ struct FQ6K {
 // Launch geometry (host-computed).
 struct Geo {
   int SB, RB;                 // superblocks per row, row blocks
-  int64_t S;                  // steps = RB * SB
+  int64_t S;                  // steps = RB * SB: at most 2^40 / (16 * 144 * 8), by gemv_wide_applicable
+  int per_cta, rest;          // S / grid, S % grid
+  float cta_per_step;         // grid / S
   int depth;                  // ring depth (steps)
   int wslot_bytes;            // 16 * pitch
   int xstage_bytes;           // XR * (512 + kOffBytes)
@@ -137,6 +141,31 @@ struct Geo {
   int row_skew;               // bytes by which consecutive rows differ modulo 16 (0: rows 16-byte aligned; else cp.async copies)
   int vec_store;              // 2-byte outputs whose 8-row runs are 16-byte aligned: stored as 16-byte vectors
 };
+
+// The offset operand of group q: its sum (times 2^S) as three bf16 terms, among the column's kOffBytes at `ob`.
+template <class F>
+__device__ __forceinline__ void put_offset(uint8_t* ob, int q, float scaled_sum) {
+  uint32_t hi, mid, lo;
+  split3(scaled_sum, hi, mid, lo);
+  if (F::kGroups == 8) {
+    // offset MMAs 1 and 2, lane group t' = q / 2: slots (hi, mid) of groups 2t', 2t'+1, then (lo, 0) of both
+    uint32_t* piece = reinterpret_cast<uint32_t*>(ob + (q >> 1) * 16);
+    piece[q & 1] = hi | (mid << 16);
+    piece[2 + (q & 1)] = lo;
+  } else {
+    // sixteen groups: lane group t' = q / 4 holds groups 4t' .. 4t'+3; three MMAs (hi, mid, lo), 8 bytes each:
+    // k-slots (2t', 2t'+1) = groups 4t', 4t'+1 and (2t'+8, 2t'+9) = groups 4t'+2, 4t'+3
+    uint16_t* piece = reinterpret_cast<uint16_t*>(ob + (q >> 2) * 32);
+    piece[0 + (q & 3)] = (uint16_t)hi;
+    piece[4 + (q & 3)] = (uint16_t)mid;
+    piece[8 + (q & 3)] = (uint16_t)lo;
+  }
+}
+// A column's power of two from the biased exponent of its largest octet sum of |x|: 2^96 suits any in about [2^-30, 2^30);
+// otherwise put the largest near 2^120.
+__device__ __forceinline__ int scale_exp_of(int emax) {
+  return (emax > 156 || (emax < 97 && emax > 0)) ? max(8, min(120, 247 - emax)) : 96;
+}
 
 // ---------------------------------------------------------------------------------------------
 // Prepare kernel: `parts` CTAs per staged batch column (columns >= M are zero-filled).  The multiply kernel waits for it, so
@@ -176,9 +205,7 @@ prepare_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int K, int M, u
   const uint32_t wmax = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(amax));      // non-negative floats order like integers
   if ((tid & 31) == 0) atomicMax(&s_max, (int)wmax);
   __syncthreads();
-  // 2^96 suits any octet sum of |x| in about [2^-30, 2^30); otherwise put the largest near 2^120
-  const int emax = min((s_max >> 23) & 0xFF, 254);
-  const int S = (emax > 156 || (emax < 97 && emax > 0)) ? max(8, min(120, 247 - emax)) : 96;
+  const int S = scale_exp_of(min((s_max >> 23) & 0xFF, 254));
   if (tid == 0 && part == 0) S_col[col] = S;
   constexpr int kE = F::kPiece / 2;                       // elements per piece: 8 or 4
   constexpr int kPiecesPerSum = F::kSumLen / kE;          // pieces (consecutive t) that make one scale group: 4
@@ -212,22 +239,64 @@ prepare_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int K, int M, u
     sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
     sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
     if (in && t == 0) {
-      uint32_t hi, mid, lo;
-      split3(sum * pow2f(S), hi, mid, lo);
-      uint8_t* ob = xo + ((int64_t)sb * XR + col) * F::kOffBytes;
-      if (F::kGroups == 8) {
-        // offset MMAs 1 and 2, lane group t' = q / 2: slots (hi, mid) of groups 2t', 2t'+1, then (lo, 0) of both
-        uint32_t* piece = reinterpret_cast<uint32_t*>(ob + (q >> 1) * 16);
-        piece[q & 1] = hi | (mid << 16);
-        piece[2 + (q & 1)] = lo;
-      } else {
-        // sixteen groups: lane group t' = q / 4 holds groups 4t' .. 4t'+3; three MMAs (hi, mid, lo), 8 bytes each:
-        // k-slots (2t', 2t'+1) = groups 4t', 4t'+1 and (2t'+8, 2t'+9) = groups 4t'+2, 4t'+3
-        uint16_t* piece = reinterpret_cast<uint16_t*>(ob + (q >> 2) * 32);
-        piece[0 + (q & 3)] = (uint16_t)hi;
-        piece[4 + (q & 3)] = (uint16_t)mid;
-        piece[8 + (q & 3)] = (uint16_t)lo;
-      }
+      put_offset<F>(xo + ((int64_t)sb * XR + col) * F::kOffBytes, q, sum * pow2f(S));
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same staging by the multiply kernel itself, for launches whose CTAs have kOwnSteps steps at most: the CTA's superblocks of x
+// go straight into the slots of its activation ring, scaled by the power of two that suits these superblocks (partial sums are
+// unscaled before CTAs add theirs up).  One warp per column; lane l has the weights 8 l .. 8 l + 7 of a superblock.
+// A launch less and its wait, 2 to 3 us (one launch / two, Q6_K 4096 x 4096 at 24 rows 23.5 / 26.0, Q4_K 2048 x 2048 at 32 11.7 / 14.5, before the
+// faster settle), for a sixth more instructions per step; two steps are also all that the rings of 32 columns have slots for.
+constexpr int kOwnSteps = 2;
+template <class F, int NT>
+__device__ __forceinline__ void stage_own(const __nv_bfloat16* __restrict__ x, int64_t ldx, int M, int SB, int k0, int n_steps, uint8_t* stages,
+                                          int stage_bytes, int* s_S, int warp, int lane) {
+  constexpr int XR = 8 * NT;
+  uint4 u[NT][kOwnSteps];
+#pragma unroll
+  for (int r = 0; r < NT; r++) {
+    const int col = r * 8 + warp;
+    int k = k0;
+#pragma unroll
+    for (int j = 0; j < kOwnSteps; j++) {
+      u[r][j] = make_uint4(0, 0, 0, 0);
+      if (col < M && j < n_steps) u[r][j] = __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)col * ldx + (int64_t)k * 256) + lane);
+      if (++k == SB) k = 0;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NT; r++) {
+    const int col = r * 8 + warp;
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < kOwnSteps; j++) {
+      const uint4 v = u[r][j];
+      const float s = (fabsf(bf16lo(v.x)) + fabsf(bf16hi(v.x))) + (fabsf(bf16lo(v.y)) + fabsf(bf16hi(v.y))) +
+                      (fabsf(bf16lo(v.z)) + fabsf(bf16hi(v.z))) + (fabsf(bf16lo(v.w)) + fabsf(bf16hi(v.w)));
+      amax = fmaxf(amax, s);
+    }
+    const int emax = min(((int)__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(amax)) >> 23) & 0xFF, 254);
+    const int S = scale_exp_of(emax);
+    if (lane == 0) s_S[col] = S;
+    const int q = F::kGroups == 8 ? lane >> 2 : lane >> 1;
+    const float up = pow2f(S + F::x_exp(q)), sum_up = pow2f(S);
+#pragma unroll
+    for (int j = 0; j < kOwnSteps; j++) {
+      if (j >= n_steps) break;
+      const uint4 w = u[r][j];
+      const float v[8] = {bf16lo(w.x), bf16hi(w.x), bf16lo(w.y), bf16hi(w.y), bf16lo(w.z), bf16hi(w.z), bf16lo(w.w), bf16hi(w.w)};
+      uint8_t* stage = stages + j * stage_bytes;
+      // a lane's 16 bytes: one piece of eight elements or two of four
+      uint8_t* dst = stage + (q * XR + col) * (4 * F::kPiece) + (F::kGroups == 8 ? lane & 3 : lane & 1) * 16;
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(v[0] * up, v[2] * up), pack_bf16(v[1] * up, v[3] * up),
+                                                  pack_bf16(v[4] * up, v[6] * up), pack_bf16(v[5] * up, v[7] * up));
+      float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+      if (F::kGroups == 8) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+      if ((lane & (F::kGroups == 8 ? 3 : 1)) == 0) put_offset<F>(stage + XR * 512 + col * F::kOffBytes, q, sum * sum_up);
     }
   }
 }
@@ -454,22 +523,25 @@ __device__ __forceinline__ void block_mul(uint32_t blk0, uint32_t blk1, int g, i
   }
 }
 
-// the CTA whose range holds step s (ranges are [S b / G, S (b + 1) / G))
-__device__ __forceinline__ int cta_of_step(int64_t s, int64_t S, int G) {
-  int b = (int)((s * G) / S);
-  while (b + 1 < G && S * (b + 1) / G <= s) ++b;
-  while (b > 0 && S * b / G > s) --b;
+// CTA b of G takes the steps [S b / G, S (b + 1) / G).  The bounds, and the CTA that holds step s, without a 64-bit division (a hundred
+// instructions; a settle that made two per contributor spent half its time on them).
+__device__ __forceinline__ int range_start(const Geo& geo, int b, int G) { return geo.per_cta * b + (int)((uint32_t)(geo.rest * b) / (uint32_t)G); }
+__device__ __forceinline__ int cta_of_step(const Geo& geo, int s, int G) {
+  int b = min((int)((float)s * geo.cta_per_step), G - 1);
+  while (b + 1 < G && range_start(geo, b + 1, G) <= s) ++b;
+  while (b > 0 && range_start(geo, b, G) > s) --b;
   return b;
 }
 
-template <class F, int NT>
+// kOwn: no prepare kernel has run; a CTA's steps (kOwnSteps and `depth` at most) all have a slot of the rings, and it stages their activations
+template <class F, int NT, bool kOwn>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
-gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __restrict__ xp, const uint8_t* __restrict__ xo,
-                 const int* __restrict__ S_col, int M, void* __restrict__ y, int y_dtype, int* __restrict__ counters,
+gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const __nv_bfloat16* __restrict__ x, int64_t ldx, const uint8_t* __restrict__ xp,
+                 const uint8_t* __restrict__ xo, const int* __restrict__ S_col, int M, void* __restrict__ y, int y_dtype, int* __restrict__ counters,
                  float* __restrict__ slots, const Geo geo, const PeerPublish pp, int* __restrict__ status,
                  const __grid_constant__ CUtensorMap w_map) {
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ int s_last;
+  __shared__ int s_last, s_S[8 * NT];
   __shared__ __align__(8) uint64_t w_bars[kWarps][4];     // one mbarrier per warp and ring slot (depth <= 4)
   constexpr int XR = 8 * NT;
   constexpr int kStageX = XR * 512, kStageO = XR * F::kOffBytes;
@@ -479,9 +551,9 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
   const int SB = geo.SB, depth = geo.depth;
   const int64_t row_bytes = (int64_t)SB * F::kTs;
   const int b = blockIdx.x, G = gridDim.x;
-  const int64_t s_begin = geo.S * b / G, s_end = geo.S * (b + 1) / G;
-  const int n_steps = (int)(s_end - s_begin);
-  const int rb_first = (int)(s_begin / SB);
+  const int s_begin = range_start(geo, b, G);
+  const int n_steps = range_start(geo, b + 1, G) - s_begin;
+  const int rb_first = s_begin / SB;
 
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t my_ring = smem_base + warp * (depth * geo.wslot_bytes);
@@ -492,7 +564,7 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
   if (tma) tma_bars_init(my_bars, depth, lane);
   // weights and activations are issued by separate cursors: the first weight copies go out before this kernel
   // waits for its predecessor (the weights are immutable), the activations only after it
-  int w_issued = 0, w_slot = 0, w_rb = rb_first, w_k = (int)(s_begin - (int64_t)rb_first * SB);
+  int w_issued = 0, w_slot = 0, w_rb = rb_first, w_k = s_begin - rb_first * SB;
   auto issue_w = [&]() {
     if (w_issued < n_steps) {
       // this warp's 16 rows of superblock w_k: a half-warp copies one row (the 16-byte aligned window around the block)
@@ -547,10 +619,17 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
       if (++x_k == SB) x_k = 0;
     }
   };
-  for (int d = 0; d < depth - 1; d++) issue_w();
+  for (int d = 0; d < (kOwn ? kOwnSteps : depth - 1); d++) issue_w();
   pdl_wait();            // the prepare kernel's output (and the previous launch's use of the scratch) is behind us
   pdl_trigger();
-  for (int d = 0; d < depth - 1; d++) { issue_x(); cp_async_commit(); }
+  if constexpr (kOwn) {
+    stage_own<F, NT>(x, ldx, M, SB, x_k, n_steps, smem + geo.off_x, geo.xstage_bytes, s_S, warp, lane);
+    cp_async_commit();
+    cp_async_wait_pending(0);
+    __syncthreads();
+  } else {
+    for (int d = 0; d < depth - 1; d++) { issue_x(); cp_async_commit(); }
+  }
   auto issue_next = [&]() { issue_w(); issue_x(); cp_async_commit(); };
 
   float out[NT][4];
@@ -561,8 +640,9 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
   float unscale[NT][2];
 #pragma unroll
   for (int nt = 0; nt < NT; nt++) {
-    unscale[nt][0] = pow2f(133 - S_col[nt * 8 + 2 * t]);
-    unscale[nt][1] = pow2f(133 - S_col[nt * 8 + 2 * t + 1]);
+    const int* S_of = kOwn ? s_S : S_col;
+    unscale[nt][0] = pow2f(133 - S_of[nt * 8 + 2 * t]);
+    unscale[nt][1] = pow2f(133 - S_of[nt * 8 + 2 * t + 1]);
   }
   auto store_rows = [&](int rb, const float (&v)[NT][4]) {
     const int row_base = rb * kBlockRows + warp * 16;
@@ -574,8 +654,7 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
       const int c = (lane >> 1) & 7, h = lane & 1;
 #pragma unroll
       for (int nt = 0; nt < NT; nt++) {
-        const float a0 = v[nt][0] * unscale[nt][0], a1 = v[nt][1] * unscale[nt][1];
-        const float a2 = v[nt][2] * unscale[nt][0], a3 = v[nt][3] * unscale[nt][1];
+        const float a0 = v[nt][0], a1 = v[nt][1], a2 = v[nt][2], a3 = v[nt][3];
         uint32_t p0, p1;       // (column 2t, column 2t + 1) of row g and of row g + 8
         if (y_dtype == GGQ_BF16) {
           const __nv_bfloat162 q0 = __floats2bfloat162_rn(a0, a1), q1 = __floats2bfloat162_rn(a2, a3);
@@ -612,7 +691,7 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
       for (int i = 0; i < 4; i++) {
         const int row = rb * kBlockRows + warp * 16 + g + 8 * (i >> 1), col = nt * 8 + 2 * t + (i & 1);
         if (row < N && col < M) {
-          const float val = v[nt][i] * unscale[nt][i & 1];
+          const float val = v[nt][i];
           if (pp.world == 0) store_out(y, y_dtype, (int64_t)col * N + row, val);
           else {            // row-sharded: this rank's rows of every rank's (M, n_total) output
 #pragma unroll 1
@@ -623,12 +702,14 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
     }
   };
 
-  int rb = rb_first, k = (int)(s_begin - (int64_t)rb_first * SB), slot = 0, seg_k = k;
+  int rb = rb_first, k = s_begin - rb_first * SB, slot = 0, seg_k = k;
   uint32_t ring_round = 0;              // how often the ring has wrapped: the parity a slot's barrier shows
   for (int i = 0; i < n_steps; i++) {
-    cp_async_wait_pending(depth - 2);
-    __syncthreads();                    // everybody's copies of step i have landed; everybody is done with step i - 1
-    issue_next();
+    if constexpr (!kOwn) {
+      cp_async_wait_pending(depth - 2);
+      __syncthreads();                  // everybody's copies of step i have landed; everybody is done with step i - 1
+      issue_next();
+    }
     if (tma) { tma_box_wait(my_bars + 8 * slot, ring_round & 1, status, lane); __syncwarp(); }
     const int row0 = rb * kBlockRows + warp * 16;
     if (row0 < N) {
@@ -645,6 +726,11 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
     if (k == SB - 1 || i == n_steps - 1) {
       // ---- the CTA's segment of row block rb ends here
       const bool whole = seg_k == 0 && k == SB - 1;
+#pragma unroll
+      for (int nt = 0; nt < NT; nt++) {
+        out[nt][0] *= unscale[nt][0]; out[nt][1] *= unscale[nt][1];
+        out[nt][2] *= unscale[nt][0]; out[nt][3] *= unscale[nt][1];
+      }
       if (whole) {
         store_rows(rb, out);
       } else {
@@ -655,8 +741,7 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
           __stcg(reinterpret_cast<float2*>(sl + g * XR + nt * 8 + 2 * t), make_float2(out[nt][0], out[nt][1]));
           __stcg(reinterpret_cast<float2*>(sl + (g + 8) * XR + nt * 8 + 2 * t), make_float2(out[nt][2], out[nt][3]));
         }
-        const int64_t rb_s0 = (int64_t)rb * SB;
-        const int c_first = cta_of_step(rb_s0, geo.S, G), c_last = cta_of_step(rb_s0 + SB - 1, geo.S, G);
+        const int c_first = cta_of_step(geo, rb * SB, G), c_last = cta_of_step(geo, rb * SB + SB - 1, G);
         __threadfence();
         __syncthreads();
         if (tid == 0) {
@@ -669,8 +754,11 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
           float sum[NT][4];
 #pragma unroll
           for (int nt = 0; nt < NT; nt++) sum[nt][0] = sum[nt][1] = sum[nt][2] = sum[nt][3] = 0.f;
+          // (the first contributor may have begun in the row block before: then this one is its second part; four slots' loads in flight)
+          const int first_part = range_start(geo, c_first, G) < rb * SB ? 1 : 0;
+#pragma unroll 4
           for (int c = c_first; c <= c_last; c++) {
-            const int cpart = (int)((geo.S * c / G) / SB) == rb ? 0 : 1;
+            const int cpart = c == c_first ? first_part : 0;
             const float* cs = slots + (((int64_t)c * 2 + cpart) * kBlockRows + warp * 16) * XR;
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
@@ -689,7 +777,7 @@ gemv_wide_kernel(const uint8_t* __restrict__ w, int N, int K, const uint8_t* __r
     }
     if (++k == SB) { k = 0; ++rb; }
   }
-  cp_async_wait_pending(0);
+  if constexpr (!kOwn) cp_async_wait_pending(0);
   peer_publish(pp, tid, gridDim.x);        // row-sharded: raise this rank's flag on every rank once the whole grid has stored
 }
 
@@ -739,7 +827,7 @@ static WsLayout ws_layout(const FormatInfo& fi, int64_t K, int M, int sm_count) 
   return l;
 }
 
-template <class F, int NT>
+template <class F, int NT, bool kOwn>
 static cudaError_t launch(const Geo& geo, int grid, cudaStream_t st, const uint8_t* w, int N, int K, const void* x, int64_t ldx, int M,
                           void* y, int y_dtype, uint8_t* ws, const WsLayout& l, const PeerPublish& pp, int* status,
                           const CUtensorMap& w_map) {
@@ -747,29 +835,32 @@ static cudaError_t launch(const Geo& geo, int grid, cudaStream_t st, const uint8
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_done[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(gemv_wide_kernel<F, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit / kCtasPerSm - 1024);
+    cudaError_t e = cudaFuncSetAttribute(gemv_wide_kernel<F, NT, kOwn>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit / kCtasPerSm - 1024);
     if (e != cudaSuccess) return e;
     attr_done[dev].store(true, std::memory_order_release);
   }
-  constexpr int XR = 8 * NT;
-  const int rounds = (K / 256 * F::kGroups * 4 + 255) / 256, parts = std::min(8, rounds);
-  cudaError_t err = launch_pdl(prepare_kernel<F, XR>, XR * parts, 256, 0, st, (const __nv_bfloat16*)x, ldx, K, M, ws + l.xp, ws + l.xo,
-                               reinterpret_cast<int*>(ws + l.scol), parts, pp, status);
-  if (err != cudaSuccess) return err;
-  err = launch_pdl(gemv_wide_kernel<F, NT>, grid, kThreads, (size_t)geo.total, st, w, N, K, (const uint8_t*)(ws + l.xp),
+  cudaError_t err = cudaSuccess;
+  if constexpr (!kOwn) {
+    constexpr int XR = 8 * NT;
+    const int rounds = (K / 256 * F::kGroups * 4 + 255) / 256, parts = std::min(8, rounds);
+    err = launch_pdl(prepare_kernel<F, XR>, XR * parts, 256, 0, st, (const __nv_bfloat16*)x, ldx, K, M, ws + l.xp, ws + l.xo,
+                     reinterpret_cast<int*>(ws + l.scol), parts, pp, status);
+    if (err != cudaSuccess) return err;
+  }
+  err = launch_pdl(gemv_wide_kernel<F, NT, kOwn>, grid, kThreads, (size_t)geo.total, st, w, N, K, (const __nv_bfloat16*)x, ldx, (const uint8_t*)(ws + l.xp),
                    (const uint8_t*)(ws + l.xo), reinterpret_cast<const int*>(ws + l.scol), M, y, y_dtype,
                    reinterpret_cast<int*>(ws + kWsCounterOffset), reinterpret_cast<float*>(ws + l.slots), geo, pp, status, w_map);
   return err != cudaSuccess ? err : cudaPeekAtLastError();
 }
 
-template <class F>
+template <class F, bool kOwn>
 static cudaError_t launch_tiles(int NT, const Geo& geo, int grid, cudaStream_t st, const uint8_t* w, int N, int K, const void* x,
                                 int64_t ldx, int M, void* y, int y_dtype, uint8_t* ws, const WsLayout& l, const PeerPublish& pp,
                                 int* status, const CUtensorMap& w_map) {
   switch (NT) {
-    case 1: return launch<F, 1>(geo, grid, st, w, N, K, x, ldx, M, y, y_dtype, ws, l, pp, status, w_map);
-    case 2: return launch<F, 2>(geo, grid, st, w, N, K, x, ldx, M, y, y_dtype, ws, l, pp, status, w_map);
-    default: return launch<F, 4>(geo, grid, st, w, N, K, x, ldx, M, y, y_dtype, ws, l, pp, status, w_map);
+    case 1: return launch<F, 1, kOwn>(geo, grid, st, w, N, K, x, ldx, M, y, y_dtype, ws, l, pp, status, w_map);
+    case 2: return launch<F, 2, kOwn>(geo, grid, st, w, N, K, x, ldx, M, y, y_dtype, ws, l, pp, status, w_map);
+    default: return launch<F, 4, kOwn>(geo, grid, st, w, N, K, x, ldx, M, y, y_dtype, ws, l, pp, status, w_map);
   }
 }
 
@@ -808,6 +899,9 @@ cudaError_t gemv_wide(int qtype, const uint8_t* w, int64_t N, int64_t K, const v
   if (!ws || ws_bytes < l.total || (uintptr_t)ws % 256) return cudaErrorInvalidValue;
   if (kWsCounterOffset + (size_t)geo.RB * sizeof(int) > kWsGemmPartialOffset) return cudaErrorInvalidValue;
   const int grid = (int)std::min<int64_t>((int64_t)sm_count * kCtasPerSm, geo.S);
+  geo.per_cta = (int)(geo.S / grid);
+  geo.rest = (int)(geo.S % grid);
+  geo.cta_per_step = (float)((double)grid / (double)geo.S);
   const int NT = tiles_of(M);
   uint8_t* base = reinterpret_cast<uint8_t*>(ws);
   PeerPublish pp = {};
@@ -832,10 +926,16 @@ cudaError_t gemv_wide(int qtype, const uint8_t* w, int64_t N, int64_t K, const v
   }
   const char* vec_env = getenv("GGQ_WIDE_VEC_STORE");       // "0": element-wise stores (read per call; the tests take both)
   geo.vec_store = vec && !(vec_env && vec_env[0] == '0') ? 1 : 0;
+  const bool own = pp.world == 0 && (geo.S + grid - 1) / grid <= std::min(geo.depth, kOwnSteps);
+  auto go = [&](auto fmt) {
+    using F = decltype(fmt);
+    auto* fn = own ? launch_tiles<F, true> : launch_tiles<F, false>;
+    return fn(NT, geo, grid, st, w, (int)N, (int)K, x, ldx, M, y, y_dtype, base, l, pp, status, w_map);
+  };
   switch (qtype) {
-    case QT_Q4_K: return launch_tiles<FQ4K>(NT, geo, grid, st, w, (int)N, (int)K, x, ldx, M, y, y_dtype, base, l, pp, status, w_map);
-    case QT_Q5_K: return launch_tiles<FQ5K>(NT, geo, grid, st, w, (int)N, (int)K, x, ldx, M, y, y_dtype, base, l, pp, status, w_map);
-    case QT_Q6_K: return launch_tiles<FQ6K>(NT, geo, grid, st, w, (int)N, (int)K, x, ldx, M, y, y_dtype, base, l, pp, status, w_map);
+    case QT_Q4_K: return go(FQ4K{});
+    case QT_Q5_K: return go(FQ5K{});
+    case QT_Q6_K: return go(FQ6K{});
     default: return cudaErrorInvalidValue;
   }
 }
