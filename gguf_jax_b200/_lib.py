@@ -119,6 +119,10 @@ class _PythonPath:
         return None
 
     @staticmethod
+    def fast_dequant(*_):
+        return None
+
+    @staticmethod
     def set_scratch(*_):
         return None
 

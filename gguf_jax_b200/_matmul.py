@@ -174,6 +174,9 @@ def _slabs(w: QuantizedArray, count: int, rows: int | None = None):
     """``(first_row, dense slab)`` for each of ``count`` equal row slabs (or slabs of ``rows`` rows, the last one
     shorter), decoded one at a time."""
     rows = w.shape[0] // count if rows is None else rows
+    if rows >= w.shape[0] > 0:
+        yield 0, QuantizedArray(w.data, w.qtype, w.shape, w.dtype).dequantize()
+        return
     for row0 in range(0, w.shape[0], rows):
         n = min(rows, w.shape[0] - row0)
         part = QuantizedArray(w.data[row0:row0 + n], w.qtype, (n, w.shape[1]), w.dtype)

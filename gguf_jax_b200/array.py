@@ -93,7 +93,7 @@ class QuantizedArray:
         want = self.dtype if dtype is None else _backend.canon_dtype(dtype)
         plain = _PLAIN.get(self.qtype)
         if plain is None:
-            return quants.dequantize(self.data, self.qtype, want).reshape(self.shape)
+            return quants.dequantize_shaped(self.data, self.qtype, want, self.shape)
         dense = self.data.reshape(self.shape)
         return dense if plain[1] else dense.to(want)
 

@@ -113,3 +113,15 @@ def dequantize(data, qtype: GGMLQuantizationType, dtype=torch.float32) -> torch.
     shape = _ref.quant_shape_from_byte_shape(tuple(data.shape), qtype)  # raises ValueError on a bad row size
     blocks = data.reshape(-1, type_size)
     return dequantize_blocks(blocks, qtype, dtype).reshape(shape)
+
+
+def dequantize_shaped(data, qtype: GGMLQuantizationType, dtype: torch.dtype, shape: tuple[int, ...]) -> torch.Tensor:
+    """``dequantize(data, qtype, dtype).reshape(shape)``; the common call (the built-in decoder, bytes on a device that has its code books,
+    nothing that watches or transforms operations) is one native function."""
+    code = _backend._DTYPE_CODE.get(dtype)
+    if (code is not None and qtype not in _replaced and type(data) is torch.Tensor and data.is_cuda and data.device.index in _lib._tables_done
+            and torch._C._len_torch_function_stack() == 0):
+        y = _lib.native().fast_dequant(data, qtype, shape, code)
+        if y is not None:
+            return y
+    return dequantize(data, qtype, dtype).reshape(shape)
