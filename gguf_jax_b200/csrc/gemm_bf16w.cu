@@ -1,5 +1,5 @@
-// Fused decode + GEMM for batches from a few dozen rows on, on the 5th-generation tensor cores (tcgen05 / TMEM): Q4_K, Q5_K and
-// Q6_K weights are decoded to float32 exactly as the decode kernel does, rounded once to bf16 and written straight into the
+// Fused decode + GEMM for batches from a few dozen rows on, on the 5th-generation tensor cores (tcgen05 / TMEM): the weights
+// of a block format (Q4_K, Q5_K, Q6_K here, the others in gemm_bf16w_b32.cu and gemm_bf16w_iq.cu; the kernel is in gemm_bf16w.cuh) are decoded to float32 exactly as the decode kernel does, rounded once to bf16 and written straight into the
 // K-major, 128-byte-swizzled A tile in shared memory; the activations are used as they are (bf16, K-major);
 // tcgen05.mma.kind::f16 accumulates in TMEM in float32.
 //

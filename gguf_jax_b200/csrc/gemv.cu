@@ -17,28 +17,22 @@ inline int tuned_max_repeat(int qtype, int64_t weight_bytes) {
   return weight_bytes < (24ll << 20) ? 1 : weight_bytes < (80ll << 20) ? 2 : 3;
 }
 inline bool is_k_quant(int qtype) { return qtype == QT_Q4_K || qtype == QT_Q5_K || qtype == QT_Q6_K; }
-// From which size on the batch-major kernel (gemv_wide.cu) takes 17 to 32 batch rows: it costs two launches and a partial-sum
-// settle, about 10 us on a weight of a few MB, and then very little per batch row (against decode + library GEMM, below).
+// From which size on the batch-major kernel (gemv_wide.cu) takes 17 to 32 batch rows: it costs a launch or two and a partial-sum
+// settle, 7 to 10 us on a weight of a few MB, and then very little per batch row (against decode + library GEMM, below).
 inline bool wide_pays(int qtype, int64_t weight_bytes) {
   return weight_bytes >= (qtype == QT_Q6_K ? (10ll << 20) : (20ll << 20));
 }
-// Above 16 batch rows the choice is between slices of 32 rows through the batch-major kernel and, in the
-// caller, the decode kernel followed by a library GEMM.  One slice wins from about 20 MB on (us, fused / decode and GEMM, on the
-// device: Q4_K 8192 x 8192 36 / 55, Q6_K 14336 x 4096 38 / 50; on smaller weights it loses, their decoded copy stays in the L2:
-// Q5_K 4096 x 4096 22 / 17 and, above Q6_K's line of 10 MB, 4096 x 4096 26 / 16); two slices or more lose, so the router's cap is
-// 32 there and 16 elsewhere.
-// The tcgen05 kernels behind ggq_gemm (integer-code and tf32 operands) are slower than both at every
+// Above 16 batch rows the choice is between a slice of 32 rows through the batch-major kernel, whose arithmetic is exact, and the dense route, whose
+// weights are rounded to bf16.  The line is where the exact kernel overtook a decoded copy and the library's GEMM (us, exact / copy and GEMM, when it
+// was drawn: Q4_K 8192 x 8192 36 / 55, Q6_K 14336 x 4096 38 / 50, Q5_K 4096 x 4096 22 / 17).  The dense route's own kernel (gemm_bf16w.cu) has since
+// become faster than both on most weights (Q6_K 4096 x 4096 at 24 rows 23 exact, 11 rounded); the line stays, because to move it would round weights that were not.
+// The tcgen05 kernels behind ggq_gemm with integer-code and tf32 operands are slower than both at every
 // batch measured and are reached only by name, above 128 rows or for the other formats.
 constexpr int kWideRouterBatch = 32;
-// Above 32 rows the bf16-weight tcgen05 kernel (gemm_bf16w.cu; the fallback's own precision) is compared with the same
-// fallback, up to 256 rows on the large weights and up to 512 where there are enough row tiles to fill the device without
-// cutting K.  us on the device at 64 / 128 / 256 / 512 rows, fused and fallback: Q4_K 14336 x 4096 37 / 39 / 47 / 65 and 47 / 47 / 56 / 73,
-// 4096 x 14336 41 / 48 / 65 / 91 and 52 / 53 / 57 / 73, 8192 x 8192 43 / 49 / 64 / 107 and 56 / 55 / 63 / 74, 28672 x 8192 146 / 171 / 164 / 262 and
-// 186 / 187 / 210 / 270; Q6_K 14336 x 4096 53 / 55 / 62 / 78 and 52 / 51 / 60 / 78, 4096 x 14336 54 / 62 / 79 / 118 and 57 / 57 / 62 / 77, 8192 x 8192 58 /
-// 64 / 79 / 119 and 61 / 59 / 68 / 80.  The caps date from a decode kernel that took 15 us longer on these weights: they still hold for Q4_K
-// and Q5_K but for 256 rows at 4096 x 14336, and lie too high for Q6_K, whose lead ends at 64 rows.  A call through the fallback
-// takes 8 us more of host time, which is what counts where the device does not lag behind.
-// On weights of a few MB the fallback's library GEMM reads a decoded copy that stays in the L2 and wins at every batch above 16.
+// Above 32 rows both sides round: the limit decides the type of the result for weights that decode to float16 or float32, and no longer which kernel
+// takes bf16 ones (the bf16-weight tcgen05 kernel on either side of it where that is faster, see gemm_bf16w_beats_dense).  us at 64 / 128 / 256 / 512 rows,
+// that kernel and decode + library GEMM: Q4_K 14336 x 4096 22 / 24 / 31 / 48 and 47 / 47 / 56 / 73, 4096 x 14336 23 / 25 / 35 / 52 and 53 / 53 / 57 / 72;
+// Q6_K 14336 x 4096 27 / 29 / 33 / 50 and 52 / 52 / 61 / 77, 4096 x 14336 28 / 29 / 38 / 56 and 58 / 58 / 61 / 76.
 constexpr int kGemmRouterBatchWide = 512;      // at least 96 row tiles of 128 rows
 constexpr int kGemmRouterBatch = 256;
 }
