@@ -188,6 +188,17 @@ def _promoted_mm(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     return torch.matmul(a.to(common), b.to(common))
 
 
+def _aligned_mm(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
+    """``a @ b`` where the contraction may be no multiple of _ROW_ELEMS, for which the library has slow kernels only, some of which add partial sums
+    in bfloat16: the last few terms become the addend of the product of the others, which is rounded once."""
+    whole = a.shape[1] // _ROW_ELEMS * _ROW_ELEMS
+    if whole in (0, a.shape[1]):
+        return _promoted_mm(a, b)
+    common = torch.promote_types(a.dtype, b.dtype)
+    a, b = a.to(common), b.to(common)
+    return torch.addmm(torch.matmul(a[:, whole:], b[whole:]), a[:, :whole], b[:whole])
+
+
 # The library GEMM reads and writes 16-byte rows: with a leading dimension that is no multiple of 8 elements it falls back
 # to kernels an order of magnitude slower (8655 x 27136 at 1336 rows: 5.8 ms against 0.6 ms for 8656).
 _ROW_ELEMS = 8
@@ -196,6 +207,13 @@ _ROW_ELEMS = 8
 # slow kernels finish in less (2445 x 1792 at 508 rows, forward and backward: 192 us unpadded, 246 us padded, both bound by
 # the host); above, they are what the call waits for.
 _PAD_FROM_OPS = 1 << 35
+
+
+# The gradient's contraction runs over the rows of the weight, and with a number of those that is no multiple of 8 the library stays slow whatever
+# the leading dimension: there the contraction is cut at the last multiple (see _aligned_mm), for a launch or two more.  us of the gradient alone
+# in one product / cut, and the distance from the exact one: 12922 x 18176 at 962 rows 3404 / 710 (0.0032 / 0.0029), 5637 x 5376 at 1000
+# 494 / 99 and at 233 138 / 81, 5003 x 2816 at 600 142 / 79 (0.0033 / 0.0028); below the line, bound by the host, 2445 x 1792 at 508 69 / 81.
+_CUT_FROM_OPS = 1 << 33
 
 
 def _pads(rows: int, w: QuantizedArray) -> bool:
@@ -259,14 +277,17 @@ def _input_cotangent(g: torch.Tensor, w: QuantizedArray, count: int) -> torch.Te
     """``g (..., N) @ w (N, K)``: the slabs cut the contraction, so their products add up (in
     float32 when there is more than one)."""
     g2 = g.reshape(-1, w.shape[0])
-    if _pads(g2.shape[0], w):           # rows of the left operand on 16-byte boundaries
+    cut = w.shape[0] % _ROW_ELEMS != 0 and 2 * g2.shape[0] * w.shape[0] * w.shape[1] >= _CUT_FROM_OPS
+    if cut:                             # rows of the left operand on 16-byte boundaries
         g2 = torch.nn.functional.pad(g2, (0, -w.shape[0] % _ROW_ELEMS))[:, :w.shape[0]]
+    mm = _aligned_mm if cut else _promoted_mm
     if count == 1:
         (_, dense), = _slabs(w, 1)
-        return _promoted_mm(g2, dense).reshape(*g.shape[:-1], w.shape[1])
+        return mm(g2, dense).reshape(*g.shape[:-1], w.shape[1])
     total = torch.zeros((g2.shape[0], w.shape[1]), dtype=torch.float32, device=g.device)
-    for row0, dense in _slabs(w, count):
-        total += _promoted_mm(g2[:, row0:row0 + dense.shape[0]], dense).float()
+    rows = w.shape[0] // count // _ROW_ELEMS * _ROW_ELEMS if cut else 0         # every slab but the last starts and ends on a boundary
+    for row0, dense in _slabs(w, count, rows or None):
+        total += mm(g2[:, row0:row0 + dense.shape[0]], dense).float()
     return total.reshape(*g.shape[:-1], w.shape[1])
 
 
