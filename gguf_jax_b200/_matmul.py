@@ -203,10 +203,11 @@ def _aligned_mm(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 # to kernels an order of magnitude slower (8655 x 27136 at 1336 rows: 5.8 ms against 0.6 ms for 8656).
 _ROW_ELEMS = 8
 
-# Padding costs an allocation and one or two launches more per product, 25 us of host time each.  Below this many operations the
-# slow kernels finish in less (2445 x 1792 at 508 rows, forward and backward: 192 us unpadded, 246 us padded, both bound by
-# the host); above, they are what the call waits for.
-_PAD_FROM_OPS = 1 << 35
+# It is slow, and adds partial sums in bfloat16, for a number of columns that is no multiple of 8 even where they are padded: from this many operations on
+# the last few rows of the weight are a product of their own, both in rows of padded length.  That costs an allocation and three launches more, 25 to 40 us of
+# host time.  us a call in one product / in two, and the distance from the exact one: Q4_0 5637 x 5408 at 233 rows 150 / 81 (0.0029 / 0.0024), 3001 x 4672 at 600 187 / 78,
+# 9001 x 5408 at 1500 982 / 153, 20001 x 1568 at 150 154 / 80, IQ4_NL 4099 x 14368 at 64 (7.5 G operations) 171 / 115; Q5_0 2445 x 1824 at 508 (4.5 G) 63 / 80.
+_PAD_FROM_OPS = 1 << 33
 
 
 # The gradient's contraction runs over the rows of the weight, and with a number of those that is no multiple of 8 the library stays slow whatever
@@ -253,7 +254,7 @@ def _materialized_forward(x: torch.Tensor, w: QuantizedArray, count: int) -> tor
         # every slab's product goes straight to its columns of the result; slab and row boundaries are multiples of
         # _ROW_ELEMS (a result whose rows are not is copied once at the end).  Slabs are rounded down, so that none
         # exceeds the budget; one of all rows stays whole.
-        rows = n_out if count == 1 else n_out // count // _ROW_ELEMS * _ROW_ELEMS or n_out // count
+        rows = n_out // count // _ROW_ELEMS * _ROW_ELEMS or n_out // count
         pitch = -(-n_out // _ROW_ELEMS) * _ROW_ELEMS
         for row0, dense in _slabs(w, count, rows):
             common = torch.promote_types(x2.dtype, dense.dtype)

@@ -58,6 +58,17 @@ def test_autocast_vmap_and_a_second_derivative(weight):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("qtype,n,k,m", [(QT.Q4_0, 3001, 4672, 600), (QT.Q8_0, 9001, 2080, 257)], ids=str)
+def test_the_product_itself_on_the_device(qtype, n, k, m):
+    assert 2 * n * k * m >= mm._PAD_FROM_OPS
+    w = synth.make_weight_on_device(n, k, qtype, seed=3, device="cuda")
+    x = torch.randn((m, k), device="cuda").to(torch.bfloat16)
+    y = gj.matmul(x, w)
+    assert y.shape == (m, n) and y.is_contiguous()
+    _close(y, x, w.dequantize().T, 2.0 ** -7)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("qtype,n,k,m,rows", [(QT.Q4_K, 2445, 1792, 1024, None), (QT.Q4_0, 2445, 1824, 1024, None), (QT.IQ2_XXS, 2442, 1792, 1200, 1221)], ids=str)
 def test_on_the_device(qtype, n, k, m, rows):
     assert 2 * n * k * m >= mm._CUT_FROM_OPS
